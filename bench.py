@@ -581,7 +581,7 @@ def reference_gpu_compare(args) -> dict:
 
 
 def ngia_classes(db_type: int) -> int:
-    return 7 if db_type == 0 else 5
+    return 3  # alignment classes in use (64 and 128 ring rows, any width)
 
 
 def run_e2e(args, db, p, S):

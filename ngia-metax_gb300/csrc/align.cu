@@ -11,31 +11,25 @@
 // their state.  The score is the number of zero bits of line[] over the net
 // length, accepted when >= ceil(L2*s).
 //
-// Two kernels reproduce that exactly:
+// Two kernels give the same accepted scores and the same rejections:
 //
-// k_align_win<P,WC>  one thread per pair.  The band window (at most WC rep
-//   blocks) lives in registers: row[m] for slot m = rep block js+m.  For each
-//   query residue the whole window is updated as one multi-word addition
+// k_align_tiled<P,RING>  one thread per pair.  The band rows live in a ring
+//   (shared memory for windows up to RING = 64 or 128 blocks, global scratch
+//   for any width with RING = 0) and are updated tile by tile in registers:
+//   for each query residue a tile of 16 row words is one multi-word addition
 //   whose carries ride the hardware carry flag (add.cc/addc.cc).  The match
 //   word of a slot comes, for DNA, from the representative's match table in
 //   shared memory (four words per rep block, one per residue code; tile.cuh),
 //   so a 32-cell word costs one load and three integer instructions (AND,
 //   IADD3.X, LOP3); protein builds it from the rep's planes held in registers
-//   (one LOP3 per plane).  When the band slides, the departing block's zero
-//   count is banked and the registers shift down one slot; an entering block
-//   starts all-ones.  Lanes claim pairs from the class queue independently
-//   (warp-aggregated atomics).
+//   (one LOP3 per plane).
 //
-// k_align_tiled<P,RING>  wider windows: one thread per pair, the band rows
-//   in a ring (shared memory for windows up to RING = 64 or 128 blocks,
-//   global scratch for any width with RING = 0), updated tile by tile with
-//   the same generated instruction sequences.
+// k_align_warp<P>  classes with few queued pairs: one warp per pair.
 //
-// Both stop a pair early once it provably cannot reach the cutoff: each query
-// residue raises the counted zeros by at most one (the bit-vector update only
-// moves a zero downwards within a run of ones, or adds one at the top of the
-// updated segment), so zeros_now + residues_left < cutoff is a rejection.
-// Accepted pairs are always computed to the end (their score is reported).
+// In clustering both keep only the rows that a score of at least the cutoff
+// can use (band_advance in tile.cuh) and stop a pair once it provably cannot
+// reach it; accepted pairs are always computed to the end (their score is
+// reported).  Pair-score mode computes the whole band.
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
@@ -47,12 +41,6 @@
 namespace ngia {
 
 constexpr int kRepPlanesOff = 32;  // planes offset inside rb.rep_rec (filter.cu)
-
-// Resident CTAs per SM requested from the register allocator for the
-// register-window kernel of P planes and WC slots.
-__host__ __device__ constexpr int win_min_blocks(int P, int WC) {
-  return P == 2 ? (WC <= 8 ? 6 : WC <= 16 ? 4 : WC <= 24 ? 3 : 2) : (WC <= 8 ? 4 : 2);
-}
 
 struct AlignHdr {
   int qn, L1, net1, nb1, word_after, rep;
@@ -193,199 +181,6 @@ __device__ __forceinline__ void flush_align_stats(RunState *st, int cls, unsigne
   if (threadIdx.x == 0 && *s_qwords) atomicAdd(&st->st_class_qwords[cls], *s_qwords);
 }
 
-template <int P, int WC>
-__global__ void __launch_bounds__(kAlignThreads, win_min_blocks(P, WC))
-    k_align_win(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ uint64_t bar;
-  AlignHdr h;
-  __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
-  if (threadIdx.x == 0) s_qw = 0;
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, 0, smem, &bar, h)) return;
-  const uint32_t *s_pl = smem;
-  const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
-  constexpr bool kEq = P == 2 && NGIA_WIN_EQ;
-  uint32_t *s_eq = smem + tiled_eq_off(P, db.max_nb, 0);
-  if constexpr (kEq) {
-    build_eq(s_pl, h.nb1, s_eq);  // the representative's match table (tile.cuh)
-    __syncthreads();
-  }
-  RunState *st = rb.st;
-  const int lane = threadIdx.x & 31;
-  const float s = prm.s;
-  const int nb1 = h.nb1;
-  const uint32_t vlast = (h.net1 & 31) ? ((1u << (h.net1 & 31)) - 1u) : 0xFFFFFFFFu;
-  // 1 and 4 as values ptxas cannot fold (nb1 is read from shared memory)
-  const uint32_t one_rt = 1u + (uint32_t)(h.nb1 < 0);
-  const FmaK fk{one_rt, one_rt << 2};
-  (void)fk;
-
-  uint32_t row[WC], pl[kEq ? 1 : P][WC], cur[P], nxt[P];
-  int state = -1, entry = 0, cand = 0;
-  int i = 0, nq = 0, B = 0, js = 0, je = -1, net2 = 0, L2 = 0, cutoff = 0, lastcols = 32, frozen = 0;
-  const uint32_t *qpl = nullptr;
-  unsigned long long n_pairs = 0, n_members = 0, n_cells = 0, n_done = 0;
-
-  for (;;) {
-    claim(st, cls, h.qn, lane, state);
-    if (__all_sync(kFullMask, state == -2)) break;
-    if (state < 0) continue;
-    // ---- start of a newly claimed pair -----------------------------------
-    if (qpl == nullptr) {
-      entry = rb.queue[cls][state];  // candidate, or pair slot in score mode
-      cand = score_mode ? rb.score_cands[entry] : entry;
-      L2 = __ldg(db.len + cand);
-      net2 = __ldg(db.net + cand);
-      nq = (net2 + 31) >> 5;
-      lastcols = (net2 & 31) ? (net2 & 31) : 32;
-      B = band_blocks(h.L1, L2, s);
-      cutoff = cutoff_of(L2, s);
-      qpl = db.words + __ldg(db.off + cand) + db.hw;
-      i = 0;
-      js = 0;
-      je = min(B, nb1 - 1);
-      frozen = 0;
-      if (!score_mode) {
-        n_pairs++;
-        n_cells += (unsigned long long)band_cells(B, nb1, net2);
-        atomicAdd(&s_qw, (unsigned long long)(nq * P));
-      }
-      if (B < 0 || je < 0 || nq == 0) {
-        finish_pair<P>(db, rb, prm, h, score_mode, entry, cand, 0, cutoff, L2, net2, qpl, s_list, n_members);
-        qpl = nullptr;
-        state = -1;
-        continue;
-      }
-#pragma unroll
-      for (int m = 0; m < WC; m++) {
-        row[m] = 0xFFFFFFFFu;
-        if constexpr (!kEq) {
-#pragma unroll
-          for (int p = 0; p < P; p++) pl[p][m] = (m <= je) ? s_pl[m * P + p] : 0u;
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < P; p++) cur[p] = __ldg(qpl + p);
-    }
-    // ---- one 32-residue query block ---------------------------------------
-    const int cols = (i == nq - 1) ? lastcols : 32;
-    n_done += (unsigned long long)(je - js + 1) * cols;
-    if (i + 1 < nq) {
-#pragma unroll
-      for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + (i + 1) * P + p);
-    }
-    uint32_t cw_unused = 0;
-    if constexpr (kEq) {
-      // match words of slot m for column k: s_eq[4 (js + m) + code_k]; slots
-      // past je read blocks not in the band (or the table's zero blocks):
-      // those rows are reset when they enter the band
-      if constexpr (NGIA_WIN_FMA) {  // the per-column bookkeeping on the FMA pipe (tile.cuh)
-        uint32_t wc[2];
-        eq_codes_top(cur, wc);
-        eq_columns_f<WC, false, NGIA_EQ_PF_WIN>(row, smem_u32(s_eq) + 16u * (uint32_t)js, wc, cols, cw_unused,
-                                                 cw_unused, fk);
-      } else {
-        uint32_t q[4];
-        eq_codes(cur, q);
-        const char *eb = reinterpret_cast<const char *>(s_eq + 4 * js);
-        eq_columns<WC, false, NGIA_EQ_PF_WIN>(row, eb, q, cols, cw_unused, cw_unused);
-      }
-    } else {
-    uint32_t rv[P];
-#pragma unroll
-    for (int p = 0; p < P; p++) rv[p] = __brev(cur[p]);
-    int k = 0;
-    for (; k + 2 <= cols; k += 2) {
-      uint32_t mk[P];
-#pragma unroll
-      for (int p = 0; p < P; p++) {
-        mk[p] = (uint32_t)((int)rv[p] >> 31);
-        rv[p] <<= 1;
-      }
-      dp_tile<P, WC, false, false>(row, pl, mk, cw_unused, cw_unused);
-#pragma unroll
-      for (int p = 0; p < P; p++) {
-        mk[p] = (uint32_t)((int)rv[p] >> 31);
-        rv[p] <<= 1;
-      }
-      dp_tile<P, WC, false, false>(row, pl, mk, cw_unused, cw_unused);
-    }
-    if (k < cols) {
-      uint32_t mk[P];
-#pragma unroll
-      for (int p = 0; p < P; p++) mk[p] = (uint32_t)((int)rv[p] >> 31);
-      dp_tile<P, WC, false, false>(row, pl, mk, cw_unused, cw_unused);
-    }
-    }
-    // ---- slide the band to query block i+1 --------------------------------
-    i++;
-    bool finished = i >= nq;
-    if (!finished) {
-      if (i - B > 0) {  // js advances: block js leaves the band for good
-        frozen += __popc(~row[0] & (js == nb1 - 1 ? vlast : 0xFFFFFFFFu));
-#pragma unroll
-        for (int m = 0; m < WC - 1; m++) {
-          row[m] = row[m + 1];
-          if constexpr (!kEq) {
-#pragma unroll
-            for (int p = 0; p < P; p++) pl[p][m] = pl[p][m + 1];
-          }
-        }
-        js++;
-      }
-      if (i + B <= nb1 - 1) {  // je advances: block je enters all-ones
-        je++;
-        const int slot = je - js;
-        uint32_t v[P];
-#pragma unroll
-        for (int p = 0; p < P; p++) v[p] = kEq ? 0u : s_pl[je * P + p];
-#pragma unroll
-        for (int m = 0; m < WC; m++)
-          if (m == slot) {
-            row[m] = 0xFFFFFFFFu;
-            if constexpr (!kEq) {
-#pragma unroll
-              for (int p = 0; p < P; p++) pl[p][m] = v[p];
-            }
-          }
-      }
-      if (js > je) finished = true;  // band ran past the representative
-    }
-    const int n = je - js + 1;
-    if (finished) {
-      int sum = frozen;
-#pragma unroll
-      for (int m = 0; m < WC; m++)
-        if (m < n) sum += __popc(~row[m] & (js + m == nb1 - 1 ? vlast : 0xFFFFFFFFu));
-      finish_pair<P>(db, rb, prm, h, score_mode, entry, cand, sum, cutoff, L2, net2, qpl, s_list, n_members);
-      qpl = nullptr;
-      state = -1;
-      continue;
-    }
-    if (!score_mode) {
-      int z = frozen;
-#pragma unroll
-      for (int m = 0; m < WC; m++) z += (m < n) ? __popc(~row[m]) : 0;
-      if (z + (net2 - 32 * i) < cutoff) {  // cannot reach the cutoff any more
-        qpl = nullptr;
-        state = -1;
-        continue;
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < P; p++) cur[p] = nxt[p];
-  }
-  flush_align_stats(st, cls, n_pairs, n_members, n_cells, n_done, &s_qw);
-}
-
-
-// One register tile of TW window slots starting at rep block `base` for all
-// `cols` residues of the current query block: rows come from and return to
-// the shared-memory ring, planes from the staged representative.  The 32
-// column carries enter in `cw` (column 0 at bit 31; zero for the lowest
-// tile) and leave in `ncw` (ignored after the highest tile).  Slots past `je`
-// are padding: computed, never stored.  Returns the change of the tile's
-// zero count (all bits).
 // Tiled window: windows of up to RING rep blocks (any width for RING = 0).
 // Each lane keeps its pair's band rows in a ring indexed by absolute rep
 // block (SmemRing / GlobalRing above) and runs each query block tile by tile in
@@ -408,7 +203,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   const uint32_t *s_pl = smem;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
   RunState *st = rb.st;
-  constexpr bool kEq = P == 2 && NGIA_ALIGN_EQ;
+  constexpr bool kEq = P == 2;
   uint32_t *s_eq = smem + tiled_eq_off(P, db.max_nb, RING);
   if constexpr (kEq) {
     build_eq(s_pl, h.nb1, s_eq);  // the representative's match table (tile.cuh)
@@ -440,7 +235,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
 
   int state = -1, entry = 0, cand = 0;
   int i = 0, nq = 0, B = 0, js = 0, je = -1, net2 = 0, L2 = 0, cutoff = 0, lastcols = 32, frozen = 0, zw = 0;
-  int zskip = 0;  // query blocks this lane's pair cannot be rejected at (NGIA_ZC_SKIP)
+  int cut = 0;  // the band rules' cutoff (none in pair-score mode)
   bool active = false;
   const uint32_t *qpl = nullptr;
   uint32_t cur[P], nxt[P];
@@ -468,12 +263,12 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       B = band_blocks(h.L1, L2, s);
       cutoff = cutoff_of(L2, s);
       qpl = db.words + __ldg(db.off + cand) + db.hw;
+      cut = score_mode ? kNoCut : cutoff;
       i = 0;
       js = 0;
-      je = min(B, nb1 - 1);
+      je = band_first_top(B, nb1, h.net1, cut);
       frozen = 0;
       zw = 0;
-      zskip = score_mode ? INT_MAX : 0;
       if (!score_mode) {
         n_pairs++;
         n_cells += (unsigned long long)band_cells(B, nb1, net2);
@@ -498,14 +293,6 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     constexpr int MT = tiled_main(P);
     const int full = (int)__reduce_min_sync(kFullMask, busy ? (unsigned)(n / MT) : 0xFFFFFFFFu);
     int rem = (int)__reduce_max_sync(kFullMask, busy ? (unsigned)(n - MT * full) : 0u);
-    // every busy lane's window ends exactly at the warp's last tile slot
-    // (all lanes vote, before the idle ones leave the body)
-    bool exact_cover = false;
-    if constexpr (kEq && NGIA_EQ_FMA && NGIA_EQ_ZCARRY) exact_cover = __all_sync(kFullMask, !busy || n - MT * full == rem);
-    (void)exact_cover;
-    // the warp counts zeros after this block when one of its lanes may be
-    // rejected there
-    const bool cnt = !(kEq && NGIA_EQ_FMA && NGIA_ZC_SKIP) || __any_sync(kFullMask, busy && zskip <= 0);
     if (!busy) continue;
     const int cols = (i == nq - 1) ? lastcols : 32;
     n_done += (unsigned long long)n * cols;
@@ -513,64 +300,24 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
 #pragma unroll
       for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + (i + 1) * P + p);
     }
-    if constexpr (kEq && NGIA_EQ_FMA) {
+    if constexpr (kEq) {
       using Ring = typename RingOf<RING>::T;
-      constexpr bool kZC = !NGIA_EQ_ZCARRY;  // tiles count zeros
       uint32_t wc[2];
       eq_codes_top(cur, wc);
-      uint32_t cw = 0, ncw = 0, last = 0;
-      int base = js;
-      if (kZC && NGIA_EQ_NOZOLD) zw = 0;  // the tiles return their rows' zero counts
-      // a one-slot remainder joins the last main tile (warp-uniform)
-      const bool merge1 = NGIA_TILED_MERGE1 && rem == 1 && full > 0;
-      for (int t = merge1 ? 1 : 0; t < full; t++, base += MT) {
-        zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring, kZC>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk, cnt);
-        last = ncw;
-        cw = ncw << (32 - cols);  // column 0's carry at bit 31
-        ncw = 0;
-      }
-      if (merge1) {
-        zw += tiled_tile_eqf<MT + 1, NGIA_EQ_PF_MAIN, Ring, kZC>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk, cnt);
-        last = ncw;
-        rem = 0;
-      }
-      for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring, kZC>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk, cnt);
-        last = ncw;
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      if (rem > 0) {
-        zw += tiled_rem_eqf<Ring, MT, kZC>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk, cnt);
-        last = ncw;
-      }
-      if constexpr (!kZC) {
-        if (exact_cover) {
-          zw += __popc(last);  // the carries out of the window's top row over the block's columns
-        } else {
-          int z = 0;
-          for (int j = js; j <= je; j++) z += __popc(~ring[j]);
-          zw = z;
-        }
-      }
-    } else if constexpr (kEq) {
-      rem = (rem + kEqRemRound - 1) / kEqRemRound * kEqRemRound;  // extra slots are padding
-      uint32_t q[4];
-      eq_codes(cur, q);
       uint32_t cw = 0, ncw = 0;
       int base = js;
+      zw = 0;  // the tiles return their rows' zero counts
       for (int t = 0; t < full; t++, base += MT) {
-        zw += tiled_tile_eq<MT, NGIA_EQ_PF_MAIN, typename RingOf<RING>::T>(ring, s_eq, base, je, nb1, cols, q, cw, ncw);
+        zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
         cw = ncw << (32 - cols);  // column 0's carry at bit 31
         ncw = 0;
       }
       for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile_eq<MT, NGIA_EQ_PF_MAIN, typename RingOf<RING>::T>(ring, s_eq, base, je, nb1, cols, q, cw, ncw);
+        zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
         cw = ncw << (32 - cols);
         ncw = 0;
       }
-      if (rem > 0)
-        zw += tiled_rem_eq<typename RingOf<RING>::T, MT>(rem, ring, s_eq, base, je, nb1, cols, q, cw, ncw);
+      if (rem > 0) zw += tiled_rem_eqf<Ring>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
     } else {
       uint32_t cw = 0, ncw = 0;
       int base = js;
@@ -589,17 +336,13 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     i++;
     bool finished = i >= nq;
     if (!finished) {
-      if (i - B > 0) {  // block js leaves the band
-        const uint32_t r0 = ring[js];
-        frozen += __popc(~r0 & (js == nb1 - 1 ? vlast : 0xFFFFFFFFu));
-        zw -= __popc(~r0);
-        js++;
+      const int step = band_advance(ring, i, B, nb1, h.net1, vlast, net2 - 32 * i, cut, js, je, frozen, zw);
+      if (step == kBandReject) {
+        active = false;
+        state = -1;
+        continue;
       }
-      if (i + B <= nb1 - 1) {  // block je enters all-ones
-        je++;
-        ring[je] = 0xFFFFFFFFu;
-      }
-      if (js > je) finished = true;
+      finished = step == kBandDone;
     }
     if (finished) {
       int sum = frozen;
@@ -609,17 +352,6 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       active = false;
       state = -1;
       continue;
-    }
-    if (cnt) {
-      const int slack = score_mode ? INT_MAX : frozen + zw + (net2 - 32 * i) - cutoff;
-      if (slack < 0) {
-        active = false;
-        state = -1;
-        continue;
-      }
-      zskip = slack >> 5;  // the next blocks whose test cannot fail
-    } else {
-      zskip--;
     }
 #pragma unroll
     for (int p = 0; p < P; p++) cur[p] = nxt[p];
@@ -832,42 +564,24 @@ typedef void (*AlignFn)(DevDB, RunBufs, RunParams, int, int, int);
 static AlignFn warp_fn(int type, int cls) {
   (void)cls;
   return type == 0 ? k_align_warp<2> : k_align_warp<5>;
-}constexpr int kWarpKernel = kNumClasses;  // index of the warp kernel in the attribute table
-
-// DNA buckets 2 and 3 (windows of 17-32 blocks) receive pairs only when
-// NGIA_DNA_WIN_CLASSES (common.cuh) keeps them; by default those windows go
-// to bucket 4, the 64-slot tiled kernel.
-static AlignFn align_fn(int type, int cls) {
-  if (type == 0) {
-    switch (cls) {
-      case 0: return k_align_win<2, 8>;
-      case 1: return k_align_win<2, 16>;
-      case 2: return k_align_win<2, 24>;
-      case 3: return k_align_win<2, 32>;
-      case 4: return k_align_tiled<2, 64>;
-      case 5: return k_align_tiled<2, 128>;
-      default: return k_align_tiled<2, 0>;
-    }
-  }
-  switch (cls) {
-    case 0: return k_align_win<5, 8>;
-    case 1: return k_align_win<5, 16>;
-    case 2: return k_align_tiled<5, 64>;
-    case 3: return k_align_tiled<5, 128>;
-    default: return k_align_tiled<5, 0>;
-  }
 }
 
-// Dynamic shared memory: rep planes | k-mer bitset | (tiled class) row ring
+constexpr int kWarpKernel = kNumClasses;  // index of the warp kernel in the attribute table
+
+static AlignFn align_fn(int type, int cls) {
+  const int ring = class_ring(type, cls);
+  if (type == 0) return ring == 64 ? k_align_tiled<2, 64> : ring == 128 ? k_align_tiled<2, 128> : k_align_tiled<2, 0>;
+  return ring == 64 ? k_align_tiled<5, 64> : ring == 128 ? k_align_tiled<5, 128> : k_align_tiled<5, 0>;
+}
+
+// Dynamic shared memory: rep planes | k-mer bitset | row ring | match table
 // | (warp kernel, cls = kWarpKernel) every row of one pair per warp.
 static size_t align_smem(int type, int max_nb, int cls) {
   const int P = type ? 5 : 2;
   size_t words = (size_t)(((max_nb * P + 3) & ~3) + kListWords);
   if (cls == kWarpKernel) return 4u * (words + (size_t)(kAlignThreads / 32) * max_nb);
-  const bool tiled = is_tiled_class(type, cls) || cls == generic_class(type);  // k_align_tiled
-  const int ring = tiled ? class_cap(type, cls) : 0;  // 64, 128, or 0 (global ring)
-  words = (size_t)tiled_eq_off(P, max_nb, ring);
-  if (P == 2 && (tiled ? NGIA_ALIGN_EQ : NGIA_WIN_EQ)) words += (size_t)eq_words(max_nb);
+  words = (size_t)tiled_eq_off(P, max_nb, class_ring(type, cls));
+  if (P == 2) words += (size_t)eq_words(max_nb);
   return 4u * words;
 }
 
@@ -884,7 +598,7 @@ cudaError_t align_configure(int type, int max_nb) {
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(mu);
   for (int c = 0; c <= kNumClasses; c++) {
-    if (c >= num_classes(type) && c != kWarpKernel) continue;
+    if ((c < first_class(type) || c >= num_classes(type)) && c != kWarpKernel) continue;
     const int want = (int)align_smem(type, max_nb, c);
     int &have = configured[dev][type ? 1 : 0][c];
     if (want <= have) continue;

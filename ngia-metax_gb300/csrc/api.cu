@@ -60,14 +60,14 @@ int enqueue_iteration(ngia_ctx *c, bool graph, cudaGraphConditionalHandle cond) 
   if (graph && !c->batch_member) {
     // classes run as parallel branches of the body graph
     CK(cudaEventRecord(c->fork_ev, c->stream));
-    for (int k = 0; k < nc; k++) {
+    for (int k = ngia::first_class(c->db.type); k < nc; k++) {
       CK(cudaStreamWaitEvent(c->side[k], c->fork_ev, 0));
       CK(ngia::launch_align(c, k, c->side[k], 0));
       CK(cudaEventRecord(c->join_ev[k], c->side[k]));
       CK(cudaStreamWaitEvent(c->stream, c->join_ev[k], 0));
     }
   } else {
-    for (int k = 0; k < nc; k++) {
+    for (int k = ngia::first_class(c->db.type); k < nc; k++) {
       if (prof) CK(cudaEventRecord(c->ev_cls[k], c->stream));
       CK(ngia::launch_align(c, k, c->stream, 0));
     }
@@ -83,7 +83,7 @@ void account_stages(ngia_ctx *c) {
   float a = 0.f, b = 0.f;
   if (cudaEventElapsedTime(&a, c->ev_p0, c->ev_p1) == cudaSuccess) c->ms_filter += a;
   if (cudaEventElapsedTime(&b, c->ev_p1, c->ev_p2) == cudaSuccess) c->ms_align += b;
-  for (int k = 0; k < ngia::num_classes(c->db.type); k++) {
+  for (int k = ngia::first_class(c->db.type); k < ngia::num_classes(c->db.type); k++) {
     float m = 0.f;
     if (cudaEventElapsedTime(&m, c->ev_cls[k], c->ev_cls[k + 1]) == cudaSuccess) c->ms_class[k] += m;
   }
@@ -278,7 +278,7 @@ int load_db(ngia_ctx *c, const ngia_db_view *v) {
 // one CTA per 128 candidates and one warp per bitmap word.
 void size_grids(ngia_ctx *c, bool by_size) {
   const int type = c->db.type;
-  for (int k = 0; k < ngia::num_classes(type); k++)
+  for (int k = ngia::first_class(type); k < ngia::num_classes(type); k++)
     c->grid_align[k] = c->num_sms * ngia::align_occupancy(type, k, c->cap_nb);
   c->grid_filter = c->num_sms * 8;
   // warp-per-pair: the whole GPU's warps; a class goes warp-per-pair when it
@@ -292,7 +292,7 @@ void size_grids(ngia_ctx *c, bool by_size) {
   if (by_size) {
     const int64_t n = std::max(1, c->db.n), nbw = (n + 31) / 32;
     const int by_n = (int)std::min<int64_t>((n + 127) / 128, INT32_MAX);
-    for (int k = 0; k < ngia::num_classes(type); k++) c->grid_align[k] = std::max(1, std::min(c->grid_align[k], by_n));
+    for (int k = ngia::first_class(type); k < ngia::num_classes(type); k++) c->grid_align[k] = std::max(1, std::min(c->grid_align[k], by_n));
     c->grid_filter = std::max(1, std::min(c->grid_filter, (int)((nbw + 7) / 8)));
     // warp-per-pair: no more warps than the job has sequences
     const int wpc = ngia::align_threads() / 32;
@@ -318,7 +318,7 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
             dalloc(&rb.scan_part, nbw) == cudaSuccess && dalloc(&rb.long_list, (size_t)cap_n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&rb.flags, 4 * std::max<size_t>(nbw, 1)) == cudaSuccess;
   ok = ok && dalloc(&rb.fstats, (size_t)ngia::kFilterStripes * ngia::kFilterStats) == cudaSuccess;
-  for (int k = 0; ok && k < ngia::num_classes(type); k++) ok = dalloc(&rb.queue[k], (size_t)cap_n) == cudaSuccess;
+  for (int k = ngia::first_class(type); ok && k < ngia::num_classes(type); k++) ok = dalloc(&rb.queue[k], (size_t)cap_n) == cudaSuccess;
   if (!ok) return fail(NGIA_E_NOMEM, "ngia_open: device allocation of run buffers failed");
   cudaMemsetAsync(rb.rep_list, 0, 4 * ngia::kListWords, c->stream);
   cudaMemsetAsync(rb.fstats, 0, 8 * ngia::kFilterStripes * ngia::kFilterStats, c->stream);
@@ -662,7 +662,7 @@ extern "C" int ngia_pair_scores(ngia_ctx *c, const ngia_params *p, int32_t rep, 
   CK(cudaMemsetAsync(c->rb.st, 0, sizeof(ngia::RunState), c->stream));
   CK(ngia::launch_prep(c, rep));
   CK(ngia::launch_score_classify(c, n));
-  for (int k = 0; k < ngia::num_classes(c->db.type); k++) CK(ngia::launch_align(c, k, c->stream, 1));
+  for (int k = ngia::first_class(c->db.type); k < ngia::num_classes(c->db.type); k++) CK(ngia::launch_align(c, k, c->stream, 1));
   CK(cudaMemcpyAsync(out, d_o, 16 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
   rc = pull_state(c);
   cudaFree(d_c);

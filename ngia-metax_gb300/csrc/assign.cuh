@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
           pass = !(word_count<P>(planes, net2, prm.w, rlist) < word_min(L2, prm.w, s));
         }
       }
-      if (pass) res = 1 + serve_class(window_of(band_blocks(L1, L2, s), nb1));
+      if (pass) res = 1 + serve_class(window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
     }
     if (q < n) s_res[q] = (uint8_t)res;
     const unsigned pm = __ballot_sync(kFullMask, res != 0);
@@ -163,34 +163,10 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
   }
 }
 
-// NGIA_SERVE_STAGE 1 (DNA): each warp copies the match table of the
-// representative its pairs use into its own shared-memory region and runs
-// the tiles with the FMA-pipe bookkeeping of the clustering kernel
-// (tile.cuh); the claimed pairs start in groups that share a representative.
-// 0 (default): every lane reads its pair's table from global memory (L1).
-// Measured on GB300: serving 56.5k vs 59.2k queries/s (200 batches of
-// 1-4,096 DNA queries against 14,077 representatives, 16 slots), speculative
-// rounds of the 20,000-sequence job 0.685 vs 0.507 s.
-// The kernel is bound by the ALU pipe (80% busy, loads 50%), so the shared
-// tables save little, while groups leave lanes idle (27.7 of 32 active): a
-// claim holds pairs of several representatives, above all in the
-// speculative rounds, whose queue interleaves the candidates.
-#ifndef NGIA_SERVE_STAGE
-#define NGIA_SERVE_STAGE 0
-#endif
-// NGIA_SERVE_FMA (DNA, without staging): the per-column bookkeeping on the FMA
-// pipe with the table in global memory (as k_align_tiled does with its
-// shared-memory table).  Measured on GB300: serving 64.3k against 58.9k
-// queries/s (serving 200 DNA query batches, p99 642 against 782 ms), the
-// speculative rounds of the 20,000-sequence job 0.489 against 0.506 s.
-// NGIA_SERVE_REM_ROUND: remainder tiles rounded up to a multiple of this width
-// (fewer tile bodies); 2, 4 and 8 gave 63.5k, 62.2k and 59.1k queries/s.
-#ifndef NGIA_SERVE_FMA
-#define NGIA_SERVE_FMA 1
-#endif
-#ifndef NGIA_SERVE_REM_ROUND
-#define NGIA_SERVE_REM_ROUND 1
-#endif
+// The match table is read from global memory through L1 (copying it to
+// shared memory per warp, with the pairs grouped by representative, was
+// slower: 56.5k against 59.2k queries/s), and the per-column bookkeeping runs
+// on the FMA pipe as in the clustering kernel (64.3k against 58.9k).
 
 // Banded LCS of the queued (representative, query) pairs of one class: the
 // loop of k_align_tiled (align.cu) with the representative taken per pair.
@@ -198,21 +174,12 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
 // query, pairs of larger reps are skipped once a smaller one accepted);
 // MASK = true: every pair runs and an accepted one sets bit r of rb.mask[q]
 // and its score.
-// A warp claims 32 queue entries once none of its lanes holds a pair.  With
-// staging (DNA), the claimed pairs start in groups: each group is the lanes
-// whose pair has the representative of the first waiting lane, that
-// representative's table is copied into the warp's region unless it is
-// there already, and the next group starts when the current one is done.
-// The filters queue the pairs of one representative next to each other (one
-// CTA per representative in serving, per-candidate pushes in the
-// speculative rounds), so a claim holds one or two groups.
 template <int P, int RING, bool MASK>
 __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     k_serve_align(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int word_after, uint32_t *scratch,
                   int64_t scratch_words, uint32_t ring_mask) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint32_t s_qn;
-  constexpr bool kStage = P == 2 && NGIA_SERVE_EQ && NGIA_SERVE_STAGE;
   if (threadIdx.x == 0) s_qn = (int64_t)rb.ctl[cls] < rb.cap ? rb.ctl[cls] : (uint32_t)rb.cap;
   __syncthreads();
   const uint32_t qn = s_qn;
@@ -227,15 +194,10 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     ring.mask = ring_mask;
     ring.stride = TL;
   }
-  // this warp's match-table region (after the shared ring)
-  uint32_t *w_eq = smem + (RING > 0 ? RING * kAlignThreads : 0) + (int64_t)(threadIdx.x >> 5) * rs.eq_stride;
-  const uint32_t w_eq_s = smem_u32(w_eq);
-  (void)w_eq_s;
   // 1 and 4 as values ptxas cannot fold (the FMA-pipe bookkeeping of tile.cuh)
   const uint32_t one_rt = 1u + (uint32_t)(qn == 0u);
   const FmaK fk{one_rt, one_rt << 2};
   (void)fk;
-  int staged = -1;  // representative whose table is in the warp's region (warp-uniform)
   const int lane = threadIdx.x & 31;
   const float s = prm.s;
   const int hw = qdb.hw;
@@ -247,9 +209,8 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   const uint32_t *qpl = nullptr, *rpl = nullptr;
   uint32_t cur[P], nxt[P];
   unsigned long long n_pairs = 0, n_cells = 0;
-  // every loop pass advances a running lane by one query block, claims, or
-  // starts a group: bounded by the queued pairs' blocks (each at most
-  // kMaxBlocks) and the groups per claim, per warp
+  // every loop pass advances a running lane by one query block or claims:
+  // bounded by the queued pairs' blocks (each at most kMaxBlocks), per warp
   const long long guard_max = ((long long)qn + 64) * (kMaxBlocks + 36);
   long long guard = 0;
   for (;;) {
@@ -258,11 +219,11 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       break;
     }
     {  // refill once prm.refill lanes are idle or none holds a pair (as in
-       // k_align_tiled; with staging only when none holds a pair); the warp
-       // votes run on all 32 lanes before they are combined per lane
+       // k_align_tiled); the warp votes run on all 32 lanes before they are
+       // combined per lane
       const bool any_held = __any_sync(kFullMask, state >= 0);
       const unsigned idle = __ballot_sync(kFullMask, state == -1);
-      const bool refill_now = !any_held || (!kStage && __popc(idle) >= prm.refill);
+      const bool refill_now = !any_held || __popc(idle) >= prm.refill;
       const bool need = state == -1 && refill_now;
       const unsigned nm = __ballot_sync(kFullMask, need);
       if (nm) {
@@ -282,28 +243,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       }
     }
     if (__all_sync(kFullMask, state == -2)) break;
-    // start claimed pairs: without staging at once; with staging in groups
-    // sharing a representative, the next group once no pair runs
-    bool start = state >= 0 && !active;
-    if constexpr (kStage) {
-      start = false;
-      if (!__any_sync(kFullMask, active)) {
-        const unsigned pm = __ballot_sync(kFullMask, state >= 0);
-        if (pm) {
-          const int rg = __shfl_sync(kFullMask, r, __ffs(pm) - 1);
-          if (rg != staged) {
-            const uint32_t *rrec = rs.words + rs.off[rg];
-            const int words = 4 * (((int)rrec[1] + 31) / 32 + kEqPad);  // table blocks + zero blocks
-            const uint4 *src = reinterpret_cast<const uint4 *>(rs.eq + (int64_t)rg * rs.eq_stride);
-            __syncwarp();
-            for (int t = lane; t < words / 4; t += 32) reinterpret_cast<uint4 *>(w_eq)[t] = __ldg(src + t);
-            __syncwarp();
-            staged = rg;
-          }
-          start = state >= 0 && r == rg;
-        }
-      }
-    }
+    const bool start = state >= 0 && !active;
     if (start) {
       const uint32_t *rrec = rs.words + rs.off[r];
       const int L1 = (int)rrec[0];
@@ -320,7 +260,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       qpl = qdb.words + __ldg(qdb.off + q) + hw;
       i = 0;
       js = 0;
-      je = min(B, nb1 - 1);
+      je = band_first_top(B, nb1, net1, cutoff);
       frozen = 0;
       zw = 0;
       if (!MASK && (rb.key[q] >> 32) < (unsigned long long)r) {
@@ -356,24 +296,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + (i + 1) * P + p);
     }
     using Ring = typename RingOf<RING>::T;
-    if constexpr (kStage) {  // match words from the warp's staged table (shared memory)
-      uint32_t wc[2];
-      eq_codes_top(cur, wc);
-      uint32_t cw = 0, ncw = 0;
-      int base = js;
-      if (NGIA_EQ_NOZOLD) zw = 0;  // the tiles return their rows' zero counts
-      for (int t = 0; t < full; t++, base += MT) {
-        zw += tiled_tile_eqf<MT, NGIA_SERVE_PF, Ring>(ring, w_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile_eqf<MT, NGIA_SERVE_PF, Ring>(ring, w_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      if (rem > 0) zw += tiled_rem_eqf<Ring, MT>(rem, ring, w_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-    } else if constexpr (P == 2 && NGIA_SERVE_EQ && NGIA_SERVE_FMA) {
+    if constexpr (P == 2) {
       // match words from the pair's representative's table (global memory,
       // L1), the per-column bookkeeping on the FMA pipe as in k_align_tiled
       const uint64_t req = (uint64_t)(rs.eq + (int64_t)r * rs.eq_stride);
@@ -392,24 +315,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
         cw = ncw << (32 - cols);
         ncw = 0;
       }
-      if (rem > 0) zw += tiled_rem_eqfg<Ring, NGIA_SERVE_REM_ROUND>(rem, ring, req, base, je, nb1, cols, wc, cw, ncw, fk);
-    } else if constexpr (P == 2 && NGIA_SERVE_EQ) {  // match words from the pair's representative's table
-      const uint32_t *req = rs.eq + (int64_t)r * rs.eq_stride;
-      uint32_t q4[4];
-      eq_codes(cur, q4);
-      uint32_t cw = 0, ncw = 0;
-      int base = js;
-      for (int t = 0; t < full; t++, base += MT) {
-        zw += tiled_tile_eq<MT, NGIA_SERVE_PF, Ring>(ring, req, base, je, nb1, cols, q4, cw, ncw);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile_eq<MT, NGIA_SERVE_PF, Ring>(ring, req, base, je, nb1, cols, q4, cw, ncw);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      if (rem > 0) zw += tiled_rem_eq<Ring, MT>(rem, ring, req, base, je, nb1, cols, q4, cw, ncw);
+      if (rem > 0) zw += tiled_rem_eqfg<Ring>(rem, ring, req, base, je, nb1, cols, wc, cw, ncw, fk);
     } else {
       uint32_t cw = 0, ncw = 0;
       int base = js;
@@ -428,17 +334,13 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     i++;
     bool finished = i >= nq;
     if (!finished) {
-      if (i - B > 0) {  // block js leaves the band
-        const uint32_t r0 = ring[js];
-        frozen += __popc(~r0 & (js == nb1 - 1 ? vlast : 0xFFFFFFFFu));
-        zw -= __popc(~r0);
-        js++;
+      const int step = band_advance(ring, i, B, nb1, net1, vlast, net2 - 32 * i, cutoff, js, je, frozen, zw);
+      if (step == kBandReject) {
+        active = false;
+        state = -1;
+        continue;
       }
-      if (i + B <= nb1 - 1) {  // block je enters all-ones
-        je++;
-        ring[je] = 0xFFFFFFFFu;
-      }
-      if (js > je) finished = true;
+      finished = step == kBandDone;
     }
     if (finished) {
       int sum = frozen;
@@ -454,11 +356,6 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
           atomicMin(&rb.key[q], ((unsigned long long)r << 32) | (uint32_t)sum);
         }
       }
-      active = false;
-      state = -1;
-      continue;
-    }
-    if (frozen + zw + (net2 - 32 * i) < cutoff) {  // cannot reach the cutoff any more
       active = false;
       state = -1;
       continue;
@@ -485,13 +382,8 @@ AlignServeFn serve_align_fn(int type, int cls) {
   return cls == 0 ? k_serve_align<5, 64, MASK> : cls == 1 ? k_serve_align<5, 128, MASK> : k_serve_align<5, 0, MASK>;
 }
 
-// Dynamic shared memory of class cls: the row ring (shared classes) and, for
-// DNA with staging, one match-table region of eq_stride words per warp.
-inline size_t serve_align_smem(int type, int cls, int64_t eq_stride) {
-  size_t b = cls == 2 ? 0 : (size_t)(cls == 0 ? 64 : 128) * kAlignThreads * 4;
-  if (type == 0 && NGIA_SERVE_EQ && NGIA_SERVE_STAGE) b += 4 * (size_t)(kAlignThreads / 32) * (size_t)eq_stride;
-  return b;
-}
+// Dynamic shared memory of class cls: the row ring (shared classes).
+inline size_t serve_align_smem(int cls) { return cls == 2 ? 0 : (size_t)(cls == 0 ? 64 : 128) * kAlignThreads * 4; }
 
 // Raises the kernel's dynamic shared memory limit to `bytes` (never lowers
 // it: launches of other open servers or contexts may need more).

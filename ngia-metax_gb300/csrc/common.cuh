@@ -14,46 +14,23 @@ constexpr int kMaxBlocks = kMaxLenDev / 32;    // 2048 plane blocks
 constexpr int kListWords = 2048;               // rep k-mer presence bitset (65,536 bits)
 constexpr int kRefGridThreads = 128 * 128;     // BLOCK*WARP of the reference launch
 
-// Alignment work classes.  Pairs are queued by the width A of their active
-// band window (rep blocks touched by one query block, min(2B+1, nb1)).  The
-// register-window classes hold the whole window in registers (capacity WC);
-// the tiled classes keep up to 64 or 128 window rows per pair in a
-// shared-memory ring and stream them through 16-slot register tiles; the last
-// class of each type (any width) runs the tiled kernel on a global-memory
-// ring.
+// Alignment work classes.  Pairs are queued by the width of the band window
+// their alignment can need (window_need, in rep blocks).  Three are in use
+// per type: up to 64 or 128 window rows per pair in a shared-memory ring, any
+// width on a global-memory ring, all through 16-slot register tiles.  The
+// numbers before first_class stand for the register-window kernels of
+// earlier versions (8 to 32 blocks); they stay unused so that class numbers
+// in saved tunings, checkpoints and statistics keep their meaning.
 constexpr int kNumClasses = 7;
-constexpr int kRingBlocks = 128;  // largest ring (the tiled classes use 64 and 128)
-__host__ __device__ inline int class_cap(int type, int c) {
-  // DNA: 8,16,24,32 | tiled 64, 128 | any;  protein: 8,16 | tiled 64, 128 | any
-  if (type == 0) {
-    const int caps[7] = {8, 16, 24, 32, 64, 128, 0};
-    return caps[c];
-  }
-  const int caps[7] = {8, 16, 64, 128, 0, 0, 0};
-  return caps[c];
-}
 __host__ __device__ inline int num_classes(int type) { return type == 0 ? 7 : 5; }
 __host__ __device__ inline int generic_class(int type) { return num_classes(type) - 1; }
-__host__ __device__ inline bool is_tiled_class(int type, int c) {
-  return c == generic_class(type) - 1 || c == generic_class(type) - 2;
+__host__ __device__ inline int first_class(int type) { return num_classes(type) - 3; }
+// Ring rows of class c: 64, 128, or 0 (global-memory ring).
+__host__ __device__ inline int class_ring(int type, int c) {
+  return c >= generic_class(type) ? 0 : c == generic_class(type) - 1 ? 128 : 64;
 }
-// DNA register-window classes in use (caps 8, 16, 24, 32 blocks, in that
-// order); windows above the last one in use go to the 64-block tiled class.
-// Two: windows of 17-64 blocks share the tiled class's persistent launch,
-// where their pairs fill the launch's tail instead of running as separate
-// latency-bound launches beside it.  Measured on GB300 (1M DNA s=0.85,
-// graph driver): 4, 3, 2 and 0 classes gave 136.1M, 137.6M, 138.0M and
-// 138.0M candidate seqs/s.
-#ifndef NGIA_DNA_WIN_CLASSES
-#define NGIA_DNA_WIN_CLASSES 2
-#endif
 __host__ __device__ inline int class_of(int type, int A) {
-  const int g = generic_class(type);
-  for (int c = 0; c < g; c++) {
-    if (type == 0 && c < 4 && c >= NGIA_DNA_WIN_CLASSES) continue;
-    if (A <= class_cap(type, c)) return c;
-  }
-  return g;
+  return first_class(type) + (A <= 64 ? 0 : A <= 128 ? 1 : 2);
 }
 
 // Device copy of the makeDB database plus per-sequence header arrays.
@@ -234,11 +211,24 @@ __device__ __forceinline__ int word_min(int L2, int w, float s) {
   return (L2 - w + 1) - length * w;
 }
 
-// Window width (rep blocks per query block) of a pair.
+// Window width (rep blocks per query block) of a pair's whole band.
 __host__ __device__ __forceinline__ int window_of(int B, int nb1) {
   if (B < 0 || nb1 <= 0) return 0;
   int a = 2 * B + 1;
   return a < nb1 ? a : nb1;
+}
+
+// Widest window the alignment of a pair can need when only scores of at
+// least `cut` matter: a chain of matches that reaches it leaves at most
+// L2 - cut query and L1 - cut rep residues unmatched, so it stays between
+// diagonals -(L2 - cut) and L1 - cut (rep position - query position); three
+// blocks cover the ends of a 32-column step (band_advance in tile.cuh keeps
+// every window within this).  Raw lengths bound the net ones.
+__host__ __device__ __forceinline__ int window_need(int L1, int L2, int cut, int B, int nb1) {
+  const int a = window_of(B, nb1);
+  const int d = L2 > cut ? L2 - cut : 0, u = L1 > cut ? L1 - cut : 0;
+  const int need = (d >> 5) + (u >> 5) + 3;
+  return a < need ? a : need;
 }
 
 // Reference band cells of one pair: sum over query blocks of

@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
             deferred = true;
           }
         }
-        if (pass) cls = class_of(db.type, window_of(band_blocks(L1, L2, s), nb1));
+        if (pass) cls = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
       }
       // long candidates go to k_filter_long, which gives each one a warp
       const unsigned dm = __ballot_sync(kFullMask, deferred);
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
             deferred = true;
           }
         }
-        if (pass && !exact) cls_of[k] = class_of(db.type, window_of(band_blocks(L1, L2, s), nb1));
+        if (pass && !exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
       }
       // long candidates: the whole warp counts each one
       for (unsigned dm = __ballot_sync(kFullMask, deferred); dm; dm &= dm - 1) {
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
           pass = !(ws < word_min(L2, prm.w, s));
           if (pass) {
             wpass++;
-            if (!exact) cls_of[k] = class_of(db.type, window_of(band_blocks(L1, L2, s), nb1));
+            if (!exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
           }
         }
       }
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(256) k_word_exact(DevDB db, RunBufs rb, RunPar
       }
       if (pass) {
         wpass++;
-        cls = class_of(db.type, window_of(band_blocks(L1, L2, prm.s), nb1));
+        cls = class_of(db.type, window_need(L1, L2, cutoff_of(L2, prm.s), band_blocks(L1, L2, prm.s), nb1));
       }
     }
     push_queue(rb, st, pass, cls, c);
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(256) k_filter_long(DevDB db, RunBufs rb, RunPa
     const int L2 = __ldg(db.len + c);
     const bool pass = lane == 0 && !(ws < word_min(L2, prm.w, s));
     if (pass) wpass++;
-    push_queue(rb, st, pass, pass ? class_of(db.type, window_of(band_blocks(L1, L2, s), nb1)) : 0, c);
+    push_queue(rb, st, pass, pass ? class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1)) : 0, c);
   }
   flush_stats(rb, 0, 0, 0, 0, wpass);
 }

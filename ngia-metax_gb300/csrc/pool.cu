@@ -143,7 +143,7 @@ __device__ void chunks_body(const PoolDev &pd, int ncls) {
   const int nj = pd.n_jobs, t = threadIdx.x;
   const int per = (nj + NT - 1) / NT;
   const int j0 = min(nj, t * per), j1 = min(nj, j0 + per);
-  for (int k = 0; k < ncls; k++) {
+  for (int k = first_class(pd.type); k < ncls; k++) {  // the classes in use
     long long tot = 0;
     for (int j = j0; j < j1; j++) tot += pd.jobs[j].rb.st->qcount[k];
 #pragma unroll
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256) k_pool_filter(PoolDev pd, int ncls) {
             deferred = true;
           }
         }
-        if (pass && !deferred) cls = class_of(type, window_of(band_blocks(L1, L2, s), nb1));
+        if (pass && !deferred) cls = class_of(type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
       }
     }
     for (unsigned dm = __ballot_sync(kFullMask, deferred); dm; dm &= dm - 1) {
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) k_pool_filter(PoolDev pd, int ncls) {
         const int L2 = __ldg(J->db.len + cc);
         pass = !(ws < word_min(L2, w, s));
         wpass = pass;
-        if (pass) cls = class_of(type, window_of(band_blocks(L1, L2, s), nb1));
+        if (pass) cls = class_of(type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
       }
     }
     push_queue(J->rb, J->rb.st, pass, cls, c);
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
   __shared__ int s_j, s_a, s_b;
   __shared__ uint32_t s_next;
   __shared__ unsigned long long s_qw;
-  constexpr bool kEq = P == 2 && NGIA_ALIGN_EQ;
+  constexpr bool kEq = P == 2;
   constexpr int MT = tiled_main(P);
   const int nj = pd.n_jobs;
   const int32_t *cb = pd.chunk_base + cls * (nj + 1);
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
         qpl = db.words + __ldg(db.off + cand) + db.hw;
         i = 0;
         js = 0;
-        je = min(B, nb1 - 1);
+        je = band_first_top(B, nb1, net1, cutoff);
         frozen = 0;
         zw = 0;
         n_pairs++;
@@ -527,12 +527,12 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
         for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + (i + 1) * P + p);
       }
       using Ring = typename RingOf<RING>::T;
-      if constexpr (kEq && NGIA_EQ_FMA) {
+      if constexpr (kEq) {
         uint32_t wc[2];
         eq_codes_top(cur, wc);
         uint32_t cw = 0, ncw = 0;
         int base = js;
-        if (NGIA_EQ_NOZOLD) zw = 0;  // the tiles return their rows' zero counts
+        zw = 0;  // the tiles return their rows' zero counts
         for (int t = 0; t < full; t++, base += MT) {
           zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
           cw = ncw << (32 - cols);  // column 0's carry at bit 31
@@ -543,23 +543,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
           cw = ncw << (32 - cols);
           ncw = 0;
         }
-        if (rem > 0) zw += tiled_rem_eqf<Ring, MT>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-      } else if constexpr (kEq) {
-        uint32_t q[4];
-        eq_codes(cur, q);
-        uint32_t cw = 0, ncw = 0;
-        int base = js;
-        for (int t = 0; t < full; t++, base += MT) {
-          zw += tiled_tile_eq<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq, base, je, nb1, cols, q, cw, ncw);
-          cw = ncw << (32 - cols);
-          ncw = 0;
-        }
-        for (; rem >= MT; rem -= MT, base += MT) {
-          zw += tiled_tile_eq<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq, base, je, nb1, cols, q, cw, ncw);
-          cw = ncw << (32 - cols);
-          ncw = 0;
-        }
-        if (rem > 0) zw += tiled_rem_eq<Ring, MT>(rem, ring, s_eq, base, je, nb1, cols, q, cw, ncw);
+        if (rem > 0) zw += tiled_rem_eqf<Ring>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
       } else {
         uint32_t cw = 0, ncw = 0;
         int base = js;
@@ -578,17 +562,13 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
       i++;
       bool finished = i >= nq;
       if (!finished) {
-        if (i - B > 0) {  // block js leaves the band
-          const uint32_t r0 = ring[js];
-          frozen += __popc(~r0 & (js == nb1 - 1 ? vlast : 0xFFFFFFFFu));
-          zw -= __popc(~r0);
-          js++;
+        const int step = band_advance(ring, i, B, nb1, net1, vlast, net2 - 32 * i, cutoff, js, je, frozen, zw);
+        if (step == kBandReject) {
+          active = false;
+          state = -1;
+          continue;
         }
-        if (i + B <= nb1 - 1) {  // block je enters all-ones
-          je++;
-          ring[je] = 0xFFFFFFFFu;
-        }
-        if (js > je) finished = true;
+        finished = step == kBandDone;
       }
       if (finished) {
         int sum = frozen;
@@ -602,11 +582,6 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
           atomicAnd(&alive[cand >> 5], ~(1u << (cand & 31)));
           n_members++;
         }
-        active = false;
-        state = -1;
-        continue;
-      }
-      if (frozen + zw + (net2 - 32 * i) < cutoff) {  // cannot reach the cutoff any more
         active = false;
         state = -1;
         continue;
@@ -652,13 +627,6 @@ __global__ void __launch_bounds__(1024) k_pool_next(PoolDev pd, cudaGraphConditi
 // ---- host side -------------------------------------------------------------------
 using PoolAlignFn = void (*)(PoolDev, int, int);
 
-// Ring per bucket: every window up to 64 blocks in the 64-slot shared ring,
-// then 128, then the global ring (the last bucket).
-int ring_of(int type, int cls) {
-  const int cap = class_cap(type, cls);
-  return cap == 0 ? 0 : cap <= 64 ? 64 : 128;
-}
-
 PoolAlignFn align_fn(int type, int ring) {
   if (type == 0) return ring == 64 ? k_pool_align<2, 64> : ring == 128 ? k_pool_align<2, 128> : k_pool_align<2, 0>;
   return ring == 64 ? k_pool_align<5, 64> : ring == 128 ? k_pool_align<5, 128> : k_pool_align<5, 0>;
@@ -667,7 +635,7 @@ PoolAlignFn align_fn(int type, int ring) {
 size_t align_smem(int type, int max_nb, int ring) {
   const int P = type ? 5 : 2;
   size_t words = (size_t)tiled_eq_off(P, max_nb, ring);
-  if (P == 2 && NGIA_ALIGN_EQ) words += (size_t)eq_words(max_nb);
+  if (P == 2) words += (size_t)eq_words(max_nb);
   return 4 * words;
 }
 
@@ -758,8 +726,8 @@ int group_open(const std::vector<ngia_ctx *> &jobs, Group **out) {
   // resident CTAs of its kernel (the global-ring bucket at most 2 per SM)
   g->grid_filter = std::max(1, std::min(g->num_sms * 8, (wbase[nj] + 7) / 8));
   PoolDev &pd = g->pd;
-  for (int k = 0; k < num_classes(type); k++) {
-    const int ring = ring_of(type, k);
+  for (int k = first_class(type); k < num_classes(type); k++) {
+    const int ring = class_ring(type, k);
     g->smem[k] = align_smem(type, g->max_nb, ring);
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)align_fn(type, ring), kAlignThreads,
@@ -777,7 +745,7 @@ int group_open(const std::vector<ngia_ctx *> &jobs, Group **out) {
     group_close(g);
     return fail(NGIA_E_NOMEM, "pool: device allocation of the alignment ring failed");
   }
-  for (int k = 0; k < num_classes(type); k++)
+  for (int k = first_class(type); k < num_classes(type); k++)
     if (cudaStreamCreateWithFlags(&g->side[k], cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&g->join[k], cudaEventDisableTiming) != cudaSuccess) {
       group_close(g);
@@ -835,13 +803,13 @@ int group_enqueue_round(Group *g, cudaStream_t s, cudaGraphConditionalHandle con
   else
     k_pool_filter<5><<<g->grid_filter, 256, fsm, s>>>(pd, nc);
   cudaError_t e = cudaEventRecord(g->fork, s);
-  for (int k = 0; e == cudaSuccess && k < nc; k++) {
+  for (int k = first_class(type); e == cudaSuccess && k < nc; k++) {
     e = cudaStreamWaitEvent(g->side[k], g->fork, 0);
     if (e != cudaSuccess) break;
     PoolDev a = pd;
     int cls = k, mnb = g->max_nb;
     void *args[] = {&a, &cls, &mnb};
-    e = cudaLaunchKernel((const void *)align_fn(type, ring_of(type, k)), dim3(pd.grid_align[k]), dim3(kAlignThreads),
+    e = cudaLaunchKernel((const void *)align_fn(type, class_ring(type, k)), dim3(pd.grid_align[k]), dim3(kAlignThreads),
                          args, g->smem[k], g->side[k]);
     if (e == cudaSuccess) e = cudaEventRecord(g->join[k], g->side[k]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, g->join[k], 0);

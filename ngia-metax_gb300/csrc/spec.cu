@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256) k_spec_filter(DevDB db, RunBufs run, Spec
       if (pass) pass = !(base_sum<A>(db.cnt, x, s_rc + i * A) < cut);
       if (pass && word_here && s_net1[i] >= 16 && net2 >= 16)
         pass = !(word_count<P>(qpl, net2, prm.w, sd.lists + (int64_t)i * list_words) < word_min(L2, prm.w, s));
-      const int res = pass ? 1 + serve_class(window_of(band_blocks(s_L1[i], L2, s), s_nb1[i])) : 0;
+      const int res = pass ? 1 + serve_class(window_need(s_L1[i], L2, cut, band_blocks(s_L1[i], L2, s), s_nb1[i])) : 0;
       const unsigned pm = __ballot_sync(kFullMask, res != 0);
       if (res) {
         const unsigned peers = __match_any_sync(pm, res);
@@ -386,7 +386,7 @@ int spec_alloc(ngia_ctx *c) {
     std::lock_guard<std::mutex> lock(mu);
     for (int k = 0; k < kServeClasses; k++) {
       const void *fn = (const void *)serve_align_fn<true>(sp->type, k);
-      const size_t smem = serve_align_smem(sp->type, k, sp->eq_stride);
+      const size_t smem = serve_align_smem(k);
       CKP(serve_align_configure<true>(sp->type, k, smem));
       int occ = 0;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kAlignThreads, smem) != cudaSuccess ||
@@ -439,7 +439,7 @@ int spec_launch_round(ngia_ctx *c, bool lists) {
     uint32_t rm = sp->ring_mask;
     void *args[] = {&db, &rs, &prm, &rb, &cls, &wa, &scr, &sw, &rm};
     CKP(cudaLaunchKernel((const void *)serve_align_fn<true>(c->db.type, k), dim3(sp->grid[k]), dim3(kAlignThreads),
-                         args, serve_align_smem(c->db.type, k, sp->eq_stride), st));
+                         args, serve_align_smem(k), st));
   }
   k_spec_resolve<<<1, 32, 0, st>>>(sp->d, sp->rb);
   CKP(cudaGetLastError());
