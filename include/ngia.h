@@ -420,12 +420,14 @@ int ngia_set_tuning(ngia_ctx *ctx, const ngia_tuning *t);
  * per job, side by side) give their jobs, by timing three policies on the
  * whole batch over the first `iters` greedy iterations of every job:
  *   NGIA_BATCH_POLICY_THREAD  every length bucket of every job aligned
- *                             thread per pair (the untuned batch default);
+ *                             thread per pair;
  *   NGIA_BATCH_POLICY_CUTOFF  each job's default warp-per-pair cut-off;
  *   NGIA_BATCH_POLICY_TUNED   each job's own ngia_autotune settings, found
  *                             with the job alone on the GPU (cached by
  *                             database shape and parameters).
- * The thread-per-pair policy stays unless another is at least 2% faster.
+ * The thread-per-pair policy is chosen unless another is at least 2% faster.
+ * (Before any choice, a job's buckets go to the group-per-pair kernels up to
+ * the default cut-off divided by the number of jobs.)
  * Later NGIA_MODE_GRAPH runs apply the chosen policy; out[j] (may be NULL)
  * receives job j's settings under it (candidates = 3, ms_per_iter and
  * default_ms_per_iter the batch's wall time per iteration under the chosen

@@ -24,7 +24,9 @@
 //   IADD3.X, LOP3); protein builds it from the rep's planes held in registers
 //   (one LOP3 per plane).
 //
-// k_align_warp<P>  classes with few queued pairs: one warp per pair.
+// k_align_wave<P,NW>, k_align_query<P>  classes with few queued pairs: a warp
+//   (windows up to 64 blocks) or a CTA of four warps per pair; 16 threads for
+//   a short query against a long representative (wave.cuh).
 //
 // In clustering both keep only the rows that a score of at least the cutoff
 // can use (band_advance in tile.cuh) and stop a pair once it provably cannot
@@ -36,7 +38,9 @@
 #include <mutex>
 
 #include "ctx.h"
+#include "kmer.cuh"
 #include "tile.cuh"
+#include "wave.cuh"
 
 namespace ngia {
 
@@ -50,21 +54,21 @@ struct AlignHdr {
 // when the short-word test follows the alignment, its k-mer bitset) into
 // shared memory with bulk copies.  Returns false when there is no work.
 template <int P>
-// warp_mode: 1 for the warp-per-pair kernel (works on classes with at most
-// warp_pairs pairs), 0 for the thread-per-pair kernels (more than that); the
-// other kernel of a class returns here, before any staging.
+// groups: pairs a CTA of the group-per-pair kernel works on at a time (it
+// takes classes with at most warp_pairs pairs), 0 for the thread-per-pair
+// kernels (classes with more); the other kernel of a class returns here,
+// before any staging.
 __device__ __forceinline__ bool align_setup(const DevDB &db, const RunBufs &rb, const RunParams &prm, int cls,
-                                            int score_mode, int warp_pairs, int warp_mode, uint32_t *smem,
+                                            int score_mode, int warp_pairs, int groups, uint32_t *smem,
                                             uint64_t *bar, AlignHdr &h) {
   __shared__ int s_hdr[6];
   RunState *st = rb.st;
   if (threadIdx.x == 0) {
     const bool skip = !score_mode && (st->done || st->iter >= st->iter_limit || st->err);
     const int qn = skip ? 0 : (int)st->qcount[cls];
-    const bool mine = warp_mode ? qn <= warp_pairs : qn > warp_pairs;
-    // warp-per-pair: one pair per warp of this CTA
-    const bool idle = warp_mode && (int)(blockIdx.x * (blockDim.x >> 5)) >= qn;
-    s_hdr[0] = mine && !idle ? qn : 0;
+    const bool mine = groups ? qn <= warp_pairs : qn > warp_pairs;
+    const bool idle = (int)blockIdx.x * groups >= qn;
+    s_hdr[0] = mine && !(groups && idle) ? qn : 0;
     s_hdr[1] = st->rep_len;
     s_hdr[2] = st->rep_net;
     s_hdr[3] = st->rep_nb;
@@ -360,200 +364,157 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
 }
 
 
-// ---- one warp per pair ------------------------------------------------------------
-// For iterations with few queued pairs of a class, the latency of one pair
-// on one thread (every residue of the query against the whole band window,
-// in order) bounds the iteration.  k_align_warp gives each pair a warp.  The
-// band's rows are cut into strips of 32, one row word per lane, and all 32
-// lanes apply the same query residue together: the strip is one 1,024-bit
-// addition row + (row & match) + carry, whose word carries are resolved with
-// carry lookahead over the lanes — lane l's word sum yields a generate bit
-// (it overflowed) and a propagate bit (it is all ones); with G and Pm the
-// ballots of those, the carry into every lane is a bit of
-// ((G | Pm) + G + carry_in) ^ (G | Pm) ^ G, and that 32-bit addition's own
-// carry is the strip's carry out.  Strips of a query block run bottom-up, the
-// column carries of one strip (a 32-bit mask) feeding the next; the lowest
-// band row takes carry 0 and the top row's carry is dropped (the reference's
-// band semantics).  Band rows live in shared memory (all nb1 rows of the
-// pair, all-ones until they enter the band), loaded at a strip's start and
-// stored at its end; after every query block the zero count (kept as the
-// sum of the lanes' row changes) gives the exact early rejection test.
-// sum = a + b over W words (word 0 lowest); returns the carry out.
-template <int W>
-__device__ __forceinline__ uint32_t add_words(const uint32_t (&a)[W], const uint32_t (&b)[W], uint32_t (&sum)[W]) {
-  uint32_t c;
-  if constexpr (W == 1) {
-    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(sum[0]), "=r"(c) : "r"(a[0]), "r"(b[0]));
-  } else if constexpr (W == 2) {
-    asm("add.cc.u32 %0, %3, %5;\n\taddc.cc.u32 %1, %4, %6;\n\taddc.u32 %2, 0, 0;"
-        : "=r"(sum[0]), "=r"(sum[1]), "=r"(c)
-        : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
-  } else {
-    static_assert(W == 4, "W is 1, 2 or 4");
-    asm("add.cc.u32 %0, %5, %9;\n\taddc.cc.u32 %1, %6, %10;\n\taddc.cc.u32 %2, %7, %11;\n\t"
-        "addc.cc.u32 %3, %8, %12;\n\taddc.u32 %4, 0, 0;"
-        : "=r"(sum[0]), "=r"(sum[1]), "=r"(sum[2]), "=r"(sum[3]), "=r"(c)
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
+// Word offset of the group kernels' match table: after the planes and the
+// k-mer bitset.
+__host__ __device__ constexpr int wave_table_off(int P, int max_nb) { return ((max_nb * P + 3) & ~3) + kListWords; }
+
+// ---- a group of threads per pair (wave.cuh) ------------------------------------------
+// For classes with few queued pairs the latency of one pair on one thread
+// bounds the iteration.  NW = 1: a warp per pair (windows up to 64 blocks);
+// NW = 4: the CTA per pair, W = 1 row word per thread for windows up to 128
+// blocks, up to 16 for any.
+template <int P, int NW, int WMAX>
+__global__ void __launch_bounds__(kAlignThreads)
+    k_align_wave(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t s_xch[4 * NW];
+  AlignHdr h;
+  __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
+  if (threadIdx.x == 0) s_qw = 0;
+  constexpr int kGroups = kAlignThreads / 32 / NW;  // pairs per CTA
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kGroups, smem, &bar, h)) return;
+  const uint32_t *s_pl = smem;
+  const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
+  const int group = (int)(threadIdx.x >> 5) / NW;
+  const bool lead = threadIdx.x % (32 * NW) == 0;
+  RunState *st = rb.st;
+  const float s = prm.s;
+  const int nb1 = h.nb1;
+  const uint32_t vlast = (h.net1 & 31) ? ((1u << (h.net1 & 31)) - 1u) : 0xFFFFFFFFu;
+  uint32_t *s_tab = smem + wave_table_off(P, db.max_nb);
+  uint32_t *s_ring = s_tab + wave_table_words(P, db.max_nb) + group * kWaveRingWords;
+  wave_table<P>(s_pl, nb1, vlast, s_tab, threadIdx.x, kAlignThreads);
+  __syncthreads();
+  unsigned long long n_pairs = 0, n_members = 0, n_cells = 0, n_done = 0;
+  for (int e = blockIdx.x * kGroups + group; e < h.qn; e += gridDim.x * kGroups) {
+    const int entry = rb.queue[cls][e];
+    const int cand = score_mode ? rb.score_cands[entry] : entry;
+    const int L2 = __ldg(db.len + cand), net2 = __ldg(db.net + cand);
+    const int nq = (net2 + 31) >> 5;
+    const int B = band_blocks(h.L1, L2, s);
+    const int cutoff = cutoff_of(L2, s);
+    const uint32_t *qpl = db.words + __ldg(db.off + cand) + db.hw;
+    if (!score_mode && lead) {
+      n_pairs++;
+      n_cells += (unsigned long long)band_cells(B, nb1, net2);
+      atomicAdd(&s_qw, (unsigned long long)(nq * P));
+    }
+    int sum = 0;  // no band: score 0
+    if (B >= 0 && nb1 > 0 && nq > 0) {
+      const int cut = score_mode ? kNoCut : cutoff;
+      int lo, hi;
+      if (!wave_band(B, h.net1, net2, cut, lo, hi)) continue;
+      sum = wave_any<P, NW, WMAX>(s_tab, nb1, qpl, nq, net2, lo, hi, cut, s_ring, s_xch, n_done);
+      if (sum < 0) continue;  // cannot reach the cutoff
+    }
+    if (score_mode) {
+      if (lead) rb.score_out[4 * entry + 2] = sum;
+      continue;
+    }
+    bool pass = !(sum < cutoff);
+    if (pass && h.word_after && threadIdx.x / 32 == group * NW) {  // short-word test (func.cu:376-396): the group's first warp
+      pass = !(word_count_warp_bits<P>(qpl, net2, prm.w, s_list) < word_min(L2, prm.w, s));
+    }
+    if (lead && pass) {
+      rb.cluster[cand] = h.rep;
+      rb.ident[cand] = sum;
+      atomicAnd(&rb.alive[cand >> 5], ~(1u << (cand & 31)));
+      n_members++;
+    }
+    __syncwarp();
   }
-  return c;
+  flush_align_stats(st, cls, n_pairs, n_members, n_cells, n_done, &s_qw);
 }
 
-// sum += c (0 or 1) over W words; the carry out is dropped.
-template <int W>
-__device__ __forceinline__ void carry_in_words(uint32_t (&sum)[W], uint32_t c) {
-  if constexpr (W == 1) {
-    sum[0] += c;
-  } else if constexpr (W == 2) {
-    asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, 0;" : "+r"(sum[0]), "+r"(sum[1]) : "r"(c));
-  } else {
-    asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.cc.u32 %2, %2, 0;\n\taddc.u32 %3, %3, 0;"
-        : "+r"(sum[0]), "+r"(sum[1]), "+r"(sum[2]), "+r"(sum[3])
-        : "r"(c));
-  }
-}
-
-// Banded LCS of one pair by one warp, W row words per lane; returns the
-// zero count, or -1 when may_reject and the pair cannot reach the cutoff.
-template <int P, int W>
-__device__ __forceinline__ int warp_pair(uint32_t *rows, const uint32_t *s_pl, int nb1, uint32_t vlast,
-                                         const uint32_t *qpl, int nq, int lastcols, int B, int net2, int cutoff,
-                                         bool may_reject, int lane, unsigned long long &n_done) {
-  for (int j = lane; j < nb1; j += 32) rows[j] = 0xFFFFFFFFu;
-  __syncwarp();
-  int delta = 0;
-  uint32_t nxt[P];
-#pragma unroll
-  for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + p);
-  for (int i = 0; i < nq; i++) {
-    uint32_t cur[P];
-#pragma unroll
-    for (int p = 0; p < P; p++) {
-      cur[p] = nxt[p];
-      if (i + 1 < nq) nxt[p] = __ldg(qpl + (i + 1) * P + p);
-    }
-    const int js = max(i - B, 0), je = min(i + B, nb1 - 1);
-    const int strips = je >= js ? (je - js + 32 * W) / (32 * W) : 0;
-    const int cols = (i == nq - 1) ? lastcols : 32;
-    if (lane == 0) n_done += (unsigned long long)(je - js + 1) * cols;
-    uint32_t cmask = 0;  // carry into the strip, bit k for column k
-    for (int sidx = 0; sidx < strips; sidx++) {
-      // lane l holds the W consecutive rows j0 .. j0+W-1 of the strip; rows
-      // above the band hold 0: they neither generate nor propagate (and no
-      // row above them could take their carry)
-      const int j0 = js + 32 * W * sidx + W * lane;
-      uint32_t row[W], row0[W], pl[W][P], rv[P];
-#pragma unroll
-      for (int w = 0; w < W; w++) {
-        const bool have = j0 + w <= je;
-        row[w] = have ? rows[j0 + w] : 0u;
-        row0[w] = row[w];
-#pragma unroll
-        for (int p = 0; p < P; p++) pl[w][p] = have ? s_pl[(j0 + w) * P + p] : 0u;
-      }
-#pragma unroll
-      for (int p = 0; p < P; p++) rv[p] = __brev(cur[p]);  // residue k's bit moves to the sign bit
-      uint32_t cout = 0;
-      for (int k = 0; k < cols; k++) {
-        uint32_t m[P], x[W], sum[W];
-#pragma unroll
-        for (int p = 0; p < P; p++) {
-          m[p] = (uint32_t)((int)rv[p] >> 31);
-          rv[p] <<= 1;
-        }
-#pragma unroll
-        for (int w = 0; w < W; w++) {
-          x[w] = row[w];
-#pragma unroll
-          for (int p = 0; p < P; p++) x[w] &= ~(pl[w][p] ^ m[p]);
-        }
-        const uint32_t gen = add_words<W>(row, x, sum);
-        uint32_t ones = sum[0];
-#pragma unroll
-        for (int w = 1; w < W; w++) ones &= sum[w];
-        const uint32_t G = __ballot_sync(kFullMask, gen);
-        const uint32_t Pm = __ballot_sync(kFullMask, ones == 0xFFFFFFFFu);
-        const uint32_t X = G | Pm;
-        const unsigned long long tot = (unsigned long long)X + G + ((cmask >> k) & 1u);
-        cout |= (uint32_t)(tot >> 32) << k;
-        carry_in_words<W>(sum, (((uint32_t)tot ^ X ^ G) >> lane) & 1u);
-#pragma unroll
-        for (int w = 0; w < W; w++) row[w] = sum[w] | (row[w] ^ x[w]);  // stored only for rows in the band
-      }
-#pragma unroll
-      for (int w = 0; w < W; w++) {
-        const int j = j0 + w;
-        if (j > je) continue;
-        rows[j] = row[w];
-        const uint32_t mk = (j == nb1 - 1) ? vlast : 0xFFFFFFFFu;
-        delta += __popc(~row[w] & mk) - __popc(~row0[w] & mk);
-      }
-      cmask = cout;
-    }
-    __syncwarp();  // this block's rows are stored before the next block loads them
-    if (may_reject && i + 1 < nq) {
-      int z = delta;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) z += __shfl_xor_sync(kFullMask, z, o);
-      if (z + (net2 - 32 * (i + 1)) < cutoff) {  // cannot reach the cutoff any more
-        return -1;
-      }
-    }
-  }
-  int sum = delta;
-#pragma unroll
-  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
-  return sum;
-}
-
+// Classes 0 and 1 with few pairs: 16 threads per pair, the query's blocks as
+// rows.  Shared memory: rep planes | k-mer bitset | rep codes | a match table
+// per warp.
 template <int P>
 __global__ void __launch_bounds__(kAlignThreads)
-    k_align_warp(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs) {
+    k_align_query(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint64_t bar;
   AlignHdr h;
   __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
   if (threadIdx.x == 0) s_qw = 0;
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, 1, smem, &bar, h)) return;
+  constexpr int kGroups = kAlignThreads / kQueryGroup;
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kGroups, smem, &bar, h)) return;
   const uint32_t *s_pl = smem;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t *rows = smem + (((db.max_nb * P + 3) & ~3) + kListWords) + warp * db.max_nb;
+  const int lane = threadIdx.x & 31, g = lane & (kQueryGroup - 1);
+  uint32_t *s_codes = smem + wave_table_off(P, db.max_nb);
+  uint32_t *tab = s_codes + 8 * db.max_nb + (threadIdx.x >> 5) * 32 * wave_codes(P);
+  const int nb1 = h.nb1;
+  for (int b = threadIdx.x; b < nb1; b += kAlignThreads) {
+    uint32_t pl[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) pl[p] = s_pl[b * P + p];
+    wave_unpack<P>(pl, reinterpret_cast<uint4 *>(s_codes) + 2 * b);
+  }
+  __syncthreads();
   RunState *st = rb.st;
   const float s = prm.s;
-  const int nb1 = h.nb1;
-  const uint32_t vlast = (h.net1 & 31) ? ((1u << (h.net1 & 31)) - 1u) : 0xFFFFFFFFu;
   unsigned long long n_pairs = 0, n_members = 0, n_cells = 0, n_done = 0;
-  const int nwarps = gridDim.x * (blockDim.x >> 5);
-  for (int e = blockIdx.x * (blockDim.x >> 5) + warp; e < h.qn; e += nwarps) {
-    const int entry = score_mode ? e : rb.queue[cls][e];
-    const int cand = score_mode ? rb.score_cands[entry] : entry;
-    const int L2 = __ldg(db.len + cand), net2 = __ldg(db.net + cand);
-    const int nq = (net2 + 31) >> 5;
-    const int lastcols = (net2 & 31) ? (net2 & 31) : 32;
-    const int B = band_blocks(h.L1, L2, s);
-    const int cutoff = cutoff_of(L2, s);
-    const uint32_t *qpl = db.words + __ldg(db.off + cand) + db.hw;
-    if (!score_mode && lane == 0) {
-      n_pairs++;
-      n_cells += (unsigned long long)band_cells(B, nb1, net2);
-      atomicAdd(&s_qw, (unsigned long long)(nq * P));
+  const int e0 = (blockIdx.x * kAlignThreads + threadIdx.x) / 32 * 2;  // the warp's first two pairs
+  for (int eb = e0; eb < h.qn; eb += (int)gridDim.x * kGroups) {       // warp-uniform
+    const int e = eb + lane / kQueryGroup;
+    const bool have = e < h.qn;
+    int entry = 0, cand = 0, L2 = 0, net2 = 0, nq = 0, B = 0, cutoff = 0, lo = 0, hi = 0, sum = 0;
+    const uint32_t *qpl = db.words;
+    bool run = false, fails = false;
+    if (have) {
+      entry = rb.queue[cls][e];
+      cand = score_mode ? rb.score_cands[entry] : entry;
+      L2 = __ldg(db.len + cand);
+      net2 = __ldg(db.net + cand);
+      nq = (net2 + 31) >> 5;
+      B = band_blocks(h.L1, L2, s);
+      cutoff = cutoff_of(L2, s);
+      qpl = db.words + __ldg(db.off + cand) + db.hw;
+      if (B >= 0 && nb1 > 0 && nq > 0) {
+        run = wave_band(B, h.net1, net2, score_mode ? kNoCut : cutoff, lo, hi);
+        fails = !run;
+      }
+      if (!score_mode && g == 0) {
+        n_pairs++;
+        n_cells += (unsigned long long)band_cells(B, nb1, net2);
+        atomicAdd(&s_qw, (unsigned long long)(nq * P));
+      }
     }
-    if (B < 0 || nq == 0) {
-      if (lane == 0) finish_pair<P>(db, rb, prm, h, score_mode, entry, cand, 0, cutoff, L2, net2, qpl, s_list, n_members);
+    const int got = wave_query<P>(s_codes, nb1, h.net1, qpl, run ? nq : 0, net2, lo, hi, tab, n_done);
+    if (run) sum = got;
+    if (score_mode) {
+      if (have && g == 0) rb.score_out[4 * entry + 2] = sum;
       continue;
     }
-    // row words per lane by this pair's band window: 32 rows per strip up to
-    // windows of 32 blocks, then 64, then 128
-    const int A = window_of(B, nb1);
-    const int sum = A <= 32   ? warp_pair<P, 1>(rows, s_pl, nb1, vlast, qpl, nq, lastcols, B, net2, cutoff, !score_mode,
-                                                lane, n_done)
-                    : A <= 64 ? warp_pair<P, 2>(rows, s_pl, nb1, vlast, qpl, nq, lastcols, B, net2, cutoff, !score_mode,
-                                                lane, n_done)
-                              : warp_pair<P, 4>(rows, s_pl, nb1, vlast, qpl, nq, lastcols, B, net2, cutoff, !score_mode,
-                                                lane, n_done);
-    if (sum < 0) continue;  // rejected early
-    if (lane == 0) finish_pair<P>(db, rb, prm, h, score_mode, entry, cand, sum, cutoff, L2, net2, qpl, s_list, n_members);
-    __syncwarp();
+    bool pass = have && !fails && !(sum < cutoff);
+    if (h.word_after) {  // short-word test (func.cu:376-396), a warp per member
+      for (int k = 0; k < 2; k++) {
+        const int src = k * kQueryGroup;
+        if (!__shfl_sync(kFullMask, (int)pass, src)) continue;
+        const uint32_t *q = reinterpret_cast<const uint32_t *>(__shfl_sync(kFullMask, (unsigned long long)qpl, src));
+        const int n2 = __shfl_sync(kFullMask, net2, src);
+        const int ws = word_count_warp_bits<P>(q, n2, prm.w, s_list);
+        if (lane / kQueryGroup == k) pass = !(ws < word_min(L2, prm.w, s));
+      }
+    }
+    if (pass && g == 0) {
+      rb.cluster[cand] = h.rep;
+      rb.ident[cand] = sum;
+      atomicAnd(&rb.alive[cand >> 5], ~(1u << (cand & 31)));
+      n_members++;
+    }
   }
   flush_align_stats(st, cls, n_pairs, n_members, n_cells, n_done, &s_qw);
 }
@@ -561,12 +522,18 @@ __global__ void __launch_bounds__(kAlignThreads)
 // ---- dispatch ---------------------------------------------------------------------
 typedef void (*AlignFn)(DevDB, RunBufs, RunParams, int, int, int);
 
-static AlignFn warp_fn(int type, int cls) {
-  (void)cls;
-  return type == 0 ? k_align_warp<2> : k_align_warp<5>;
+static AlignFn wave_fn(int type, int cls) {
+  if (is_query_class(cls)) return type == 0 ? k_align_query<2> : k_align_query<5>;
+  const int ring = class_ring(type, cls);
+  if (type == 0)
+    return ring == 64 ? k_align_wave<2, 1, 2> : ring == 128 ? k_align_wave<2, 4, 1> : k_align_wave<2, 4, 16>;
+  return ring == 64 ? k_align_wave<5, 1, 2> : ring == 128 ? k_align_wave<5, 4, 1> : k_align_wave<5, 4, 16>;
 }
 
-constexpr int kWarpKernel = kNumClasses;  // index of the warp kernel in the attribute table
+// Pairs a CTA of the class's group-per-pair kernel takes at a time.
+int wave_pairs_per_cta(int type, int cls) {
+  return is_query_class(cls) ? kAlignThreads / kQueryGroup : class_ring(type, cls) == 64 ? kAlignThreads / 32 : 1;
+}
 
 static AlignFn align_fn(int type, int cls) {
   const int ring = class_ring(type, cls);
@@ -575,12 +542,24 @@ static AlignFn align_fn(int type, int cls) {
 }
 
 // Dynamic shared memory: rep planes | k-mer bitset | row ring | match table
-// | (warp kernel, cls = kWarpKernel) every row of one pair per warp.
+// (the group-per-pair kernels: rep planes | bitset | match table by code |
+// code rings, or rep codes | match tables).
+static size_t wave_smem(int type, int cls, int max_nb) {
+  const int P = type ? 5 : 2;
+  size_t words = (size_t)wave_table_off(P, max_nb);
+  if (is_query_class(cls))
+    words += 8 * (size_t)max_nb + kAlignThreads * wave_codes(P);
+  else
+    words += (size_t)wave_table_words(P, max_nb) + (size_t)wave_pairs_per_cta(type, cls) * kWaveRingWords;
+  return 4u * words;
+}
+// Records of up to this many bytes of shared memory per CTA take the
+// group-per-pair kernels (proteins up to about 45,000 residues).
+constexpr size_t kWaveSmemMost = 226 * 1024;
+bool wave_fits(int type, int max_nb) { return wave_smem(type, base_class(type), max_nb) <= kWaveSmemMost; }
 static size_t align_smem(int type, int max_nb, int cls) {
   const int P = type ? 5 : 2;
-  size_t words = (size_t)(((max_nb * P + 3) & ~3) + kListWords);
-  if (cls == kWarpKernel) return 4u * (words + (size_t)(kAlignThreads / 32) * max_nb);
-  words = (size_t)tiled_eq_off(P, max_nb, class_ring(type, cls));
+  size_t words = (size_t)tiled_eq_off(P, max_nb, class_ring(type, cls));
   if (P == 2) words += (size_t)eq_words(max_nb);
   return 4u * words;
 }
@@ -591,37 +570,34 @@ static size_t align_smem(int type, int max_nb, int cls) {
 // longer ones.
 cudaError_t align_configure(int type, int max_nb) {
   static std::mutex mu;
-  static int configured[64][2][kNumClasses + 1] = {};
+  static int configured[64][2][2][kNumClasses] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(mu);
-  for (int c = 0; c <= kNumClasses; c++) {
-    if ((c < first_class(type) || c >= num_classes(type)) && c != kWarpKernel) continue;
-    const int want = (int)align_smem(type, max_nb, c);
-    int &have = configured[dev][type ? 1 : 0][c];
-    if (want <= have) continue;
-    if (c == kWarpKernel) {
-      for (int k = 0; k < num_classes(type); k++) {
-        e = cudaFuncSetAttribute((const void *)warp_fn(type, k), cudaFuncAttributeMaxDynamicSharedMemorySize, want);
-        if (e != cudaSuccess) return e;
-      }
-    } else {
-      e = cudaFuncSetAttribute((const void *)align_fn(type, c), cudaFuncAttributeMaxDynamicSharedMemorySize, want);
+  for (int c = 0; c < num_classes(type); c++) {
+    if (!class_used(type, c, max_nb)) continue;
+    for (int wave = 0; wave < (wave_fits(type, max_nb) ? 2 : 1); wave++) {
+      const int want = (int)(wave ? wave_smem(type, c, max_nb) : align_smem(type, max_nb, c));
+      int &have = configured[dev][type ? 1 : 0][wave][c];
+      if (want <= have) continue;
+      e = cudaFuncSetAttribute((const void *)(wave ? wave_fn(type, c) : align_fn(type, c)),
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, want);
       if (e != cudaSuccess) return e;
+      have = want;
     }
-    have = want;
   }
   return cudaSuccess;
 }
 
-// Resident CTAs per SM of class `cls` (persistent grid = that x SM count).
-// (cls = kNumClasses: the warp kernel.)
-int align_occupancy(int type, int cls, int max_nb) {
+// Resident CTAs per SM of class `cls` (persistent grid = that x SM count);
+// wave: of its group-per-pair kernel.
+int align_occupancy(int type, int cls, int max_nb, bool wave) {
   int nb = 0;
-  const void *fn = cls == kWarpKernel ? (const void *)warp_fn(type, num_classes(type) - 1) : (const void *)align_fn(type, cls);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kAlignThreads, align_smem(type, max_nb, cls)) !=
+  const void *fn = (const void *)(wave ? wave_fn(type, cls) : align_fn(type, cls));
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kAlignThreads,
+                                                    wave ? wave_smem(type, cls, max_nb) : align_smem(type, max_nb, cls)) !=
       cudaSuccess)
     return 1;
   return nb < 1 ? 1 : nb;
@@ -629,25 +605,30 @@ int align_occupancy(int type, int cls, int max_nb) {
 
 int align_threads() { return kAlignThreads; }
 
-// Launches class `cls`: the thread-per-pair kernel, and (in clustering) the
-// warp-per-pair kernel; which of the two works is decided on the device from
-// the class's queued pair count against c->warp_pairs.
+// Launches class `cls`: the thread-per-pair kernel and the group-per-pair
+// kernel; which of the two works is decided on the device from the class's
+// queued pair count against the cut-off.  score_mode: 0 in clustering, else
+// the pairs of a pair-score call.
 cudaError_t launch_align(ngia_ctx *c, int cls, cudaStream_t s, int score_mode) {
-  AlignFn fn = align_fn(c->db.type, cls);
   DevDB db = c->db;
   RunBufs rb = c->rb;
   RunParams prm = c->prm;
-  // per length bucket (class): its own warp-per-pair cut-off and CTA count
-  // when the tuner chose them
-  int wp = score_mode ? -1 : (c->cls_warp_pairs[cls] >= 0 ? c->cls_warp_pairs[cls] : c->warp_pairs);
-  const int grid = std::max(1, c->grid_align[cls] / std::max(1, c->cls_grid_div[cls]));
+  // per length bucket (class): its own cut-off and CTA count when the tuner
+  // chose them; pair scores go by the context's grids
+  int wp = score_mode ? c->warp_pairs_default : c->cls_warp_pairs[cls] >= 0 ? c->cls_warp_pairs[cls] : c->warp_pairs;
+  if (!wave_fits(c->db.type, c->cap_nb)) wp = -1;
+  int grid = std::max(1, c->grid_align[cls] / std::max(1, c->cls_grid_div[cls]));
+  int grid_wave = c->grid_wave[cls];
+  if (score_mode) {  // no more CTAs than the call's pairs can use
+    grid = std::min(grid, (score_mode + kAlignThreads - 1) / kAlignThreads);
+    grid_wave = std::min(grid_wave, score_mode);
+  }
   void *args[] = {&db, &rb, &prm, &cls, &score_mode, &wp};
-  cudaError_t e = cudaLaunchKernel((const void *)fn, dim3(grid), dim3(kAlignThreads), args,
+  cudaError_t e = cudaLaunchKernel((const void *)align_fn(c->db.type, cls), dim3(grid), dim3(kAlignThreads), args,
                                    align_smem(c->db.type, c->db.max_nb, cls), s);
-  if (e != cudaSuccess || wp <= 0) return e;  // no class can go warp-per-pair
-  return cudaLaunchKernel((const void *)warp_fn(c->db.type, cls), dim3(c->grid_warp), dim3(kAlignThreads), args,
-                          align_smem(c->db.type, c->db.max_nb, kWarpKernel), s);
+  if (e != cudaSuccess || wp <= 0) return e;  // no class goes to the group kernel
+  return cudaLaunchKernel((const void *)wave_fn(c->db.type, cls), dim3(grid_wave), dim3(kAlignThreads), args,
+                          wave_smem(c->db.type, cls, c->db.max_nb), s);
 }
-
 
 }  // namespace ngia

@@ -60,16 +60,18 @@ int enqueue_iteration(ngia_ctx *c, bool graph, cudaGraphConditionalHandle cond) 
   if (graph && !c->batch_member) {
     // classes run as parallel branches of the body graph
     CK(cudaEventRecord(c->fork_ev, c->stream));
-    for (int k = ngia::first_class(c->db.type); k < nc; k++) {
-      CK(cudaStreamWaitEvent(c->side[k], c->fork_ev, 0));
-      CK(ngia::launch_align(c, k, c->side[k], 0));
-      CK(cudaEventRecord(c->join_ev[k], c->side[k]));
+    for (int k = 0; k < nc; k++) {
+      if (!ngia::class_used(c->db.type, k, c->db.max_nb)) continue;
+      cudaStream_t side = c->side[ngia::class_stream(c->db.type, k)];
+      CK(cudaStreamWaitEvent(side, c->fork_ev, 0));
+      CK(ngia::launch_align(c, k, side, 0));
+      CK(cudaEventRecord(c->join_ev[k], side));
       CK(cudaStreamWaitEvent(c->stream, c->join_ev[k], 0));
     }
   } else {
-    for (int k = ngia::first_class(c->db.type); k < nc; k++) {
+    for (int k = 0; k < nc; k++) {
       if (prof) CK(cudaEventRecord(c->ev_cls[k], c->stream));
-      CK(ngia::launch_align(c, k, c->stream, 0));
+      if (ngia::class_used(c->db.type, k, c->db.max_nb)) CK(ngia::launch_align(c, k, c->stream, 0));
     }
     if (prof) CK(cudaEventRecord(c->ev_cls[nc], c->stream));
   }
@@ -83,7 +85,7 @@ void account_stages(ngia_ctx *c) {
   float a = 0.f, b = 0.f;
   if (cudaEventElapsedTime(&a, c->ev_p0, c->ev_p1) == cudaSuccess) c->ms_filter += a;
   if (cudaEventElapsedTime(&b, c->ev_p1, c->ev_p2) == cudaSuccess) c->ms_align += b;
-  for (int k = ngia::first_class(c->db.type); k < ngia::num_classes(c->db.type); k++) {
+  for (int k = 0; k < ngia::num_classes(c->db.type); k++) {
     float m = 0.f;
     if (cudaEventElapsedTime(&m, c->ev_cls[k], c->ev_cls[k + 1]) == cudaSuccess) c->ms_class[k] += m;
   }
@@ -278,27 +280,29 @@ int load_db(ngia_ctx *c, const ngia_db_view *v) {
 // one CTA per 128 candidates and one warp per bitmap word.
 void size_grids(ngia_ctx *c, bool by_size) {
   const int type = c->db.type;
-  for (int k = ngia::first_class(type); k < ngia::num_classes(type); k++)
-    c->grid_align[k] = c->num_sms * ngia::align_occupancy(type, k, c->cap_nb);
+  const int nc = ngia::num_classes(type);
+  const bool wave = ngia::wave_fits(type, c->cap_nb);
+  for (int k = 0; k < nc; k++) {
+    if (!ngia::class_used(type, k, c->cap_nb)) continue;
+    c->grid_align[k] = c->num_sms * ngia::align_occupancy(type, k, c->cap_nb, false);
+    c->grid_wave[k] = wave ? c->num_sms * ngia::align_occupancy(type, k, c->cap_nb, true) : 1;
+  }
   c->grid_filter = c->num_sms * 8;
-  // warp-per-pair: the whole GPU's warps; a class goes warp-per-pair when it
-  // has at most one pair per warp (a wide pair's latency on a warp is a few
-  // times shorter than on a thread, at ~6x the instructions per cell; swept
-  // on GB300: 0.25, 0.5, 1 and 2 pairs per warp gave 41, 47, 47 and 40M
-  // candidate seqs/s on the 20,000-sequence DNA workload and within 1% of
-  // each other on the 1M DNA and 200k protein workloads)
-  c->grid_warp = c->num_sms * ngia::align_occupancy(type, ngia::kNumClasses, c->cap_nb);
-  c->warp_pairs = c->grid_warp * (ngia::align_threads() / 32);
   if (by_size) {
     const int64_t n = std::max(1, c->db.n), nbw = (n + 31) / 32;
-    const int by_n = (int)std::min<int64_t>((n + 127) / 128, INT32_MAX);
-    for (int k = ngia::first_class(type); k < ngia::num_classes(type); k++) c->grid_align[k] = std::max(1, std::min(c->grid_align[k], by_n));
+    for (int k = 0; k < nc; k++) {
+      c->grid_align[k] = (int)std::max<int64_t>(1, std::min<int64_t>(c->grid_align[k], (n + 127) / 128));
+      const int per = ngia::wave_pairs_per_cta(type, k);
+      c->grid_wave[k] = (int)std::max<int64_t>(1, std::min<int64_t>(c->grid_wave[k], (n + per - 1) / per));
+    }
     c->grid_filter = std::max(1, std::min(c->grid_filter, (int)((nbw + 7) / 8)));
-    // warp-per-pair: no more warps than the job has sequences
-    const int wpc = ngia::align_threads() / 32;
-    c->grid_warp = std::max(1, std::min(c->grid_warp, (int)((n + wpc - 1) / wpc)));
-    c->warp_pairs = c->grid_warp * wpc;
   }
+  // A class with at most this many pairs goes to its group-per-pair kernel.
+  // One thread per pair takes a pair's latency whatever their number (DNA
+  // 1,450 residues: 275-345 us from 1,500 to 24,000 pairs on GB300), a group
+  // per pair 33 us per 1,000 pairs once it fills the GPU: equal at about
+  // 9,000 (150 SMs x 56).
+  c->warp_pairs = 56 * c->num_sms;
   if (const char *w = getenv("NGIA_WARP_PAIRS")) c->warp_pairs = atoi(w);
   c->warp_pairs_default = c->warp_pairs;
 }
@@ -318,7 +322,8 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
             dalloc(&rb.scan_part, nbw) == cudaSuccess && dalloc(&rb.long_list, (size_t)cap_n) == cudaSuccess;
   ok = ok && cudaMalloc((void **)&rb.flags, 4 * std::max<size_t>(nbw, 1)) == cudaSuccess;
   ok = ok && dalloc(&rb.fstats, (size_t)ngia::kFilterStripes * ngia::kFilterStats) == cudaSuccess;
-  for (int k = ngia::first_class(type); ok && k < ngia::num_classes(type); k++) ok = dalloc(&rb.queue[k], (size_t)cap_n) == cudaSuccess;
+  for (int k = 0; ok && k < ngia::num_classes(type); k++)
+    if (ngia::class_used(type, k, c->cap_nb)) ok = dalloc(&rb.queue[k], (size_t)cap_n) == cudaSuccess;
   if (!ok) return fail(NGIA_E_NOMEM, "ngia_open: device allocation of run buffers failed");
   cudaMemsetAsync(rb.rep_list, 0, 4 * ngia::kListWords, c->stream);
   cudaMemsetAsync(rb.fstats, 0, 8 * ngia::kFilterStripes * ngia::kFilterStats, c->stream);
@@ -330,8 +335,8 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
   c->db.n = (int32_t)cap_n;
   size_grids(c, c->batch_member);
   c->db.n = saved_n;
-  const int g = ngia::generic_class(type);
-  rb.generic_lanes = c->grid_align[g] * ngia::align_threads();
+  const int g = ngia::generic_class(type);  // (class 1 is on the global ring too)
+  rb.generic_lanes = std::max(c->grid_align[1], c->grid_align[g]) * ngia::align_threads();
   uint32_t ring = 1;
   while ((int)ring < c->cap_nb) ring <<= 1;
   rb.ring_mask = ring - 1;
@@ -407,7 +412,7 @@ int ngia::drv::reload_ctx(ngia_ctx *c, const ngia_db_view *v) {
   if (nb > c->cap_nb)
     return fail(NGIA_E_LIMIT, "reload: a record of %d blocks exceeds the capacity of %d", nb, c->cap_nb);
   const ngia::DevDB before = c->db;
-  const int grids_before = c->grid_filter, warp_before = c->grid_warp;
+  const int grids_before = c->grid_filter, warp_before = c->warp_pairs_default;
   c->begun = false;
   int rc = load_db(c, v);
   if (rc) {
@@ -422,7 +427,7 @@ int ngia::drv::reload_ctx(ngia_ctx *c, const ngia_db_view *v) {
   // a captured graph holds the kernel arguments (sizes) and grids: it stays
   // valid when the database has the same shape
   const bool same = before.n == c->db.n && before.max_nb == c->db.max_nb && before.has_short == c->db.has_short &&
-                    grids_before == c->grid_filter && warp_before == c->grid_warp;
+                    grids_before == c->grid_filter && warp_before == c->warp_pairs_default;
   if (!same) destroy_graph(c);
   return NGIA_OK;
 }
@@ -662,7 +667,8 @@ extern "C" int ngia_pair_scores(ngia_ctx *c, const ngia_params *p, int32_t rep, 
   CK(cudaMemsetAsync(c->rb.st, 0, sizeof(ngia::RunState), c->stream));
   CK(ngia::launch_prep(c, rep));
   CK(ngia::launch_score_classify(c, n));
-  for (int k = ngia::first_class(c->db.type); k < ngia::num_classes(c->db.type); k++) CK(ngia::launch_align(c, k, c->stream, 1));
+  for (int k = 0; k < ngia::num_classes(c->db.type); k++)
+    if (ngia::class_used(c->db.type, k, c->db.max_nb)) CK(ngia::launch_align(c, k, c->stream, n));
   CK(cudaMemcpyAsync(out, d_o, 16 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
   rc = pull_state(c);
   cudaFree(d_c);

@@ -353,17 +353,17 @@ extern "C" int ngia_batch_run(ngia_batch *b, const ngia_params *params, int32_t 
     bool rebuild = !b->exec || b->prm.size() != nj;
     for (size_t j = 0; j < nj; j++) {
       ngia_ctx *c = b->jobs[j];
-      // jobs running side by side fill the GPU: one thread per pair, the
-      // form with the fewest instructions per cell (256-job batch on GB300:
-      // 15.4M vs 13.0M candidate seqs/s with warp-per-pair classes);
-      // NGIA_BATCH_WARP=1 keeps each job's own warp-per-pair cut-off:
-      // 17.97M against 20.97M over the first 8 iterations, 4.23 against
-      // 4.31 s for 256 small jobs clustered to the end
+      // jobs running side by side share the GPU: each class of a job goes to
+      // the group-per-pair kernels up to the job's share of the pairs at
+      // which they pay (many jobs: thread per pair, the form with the fewest
+      // instructions per cell; 12 jobs of 1,000-4,000 sequences on GB300, 32
+      // iterations each: 281 ms with every class thread per pair, 52
+      // with the share); NGIA_BATCH_WARP=1 keeps each job's own cut-off
       // after ngia_batch_autotune, the chosen policy's settings
       if (b->policy >= 0 && b->policy_wp.size() == nj)
         c->tuned_warp_pairs = b->policy_wp[j];
       else
-        c->tuned_warp_pairs = batch_warp() ? -1 : 0;
+        c->tuned_warp_pairs = batch_warp() ? -1 : c->warp_pairs_default / (int)nj;
       int rc = ngia_cluster_begin(c, &params[j], NGIA_MODE_PLAIN);  // no per-job graph
       if (rc) return rc;
       c->mode = NGIA_MODE_GRAPH;

@@ -15,22 +15,44 @@ constexpr int kListWords = 2048;               // rep k-mer presence bitset (65,
 constexpr int kRefGridThreads = 128 * 128;     // BLOCK*WARP of the reference launch
 
 // Alignment work classes.  Pairs are queued by the width of the band window
-// their alignment can need (window_need, in rep blocks).  Three are in use
-// per type: up to 64 or 128 window rows per pair in a shared-memory ring, any
-// width on a global-memory ring, all through 16-slot register tiles.  The
-// numbers before first_class stand for the register-window kernels of
-// earlier versions (8 to 32 blocks); they stay unused so that class numbers
-// in saved tunings, checkpoints and statistics keep their meaning.
+// their alignment can need (window_need, in rep blocks): the last three
+// classes of a type hold windows of up to 64 or 128 rows in a shared-memory
+// ring, or of any width on a global-memory ring.  Classes 0 and 1 are the
+// pairs of windows up to 128 and of any width whose query has at most
+// kQueryRows blocks: short queries against a long representative, aligned by
+// 16 threads with the query's blocks as rows (wave.cuh) while they are few.
+// DNA numbers 2 and 3 are unused: class numbers in saved tunings, checkpoints
+// and statistics keep their meaning.
 constexpr int kNumClasses = 7;
+constexpr int kQueryRows = 16;
 __host__ __device__ inline int num_classes(int type) { return type == 0 ? 7 : 5; }
 __host__ __device__ inline int generic_class(int type) { return num_classes(type) - 1; }
-__host__ __device__ inline int first_class(int type) { return num_classes(type) - 3; }
+__host__ __device__ inline int base_class(int type) { return num_classes(type) - 3; }
+// Classes 0 and 1: rows are the query's.
+__host__ __device__ inline bool is_query_class(int c) { return c < 2; }
 // Ring rows of class c: 64, 128, or 0 (global-memory ring).
 __host__ __device__ inline int class_ring(int type, int c) {
+  if (is_query_class(c)) return c == 0 ? 128 : 0;
   return c >= generic_class(type) ? 0 : c == generic_class(type) - 1 ? 128 : 64;
 }
-__host__ __device__ inline int class_of(int type, int A) {
-  return first_class(type) + (A <= 64 ? 0 : A <= 128 ? 1 : 2);
+// Whether a database whose records have up to max_nb blocks can queue pairs
+// in class c.
+__host__ __device__ inline bool class_used(int type, int c, int max_nb) {
+  if (c >= num_classes(type) || (c >= 2 && c < base_class(type))) return false;
+  const int ring = class_ring(type, c);
+  return ring == 64 || max_nb > (ring == 128 ? 64 : 128);
+}
+// Parallel branch class c runs in: the two classes on the global ring share
+// its scratch and run one after the other.
+__host__ __device__ inline int class_stream(int type, int c) {
+  return class_ring(type, c) == 0 ? generic_class(type) : c;
+}
+// The class of a pair whose window is A blocks and whose query has L2 (raw)
+// residues.
+__host__ __device__ inline int class_of(int type, int A, int L2) {
+  if (A <= 64) return base_class(type);
+  if (L2 <= 32 * kQueryRows) return A <= 128 ? 0 : 1;
+  return base_class(type) + (A <= 128 ? 1 : 2);
 }
 
 // Device copy of the makeDB database plus per-sequence header arrays.

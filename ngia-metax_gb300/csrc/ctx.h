@@ -39,8 +39,8 @@ struct ngia_ctx {
   // launch shapes
   int grid_filter = 0;
   int grid_align[ngia::kNumClasses] = {0};
-  int grid_warp = 0;    // CTAs of the warp-per-pair kernel
-  int warp_pairs = -1;  // a class with at most this many pairs runs warp-per-pair
+  int grid_wave[ngia::kNumClasses] = {0};  // CTAs of the group-per-pair kernels
+  int warp_pairs = -1;  // a class with at most this many pairs runs a group per pair
   int warp_pairs_default = -1;  // the above as sized for this context's grids
   // settings that change speed only (set by ngia_autotune / ngia_set_tuning):
   // test order (0 auto, 1 short words first, 2 alignment first), lockstep
@@ -109,8 +109,10 @@ cudaError_t launch_subset_start(ngia_ctx *c, const uint32_t *d_alive);
 cudaError_t launch_score_classify(ngia_ctx *c, int n);
 // align.cu
 cudaError_t launch_align(ngia_ctx *c, int cls, cudaStream_t s, int score_mode);
-int align_occupancy(int type, int cls, int max_nb);
+int align_occupancy(int type, int cls, int max_nb, bool wave);
 int align_threads();
+int wave_pairs_per_cta(int type, int cls);
+bool wave_fits(int type, int max_nb);  // group-per-pair kernels hold records of this many blocks
 cudaError_t align_configure(int type, int max_nb);
 cudaError_t filter_configure();
 // pool.cu: the pooled batch form (NGIA_MODE_POOL), one pool per record type

@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
             deferred = true;
           }
         }
-        if (pass) cls = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
+        if (pass) cls = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
       }
       // long candidates go to k_filter_long, which gives each one a warp
       const unsigned dm = __ballot_sync(kFullMask, deferred);
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
             deferred = true;
           }
         }
-        if (pass && !exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
+        if (pass && !exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
       }
       // long candidates: the whole warp counts each one
       for (unsigned dm = __ballot_sync(kFullMask, deferred); dm; dm &= dm - 1) {
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
           pass = !(ws < word_min(L2, prm.w, s));
           if (pass) {
             wpass++;
-            if (!exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
+            if (!exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
           }
         }
       }
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(256) k_word_exact(DevDB db, RunBufs rb, RunPar
       }
       if (pass) {
         wpass++;
-        cls = class_of(db.type, window_need(L1, L2, cutoff_of(L2, prm.s), band_blocks(L1, L2, prm.s), nb1));
+        cls = class_of(db.type, window_need(L1, L2, cutoff_of(L2, prm.s), band_blocks(L1, L2, prm.s), nb1), L2);
       }
     }
     push_queue(rb, st, pass, cls, c);
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(256) k_filter_long(DevDB db, RunBufs rb, RunPa
     const int L2 = __ldg(db.len + c);
     const bool pass = lane == 0 && !(ws < word_min(L2, prm.w, s));
     if (pass) wpass++;
-    push_queue(rb, st, pass, pass ? class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1)) : 0, c);
+    push_queue(rb, st, pass, pass ? class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2) : 0, c);
   }
   flush_stats(rb, 0, 0, 0, 0, wpass);
 }
@@ -977,37 +977,36 @@ cudaError_t launch_next(ngia_ctx *c, unsigned long long cond, int use_cond) {
 }
 
 // ---- pair-score mode: per-pair composition / word values and queueing ----------
+// A warp per candidate: one thread's short-word count of 1,450 residues took
+// 58 us of a 32-pair call's 150.
 template <int P>
-__global__ void k_score_classify(DevDB db, RunBufs rb, RunParams prm, int n) {
+__global__ void __launch_bounds__(256) k_score_classify(DevDB db, RunBufs rb, RunParams prm, int n) {
   RunState *st = rb.st;
   constexpr int A = P == 2 ? 4 : 28;
   __shared__ uint32_t s_rc[28];
   if (threadIdx.x < A) s_rc[threadIdx.x] = rb.rep_rec[2 + threadIdx.x];
   __syncthreads();
   const int L1 = st->rep_len, nb1 = st->rep_nb, net1 = st->rep_net;
-  const int iters = (n + blockDim.x * gridDim.x - 1) / (blockDim.x * gridDim.x);
-  for (int it = 0; it < iters; it++) {
-    const int k = it * blockDim.x * gridDim.x + blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = k < n;
-    int cls = 0;
-    if (valid) {
-      const int c = rb.score_cands[k];
-      const int L2 = db.len[c], net2 = db.net[c];
-      rb.score_out[4 * k + 0] = base_sum<A>(db.cnt, c, s_rc);
-      if (net1 < 16 || net2 < 16)
-        rb.score_out[4 * k + 1] = -1;
-      else
-        rb.score_out[4 * k + 1] = word_count<P>(db.words + db.off[c] + db.hw, net2, prm.w, rb.rep_list);
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += warps) {
+    const int c = rb.score_cands[k];
+    const int L2 = db.len[c], net2 = db.net[c];
+    const int ws = net1 < 16 || net2 < 16
+                       ? -1
+                       : word_count_warp_bits<P>(db.words + db.off[c] + db.hw, net2, prm.w, rb.rep_list);
+    if ((threadIdx.x & 31) == 0) {
       const int B = band_blocks(L1, L2, prm.s);
+      const int cls = class_of(db.type, window_of(B, nb1), L2);
+      rb.score_out[4 * k + 0] = base_sum<A>(db.cnt, c, s_rc);
+      rb.score_out[4 * k + 1] = ws;
       rb.score_out[4 * k + 3] = B;
-      cls = class_of(db.type, window_of(B, nb1));
+      rb.queue[cls][atomicAdd(&st->qcount[cls], 1u)] = k;
     }
-    push_queue(rb, st, valid, cls, k);
   }
 }
 
 cudaError_t launch_score_classify(ngia_ctx *c, int n) {
-  const int grid = std::max(1, std::min(c->num_sms * 4, (n + 255) / 256));
+  const int grid = std::max(1, std::min(c->num_sms * 8, (n + 7) / 8));
   if (c->db.P == 2)
     k_score_classify<2><<<grid, 256, 0, c->stream>>>(c->db, c->rb, c->prm, n);
   else

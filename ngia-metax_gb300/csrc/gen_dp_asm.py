@@ -61,6 +61,22 @@ def one_eqf(TW: int) -> str:
                  f"const uint32_t (&e)[{TW}], uint32_t &cw, uint32_t &ncw, uint32_t one)", outs, ins, lines)
 
 
+def one_wave(W: int) -> str:
+    """The update with a mask per row word (act[m]) on the match word: a row
+    whose mask is 0 stays as it is."""
+    outs = [f'"+r"(row[{m}])' for m in range(W)] + ['"+r"(cw)', '"+r"(ncw)']
+    ins = [f'"r"(e[{m}])' for m in range(W)] + [f'"r"(act[{m}])' for m in range(W)]
+    cw, ncw, e, act = W, W + 1, W + 2, 2 * W + 2
+    lines = [".reg .u32 x, t;", f"add.cc.u32 %{cw}, %{cw}, %{cw};"]
+    for m in range(W):
+        lines += [f"lop3.b32 x, %{m}, %{e + m}, %{act + m}, 0x80;", f"addc.cc.u32 t, %{m}, x;",
+                  f"lop3.b32 %{m}, t, %{m}, x, 0xF6;"]
+    lines.append(f"addc.u32 %{ncw}, %{ncw}, %{ncw};")
+    return block(f"template <>\n__device__ __forceinline__ void dp_wave<{W}>(uint32_t (&row)[{W}], "
+                 f"const uint32_t (&e)[{W}], const uint32_t (&act)[{W}], uint32_t &cw, uint32_t &ncw)",
+                 outs, ins, lines)
+
+
 def main() -> None:
     parts = ["// dp_asm.cuh — generated by gen_dp_asm.py; do not edit by hand.\n"
              "// One residue (column) update of a TW-slot register tile of the banded\n"
@@ -71,9 +87,13 @@ def main() -> None:
              "                                        const uint32_t (&mk)[P], uint32_t &cw, uint32_t &ncw);\n\n"
              "template <int TW>\n"
              "__device__ __forceinline__ void dp_tile_eqf(uint32_t (&row)[TW], const uint32_t (&e)[TW], uint32_t &cw,\n"
-             "                                            uint32_t &ncw, uint32_t one);\n\n"]
+             "                                            uint32_t &ncw, uint32_t one);\n\n"
+             "template <int W>\n"
+             "__device__ __forceinline__ void dp_wave(uint32_t (&row)[W], const uint32_t (&e)[W], const uint32_t (&act)[W],\n"
+             "                                        uint32_t &cw, uint32_t &ncw);\n\n"]
     parts += [one(P, TW) for P in PLANES for TW in WIDTHS]
     parts += [one_eqf(TW) for TW in WIDTHS]
+    parts += [one_wave(W) for W in (1, 2, 4, 8, 16)]
     parts.append("}  // namespace ngia\n")
     (Path(__file__).resolve().parent / "dp_asm.cuh").write_text("".join(parts))
 

@@ -41,6 +41,54 @@ __device__ int word_count(const uint32_t *__restrict__ planes, int net2, int w, 
   return sum;
 }
 
+// Short-word count of one candidate by the whole warp against a k-mer
+// bitset: lane l takes blocks l, l+32, ...; each block's
+// history (the last w-1 residues of the block below) comes from the lane
+// below by a shuffle.  Counts positions q >= w-1 (func.cu:376-396).  All 32
+// lanes call it with the same arguments.
+template <int P>
+__device__ int word_count_warp_bits(const uint32_t *__restrict__ planes, int net2, int w, const uint32_t *list) {
+  constexpr int bits = P == 2 ? 2 : 5;
+  const uint32_t mask = (1u << (w * bits)) - 1u;
+  const int lane = threadIdx.x & 31;
+  const int nb = (net2 + 31) >> 5;
+  int sum = 0;
+  uint32_t carry[P];
+#pragma unroll
+  for (int p = 0; p < P; p++) carry[p] = 0u;
+  for (int b0 = 0; b0 < nb; b0 += 32) {
+    const int b = b0 + lane;
+    const bool have = b < nb;
+    const int lim = have ? min(32, net2 - 32 * b) : 0;
+    uint32_t pl[P], pv[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+      pl[p] = have ? __ldg(planes + b * P + p) : 0u;
+      pv[p] = __shfl_up_sync(kFullMask, pl[p], 1);
+      if (lane == 0) pv[p] = carry[p];
+    }
+    uint32_t word = 0;
+    for (int k = 32 - (w - 1); k < 32; k++) {  // history: the block below's last w-1 residues
+      uint32_t c = 0;
+#pragma unroll
+      for (int p = 0; p < P; p++) c |= ((pv[p] >> k) & 1u) << p;
+      word = ((word << bits) | c) & mask;
+    }
+    for (int k = 0; k < lim; k++) {
+      uint32_t c = 0;
+#pragma unroll
+      for (int p = 0; p < P; p++) c |= ((pl[p] >> k) & 1u) << p;
+      word = ((word << bits) | c) & mask;
+      if (32 * b + k >= w - 1) sum += (list[word >> 5] >> (word & 31)) & 1u;
+    }
+#pragma unroll
+    for (int p = 0; p < P; p++) carry[p] = __shfl_sync(kFullMask, pl[p], 31);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
+  return sum;
+}
+
 // Composition sum of candidate c against the representative counts rc[].
 template <int A>
 __device__ __forceinline__ int base_sum(const uint32_t *__restrict__ cnt, int c, const uint32_t *rc) {

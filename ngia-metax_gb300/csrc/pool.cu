@@ -143,7 +143,8 @@ __device__ void chunks_body(const PoolDev &pd, int ncls) {
   const int nj = pd.n_jobs, t = threadIdx.x;
   const int per = (nj + NT - 1) / NT;
   const int j0 = min(nj, t * per), j1 = min(nj, j0 + per);
-  for (int k = first_class(pd.type); k < ncls; k++) {  // the classes in use
+  for (int k = 0; k < ncls; k++) {
+    if (pd.grid_align[k] == 0) continue;  // a class the pool cannot queue pairs in
     long long tot = 0;
     for (int j = j0; j < j1; j++) tot += pd.jobs[j].rb.st->qcount[k];
 #pragma unroll
@@ -200,54 +201,6 @@ __device__ __forceinline__ bool last_cta(uint32_t *done) {
 }
 
 // ---- filter -------------------------------------------------------------------
-// Short-word count of one candidate by the whole warp against a k-mer
-// bitset in global memory: lane l takes blocks l, l+32, ...; each block's
-// history (the last w-1 residues of the block below) comes from the lane
-// below by a shuffle.  Counts positions q >= w-1 (func.cu:376-396).  All 32
-// lanes call it with the same arguments.
-template <int P>
-__device__ int word_count_warp_bits(const uint32_t *__restrict__ planes, int net2, int w, const uint32_t *list) {
-  constexpr int bits = P == 2 ? 2 : 5;
-  const uint32_t mask = (1u << (w * bits)) - 1u;
-  const int lane = threadIdx.x & 31;
-  const int nb = (net2 + 31) >> 5;
-  int sum = 0;
-  uint32_t carry[P];
-#pragma unroll
-  for (int p = 0; p < P; p++) carry[p] = 0u;
-  for (int b0 = 0; b0 < nb; b0 += 32) {
-    const int b = b0 + lane;
-    const bool have = b < nb;
-    const int lim = have ? min(32, net2 - 32 * b) : 0;
-    uint32_t pl[P], pv[P];
-#pragma unroll
-    for (int p = 0; p < P; p++) {
-      pl[p] = have ? __ldg(planes + b * P + p) : 0u;
-      pv[p] = __shfl_up_sync(kFullMask, pl[p], 1);
-      if (lane == 0) pv[p] = carry[p];
-    }
-    uint32_t word = 0;
-    for (int k = 32 - (w - 1); k < 32; k++) {  // history: the block below's last w-1 residues
-      uint32_t c = 0;
-#pragma unroll
-      for (int p = 0; p < P; p++) c |= ((pv[p] >> k) & 1u) << p;
-      word = ((word << bits) | c) & mask;
-    }
-    for (int k = 0; k < lim; k++) {
-      uint32_t c = 0;
-#pragma unroll
-      for (int p = 0; p < P; p++) c |= ((pl[p] >> k) & 1u) << p;
-      word = ((word << bits) | c) & mask;
-      if (32 * b + k >= w - 1) sum += (list[word >> 5] >> (word & 31)) & 1u;
-    }
-#pragma unroll
-    for (int p = 0; p < P; p++) carry[p] = __shfl_sync(kFullMask, pl[p], 31);
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
-  return sum;
-}
-
 template <int P>
 __global__ void __launch_bounds__(256) k_pool_filter(PoolDev pd, int ncls) {
   constexpr int A = P == 2 ? 4 : 28;
@@ -297,7 +250,7 @@ __global__ void __launch_bounds__(256) k_pool_filter(PoolDev pd, int ncls) {
             deferred = true;
           }
         }
-        if (pass && !deferred) cls = class_of(type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
+        if (pass && !deferred) cls = class_of(type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
       }
     }
     for (unsigned dm = __ballot_sync(kFullMask, deferred); dm; dm &= dm - 1) {
@@ -309,7 +262,7 @@ __global__ void __launch_bounds__(256) k_pool_filter(PoolDev pd, int ncls) {
         const int L2 = __ldg(J->db.len + cc);
         pass = !(ws < word_min(L2, w, s));
         wpass = pass;
-        if (pass) cls = class_of(type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
+        if (pass) cls = class_of(type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
       }
     }
     push_queue(J->rb, J->rb.st, pass, cls, c);
@@ -726,7 +679,8 @@ int group_open(const std::vector<ngia_ctx *> &jobs, Group **out) {
   // resident CTAs of its kernel (the global-ring bucket at most 2 per SM)
   g->grid_filter = std::max(1, std::min(g->num_sms * 8, (wbase[nj] + 7) / 8));
   PoolDev &pd = g->pd;
-  for (int k = first_class(type); k < num_classes(type); k++) {
+  for (int k = 0; k < num_classes(type); k++) {
+    if (!class_used(type, k, g->max_nb)) continue;
     const int ring = class_ring(type, k);
     g->smem[k] = align_smem(type, g->max_nb, ring);
     int occ = 0;
@@ -738,14 +692,15 @@ int group_open(const std::vector<ngia_ctx *> &jobs, Group **out) {
   }
   uint32_t rs = 1;
   while ((int)rs < g->max_nb) rs <<= 1;
+  // (class 1 is on the global ring too: it runs on the same stream)
   const int gcls = generic_class(type);
-  pd.scratch_words = (int64_t)pd.grid_align[gcls] * kAlignThreads * rs;
+  pd.scratch_words = (int64_t)std::max(pd.grid_align[1], pd.grid_align[gcls]) * kAlignThreads * rs;
   pd.ring_mask = rs - 1;
   if (dalloc(&g->d_scratch, (size_t)pd.scratch_words) != cudaSuccess) {
     group_close(g);
     return fail(NGIA_E_NOMEM, "pool: device allocation of the alignment ring failed");
   }
-  for (int k = first_class(type); k < num_classes(type); k++)
+  for (int k = 0; k < num_classes(type); k++)
     if (cudaStreamCreateWithFlags(&g->side[k], cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&g->join[k], cudaEventDisableTiming) != cudaSuccess) {
       group_close(g);
@@ -803,15 +758,17 @@ int group_enqueue_round(Group *g, cudaStream_t s, cudaGraphConditionalHandle con
   else
     k_pool_filter<5><<<g->grid_filter, 256, fsm, s>>>(pd, nc);
   cudaError_t e = cudaEventRecord(g->fork, s);
-  for (int k = first_class(type); e == cudaSuccess && k < nc; k++) {
-    e = cudaStreamWaitEvent(g->side[k], g->fork, 0);
+  for (int k = 0; e == cudaSuccess && k < nc; k++) {
+    if (pd.grid_align[k] == 0) continue;
+    cudaStream_t side = g->side[class_stream(type, k)];
+    e = cudaStreamWaitEvent(side, g->fork, 0);
     if (e != cudaSuccess) break;
     PoolDev a = pd;
     int cls = k, mnb = g->max_nb;
     void *args[] = {&a, &cls, &mnb};
     e = cudaLaunchKernel((const void *)align_fn(type, class_ring(type, k)), dim3(pd.grid_align[k]), dim3(kAlignThreads),
-                         args, g->smem[k], g->side[k]);
-    if (e == cudaSuccess) e = cudaEventRecord(g->join[k], g->side[k]);
+                         args, g->smem[k], side);
+    if (e == cudaSuccess) e = cudaEventRecord(g->join[k], side);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, g->join[k], 0);
   }
   if (e != cudaSuccess) return fail(NGIA_E_CUDA, "pool: alignment launches: %s", cudaGetErrorString(e));

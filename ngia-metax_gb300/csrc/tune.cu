@@ -173,7 +173,7 @@ extern "C" int ngia_autotune(ngia_ctx *c, const ngia_params *p, int32_t iters, n
   }
   // per length bucket: the classes that queued pairs in the default run
   const int cut = best_s.wp >= 0 ? best_s.wp : def_wp;
-  for (int k = ngia::first_class(c->db.type); k < ngia::num_classes(c->db.type) && !rc; k++) {
+  for (int k = 0; k < ngia::num_classes(c->db.type) && !rc; k++) {
     if (!pairs[k]) continue;
     for (int v = 0; v < 3 && !rc; v++) {
       Setting s = best_s;

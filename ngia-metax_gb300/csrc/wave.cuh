@@ -1,0 +1,346 @@
+// wave.cuh — the banded bit-parallel LCS of one pair by a group of 32 or 128
+// threads, for launches whose pairs are too few to give every thread its own.
+//
+// The band is a grid of 32 x 32 blocks (query block i, rep block j).  A chunk
+// of W rep blocks belongs to one thread of the group, chunk q to thread
+// q mod GS, its W row words in registers; the columns of a query block are
+// taken in units of 16.  Thread g works on unit u = t - q of its chunk at
+// step t, so that the carries chunk q-1 put out at unit u reach it one step
+// later: a systolic wavefront with one shuffle per step (and one shared word
+// per warp for groups of 128), instead of a vote over all lanes per column.
+// A thread whose chunk has left the band banks its zeros and opens chunk
+// q + GS.  Units the thread's chunk does not take part in run with masked
+// match words and no carry in, which leaves the rows as they are and puts no
+// carry out.
+//
+// Match words come from a table of the representative in shared memory, one
+// row of words per residue code, so that the 32 lanes (consecutive rep
+// blocks, any codes) hit 32 banks; the query's codes from a ring of bytes the
+// group fills 32 blocks at a time.
+//
+// What bounds it: a lone warp per scheduler issues its instructions one
+// after the other, about three cycles each: nine per column and 80 per step
+// of 16 columns; a pair takes 2 nq + nb1 / W steps.  GB300: a 6,600-residue
+// protein pair 375 -> 195 us against a form that resolved every column's
+// carries over the lanes with two votes, 500 DNA pairs of 1,450 residues
+// 100-275 -> 65 us.  Tried: planes in registers instead of the table (370
+// us), the columns rolled by four (250), the carry as a value instead of the
+// carry flag (231), two row words per thread where one is enough (292).
+#pragma once
+#include <stdint.h>
+
+#include "common.cuh"
+#include "dp_asm.cuh"
+
+namespace ngia {
+
+constexpr int kWaveCols = 16, kWaveUnits = 2;  // columns per unit, units per query block
+constexpr int kWaveRing = 128;                 // query blocks of codes a group keeps
+constexpr int kWaveRingWords = kWaveRing * 8;  // one byte per residue
+
+__host__ __device__ constexpr int wave_codes(int P) { return 1 << P; }               // residue codes the planes can hold
+// Words of a match table of max_nb blocks (rows of whole 32-block lines, so
+// that the last chunk's missing blocks read zeros).
+__host__ __device__ constexpr int wave_stride(int nb) { return (nb + 31) & ~31; }
+__host__ __device__ constexpr int wave_table_words(int P, int nb) { return wave_codes(P) * wave_stride(nb); }
+
+// Widest band (blocks a query block covers) a group of GS threads can take
+// with W row words per thread when chunks are reused: a thread must have left
+// chunk q - 1 + GS alone until its neighbour is through with chunk q.
+__host__ __device__ constexpr int wave_cap(int GS, int W) { return W * (GS - 2) + GS / kWaveUnits + 1; }
+
+// Band of one pair in blocks below and above the diagonal.  With a cutoff,
+// only the diagonals a chain of that many matches can touch; false when no
+// chain can reach it.
+__device__ __forceinline__ bool wave_band(int B, int net1, int net2, int cut, int &lo, int &hi) {
+  lo = hi = B;
+  if (cut == kNoCut) return true;
+  if (net1 < cut || net2 < cut) return false;
+  lo = min(B, 1 + ((net2 - cut) >> 5));
+  hi = min(B, 1 + ((net1 - cut) >> 5));
+  return true;
+}
+
+// Builds the match table of a representative (planes rp, nb1 blocks, vlast
+// the valid rows of the last) at tab with `threads` threads, t of them;
+// the caller synchronises.
+template <int P>
+__device__ __forceinline__ void wave_table(const uint32_t *rp, int nb1, uint32_t vlast, uint32_t *tab, int t,
+                                           int threads) {
+  const int stride = wave_stride(nb1);
+  for (int j = t; j < stride; j += threads) {
+    uint32_t pl[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) pl[p] = j < nb1 ? rp[j * P + p] : 0u;
+    const uint32_t valid = j < nb1 - 1 ? 0xFFFFFFFFu : j == nb1 - 1 ? vlast : 0u;
+#pragma unroll
+    for (int a = 0; a < wave_codes(P); a++) {
+      uint32_t m = valid;
+#pragma unroll
+      for (int p = 0; p < P; p++) m &= (a >> p) & 1 ? pl[p] : ~pl[p];
+      tab[a * stride + j] = m;
+    }
+  }
+}
+
+// The residue codes of one query block (planes pl) as 32 bytes.
+template <int P>
+__device__ __forceinline__ void wave_unpack(const uint32_t (&pl)[P], uint4 *out) {
+  uint32_t v[8];
+#pragma unroll
+  for (int x = 0; x < 8; x++) {
+    v[x] = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+      for (int p = 0; p < P; p++) v[x] |= ((pl[p] >> (4 * x + c)) & 1u) << (8 * c + p);
+  }
+  out[0] = make_uint4(v[0], v[1], v[2], v[3]);
+  out[1] = make_uint4(v[4], v[5], v[6], v[7]);
+}
+
+// W consecutive match words (W-word aligned, at most four at a time).
+template <int W>
+__device__ __forceinline__ void wave_load(uint32_t (&e)[W], const char *a) {
+  if constexpr (W == 1) {
+    e[0] = *reinterpret_cast<const uint32_t *>(a);
+  } else if constexpr (W == 2) {
+    const uint2 v = *reinterpret_cast<const uint2 *>(a);
+    e[0] = v.x;
+    e[1] = v.y;
+  } else {
+#pragma unroll
+    for (int w = 0; w < W; w += 4) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(a + 4 * w);
+      e[w] = v.x;
+      e[w + 1] = v.y;
+      e[w + 2] = v.z;
+      e[w + 3] = v.w;
+    }
+  }
+}
+
+// Zero count of the pair over its band, the same in every thread of the
+// group, or -1 once it cannot reach `cut`.  All GS = 32 NW threads call it
+// with the same arguments (NW > 1: the whole CTA, xch = 4 NW shared words).
+// tab: the representative's match table, ring: the group's code ring (both
+// shared, 16-byte aligned), qp: query planes.  B >= 0, nb1 > 0 and nq > 0.
+template <int P, int W, int NW>
+__device__ __forceinline__ int wave_pair(const uint32_t *tab, int nb1, const uint32_t *qp, int nq, int net2, int lo,
+                                         int hi, int cut, uint32_t *ring, uint32_t *xch, unsigned long long &n_done) {
+  constexpr int GS = 32 * NW, C = kWaveCols, S = kWaveUnits;
+  const int lane = threadIdx.x & 31, warp = NW > 1 ? (int)(threadIdx.x >> 5) : 0;
+  const int g = warp * 32 + lane;
+  const int q_last = min(nb1 - 1, nq - 1 + hi) / W;
+  const uint32_t row_bytes = 4u * (uint32_t)wave_stride(nb1);
+  uint32_t row[W];
+  const char *base = nullptr;
+  int q = g, u0 = 0, u1 = 0, acc = 0;
+  auto open = [&]() {  // chunk q: rows all-ones
+    const bool used = q <= q_last;
+    u0 = used ? S * max(0, q * W - hi) : 0;
+    u1 = used ? min(S * nq, S * (q * W + W + lo)) : 0;
+    base = reinterpret_cast<const char *>(tab + (used ? q * W : 0));
+#pragma unroll
+    for (int w = 0; w < W; w++) row[w] = 0xFFFFFFFFu;
+  };
+  open();
+  uint32_t cout = 0, cells = 0;
+  const int steps = S * nq + q_last;
+  if constexpr (NW == 1) __syncwarp();  // the group is through with the last pair's ring
+  for (int t = 0; t < steps; t++) {
+    if ((t & (32 * S - 1)) == 0) {  // the next 32 query blocks' codes
+      const int b = (t >> 1) + g;
+      if (g < 32 && b < nq) {
+        uint32_t pl[P];
+#pragma unroll
+        for (int p = 0; p < P; p++) pl[p] = __ldg(qp + b * P + p);
+        wave_unpack<P>(pl, reinterpret_cast<uint4 *>(ring) + 2 * (b & (kWaveRing - 1)));
+      }
+      if constexpr (NW == 1) __syncwarp();
+    }
+    // carries of the chunk below at this unit
+    uint32_t cin = __shfl_sync(kFullMask, cout, (lane + 31) & 31);
+    if constexpr (NW > 1) {
+      if (lane == 31) xch[(t & 1) * NW + warp] = cout;
+      if ((t & 7) == 7 && cut != kNoCut) {
+        int z = acc;
+#pragma unroll
+        for (int w = 0; w < W; w++) z += __popc(~row[w]);
+        z = __reduce_add_sync(kFullMask, z);
+        if (lane == 0) xch[2 * NW + ((t >> 3) & 1) * NW + warp] = (uint32_t)z;
+      }
+      __syncthreads();
+      if (lane == 0) cin = xch[(t & 1) * NW + (warp + NW - 1) % NW];
+    }
+    if (cut != kNoCut && (t & 7) == 7) {
+      // Every row's zeros up to its own unit of the last step bound the
+      // longest chain that ends at the top row reached so far, and each
+      // column after that row's unit adds at most one.
+      int z = 0;
+      if constexpr (NW > 1) {
+#pragma unroll
+        for (int k = 0; k < NW; k++) z += (int)xch[2 * NW + ((t >> 3) & 1) * NW + k];
+      } else {
+        z = acc;
+#pragma unroll
+        for (int w = 0; w < W; w++) z += __popc(~row[w]);
+        z = __reduce_add_sync(kFullMask, z);
+      }
+      int top = (t - 1 + S * hi) / (S * W + 1);
+      if (top * W <= hi) top = min(t - 1, hi / W);
+      top = min(top, q_last);
+      if (z + max(0, net2 - C * (t - top)) < cut) {  // the group decides alike
+        n_done += cells;
+        return -1;
+      }
+    }
+    const int u = t - q, i = u >> 1;
+    const bool active = u >= u0 && u < u1;
+    const int ncol = active ? max(0, min(C, net2 - C * u)) : 0;
+    uint32_t act[W];
+    int rows = 0;
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+      const int j = q * W + w;
+      const bool in = active && (W == 1 || (j >= i - lo && j <= i + hi));
+      act[w] = in ? 0xFFFFFFFFu : 0u;
+      rows += in ? 1 : 0;
+    }
+    cells += (uint32_t)(rows * ncol);
+    // idle threads take code 0: the ring's other bytes may be from nowhere
+    uint4 codes = make_uint4(0u, 0u, 0u, 0u);
+    if (active) codes = reinterpret_cast<const uint4 *>(ring)[2 * (i & (kWaveRing - 1)) + (u & 1)];
+    const uint32_t code[4] = {codes.x, codes.y, codes.z, codes.w};
+    uint32_t cw = ncol > 0 && q > 0 ? cin << (32 - ncol) : 0u, ncw = 0;
+    auto column = [&](uint32_t c) {  // one column of residue code c
+      uint32_t e[W];
+      wave_load<W>(e, base + c * row_bytes);
+      dp_wave<W>(row, e, act, cw, ncw);
+    };
+    if (t < S * nq - 2 || __all_sync(kFullMask, !active || ncol == C)) {
+#pragma unroll(W <= 2 ? C : 4)
+      for (int k = 0; k < C; k++) column(__byte_perm(code[k >> 2], 0, 0x4440 | (k & 3)));
+    } else {  // the query's last columns
+#pragma unroll 1
+      for (int k = 0; k < ncol; k++) {
+        const uint32_t w = k < 4 ? code[0] : k < 8 ? code[1] : k < 12 ? code[2] : code[3];
+        column((w >> (8 * (k & 3))) & 0xFFu);
+      }
+    }
+    cout = ncw;
+    if (u >= 0 && u + 1 >= u1 && q <= q_last) {  // the chunk has left the band
+#pragma unroll
+      for (int w = 0; w < W; w++) acc += __popc(~row[w]);
+      q += GS;
+      open();
+    }
+  }
+  n_done += cells;
+  int sum = __reduce_add_sync(kFullMask, acc);
+  if constexpr (NW > 1) {
+    __syncthreads();
+    if (lane == 0) xch[warp] = (uint32_t)sum;
+    __syncthreads();
+    sum = 0;
+#pragma unroll
+    for (int k = 0; k < NW; k++) sum += (int)xch[k];
+    __syncthreads();
+  }
+  return sum;
+}
+
+// The same with the fewest row words per thread (up to WMAX) the band allows;
+// a group that holds every rep block at once takes any band.  The caller
+// makes sure that WMAX words do.
+template <int P, int NW, int WMAX>
+__device__ __forceinline__ int wave_any(const uint32_t *tab, int nb1, const uint32_t *qp, int nq, int net2, int lo,
+                                        int hi, int cut, uint32_t *ring, uint32_t *xch, unsigned long long &n_done) {
+  constexpr int GS = 32 * NW;
+  const int n = lo + hi + 1;
+#define NGIA_WAVE(W)                                        \
+  if constexpr (W <= WMAX)                                  \
+    if (W == WMAX || n <= wave_cap(GS, W) || nb1 <= GS * W) \
+      return wave_pair<P, W, NW>(tab, nb1, qp, nq, net2, lo, hi, cut, ring, xch, n_done);
+  NGIA_WAVE(1) NGIA_WAVE(2) NGIA_WAVE(4) NGIA_WAVE(8) NGIA_WAVE(16)
+#undef NGIA_WAVE
+  return -1;
+}
+
+// ---- the query's blocks as rows -------------------------------------------------
+// Short queries against a long representative: GS = 16 threads per pair, two
+// pairs per warp, one query block per thread as its row word, the
+// representative's residues as columns.  The band and the recurrence are
+// symmetric in the two sequences, so the count is the same; a pair takes
+// 2 nb1 + nq steps of two lanes' groups instead of 2 nq + nb1 / W of 128
+// threads.  No early rejection: while the representative is long, every
+// query residue can still find its match.
+// rep_codes: the representative's residue codes, 32 bytes per block (shared
+// by the CTA); tab: the warp's match table, one word per code and lane.
+// Lanes of a group without a pair pass nq = 0.  Returns the zero count to
+// every lane of the pair's group.
+constexpr int kQueryGroup = 16;
+static_assert(kQueryRows <= kQueryGroup, "a query block per thread");
+
+template <int P>
+__device__ __forceinline__ int wave_query(const uint32_t *rep_codes, int nb1, int net1, const uint32_t *qp, int nq,
+                                          int net2, int lo, int hi, uint32_t *tab, unsigned long long &n_done) {
+  constexpr int C = kWaveCols, S = kWaveUnits;
+  const int lane = threadIdx.x & 31, g = lane & (kQueryGroup - 1);
+  // row word g: the query's block g; its match words by code
+  uint32_t pl[P];
+  const bool used = g < nq;
+#pragma unroll
+  for (int p = 0; p < P; p++) pl[p] = used ? __ldg(qp + g * P + p) : 0u;
+  const uint32_t valid = !used ? 0u : g == nq - 1 && (net2 & 31) ? (1u << (net2 & 31)) - 1u : 0xFFFFFFFFu;
+  __syncwarp();  // the last pair's table is read
+#pragma unroll
+  for (int a = 0; a < wave_codes(P); a++) {
+    uint32_t m = valid;
+#pragma unroll
+    for (int p = 0; p < P; p++) m &= (a >> p) & 1 ? pl[p] : ~pl[p];
+    tab[32 * a + lane] = m;
+  }
+  __syncwarp();
+  // units of the rep this row takes part in (row block g, rep block i:
+  // -lo <= i - g <= hi), and the steps the warp needs
+  const int u0 = used ? S * max(0, g - lo) : 0, u1 = used ? min(S * nb1, S * (g + 1 + hi)) : 0;
+  const int steps = (int)__reduce_max_sync(kFullMask, (unsigned)(u1 > u0 ? u1 + g : 0));
+  uint32_t row[1] = {0xFFFFFFFFu}, cout = 0, cells = 0;
+  const char *base = reinterpret_cast<const char *>(tab + lane);
+  for (int t = 0; t < steps; t++) {
+    const uint32_t cin = __shfl_sync(kFullMask, cout, (lane + 31) & 31);
+    const int u = t - g;
+    const bool active = u >= u0 && u < u1;
+    const int ncol = active ? max(0, min(C, net1 - C * u)) : 0;
+    const uint32_t act[1] = {active ? 0xFFFFFFFFu : 0u};
+    cells += (uint32_t)ncol;
+    uint4 codes = make_uint4(0u, 0u, 0u, 0u);
+    if (active) codes = reinterpret_cast<const uint4 *>(rep_codes)[u];
+    const uint32_t code[4] = {codes.x, codes.y, codes.z, codes.w};
+    uint32_t cw = ncol > 0 && g > 0 ? cin << (32 - ncol) : 0u, ncw = 0;
+    auto column = [&](uint32_t c) {
+      uint32_t e[1];
+      wave_load<1>(e, base + c * 128u);
+      dp_wave<1>(row, e, act, cw, ncw);
+    };
+    if (__all_sync(kFullMask, !active || ncol == C)) {
+#pragma unroll
+      for (int k = 0; k < C; k++) column(__byte_perm(code[k >> 2], 0, 0x4440 | (k & 3)));
+    } else {  // the representative's last columns
+#pragma unroll 1
+      for (int k = 0; k < ncol; k++) {
+        const uint32_t w = k < 4 ? code[0] : k < 8 ? code[1] : k < 12 ? code[2] : code[3];
+        column((w >> (8 * (k & 3))) & 0xFFu);
+      }
+    }
+    cout = ncw;
+  }
+  n_done += cells;
+  int sum = __popc(~row[0]);
+#pragma unroll
+  for (int o = kQueryGroup / 2; o; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
+  return sum;
+}
+
+}  // namespace ngia
