@@ -146,17 +146,26 @@ __device__ __forceinline__ int wave_pair(const uint32_t *tab, int nb1, const uin
   };
   open();
   uint32_t cout = 0, cells = 0;
+  int low = 0, low_end = S * (W + lo), filled = 0;  // lowest active chunk, the step it ends at; blocks of codes fetched
   const int steps = S * nq + q_last;
   if constexpr (NW == 1) __syncwarp();  // the group is through with the last pair's ring
   for (int t = 0; t < steps; t++) {
-    if ((t & (32 * S - 1)) == 0) {  // the next 32 query blocks' codes
-      const int b = (t >> 1) + g;
+    // The lowest chunk still in the band is furthest along the query, the
+    // GS chunks from it at most GS / 2 blocks behind: the next 32 blocks'
+    // codes are fetched when it reaches them, over blocks no thread needs.
+    if (t >= low_end) {
+      low++;
+      low_end += S * W + 1;
+    }
+    if (((t - low) >> 1) >= filled && filled < nq) {
+      const int b = filled + g;
       if (g < 32 && b < nq) {
         uint32_t pl[P];
 #pragma unroll
         for (int p = 0; p < P; p++) pl[p] = __ldg(qp + b * P + p);
         wave_unpack<P>(pl, reinterpret_cast<uint4 *>(ring) + 2 * (b & (kWaveRing - 1)));
       }
+      filled += 32;
       if constexpr (NW == 1) __syncwarp();
     }
     // carries of the chunk below at this unit

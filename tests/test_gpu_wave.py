@@ -33,6 +33,11 @@ def _seq(rng, alpha, L, base=None):
     (0, 4097, 0.5, (4096, 4081, 2100, 530, 512, 480, 16)),
     (0, 10001, 0.6, (9999, 6000, 1010, 512, 511, 65)),
     (0, 60003, 0.5, (50000, 20000, 500, 31)),
+    (0, 20000, 0.97, (19990, 19500)),  # long pairs: every form's code ring wraps many times
+    (0, 16000, 0.95, (15990, 15600)),
+    (0, 30000, 0.93, (29990, 28500)),
+    (1, 33000, 0.9, (32990, 31000)),
+    (1, 40000, 0.8, (39000,)),
     (1, 1520, 0.9, (1520, 1400, 1040, 512, 500)),
     (1, 4100, 0.6, (4100, 2049, 544, 512, 496, 17)),
     (1, 9000, 0.5, (8990, 3000, 513, 512, 90)),
