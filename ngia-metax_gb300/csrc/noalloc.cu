@@ -8,12 +8,22 @@
 // Such a caller already holds its inputs and outputs in device memory; this
 // entry point uses them as given and allocates nothing.
 //
-// The alignment needs per-thread working rows (one 32-bit word per 32
-// representative residues).  Here they live in a fixed file-scope device
-// array, g_noalloc_rows, of kNoAllocWords words (4 MiB).  Every GPU that loads
-// this library keeps that array until the process exits.  Its size caps the
-// representative at 65,536 residues (2,048 words per thread row); the grid is
-// sized so that every thread's row fits.
+// Three kernels:
+//  * up to noalloc_groups pairs per SM, a group of threads per pair (wave.cuh:
+//    rows in registers, match table and query codes in shared memory);
+//  * above that, representatives of up to 128 blocks: a thread per pair, the
+//    band rows in a shared-memory ring, register tiles (tile.cuh);
+//  * proteins whose match table does not fit shared memory: a thread per
+//    pair with its working row (one 32-bit word per 32 representative
+//    residues) in a fixed file-scope device array, g_noalloc_rows, of
+//    kNoAllocWords words (4 MiB).
+// GB300, whole calls: 4,096 DNA queries of 1,450 residues 810 -> 168 us, 1,000
+// proteins of 380 residues 300 -> 49 us (against the third kernel for all).
+//
+// Every GPU that loads this library keeps that array until the process
+// exits.  Its size caps the representative at 65,536 residues (2,048 words
+// per thread row); the grid of the third kernel is sized so that every
+// thread's row fits.
 //
 // Host code must not use the array's name as a device address: the first call
 // on each device looks its address up with cudaGetSymbolAddress (with that
@@ -33,11 +43,21 @@
 
 #include "../host/host_common.h"
 #include "common.cuh"
+#include "tile.cuh"
+#include "wave.cuh"
 
 namespace {
 
 constexpr int kNoAllocWords = 1 << 20;  // 4 MiB of per-thread rows
 constexpr int kThreads = 128;
+static_assert(kThreads == ngia::kAlignThreads, "the ring and the groups of four warps");
+// Pairs per SM up to which a group per pair is faster than a thread per pair,
+// which takes a pair's latency whatever their number.  GB300: DNA 1,450
+// residues 238 us for 6,000 pairs by groups, 292 from 9,000 to 16,000 by
+// threads; 300 residues 69 against 47; protein 380 residues 118 against 132,
+// 900 residues 232 against 525.
+constexpr int noalloc_groups(int P, int nb1) { return P == 2 && nb1 <= 16 ? 26 : 50; }
+constexpr size_t kNoAllocSmemMost = 226 * 1024;
 
 __device__ __align__(256) uint32_t g_noalloc_rows[kNoAllocWords];
 
@@ -113,6 +133,162 @@ __global__ void __launch_bounds__(kThreads) k_noalloc_scores(const uint32_t *__r
   }
 }
 
+// Length and score of a query that needs no alignment: -1 for a record that
+// makeDB cannot have written, 0 where the band or a sequence is empty.
+// Returns true when there is an alignment to do.
+__device__ __forceinline__ bool noalloc_pair(const uint32_t *q, int nb1, int L1, float s, int &net2, int &B, int *score) {
+  const uint32_t L2 = q[0];
+  net2 = (int)q[1];
+  if (L2 > (uint32_t)ngia::kMaxLenDev || (uint32_t)net2 > L2) {
+    *score = -1;
+    return false;
+  }
+  B = ngia::band_blocks(L1, (int)L2, s);
+  *score = 0;
+  return B >= 0 && nb1 > 0 && net2 > 0;
+}
+
+// A group of 32 NW threads per pair.  Shared memory: match table | code rings.
+template <int P, int NW, int WMAX>
+__global__ void __launch_bounds__(kThreads) k_noalloc_wave(const uint32_t *__restrict__ words, int64_t rep_off,
+                                                           const int64_t *__restrict__ query_off, int n, float s,
+                                                           int *__restrict__ scores, int cap_blocks) {
+  extern __shared__ __align__(16) uint32_t s_mem[];
+  __shared__ uint32_t s_xch[4 * NW];
+  constexpr int hw = P == 2 ? 6 : 30, kGroups = kThreads / 32 / NW;
+  const uint32_t *rep = words + rep_off;
+  const int L1 = (int)rep[0], net1 = (int)rep[1], nb1 = (net1 + 31) / 32;
+  if (nb1 > cap_blocks) return;  // the host sized shared memory for this many
+  const int group = (int)(threadIdx.x >> 5) / NW;
+  const bool lead = threadIdx.x % (32 * NW) == 0;
+  const uint32_t vlast = (net1 & 31) ? ((1u << (net1 & 31)) - 1u) : 0xFFFFFFFFu;
+  uint32_t *ring = s_mem + ngia::wave_table_words(P, nb1) + group * ngia::kWaveRingWords;
+  ngia::wave_table<P>(rep + hw, nb1, vlast, s_mem, threadIdx.x, kThreads);
+  __syncthreads();
+  unsigned long long cells = 0;
+  for (int k = blockIdx.x * kGroups + group; k < n; k += gridDim.x * kGroups) {
+    const uint32_t *q = words + query_off[k];
+    int net2 = 0, B = 0, score = 0;
+    if (noalloc_pair(q, nb1, L1, s, net2, B, &score))
+      score = ngia::wave_any<P, NW, WMAX>(s_mem, nb1, q + hw, (net2 + 31) / 32, net2, B, B, ngia::kNoCut, ring, s_xch,
+                                          cells);
+    if (lead) scores[k] = score;
+  }
+}
+
+// A thread per pair, 32 neighbouring queries per warp.  Shared memory: rep
+// planes | row ring | match table (the layout of the clustering kernel
+// without its k-mer bitset).
+template <int P, int RING>
+__global__ void __launch_bounds__(kThreads, ngia::tiled_min_blocks(P))
+    k_noalloc_tiled(const uint32_t *__restrict__ words, int64_t rep_off, const int64_t *__restrict__ query_off, int n,
+                    float s, int *__restrict__ scores, int cap_blocks) {
+  using Ring = typename ngia::RingOf<RING>::T;
+  extern __shared__ __align__(16) uint32_t s_mem[];
+  constexpr int hw = P == 2 ? 6 : 30, MT = ngia::tiled_main(P);
+  constexpr unsigned kAll = ngia::kFullMask;
+  const uint32_t *rep = words + rep_off;
+  const int L1 = (int)rep[0], net1 = (int)rep[1], nb1 = (net1 + 31) / 32;
+  if (nb1 > cap_blocks) return;
+  const uint32_t vlast = (net1 & 31) ? ((1u << (net1 & 31)) - 1u) : 0xFFFFFFFFu;
+  const int planes = (cap_blocks * P + 3) & ~3;
+  for (int t = threadIdx.x; t < nb1 * P; t += kThreads) s_mem[t] = rep[hw + t];
+  __syncthreads();
+  uint32_t *s_eq = s_mem + planes + RING * kThreads;
+  if constexpr (P == 2) {
+    ngia::build_eq(s_mem, nb1, s_eq);
+    __syncthreads();
+  }
+  const uint32_t s_eq_s = ngia::smem_u32(s_eq);
+  (void)s_eq_s;
+  const uint32_t one_rt = 1u + (uint32_t)(nb1 < 0);
+  const ngia::FmaK fk{one_rt, one_rt << 2};
+  (void)fk;
+  Ring ring;
+  ring.base = s_mem + planes + threadIdx.x;
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (kThreads / 32);
+  for (int k0 = (blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * 32; k0 < n; k0 += warps * 32) {
+    const int k = k0 + lane;
+    int net2 = 0, B = 0, score = 0, nq = 0, js = 0, je = -1, frozen = 0, zw = 0;
+    const uint32_t *qpl = words;
+    if (k < n) {
+      const uint32_t *q = words + query_off[k];
+      if (noalloc_pair(q, nb1, L1, s, net2, B, &score)) {
+        qpl = q + hw;
+        nq = (net2 + 31) / 32;
+        je = min(B, nb1 - 1);
+        for (int j = 0; j <= je; j++) ring[j] = 0xFFFFFFFFu;
+      }
+    }
+    for (int i = 0; __any_sync(kAll, i < nq); i++) {  // warp-uniform
+      const bool busy = i < nq;
+      const int rows = busy ? je - js + 1 : 0;
+      const int full = (int)__reduce_min_sync(kAll, busy ? (unsigned)(rows / MT) : 0xFFFFFFFFu);
+      int rem = (int)__reduce_max_sync(kAll, busy ? (unsigned)(rows - MT * full) : 0u);
+      if (busy) {
+        const int cols = min(32, net2 - 32 * i);
+        uint32_t cur[P], cw = 0, ncw = 0;
+#pragma unroll
+        for (int p = 0; p < P; p++) cur[p] = __ldg(qpl + i * P + p);
+        int base = js;
+        if constexpr (P == 2) {
+          uint32_t wc[2];
+          ngia::eq_codes_top(cur, wc);
+          zw = 0;
+          for (int t = 0; t < full; t++, base += MT) {
+            zw += ngia::tiled_tile_eqf<MT, true, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
+            cw = ncw << (32 - cols);
+            ncw = 0;
+          }
+          for (; rem >= MT; rem -= MT, base += MT) {
+            zw += ngia::tiled_tile_eqf<MT, true, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
+            cw = ncw << (32 - cols);
+            ncw = 0;
+          }
+          if (rem > 0) zw += ngia::tiled_rem_eqf<Ring>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
+        } else {
+          for (int t = 0; t < full; t++, base += MT) {
+            zw += ngia::tiled_tile<P, MT, Ring>(ring, s_mem, base, je, cols, cur, cw, ncw);
+            cw = ncw << (32 - cols);
+            ncw = 0;
+          }
+          for (; rem >= MT; rem -= MT, base += MT) {
+            zw += ngia::tiled_tile<P, MT, Ring>(ring, s_mem, base, je, cols, cur, cw, ncw);
+            cw = ncw << (32 - cols);
+            ncw = 0;
+          }
+          if (rem > 0) zw += ngia::tiled_rem<P, Ring, MT>(rem, ring, s_mem, base, je, cols, cur, cw, ncw);
+        }
+        const bool last = i + 1 >= nq || ngia::band_advance(ring, i + 1, B, nb1, net1, vlast, net2 - 32 * (i + 1),
+                                                            ngia::kNoCut, js, je, frozen, zw) != ngia::kBandGo;
+        if (last) {
+          score = frozen;
+          for (int j = js; j <= je; j++) score += __popc(~ring[j] & (j == nb1 - 1 ? vlast : 0xFFFFFFFFu));
+          nq = 0;
+        }
+      }
+    }
+    if (k < n) scores[k] = score;
+  }
+}
+
+using NoAllocFn = void (*)(const uint32_t *, int64_t, const int64_t *, int, float, int *, int);
+
+// Raises a kernel's dynamic shared memory limit to `bytes` (never lowers it).
+cudaError_t noalloc_configure(NoAllocFn fn, int slot, size_t bytes) {
+  static std::mutex mu;
+  static size_t have[64][16] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (bytes <= have[dev][slot]) return cudaSuccess;
+  e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) have[dev][slot] = bytes;
+  return e;
+}
+
 // Address of g_noalloc_rows on the current device, looked up once per device.
 int rows_address(uint32_t **out) {
   int dev = 0;
@@ -160,20 +336,39 @@ extern "C" int ngia_rep_scores_noalloc(const uint32_t *d_words, int64_t rep_off,
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Every thread owns one row of nb1 words; the grid is as large as the
-  // array allows (at least 4 CTAs: 2,048-word rows x 512 threads).
-  const int64_t max_lanes = kNoAllocWords / (nb1 > 0 ? nb1 : 1);
-  int grid = (int)std::min<int64_t>((int64_t)std::max(sms, 1) * 4, max_lanes / kThreads);
-  grid = std::max(1, std::min(grid, (n + kThreads - 1) / kThreads));
-  const int64_t lanes = (int64_t)grid * kThreads;
-  const int cap_blocks = (int)(kNoAllocWords / lanes);
-  const size_t smem = sizeof(uint32_t) * (size_t)std::max(1, nb1 * P);
-  if (type == 0)
-    k_noalloc_scores<2><<<grid, kThreads, smem, st>>>(d_words, rep_off, d_query_off, n, similarity, d_scores, rows,
-                                                      lanes, cap_blocks);
-  else
-    k_noalloc_scores<5><<<grid, kThreads, smem, st>>>(d_words, rep_off, d_query_off, n, similarity, d_scores, rows,
-                                                      lanes, cap_blocks);
+  const bool many = n > noalloc_groups(P, nb1) * std::max(sms, 1) && nb1 <= 128;
+  const int form = nb1 <= 64 ? 0 : nb1 <= 128 ? 1 : 2;  // a warp, a CTA of one row word per thread, of up to 16
+  NoAllocFn fn;
+  size_t smem;
+  int per;  // pairs per CTA
+  if (many) {
+    const int ring = form == 0 ? 64 : 128;
+    fn = P == 2 ? (form == 0 ? k_noalloc_tiled<2, 64> : k_noalloc_tiled<2, 128>)
+                : (form == 0 ? k_noalloc_tiled<5, 64> : k_noalloc_tiled<5, 128>);
+    smem = 4 * (size_t)(((nb1 * P + 3) & ~3) + ring * kThreads + (P == 2 ? ngia::eq_words(nb1) : 0));
+    per = kThreads;
+  } else {
+    fn = P == 2 ? (form == 0 ? k_noalloc_wave<2, 1, 2> : form == 1 ? k_noalloc_wave<2, 4, 1> : k_noalloc_wave<2, 4, 16>)
+                : (form == 0 ? k_noalloc_wave<5, 1, 2> : form == 1 ? k_noalloc_wave<5, 4, 1> : k_noalloc_wave<5, 4, 16>);
+    per = form == 0 ? kThreads / 32 : 1;
+    smem = 4 * ((size_t)ngia::wave_table_words(P, nb1) + (size_t)per * ngia::kWaveRingWords);
+  }
+  if (smem <= kNoAllocSmemMost) {
+    e = noalloc_configure(fn, (P == 2 ? 0 : 8) + (many ? 4 : 0) + form, smem);
+    if (e != cudaSuccess) return ngia::fail(NGIA_E_CUDA, "ngia_rep_scores_noalloc: %s", cudaGetErrorString(e));
+    const int grid = std::max(1, std::min(std::max(sms, 1) * 8, (n + per - 1) / per));
+    fn<<<grid, kThreads, smem, st>>>(d_words, rep_off, d_query_off, n, similarity, d_scores, nb1);
+  } else {  // a protein's table of more than 1,700 blocks
+    // Every thread owns one row of nb1 words; the grid is as large as the
+    // array allows (at least 4 CTAs: 2,048-word rows x 512 threads).
+    const int64_t max_lanes = kNoAllocWords / (nb1 > 0 ? nb1 : 1);
+    int grid = (int)std::min<int64_t>((int64_t)std::max(sms, 1) * 4, max_lanes / kThreads);
+    grid = std::max(1, std::min(grid, (n + kThreads - 1) / kThreads));
+    const int64_t lanes = (int64_t)grid * kThreads;
+    const int cap_blocks = (int)(kNoAllocWords / lanes);
+    k_noalloc_scores<5><<<grid, kThreads, sizeof(uint32_t) * (size_t)(nb1 * P), st>>>(
+        d_words, rep_off, d_query_off, n, similarity, d_scores, rows, lanes, cap_blocks);
+  }
   e = cudaGetLastError();
   if (e != cudaSuccess) return ngia::fail(NGIA_E_CUDA, "ngia_rep_scores_noalloc: %s", cudaGetErrorString(e));
   return NGIA_OK;
