@@ -5,6 +5,14 @@
 // sequences as representatives, every accepting one per query as a bit
 // mask).  The per-pair tests are the reference's (composition,
 // func.cu:323-354; short words, 357-447; banded LCS, 450-604).
+//
+// The filters queue the pairs of one representative in groups of 32 entries
+// that start at a multiple of 32, the last one padded: a warp of the
+// alignment kernel takes a group, so its lanes share the representative and
+// its match table lies in shared memory.  (With entries of several
+// representatives in a warp the table was read from global memory through
+// L1, several cache lines per load.  GB300, 20,000 DNA sequences to the end:
+// 313 -> 287 ms, 250 with remainder tiles of even width.)
 #pragma once
 #include <stdint.h>
 
@@ -13,12 +21,17 @@
 #include "common.cuh"
 #include "kmer.cuh"
 #include "tile.cuh"
+#include "wave.cuh"
 
 namespace ngia {
 namespace {
 
-constexpr int kServeClasses = 3;    // band windows <= 64 blocks, <= 128, wider
+// Pair classes: band windows <= 64 blocks, <= 128, wider, and queries of at
+// most kQueryRows blocks with a window above 64 (the query's blocks are the
+// rows then).
+constexpr int kServeClasses = 4;
 constexpr unsigned long long kNoRep = ~0ull;
+constexpr int kCtlWords = 16;  // RoundBufs::ctl
 
 // Device view of the resident representatives.
 struct RepStore {
@@ -29,48 +42,33 @@ struct RepStore {
   const uint32_t *lists;  // n x list_words k-mer bitsets (empty when net < 16)
   int32_t n, list_words;
   const int32_t *count;   // when set: the representatives in use (on the device, <= n)
-  const uint32_t *eq;     // DNA: match table of representative r at r * eq_stride (tile.cuh layout)
-  int64_t eq_stride;      // words per table: 4 x (largest plane blocks + kEqPad)
 };
-
-// DNA match tables (tile.cuh) of the representatives, one CTA each: four
-// words per plane block, zero from the representative's last block to the
-// end of its table.
-__global__ void k_rep_eq(RepStore rs, uint32_t *eq) {
-  const int r = blockIdx.x;
-  if (rs.count && r >= *rs.count) return;
-  const uint32_t *rec = rs.words + rs.off[r];
-  const int nb1 = ((int)rec[1] + 31) / 32;
-  const uint32_t *pl = rec + 6;  // DNA header words
-  uint4 *t = reinterpret_cast<uint4 *>(eq + (int64_t)r * rs.eq_stride);
-  const int blocks = (int)(rs.eq_stride / 4);
-  for (int j = threadIdx.x; j < blocks; j += blockDim.x) {
-    const bool real = j < nb1;
-    const uint32_t p0 = real ? pl[2 * j] : 0u, p1 = real ? pl[2 * j + 1] : 0u;
-    uint4 e;
-    e.x = real ? ~p0 & ~p1 : 0u;
-    e.y = p0 & ~p1;
-    e.z = ~p0 & p1;
-    e.w = p0 & p1;
-    t[j] = e;
-  }
-}
 
 // Buffers of the assignment rounds of one slot.
 struct RoundBufs {
-  int2 *queue[kServeClasses];  // (representative, query) pairs of a round
-  uint32_t *ctl;               // [0..2] pairs queued per class, [3..5] claimed, [6] queries left
+  int2 *queue[kServeClasses];  // (representative, query) pairs of a round, query -1 = padding
+  uint32_t *ctl;               // [0..3] entries queued per class (groups of 32), [4..7] claimed,
+                               // [8..11] pairs queued, [12] queries left, [13] error
   unsigned long long *key;     // per query: rep << 32 | score of the best accepting rep
   uint32_t *todo;              // bitmap of the queries not assigned yet
   unsigned long long *stats;   // [0] pairs aligned, [1] in-band cells computed
-  int64_t cap;                 // pairs per class queue
+  int64_t cap;                 // entries per class queue
   // mask form (speculative rounds): every accepting representative is kept
+  const int32_t *list;         // queries are positions in this list of sequences (null: sequences)
   unsigned long long *mask;    // per query: bit r = representative r accepts it
   int32_t *score;              // score of (r, q) at r * score_stride + q, for accepted pairs
   int64_t score_stride;
 };
+constexpr int kCtlClaimed = 4, kCtlPairs = 8, kCtlLeft = 12, kCtlErr = 13;
 
 __host__ __device__ inline int serve_class(int A) { return A <= 64 ? 0 : A <= 128 ? 1 : 2; }
+__host__ __device__ inline int round_class(int A, int L2) {
+  return A > 64 && L2 <= 32 * kQueryRows ? 3 : serve_class(A);
+}
+// Whether windows of up to max_nb blocks can put a pair in class c.
+__host__ __device__ inline bool serve_class_used(int c, int max_nb, bool rounds) {
+  return c == 0 || (max_nb > (c == 2 ? 128 : 64) && (c < 3 || rounds));
+}
 
 // k-mer presence bitset of every representative (the list of k_prep).
 template <int P>
@@ -98,10 +96,43 @@ __global__ void k_rep_lists(RepStore rs, int w, uint32_t *lists) {
   for (int i = threadIdx.x; i < lw; i += blockDim.x) lists[(int64_t)r * lw + i] = s_list[i];
 }
 
+// Queues the survivors of one representative r among n_res tested queries of
+// a CTA: s_res[k] = 0 or 1 + class of query q0 + k.  One reservation per class
+// (whole groups of 32), then the entries and the padding.  Every thread of the
+// CTA calls it after s_res and s_cnt (survivors per class) are complete.
+__device__ __forceinline__ void queue_groups(const RoundBufs &rb, int r, int q0, int n_res, const uint8_t *s_res,
+                                             const uint32_t *s_cnt, uint32_t *s_base, uint32_t *s_pos) {
+  if (threadIdx.x < kServeClasses) {
+    const uint32_t cnt = s_cnt[threadIdx.x], padded = (cnt + 31u) & ~31u;
+    uint32_t base = 0;
+    if (cnt) {
+      base = atomicAdd(&rb.ctl[threadIdx.x], padded);
+      atomicAdd(&rb.ctl[kCtlPairs + threadIdx.x], cnt);
+    }
+    s_base[threadIdx.x] = base;
+    s_pos[threadIdx.x] = 0;
+    for (uint32_t k = cnt; k < padded; k++)
+      if ((int64_t)base + k < rb.cap) rb.queue[threadIdx.x][(int64_t)base + k] = make_int2(r, -1);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int k0 = (threadIdx.x >> 5) * 32; k0 < n_res; k0 += blockDim.x) {
+    const int k = k0 + lane;
+    const int res = k < n_res ? s_res[k] : 0;
+    const unsigned pm = __ballot_sync(kFullMask, res != 0);
+    if (!res) continue;
+    const unsigned peers = __match_any_sync(pm, res);
+    const int leader = __ffs(peers) - 1;
+    uint32_t b = 0;
+    if (lane == leader) b = atomicAdd(&s_pos[res - 1], (uint32_t)__popc(peers));
+    b = __shfl_sync(peers, b, leader);
+    const int64_t slot = (int64_t)s_base[res - 1] + b + __popc(peers & ((1u << lane) - 1u));
+    if (slot < rb.cap) rb.queue[res - 1][slot] = make_int2(r, q0 + k);
+  }
+}
+
 // One CTA per representative of the chunk: composition test (and the
-// short-word test in word-first order) for every unassigned query; the
-// survivors are queued per class with one global atomic per class and CTA
-// (two passes over the queries: decide into shared memory, then write).
+// short-word test in word-first order) for every unassigned query.
 template <int P>
 __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int r0,
                                                       int word_first) {
@@ -111,7 +142,7 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
   const int r = r0 + blockIdx.x;
   const uint32_t *rec = rs.words + rs.off[r];
   if (threadIdx.x < A) s_rc[threadIdx.x] = rec[2 + threadIdx.x];
-  if (threadIdx.x < kServeClasses) s_cnt[threadIdx.x] = s_pos[threadIdx.x] = 0;
+  if (threadIdx.x < kServeClasses) s_cnt[threadIdx.x] = 0;
   __syncthreads();
   const int L1 = (int)rec[0], net1 = (int)rec[1], nb1 = (net1 + 31) / 32;
   const float s = prm.s;
@@ -127,7 +158,8 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
       // a smaller representative of this round may already hold q
       const bool open = (rb.key[q] >> 32) > (unsigned long long)r;
       const int L2 = __ldg(qdb.len + q);
-      bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cutoff_of(L2, s));
+      const int cut = cutoff_of(L2, s);
+      bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cut);
       if (pass && word_here) {
         const int net2 = __ldg(qdb.net + q);
         if (net2 >= 16) {
@@ -135,7 +167,7 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
           pass = !(word_count<P>(planes, net2, prm.w, rlist) < word_min(L2, prm.w, s));
         }
       }
-      if (pass) res = 1 + serve_class(window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1));
+      if (pass) res = 1 + serve_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1));
     }
     if (q < n) s_res[q] = (uint8_t)res;
     const unsigned pm = __ballot_sync(kFullMask, res != 0);
@@ -145,46 +177,52 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
     }
   }
   __syncthreads();
-  if (threadIdx.x < kServeClasses)
-    s_base[threadIdx.x] = s_cnt[threadIdx.x] ? atomicAdd(&rb.ctl[threadIdx.x], s_cnt[threadIdx.x]) : 0u;
-  __syncthreads();
-  for (int wi = warp; wi < nbw; wi += blockDim.x >> 5) {
-    const int q = wi * 32 + lane;
-    const int res = q < n ? s_res[q] : 0;
-    const unsigned pm = __ballot_sync(kFullMask, res != 0);
-    if (!res) continue;
-    const unsigned peers = __match_any_sync(pm, res);
-    const int leader = __ffs(peers) - 1;
-    uint32_t b = 0;
-    if (lane == leader) b = atomicAdd(&s_pos[res - 1], (uint32_t)__popc(peers));
-    b = __shfl_sync(peers, b, leader);
-    const int64_t slot = (int64_t)s_base[res - 1] + b + __popc(peers & ((1u << lane) - 1u));
-    if (slot < rb.cap) rb.queue[res - 1][slot] = make_int2(r, q);
+  queue_groups(rb, r, 0, n, s_res, s_cnt, s_base, s_pos);
+}
+
+// Whether the class's pairs of this round go to the group-per-pair kernel
+// (few pairs) or to the thread-per-pair kernel.
+__device__ __forceinline__ bool round_wave(const RoundBufs &rb, int cls, int wave_pairs) {
+  return rb.ctl[kCtlPairs + cls] <= (uint32_t)wave_pairs;
+}
+
+// A pair's score reached its cutoff.  MASK = false: the query's key keeps the
+// smallest accepting representative; MASK = true: one bit per representative.
+template <bool MASK>
+__device__ __forceinline__ void round_accept(const RoundBufs &rb, int r, int q, int sum) {
+  if (MASK) {
+    rb.score[(int64_t)r * rb.score_stride + q] = sum;
+    atomicOr(&rb.mask[q], 1ull << r);
+  } else {
+    atomicMin(&rb.key[q], ((unsigned long long)r << 32) | (uint32_t)sum);
   }
 }
 
-// The match table is read from global memory through L1 (copying it to
-// shared memory per warp, with the pairs grouped by representative, was
-// slower: 56.5k against 59.2k queries/s), and the per-column bookkeeping runs
-// on the FMA pipe as in the clustering kernel (64.3k against 58.9k).
+// Representatives of up to this many blocks (8,192 residues) have their DNA
+// match table in the warp's shared memory; longer ones are matched from their
+// planes (one more operation per word).
+constexpr int kRoundTable = 256;
+__host__ __device__ constexpr int round_table_blocks(int max_nb) {
+  return (max_nb < kRoundTable ? max_nb : kRoundTable) + kEqPad;
+}
 
-// Banded LCS of the queued (representative, query) pairs of one class: the
-// loop of k_align_tiled (align.cu) with the representative taken per pair.
-// MASK = false: first match (rb.key keeps the smallest accepting rep per
-// query, pairs of larger reps are skipped once a smaller one accepted);
-// MASK = true: every pair runs and an accepted one sets bit r of rb.mask[q]
-// and its score.
-template <int P, int RING, bool MASK>
+// Banded LCS of the queued pairs of one class, one thread per pair: the loop
+// of k_align_tiled (align.cu) with a warp's 32 entries sharing their
+// representative.  Class 3: the query's blocks are the rows and the
+// representative's residues the columns (the band is symmetric), always from
+// the planes.
+template <int P, int RING, bool MASK, bool QROWS>
 __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
-    k_serve_align(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int word_after, uint32_t *scratch,
-                  int64_t scratch_words, uint32_t ring_mask) {
+    k_round_align(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int word_after, int wave_pairs,
+                  uint32_t *scratch, int64_t scratch_words, uint32_t ring_mask, int table_blocks) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint32_t s_qn;
-  if (threadIdx.x == 0) s_qn = (int64_t)rb.ctl[cls] < rb.cap ? rb.ctl[cls] : (uint32_t)rb.cap;
+  if (threadIdx.x == 0) s_qn = round_wave(rb, cls, wave_pairs) ? 0u : (uint32_t)min((int64_t)rb.ctl[cls], rb.cap);
   __syncthreads();
   const uint32_t qn = s_qn;
   if (qn == 0) return;
-  typename RingOf<RING>::T ring;
+  using Ring = typename RingOf<RING>::T;
+  Ring ring;
   if constexpr (RING > 0) {
     ring.base = smem + threadIdx.x;
   } else {
@@ -194,6 +232,10 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     ring.mask = ring_mask;
     ring.stride = TL;
   }
+  constexpr bool kTable = P == 2 && !QROWS;
+  uint32_t *w_eq = smem + RING * kAlignThreads + (threadIdx.x >> 5) * 4 * table_blocks;  // this warp's match table
+  const uint32_t w_eq_s = smem_u32(w_eq);
+  (void)w_eq_s;
   // 1 and 4 as values ptxas cannot fold (the FMA-pipe bookkeeping of tile.cuh)
   const uint32_t one_rt = 1u + (uint32_t)(qn == 0u);
   const FmaK fk{one_rt, one_rt << 2};
@@ -201,167 +243,133 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   const int lane = threadIdx.x & 31;
   const float s = prm.s;
   const int hw = qdb.hw;
-  int state = -1;  // -1 idle, -2 queue exhausted, >= 0 a claimed entry (waiting or running)
-  int r = 0, q = 0, i = 0, nq = 0, B = 0, js = 0, je = -1, net1 = 0, nb1 = 0, net2 = 0, L2 = 0, cutoff = 0;
-  int lastcols = 32, frozen = 0, zw = 0;
-  uint32_t vlast = 0;
-  bool active = false;
-  const uint32_t *qpl = nullptr, *rpl = nullptr;
-  uint32_t cur[P], nxt[P];
+  constexpr int MT = tiled_main(P);
   unsigned long long n_pairs = 0, n_cells = 0;
-  // every loop pass advances a running lane by one query block or claims:
-  // bounded by the queued pairs' blocks (each at most kMaxBlocks), per warp
-  const long long guard_max = ((long long)qn + 64) * (kMaxBlocks + 36);
-  long long guard = 0;
+  int staged = -1, L1 = 0, net1 = 0, nb1 = 0;  // the warp's representative
+  const uint32_t *rpl = nullptr;
+  bool table = false;
   for (;;) {
-    if (++guard > guard_max) {
-      if (lane == 0) atomicExch(&rb.ctl[7], 1u);
-      break;
-    }
-    {  // refill once prm.refill lanes are idle or none holds a pair (as in
-       // k_align_tiled); the warp votes run on all 32 lanes before they are
-       // combined per lane
-      const bool any_held = __any_sync(kFullMask, state >= 0);
-      const unsigned idle = __ballot_sync(kFullMask, state == -1);
-      const bool refill_now = !any_held || __popc(idle) >= prm.refill;
-      const bool need = state == -1 && refill_now;
-      const unsigned nm = __ballot_sync(kFullMask, need);
-      if (nm) {
-        const int leader = __ffs(nm) - 1;
-        uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(&rb.ctl[3 + cls], (uint32_t)__popc(nm));
-        base = __shfl_sync(kFullMask, base, leader);
-        if (need) {
-          const uint32_t idx = base + (uint32_t)__popc(nm & ((1u << lane) - 1u));
-          state = idx < qn ? (int)idx : -2;
-          if (state >= 0) {
-            const int2 e = rb.queue[cls][state];
-            r = e.x;
-            q = e.y;
-          }
-        }
-      }
-    }
-    if (__all_sync(kFullMask, state == -2)) break;
-    const bool start = state >= 0 && !active;
-    if (start) {
+    uint32_t e0 = 0;
+    if (lane == 0) e0 = atomicAdd(&rb.ctl[kCtlClaimed + cls], 32u);
+    e0 = __shfl_sync(kFullMask, e0, 0);
+    if (e0 >= qn) break;
+    const int2 e = rb.queue[cls][e0 + lane];
+    const int r = __shfl_sync(kFullMask, e.x, 0), q = e.y;
+    if (r != staged) {
       const uint32_t *rrec = rs.words + rs.off[r];
-      const int L1 = (int)rrec[0];
+      L1 = (int)rrec[0];
       net1 = (int)rrec[1];
       nb1 = (net1 + 31) >> 5;
       rpl = rrec + hw;
-      vlast = (net1 & 31) ? ((1u << (net1 & 31)) - 1u) : 0xFFFFFFFFu;
-      L2 = __ldg(qdb.len + q);
-      net2 = __ldg(qdb.net + q);
-      nq = (net2 + 31) >> 5;
-      lastcols = (net2 & 31) ? (net2 & 31) : 32;
+      staged = r;
+      if constexpr (kTable) {
+        table = nb1 + kEqPad <= table_blocks;
+        if (table) {
+          __syncwarp();
+          for (int j = lane; j < nb1 + kEqPad; j += 32) {
+            const bool real = j < nb1;
+            const uint32_t p0 = real ? rpl[2 * j] : 0u, p1 = real ? rpl[2 * j + 1] : 0u;
+            *reinterpret_cast<uint4 *>(w_eq + 4 * j) =
+                make_uint4(real ? ~p0 & ~p1 : 0u, p0 & ~p1, ~p0 & p1, p0 & p1);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    // rows (their planes rp, blocks nbr, residues nr) and columns (cp, nqc, nc)
+    int L2 = 0, net2 = 0, B = 0, cutoff = 0;
+    const uint32_t *qpl = nullptr;
+    bool active = false;
+    if (q >= 0 && (MASK || (rb.key[q] >> 32) > (unsigned long long)r)) {  // else a smaller representative holds q
+      const int x = MASK ? rb.list[q] : q;
+      L2 = __ldg(qdb.len + x);
+      net2 = __ldg(qdb.net + x);
       B = band_blocks(L1, L2, s);
       cutoff = cutoff_of(L2, s);
-      qpl = qdb.words + __ldg(qdb.off + q) + hw;
-      i = 0;
-      js = 0;
-      je = band_first_top(B, nb1, net1, cutoff);
-      frozen = 0;
-      zw = 0;
-      if (!MASK && (rb.key[q] >> 32) < (unsigned long long)r) {
-        state = -1;  // a smaller representative already holds q
-      } else if (B < 0 || je < 0 || nq == 0) {
-        if (!(0 < cutoff)) {
-          if (MASK) {
-            rb.score[(int64_t)r * rb.score_stride + q] = 0;
-            atomicOr(&rb.mask[q], 1ull << r);
-          } else {
-            atomicMin(&rb.key[q], (unsigned long long)r << 32);
+      qpl = qdb.words + __ldg(qdb.off + x) + hw;
+      active = B >= 0 && nb1 > 0 && net2 > 0;
+      if (!active && !(0 < cutoff)) round_accept<MASK>(rb, r, q, 0);  // no band: score 0
+    }
+    const uint32_t *rp = QROWS ? qpl : rpl, *cp = QROWS ? rpl : qpl;
+    const int nr = QROWS ? net2 : net1, nbr = (nr + 31) >> 5;
+    const int nc = QROWS ? net1 : net2, ncb = (nc + 31) >> 5;
+    const uint32_t vlast = (nr & 31) ? ((1u << (nr & 31)) - 1u) : 0xFFFFFFFFu;
+    int i = 0, js = 0, je = 0, frozen = 0, zw = 0;
+    uint32_t cur[P], nxt[P];
+    if (active) {
+      n_pairs++;
+      je = band_first_top(B, nbr, nr, cutoff);
+      for (int j = 0; j <= je; j++) ring[j] = 0xFFFFFFFFu;
+#pragma unroll
+      for (int p = 0; p < P; p++) cur[p] = __ldg(cp + p);
+    }
+    // the group's lanes in step, one column block at a time (at most kMaxBlocks)
+    while (__any_sync(kFullMask, active)) {
+      const int n = active ? je - js + 1 : 0;
+      const int full = (int)__reduce_min_sync(kFullMask, active ? (unsigned)(n / MT) : 0xFFFFFFFFu);
+      int rem = (int)__reduce_max_sync(kFullMask, active ? (unsigned)(n - MT * full) : 0u);
+      if (!active) continue;
+      const int cols = min(32, nc - 32 * i);
+      n_cells += (unsigned long long)n * cols * 32;
+      if (i + 1 < ncb) {
+#pragma unroll
+        for (int p = 0; p < P; p++) nxt[p] = __ldg(cp + (i + 1) * P + p);
+      }
+      uint32_t cw = 0, ncw = 0;
+      int base = js;
+      if (kTable && table) {
+        if constexpr (kTable) {
+          uint32_t wc[2];
+          eq_codes_top(cur, wc);
+          zw = 0;  // the tiles return their rows' zero counts
+          for (int t = 0; t < full; t++, base += MT) {
+            zw += tiled_tile_eqf<MT, NGIA_SERVE_PF, Ring>(ring, w_eq_s, base, je, nbr, cols, wc, cw, ncw, fk);
+            cw = ncw << (32 - cols);
+            ncw = 0;
           }
+          for (; rem >= MT; rem -= MT, base += MT) {
+            zw += tiled_tile_eqf<MT, NGIA_SERVE_PF, Ring>(ring, w_eq_s, base, je, nbr, cols, wc, cw, ncw, fk);
+            cw = ncw << (32 - cols);
+            ncw = 0;
+          }
+          if (rem > 0) zw += tiled_rem_eqf<Ring>(rem, ring, w_eq_s, base, je, nbr, cols, wc, cw, ncw, fk);
         }
-        state = -1;
       } else {
-        for (int j = 0; j <= je; j++) ring[j] = 0xFFFFFFFFu;
-#pragma unroll
-        for (int p = 0; p < P; p++) cur[p] = __ldg(qpl + p);
-        active = true;
-        n_pairs++;
+        for (int t = 0; t < full; t++, base += MT) {
+          zw += tiled_tile<P, MT, Ring>(ring, rp, base, je, cols, cur, cw, ncw);
+          cw = ncw << (32 - cols);
+          ncw = 0;
+        }
+        for (; rem >= MT; rem -= MT, base += MT) {
+          zw += tiled_tile<P, MT, Ring>(ring, rp, base, je, cols, cur, cw, ncw);
+          cw = ncw << (32 - cols);
+          ncw = 0;
+        }
+        if (rem > 0) zw += tiled_rem<P, Ring, MT>(rem, ring, rp, base, je, cols, cur, cw, ncw);
       }
-    }
-    const bool busy = active;
-    constexpr int MT = tiled_main(P);
-    const int n = busy ? je - js + 1 : 0;
-    const int full = (int)__reduce_min_sync(kFullMask, busy ? (unsigned)(n / MT) : 0xFFFFFFFFu);
-    int rem = (int)__reduce_max_sync(kFullMask, busy ? (unsigned)(n - MT * full) : 0u);
-    if (!busy) continue;
-    const int cols = (i == nq - 1) ? lastcols : 32;
-    n_cells += (unsigned long long)n * cols * 32;
-    if (i + 1 < nq) {
-#pragma unroll
-      for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + (i + 1) * P + p);
-    }
-    using Ring = typename RingOf<RING>::T;
-    if constexpr (P == 2) {
-      // match words from the pair's representative's table (global memory,
-      // L1), the per-column bookkeeping on the FMA pipe as in k_align_tiled
-      const uint64_t req = (uint64_t)(rs.eq + (int64_t)r * rs.eq_stride);
-      uint32_t wc[2];
-      eq_codes_top(cur, wc);
-      uint32_t cw = 0, ncw = 0;
-      int base = js;
-      zw = 0;  // the tiles return their rows' zero counts
-      for (int t = 0; t < full; t++, base += MT) {
-        zw += tiled_tile_eqfg<MT, NGIA_SERVE_PF, Ring>(ring, req, base, je, nb1, cols, wc, cw, ncw, fk);
-        cw = ncw << (32 - cols);
-        ncw = 0;
+      i++;
+      bool finished = i >= ncb;
+      if (!finished) {
+        const int step = band_advance(ring, i, B, nbr, nr, vlast, nc - 32 * i, cutoff, js, je, frozen, zw);
+        if (step == kBandReject) {
+          active = false;
+          continue;
+        }
+        finished = step == kBandDone;
       }
-      for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile_eqfg<MT, NGIA_SERVE_PF, Ring>(ring, req, base, je, nb1, cols, wc, cw, ncw, fk);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      if (rem > 0) zw += tiled_rem_eqfg<Ring>(rem, ring, req, base, je, nb1, cols, wc, cw, ncw, fk);
-    } else {
-      uint32_t cw = 0, ncw = 0;
-      int base = js;
-      for (int t = 0; t < full; t++, base += MT) {
-        zw += tiled_tile<P, MT, Ring>(ring, rpl, base, je, cols, cur, cw, ncw);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile<P, MT, Ring>(ring, rpl, base, je, cols, cur, cw, ncw);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      if (rem > 0) zw += tiled_rem<P, Ring, MT>(rem, ring, rpl, base, je, cols, cur, cw, ncw);
-    }
-    i++;
-    bool finished = i >= nq;
-    if (!finished) {
-      const int step = band_advance(ring, i, B, nb1, net1, vlast, net2 - 32 * i, cutoff, js, je, frozen, zw);
-      if (step == kBandReject) {
+      if (finished) {
+        int sum = frozen;
+        for (int j = js; j <= je; j++) sum += __popc(~ring[j] & (j == nbr - 1 ? vlast : 0xFFFFFFFFu));
+        bool pass = !(sum < cutoff);
+        if (pass && word_after && net1 >= 16 && net2 >= 16)
+          pass = !(word_count<P>(qpl, net2, prm.w, rs.lists + (int64_t)r * rs.list_words) < word_min(L2, prm.w, s));
+        if (pass) round_accept<MASK>(rb, r, q, sum);
         active = false;
-        state = -1;
         continue;
       }
-      finished = step == kBandDone;
-    }
-    if (finished) {
-      int sum = frozen;
-      for (int j = js; j <= je; j++) sum += __popc(~ring[j] & (j == nb1 - 1 ? vlast : 0xFFFFFFFFu));
-      bool pass = !(sum < cutoff);
-      if (pass && word_after && net1 >= 16 && net2 >= 16)
-        pass = !(word_count<P>(qpl, net2, prm.w, rs.lists + (int64_t)r * rs.list_words) < word_min(L2, prm.w, s));
-      if (pass) {
-        if (MASK) {
-          rb.score[(int64_t)r * rb.score_stride + q] = sum;
-          atomicOr(&rb.mask[q], 1ull << r);
-        } else {
-          atomicMin(&rb.key[q], ((unsigned long long)r << 32) | (uint32_t)sum);
-        }
-      }
-      active = false;
-      state = -1;
-      continue;
-    }
 #pragma unroll
-    for (int p = 0; p < P; p++) cur[p] = nxt[p];
+      for (int p = 0; p < P; p++) cur[p] = nxt[p];
+    }
   }
   for (int o = 16; o; o >>= 1) {
     n_pairs += __shfl_down_sync(kFullMask, n_pairs, o);
@@ -373,35 +381,231 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   }
 }
 
-using AlignServeFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, uint32_t *, int64_t, uint32_t);
-
-template <bool MASK>
-AlignServeFn serve_align_fn(int type, int cls) {
-  if (type == 0)
-    return cls == 0 ? k_serve_align<2, 64, MASK> : cls == 1 ? k_serve_align<2, 128, MASK> : k_serve_align<2, 0, MASK>;
-  return cls == 0 ? k_serve_align<5, 64, MASK> : cls == 1 ? k_serve_align<5, 128, MASK> : k_serve_align<5, 0, MASK>;
+// The same for classes with few pairs, a group of threads per pair (wave.cuh).
+// NW 1 or 4: rows are the representative's; NW 0: 16 threads per pair, the
+// query's blocks as rows.  A CTA takes as many neighbouring entries as it has
+// groups: they share their representative.
+// Shared memory: match table | code rings, or rep codes | match tables.
+template <int P, int NW, int WMAX, bool MASK>
+__global__ void __launch_bounds__(kAlignThreads)
+    k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int word_after, int wave_pairs,
+                 int cap_blocks) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  constexpr bool kQ = NW == 0;
+  constexpr int GS = kQ ? kQueryGroup : 32 * NW, kGroups = kAlignThreads / GS;
+  __shared__ uint32_t s_xch[kQ ? 1 : 4 * NW];
+  __shared__ uint32_t s_qn;
+  if (threadIdx.x == 0) s_qn = round_wave(rb, cls, wave_pairs) ? (uint32_t)min((int64_t)rb.ctl[cls], rb.cap) : 0u;
+  __syncthreads();
+  const uint32_t qn = s_qn;
+  const int group = threadIdx.x / GS;
+  const bool lead = threadIdx.x % GS == 0;
+  const float s = prm.s;
+  const int hw = qdb.hw, lane = threadIdx.x & 31;
+  unsigned long long n_pairs = 0, n_cells = 0;
+  int staged = -1, L1 = 0, net1 = 0, nb1 = 0;
+  for (uint32_t e0 = blockIdx.x * kGroups; e0 < qn; e0 += gridDim.x * kGroups) {
+    const int2 first = rb.queue[cls][e0];  // entries of one group: the padding comes last
+    if (first.y < 0) continue;             // CTA-uniform
+    const int r = first.x;
+    if (r != staged) {
+      __syncthreads();  // every group is through with the last representative
+      const uint32_t *rrec = rs.words + rs.off[r];
+      L1 = (int)rrec[0];
+      net1 = (int)rrec[1];
+      nb1 = (net1 + 31) >> 5;
+      const uint32_t vlast = (net1 & 31) ? ((1u << (net1 & 31)) - 1u) : 0xFFFFFFFFu;
+      if constexpr (kQ) {
+        for (int b = threadIdx.x; b < nb1; b += kAlignThreads) {
+          uint32_t pl[P];
+#pragma unroll
+          for (int p = 0; p < P; p++) pl[p] = rrec[hw + b * P + p];
+          wave_unpack<P>(pl, reinterpret_cast<uint4 *>(smem) + 2 * b);
+        }
+      } else {
+        wave_table<P>(rrec + hw, nb1, vlast, smem, threadIdx.x, kAlignThreads);
+      }
+      __syncthreads();
+      staged = r;
+    }
+    const int2 e = rb.queue[cls][e0 + group];
+    const int q = e.y;
+    int L2 = 0, net2 = 0, nq = 0, B = 0, cutoff = 1, lo = 0, hi = 0, sum = 0;
+    const uint32_t *qpl = qdb.words;
+    // (a key can change while the group's threads look at it: one answer)
+    bool have = q >= 0 && (MASK || (rb.key[q] >> 32) > (unsigned long long)r), run = false;
+    if constexpr (!MASK) {
+      if constexpr (NW == 4)
+        have = __syncthreads_or(have) != 0;
+      else
+        have = __shfl_sync(kFullMask, (int)have, 0, GS) != 0;
+    }
+    if (have) {
+      const int x = MASK ? rb.list[q] : q;
+      L2 = __ldg(qdb.len + x);
+      net2 = __ldg(qdb.net + x);
+      nq = (net2 + 31) >> 5;
+      B = band_blocks(L1, L2, s);
+      cutoff = cutoff_of(L2, s);
+      qpl = qdb.words + __ldg(qdb.off + x) + hw;
+      if (B >= 0 && nb1 > 0 && nq > 0) {
+        run = wave_band(B, net1, net2, cutoff, lo, hi);
+        have = run;
+        if (lead) n_pairs++;
+      }
+    }
+    unsigned long long cells = 0;
+    if constexpr (kQ) {
+      uint32_t *tab = smem + 8 * cap_blocks + (threadIdx.x >> 5) * 32 * wave_codes(P);
+      const int got = wave_query<P>(smem, nb1, net1, qpl, run ? nq : 0, net2, lo, hi, tab, cells);
+      if (run) sum = got;
+    } else if (run) {  // uniform in the group
+      uint32_t *ring = smem + wave_table_words(P, cap_blocks) + group * kWaveRingWords;
+      sum = wave_any<P, NW, WMAX>(smem, nb1, qpl, nq, net2, lo, hi, cutoff, ring, s_xch, cells);
+    }
+    n_cells += 32 * cells;
+    bool pass = have && !(sum < cutoff);
+    if (word_after && net1 >= 16) {  // short-word test (func.cu:376-396), a warp per member
+      const uint32_t *list = rs.lists + (int64_t)r * rs.list_words;
+#pragma unroll
+      for (int k = 0; k < (kQ ? 2 : 1); k++) {
+        const int src = k * kQueryGroup;
+        if (!__shfl_sync(kFullMask, (int)(pass && net2 >= 16), src)) continue;
+        const uint32_t *qp = reinterpret_cast<const uint32_t *>(__shfl_sync(kFullMask, (unsigned long long)qpl, src));
+        const int n2 = __shfl_sync(kFullMask, net2, src);
+        const int ws = word_count_warp_bits<P>(qp, n2, prm.w, list);
+        if (!kQ || lane / kQueryGroup == k) pass = !(ws < word_min(L2, prm.w, s));
+      }
+    }
+    if (pass && lead) round_accept<MASK>(rb, r, q, sum);
+  }
+  for (int o = 16; o; o >>= 1) {
+    n_pairs += __shfl_down_sync(kFullMask, n_pairs, o);
+    n_cells += __shfl_down_sync(kFullMask, n_cells, o);
+  }
+  if (lane == 0 && (n_pairs || n_cells)) {
+    atomicAdd(&rb.stats[0], n_pairs);
+    atomicAdd(&rb.stats[1], n_cells);
+  }
 }
 
-// Dynamic shared memory of class cls: the row ring (shared classes).
-inline size_t serve_align_smem(int cls) { return cls == 2 ? 0 : (size_t)(cls == 0 ? 64 : 128) * kAlignThreads * 4; }
+// ---- launch ---------------------------------------------------------------------
+using RoundAlignFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, uint32_t *, int64_t, uint32_t, int);
+using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, int);
 
-// Raises the kernel's dynamic shared memory limit to `bytes` (never lowers
-// it: launches of other open servers or contexts may need more).
+template <int P, bool MASK>
+RoundAlignFn round_align_fn(int cls) {
+  switch (cls) {
+    case 0: return k_round_align<P, 64, MASK, false>;
+    case 1: return k_round_align<P, 128, MASK, false>;
+    case 2: return k_round_align<P, 0, MASK, false>;
+    default: return k_round_align<P, 64, MASK, true>;
+  }
+}
+template <int P, bool MASK>
+RoundWaveFn round_wave_fn(int cls) {
+  switch (cls) {
+    case 0: return k_round_wave<P, 1, 2, MASK>;
+    case 1: return k_round_wave<P, 4, 1, MASK>;
+    case 2: return k_round_wave<P, 4, 16, MASK>;
+    default: return k_round_wave<P, 0, 1, MASK>;
+  }
+}
+inline int round_wave_groups(int cls) { return cls == 0 ? 4 : cls == 3 ? kAlignThreads / kQueryGroup : 1; }
+
+inline size_t round_align_smem(int type, int cls, int rep_nb) {
+  const size_t ring = cls == 2 ? 0 : (size_t)(cls == 1 ? 128 : 64) * kAlignThreads;
+  const size_t table = type == 0 && cls != 3 ? (size_t)(kAlignThreads / 32) * 4 * (size_t)round_table_blocks(rep_nb) : 0;
+  return 4 * (ring + table);
+}
+inline size_t round_wave_smem(int type, int cls, int rep_nb) {
+  const int P = type ? 5 : 2;
+  return 4 * (cls == 3 ? 8 * (size_t)rep_nb + kAlignThreads * wave_codes(P)
+                       : (size_t)wave_table_words(P, rep_nb) + (size_t)round_wave_groups(cls) * kWaveRingWords);
+}
+
+// The alignment launches of a round: shapes for representatives of up to
+// rep_nb blocks, and per class the pairs up to which a group per pair is
+// faster (0: its kernel does not fit).
+struct RoundPlan {
+  int type = 0, rep_nb = 1;
+  int grid[kServeClasses] = {0, 0, 0, 0}, wave_grid[kServeClasses] = {0, 0, 0, 0};
+  int wave_pairs[kServeClasses] = {0, 0, 0, 0};
+  uint32_t *scratch = nullptr;  // global ring of class 2
+  int64_t scratch_words = 0;
+  uint32_t ring_mask = 0;
+};
+
 template <bool MASK>
-cudaError_t serve_align_configure(int type, int cls, size_t bytes) {
+const void *round_fn(int type, int cls, bool wave) {
+  if (wave) return type == 0 ? (const void *)round_wave_fn<2, MASK>(cls) : (const void *)round_wave_fn<5, MASK>(cls);
+  return type == 0 ? (const void *)round_align_fn<2, MASK>(cls) : (const void *)round_align_fn<5, MASK>(cls);
+}
+
+// Kernel attributes (the dynamic shared memory limit only grows: launches of
+// other open servers or contexts may need more) and grids.  The scratch is the
+// caller's to allocate (scratch_words) and free.
+template <bool MASK>
+cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
   static std::mutex mu;
-  static size_t have[64][2][kServeClasses] = {};
+  static size_t have[64][2][2][kServeClasses] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  pl.type = type;
+  pl.rep_nb = rep_nb;
   std::lock_guard<std::mutex> lock(mu);
-  size_t &h = have[dev][type ? 1 : 0][cls];
-  if (bytes <= h) return cudaSuccess;
-  e = cudaFuncSetAttribute((const void *)serve_align_fn<MASK>(type, cls), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)bytes);
-  if (e == cudaSuccess) h = bytes;
-  return e;
+  for (int c = 0; c < kServeClasses; c++)
+    for (int wave = 0; wave < 2; wave++) {
+      const void *fn = round_fn<MASK>(type, c, wave != 0);
+      const size_t bytes = wave ? round_wave_smem(type, c, rep_nb) : round_align_smem(type, c, rep_nb);
+      if (wave && bytes > 226 * 1024) continue;  // wave_pairs stays 0: a thread per pair
+      size_t &h = have[dev][type ? 1 : 0][wave][c];
+      if (bytes > h) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+        h = bytes;
+      }
+      int occ = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kAlignThreads, bytes) != cudaSuccess || occ < 1) occ = 1;
+      (wave ? pl.wave_grid : pl.grid)[c] = num_sms * occ;
+      // the clustering kernels' cut-off (api.cu)
+      if (wave) pl.wave_pairs[c] = 56 * num_sms;
+    }
+  uint32_t ring = 1;
+  while ((int)ring < rep_nb) ring <<= 1;
+  pl.ring_mask = ring - 1;
+  pl.scratch_words = serve_class_used(2, rep_nb, MASK) ? (int64_t)pl.grid[2] * kAlignThreads * ring : 1;
+  return cudaSuccess;
+}
+
+// Launches both kernels of every class the representatives' lengths allow;
+// the round's pair counts decide on the device which of the two works.
+template <bool MASK>
+cudaError_t round_launch(const RoundPlan &pl, const DevDB &qdb, const RepStore &rs, const RunParams &prm,
+                         const RoundBufs &rb, int word_after, cudaStream_t st) {
+  for (int c = 0; c < kServeClasses; c++) {
+    if (!serve_class_used(c, pl.rep_nb, MASK)) continue;
+    DevDB db = qdb;
+    RepStore r = rs;
+    RunParams p = prm;
+    RoundBufs b = rb;
+    int cls = c, wa = word_after, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb;
+    uint32_t *scr = pl.scratch;
+    int64_t sw = pl.scratch_words;
+    uint32_t rm = pl.ring_mask;
+    void *args[] = {&db, &r, &p, &b, &cls, &wa, &wp, &scr, &sw, &rm, &tb};
+    cudaError_t e = cudaLaunchKernel(round_fn<MASK>(pl.type, c, false), dim3(pl.grid[c]), dim3(kAlignThreads), args,
+                                     round_align_smem(pl.type, c, pl.rep_nb), st);
+    if (e != cudaSuccess) return e;
+    if (wp <= 0) continue;
+    void *wargs[] = {&db, &r, &p, &b, &cls, &wa, &wp, &cap};
+    e = cudaLaunchKernel(round_fn<MASK>(pl.type, c, true), dim3(pl.wave_grid[c]), dim3(kAlignThreads), wargs,
+                         round_wave_smem(pl.type, c, pl.rep_nb), st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace

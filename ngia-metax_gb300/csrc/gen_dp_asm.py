@@ -21,7 +21,7 @@ Run `python gen_dp_asm.py` after editing; the output is committed.
 """
 from pathlib import Path
 
-PLANES = (5,)
+PLANES = (2, 5)
 WIDTHS = tuple(range(1, 17))
 
 

@@ -6,8 +6,8 @@
 //
 // Resident state (ngia_serve_open): the representatives as a device
 // database (records and header arrays, loaded by the same loader as
-// ngia_open) plus one k-mer bitset and, for DNA, one match table per
-// representative, built on the device.  The per-pair kernels are shared with
+// ngia_open) plus one k-mer bitset per representative, built on the device.
+// The per-pair kernels are shared with
 // the speculative rounds (assign.cuh).
 //
 // One batch runs on one slot — a context of fixed capacity with its own
@@ -16,8 +16,8 @@
 //     (64, 128, ... doubling up to 1,024): k_serve_filter tests every unassigned
 //     query against every representative of the chunk (composition, and the
 //     short-word test when it goes first) and queues the surviving pairs by
-//     band-window width; k_serve_align runs the banded LCS of each pair with
-//     the tiled register update (tile.cuh, lanes in lockstep) and keeps per
+//     band-window width in groups of one representative; k_round_align (or,
+//     for few pairs, k_round_wave) runs the banded LCS and keeps per
 //     query the smallest accepting representative with its score (one 64-bit
 //     atomicMin of rep << 32 | score); k_serve_round_end drops assigned
 //     queries and counts the rest.  A later round only holds later
@@ -58,6 +58,7 @@ namespace {
 
 constexpr int kFirstChunk = 64;     // representatives in the first round
 constexpr int kMaxChunk = 1024;     // ... doubling up to this many per round
+constexpr int64_t kFirstPairs = 1 << 16, kMaxPairs = 1 << 18;  // pairs a round takes more representatives for
 
 __global__ void k_serve_init(int n, RoundBufs rb) {
   const int nbw = (n + 31) / 32;
@@ -84,7 +85,7 @@ __global__ void k_serve_round_end(int n, RoundBufs rb) {
     left += __popc(bits);
   }
   for (int o = 16; o; o >>= 1) left += __shfl_xor_sync(kFullMask, left, o);
-  if ((threadIdx.x & 31) == 0 && left) atomicAdd(&rb.ctl[6], left);
+  if ((threadIdx.x & 31) == 0 && left) atomicAdd(&rb.ctl[kCtlLeft], left);
 }
 
 // NGIA_SERVE_TRACE=1 prints the phases of every batch to stderr.
@@ -146,9 +147,7 @@ struct Slot {
   uint32_t *h_ctl = nullptr;                  // pinned
   unsigned long long *h_key = nullptr;        // pinned, cap_n
   unsigned long long *h_stats = nullptr;      // pinned, 2
-  uint32_t *scratch = nullptr;
-  int64_t scratch_words = 0;
-  int grid[kServeClasses] = {0, 0, 0};
+  RoundPlan plan;
   std::vector<int32_t> cl, id;
   std::thread worker;
 };
@@ -163,11 +162,9 @@ struct ngia_server {
   int word_first = 0;
   ngia_ctx *reps = nullptr;  // the resident representatives' database
   uint32_t *d_lists = nullptr;
-  uint32_t *d_eq = nullptr;  // DNA match tables of the representatives
   ngia::RepStore store{};
   int64_t cap_n = 0, cap_words = 0;
   int32_t cap_nb = 0;
-  uint32_t ring_mask = 0;
   std::vector<std::unique_ptr<ngia::Slot>> slots;
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
@@ -205,25 +202,32 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
   k_serve_init<<<std::max(1, std::min(c->num_sms, (n + 255) / 256)), 256, 0, st>>>(n, rb);
   CKS(cudaGetLastError());
   const int word_after = !sv->word_first && !sv->prm.precise;
-  // largest round (NGIA_SERVE_MAX_CHUNK, at most kMaxChunk, which sizes the
-  // slot's pair queues): a query accepted by a representative of a round can
-  // still have its pairs with the round's later representatives aligned.
-  // Swept on GB300 (200 DNA query batches, 14,077 representatives): 1,024,
-  // 512, 256 and 128 aligned 300.2M, 299.3M, 298.5M and 298.0M pairs at
-  // 53.1k, 53.0k, 52.3k and 51.3k queries/s: nearly every pair is one the
-  // first-match rule needs.
+  // Representatives per round: kFirstChunk doubling up to kMaxChunk, and more
+  // while the unassigned queries are few, so that a round holds at least
+  // kFirstPairs (later kMaxPairs) pairs: a round takes a pair's latency
+  // however few there are (24 queries against 6,000 representatives: 9 rounds
+  // of 290 us, now 2; the batch 5.2 -> 1.4 ms).  A query accepted by a representative of a round can
+  // still have its pairs with the round's later representatives aligned:
+  // chunks of 1,024, 512, 256 and 128 aligned 300.2M, 299.3M, 298.5M and
+  // 298.0M pairs (200 DNA query batches, 14,077 representatives), so nearly
+  // every pair is one the first-match rule needs.  NGIA_SERVE_MAX_CHUNK lowers
+  // the largest round.
   static const int max_chunk = [] {
     const char *m = getenv("NGIA_SERVE_MAX_CHUNK");
-    return m ? std::max(kFirstChunk, std::min(kMaxChunk, atoi(m))) : kMaxChunk;
+    return m ? std::max(kFirstChunk, std::min(kMaxChunk, atoi(m))) : INT_MAX;
   }();
-  int r0 = 0, chunk = std::min(kFirstChunk, max_chunk);
+  int r0 = 0, chunk = kFirstChunk;
+  int64_t pairs = kFirstPairs;
   uint32_t left = (uint32_t)n;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   if (trace())
     for (auto &e : ev) cudaEventCreate(&e);
   while (r0 < sv->store.n && left > 0) {
-    const int nr = std::min(chunk, sv->store.n - r0);
-    CKS(cudaMemsetAsync(rb.ctl, 0, 8 * sizeof(uint32_t), st));
+    // at most the queue's capacity: a representative's entries pad to 32
+    const int64_t fit = rb.cap / (((int64_t)left + 31) & ~31ll);
+    const int64_t want = std::min<int64_t>({std::max<int64_t>(chunk, pairs / left), fit, (int64_t)max_chunk});
+    const int nr = (int)std::min<int64_t>(want, sv->store.n - r0);
+    CKS(cudaMemsetAsync(rb.ctl, 0, kCtlWords * sizeof(uint32_t), st));
     if (ev[0]) cudaEventRecord(ev[0], st);
     if (sv->type == 0)
       k_serve_filter<2><<<nr, 256, (size_t)nbw * 32, st>>>(c->db, sv->store, sv->prm, rb, r0, sv->word_first);
@@ -231,42 +235,32 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
       k_serve_filter<5><<<nr, 256, (size_t)nbw * 32, st>>>(c->db, sv->store, sv->prm, rb, r0, sv->word_first);
     CKS(cudaGetLastError());
     if (ev[1]) cudaEventRecord(ev[1], st);
-    for (int k = 0; k < kServeClasses; k++) {
-      AlignServeFn fn = serve_align_fn<false>(sv->type, k);
-      DevDB db = c->db;
-      RepStore rs = sv->store;
-      RunParams prm = sv->prm;
-      int cls = k, wa = word_after;
-      uint32_t *scr = sl.scratch;
-      int64_t sw = sl.scratch_words;
-      uint32_t rm = sv->ring_mask;
-      void *args[] = {&db, &rs, &prm, &rb, &cls, &wa, &scr, &sw, &rm};
-      CKS(cudaLaunchKernel((const void *)fn, dim3(sl.grid[k]), dim3(kAlignThreads), args,
-                           serve_align_smem(k), st));
-    }
+    CKS(round_launch<false>(sl.plan, c->db, sv->store, sv->prm, rb, word_after, st));
     if (ev[2]) cudaEventRecord(ev[2], st);
     k_serve_round_end<<<std::max(1, std::min(c->num_sms, (nbw + 255) / 256)), 256, 0, st>>>(n, rb);
     CKS(cudaGetLastError());
     if (ev[3]) cudaEventRecord(ev[3], st);
-    CKS(cudaMemcpyAsync(sl.h_ctl, rb.ctl, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    CKS(cudaMemcpyAsync(sl.h_ctl, rb.ctl, kCtlWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CKS(cudaStreamSynchronize(st));
-    if (sl.h_ctl[7]) return fail(NGIA_E_DEVICE, "serve: alignment loop bound exceeded (round at rep %d)", r0);
-    if (sl.h_ctl[0] > rb.cap || sl.h_ctl[1] > rb.cap || sl.h_ctl[2] > rb.cap)
-      return fail(NGIA_E_LIMIT, "serve: %u pairs in one round exceed the queue capacity", sl.h_ctl[0]);
-    left = sl.h_ctl[6];
+    for (int k = 0; k < kServeClasses; k++)
+      if (sl.h_ctl[k] > rb.cap)
+        return fail(NGIA_E_LIMIT, "serve: %u pairs in one round exceed the queue capacity", sl.h_ctl[k]);
+    left = sl.h_ctl[kCtlLeft];
     if (trace()) {
       float f = 0, a = 0, e = 0;
       cudaEventElapsedTime(&f, ev[0], ev[1]);
       cudaEventElapsedTime(&a, ev[1], ev[2]);
       cudaEventElapsedTime(&e, ev[2], ev[3]);
       fprintf(stderr,
-              "[serve] slot %d ticket %lld round %d reps %d..%d pairs %u/%u/%u left %u  filter %.3f align %.3f end "
+              "[serve] slot %d ticket %lld round %d reps %d..%d pairs %u/%u/%u/%u left %u  filter %.3f align %.3f end "
               "%.3f ms\n",
-              sl.index, (long long)rq.ticket, rq.rounds, r0, r0 + nr - 1, sl.h_ctl[0], sl.h_ctl[1], sl.h_ctl[2], left,
+              sl.index, (long long)rq.ticket, rq.rounds, r0, r0 + nr - 1, sl.h_ctl[kCtlPairs],
+              sl.h_ctl[kCtlPairs + 1], sl.h_ctl[kCtlPairs + 2], sl.h_ctl[kCtlPairs + 3], left,
               f, a, e);
     }
     r0 += nr;
-    chunk = std::min(chunk * 2, max_chunk);
+    chunk = std::min(chunk * 2, kMaxChunk);
+    pairs = std::min(pairs * 2, kMaxPairs);
     rq.rounds++;
   }
   for (auto &e : ev)
@@ -355,19 +349,18 @@ void free_slot(Slot &sl) {
   cudaFree(sl.rb.todo);
   cudaFree(sl.rb.stats);
   if (sl.h_stats) cudaFreeHost(sl.h_stats);
-  cudaFree(sl.scratch);
+  cudaFree(sl.plan.scratch);
   if (sl.h_ctl) cudaFreeHost(sl.h_ctl);
   if (sl.h_key) cudaFreeHost(sl.h_key);
   sl = Slot{};
 }
 
 // Device bytes of one slot (context, round buffers, scratch).
-int64_t slot_bytes(const ngia_server *sv, int grid2) {
+int64_t slot_bytes(const ngia_server *sv, int64_t scratch) {
   const int A = sv->type ? 28 : 4;
   const int64_t ctx = 4 * sv->cap_words + sv->cap_n * (8 + 4 + 4 + 4 * A) +
                       sv->cap_n * (4 + 4 + 4 * ngia::kNumClasses) + (int64_t)sv->cap_n / 8 * 3;
-  const int64_t rounds = (int64_t)kServeClasses * kMaxChunk * sv->cap_n * 8 + sv->cap_n * 8 + sv->cap_n / 8;
-  const int64_t scratch = (int64_t)grid2 * kAlignThreads * (sv->ring_mask + 1) * 4;
+  const int64_t rounds = 3ll * kMaxChunk * sv->cap_n * 8 + sv->cap_n * 8 + sv->cap_n / 8;
   // speculative leftover rounds: masks, up to 64 scores per record, pair
   // queues of 2^20 pairs per class, their own global ring
   const int64_t spec = sv->cap_n * (8 + 64 * 4) + (int64_t)kServeClasses * (1 << 20) * 8 + scratch;
@@ -378,29 +371,23 @@ int open_slot(ngia_server *sv, Slot &sl, int index) {
   sl.index = index;
   int rc = drv::open_ctx_capacity(sv->type, sv->cap_n, sv->cap_words, sv->cap_nb, &sl.ctx);
   if (rc) return rc;
-  const int64_t cap = (int64_t)kMaxChunk * sv->cap_n;
-  for (auto *&q : sl.rb.queue)
-    if (cudaMalloc((void **)&q, sizeof(int2) * (size_t)cap) != cudaSuccess)
+  const int64_t cap = (int64_t)kMaxChunk * ((sv->cap_n + 31) & ~31ll);  // a representative's pairs pad to 32
+  for (int k = 0; k < kServeClasses; k++)
+    if (serve_class_used(k, sv->reps->db.max_nb, false) &&
+        cudaMalloc((void **)&sl.rb.queue[k], sizeof(int2) * (size_t)cap) != cudaSuccess)
       return fail(NGIA_E_NOMEM, "serve: queue allocation failed");
-  if (cudaMalloc((void **)&sl.rb.ctl, 8 * sizeof(uint32_t)) != cudaSuccess ||
+  if (cudaMalloc((void **)&sl.rb.ctl, kCtlWords * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc((void **)&sl.rb.key, sizeof(unsigned long long) * (size_t)sv->cap_n) != cudaSuccess ||
       cudaMalloc((void **)&sl.rb.todo, 4 * (size_t)((sv->cap_n + 31) / 32)) != cudaSuccess ||
-      cudaMallocHost((void **)&sl.h_ctl, 8 * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMallocHost((void **)&sl.h_ctl, kCtlWords * sizeof(uint32_t)) != cudaSuccess ||
       cudaMallocHost((void **)&sl.h_key, sizeof(unsigned long long) * (size_t)sv->cap_n) != cudaSuccess ||
       cudaMalloc((void **)&sl.rb.stats, 2 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMallocHost((void **)&sl.h_stats, 2 * sizeof(unsigned long long)) != cudaSuccess)
     return fail(NGIA_E_NOMEM, "serve: slot allocation failed");
   sl.rb.cap = cap;
-  for (int k = 0; k < kServeClasses; k++) {
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)serve_align_fn<false>(sv->type, k), kAlignThreads,
-                                                      serve_align_smem(k)) != cudaSuccess ||
-        occ < 1)
-      occ = 1;
-    sl.grid[k] = sv->num_sms * occ;
-  }
-  sl.scratch_words = (int64_t)sl.grid[2] * kAlignThreads * (sv->ring_mask + 1);
-  if (cudaMalloc((void **)&sl.scratch, 4 * (size_t)sl.scratch_words) != cudaSuccess)
+  if (round_plan<false>(sl.plan, sv->type, sv->reps->db.max_nb, sv->num_sms) != cudaSuccess)
+    return fail(NGIA_E_CUDA, "serve: kernel attributes");
+  if (cudaMalloc((void **)&sl.plan.scratch, 4 * (size_t)sl.plan.scratch_words) != cudaSuccess)
     return fail(NGIA_E_NOMEM, "serve: scratch allocation failed");
   if (leftover_mode() == NGIA_MODE_SPEC) {  // the leftover driver's buffers, before any request
     rc = drv::spec_prepare(sl.ctx);
@@ -420,7 +407,6 @@ void destroy(ngia_server *sv) {
   for (auto &sl : sv->slots) free_slot(*sl);
   if (sv->reps) ngia_close(sv->reps);
   cudaFree(sv->d_lists);
-  cudaFree(sv->d_eq);
   delete sv;
 }
 
@@ -489,43 +475,27 @@ extern "C" int ngia_serve_open(const ngia_db_view *reps, const ngia_params *para
   }
   sv->store = ngia::RepStore{rc_ctx->db.words, rc_ctx->db.off, rc_ctx->db.len, rc_ctx->db.net, rc_ctx->db.cnt,
                              sv->d_lists, rc_ctx->db.n, lw};
-  if (sv->type == 0) {
-    sv->store.eq_stride = (int64_t)ngia::eq_words(rc_ctx->db.max_nb);
-    if (cudaMalloc((void **)&sv->d_eq, 4 * (size_t)sv->store.eq_stride * (size_t)reps->n) != cudaSuccess) {
-      ngia::destroy(sv);
-      return fail(NGIA_E_NOMEM, "ngia_serve_open: match table allocation failed");
-    }
-    sv->store.eq = sv->d_eq;
-    ngia::k_rep_eq<<<reps->n, 256, 0, rc_ctx->stream>>>(sv->store, sv->d_eq);
+  if (sv->type == 0)
     ngia::k_rep_lists<2><<<reps->n, 256, 0, rc_ctx->stream>>>(sv->store, params->word_length, sv->d_lists);
-  } else {
+  else
     ngia::k_rep_lists<5><<<reps->n, 256, 0, rc_ctx->stream>>>(sv->store, params->word_length, sv->d_lists);
-  }
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(rc_ctx->stream);
   if (e != cudaSuccess) {
     ngia::destroy(sv);
     return fail(NGIA_E_CUDA, "ngia_serve_open: k-mer tables: %s", cudaGetErrorString(e));
   }
-  uint32_t ring = 1;
-  while ((int)ring < rc_ctx->db.max_nb) ring <<= 1;
-  sv->ring_mask = ring - 1;
-  for (int k = 0; k < ngia::kServeClasses; k++) {
-    e = ngia::serve_align_configure<false>(sv->type, k, ngia::serve_align_smem(k));
-    if (e != cudaSuccess) {
-      ngia::destroy(sv);
-      return fail(NGIA_E_CUDA, "ngia_serve_open: kernel attributes: %s", cudaGetErrorString(e));
-    }
-  }
   // slots: as many as asked for and as fit the memory budget
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   const int64_t budget = cf.memory_budget > 0 ? cf.memory_budget : (int64_t)(free_b / 2);
-  int occ2 = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, (const void *)ngia::serve_align_fn<false>(sv->type, 2),
-                                                ngia::kAlignThreads,
-                                                ngia::serve_align_smem(2));
-  const int64_t per = ngia::slot_bytes(sv, sv->num_sms * std::max(1, occ2));
+  ngia::RoundPlan plan;
+  e = ngia::round_plan<false>(plan, sv->type, rc_ctx->db.max_nb, sv->num_sms);
+  if (e != cudaSuccess) {
+    ngia::destroy(sv);
+    return fail(NGIA_E_CUDA, "ngia_serve_open: kernel attributes: %s", cudaGetErrorString(e));
+  }
+  const int64_t per = ngia::slot_bytes(sv, 4 * plan.scratch_words);
   const int n_slots = (int)std::min<int64_t>(cf.slots, budget / per);
   if (n_slots < 1) {
     ngia::destroy(sv);

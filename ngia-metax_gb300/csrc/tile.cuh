@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "dp_asm.cuh"
+#include "kmer.cuh"
 
 // Build-time tuning of the DNA alignment kernels (swept on GB300, 1M DNA):
 //  NGIA_TILED_MAIN_DNA / NGIA_TILED_BLOCKS_DNA  main tile width and resident
@@ -33,9 +34,12 @@
 #ifndef NGIA_SERVE_PF
 #define NGIA_SERVE_PF 0
 #endif
-// Remainder tiles: rounded up to a multiple of this many slots.
+// Remainder tiles: rounded up to a multiple of this many slots.  Two: windows
+// that follow their pair end at any width, and half as many tile bodies miss
+// less in the instruction cache (20,000 DNA to the end 286 -> 250 ms, four
+// 258 ms; 400k DNA, 12 iterations 27.3 -> 24.4, four 25.4).
 #ifndef NGIA_REM_ROUND
-#define NGIA_REM_ROUND 1
+#define NGIA_REM_ROUND 2
 #endif
 
 namespace ngia {
@@ -151,16 +155,6 @@ __device__ __forceinline__ void build_eq(const uint32_t *s_pl, int nb1, uint32_t
 struct FmaK {
   uint32_t one, four;
 };
-
-// Bit i of x (i < 16) to bit 2i.
-__device__ __forceinline__ uint32_t spread16(uint32_t x) {
-  x &= 0xFFFFu;
-  x = (x | (x << 8)) & 0x00FF00FFu;
-  x = (x | (x << 4)) & 0x0F0F0F0Fu;
-  x = (x | (x << 2)) & 0x33333333u;
-  x = (x | (x << 1)) & 0x55555555u;
-  return x;
-}
 
 // Column codes of one 32-residue query block, first column on top: w[h]
 // holds columns 16h..16h+15, two bits each (plane-1 bit above plane-0 bit),
@@ -308,101 +302,6 @@ __device__ __forceinline__ int tiled_rem_eqf(int rem, const Ring &ring, uint32_t
 #define NGIA_REM(W) \
   case W:           \
     if (W % R == 0) return tiled_tile_eqf<W % R == 0 ? W : 1, false, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, k); \
-    return 0;
-    NGIA_REM_CASES(NGIA_REM)
-#undef NGIA_REM
-    default:
-      return 0;
-  }
-}
-
-// ---- the same bookkeeping with the match table in global memory ------------
-// (kernels that take the representative per pair read its table through L1)
-__device__ __forceinline__ uint64_t eq_next_addr_g(uint32_t &w, uint64_t eb, const FmaK &k) {
-  uint32_t c;
-  uint64_t a;
-  asm("mul.hi.u32 %0, %1, %2;" : "=r"(c) : "r"(w), "r"(k.four));
-  asm("mul.lo.u32 %0, %0, %1;" : "+r"(w) : "r"(k.four));
-  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(c), "r"(k.four), "l"(eb));
-  return a;
-}
-
-template <int M, int TW>
-struct EqLoadG {
-  static __device__ __forceinline__ void run(uint32_t (&e)[TW], uint64_t a) {
-    EqLoadG<M - 1, TW>::run(e, a);
-    asm volatile("ld.global.nc.u32 %0, [%1+%2];" : "=r"(e[M - 1]) : "l"(a), "n"(16 * (M - 1)));
-  }
-};
-template <int TW>
-struct EqLoadG<0, TW> {
-  static __device__ __forceinline__ void run(uint32_t (&)[TW], uint64_t) {}
-};
-
-template <int TW, bool PF>
-__device__ __forceinline__ void eq_columns_fg(uint32_t (&row)[TW], uint64_t eb, const uint32_t (&wc)[2], int cols,
-                                              uint32_t &cw, uint32_t &ncw, const FmaK &k) {
-#pragma unroll 1
-  for (int h = 0; h < 2; h++) {
-    const int n = min(16, cols - 16 * h);
-    if (n <= 0) break;
-    uint32_t w = wc[h];
-    if constexpr (PF) {
-      uint32_t ea[TW], eo[TW];
-      EqLoadG<TW, TW>::run(ea, eq_next_addr_g(w, eb, k));
-      int c = 0;
-#pragma unroll 1
-      for (; c + 2 <= n; c += 2) {
-        EqLoadG<TW, TW>::run(eo, eq_next_addr_g(w, eb, k));
-        dp_tile_eqf<TW>(row, ea, cw, ncw, k.one);
-        EqLoadG<TW, TW>::run(ea, eq_next_addr_g(w, eb, k));  // past the last column: code 0, in bounds
-        dp_tile_eqf<TW>(row, eo, cw, ncw, k.one);
-      }
-      if (c < n) dp_tile_eqf<TW>(row, ea, cw, ncw, k.one);
-    } else {
-#pragma unroll 1
-      for (int c = 0; c < n; c++) {
-        uint32_t ev[TW];
-        EqLoadG<TW, TW>::run(ev, eq_next_addr_g(w, eb, k));
-        dp_tile_eqf<TW>(row, ev, cw, ncw, k.one);
-      }
-    }
-  }
-}
-
-// tiled_tile_eqf with the table at global address eqb; returns the zero
-// count of the tile's rows after the block.
-template <int TW, bool PF, class Ring>
-__device__ __forceinline__ int tiled_tile_eqfg(const Ring &ring, uint64_t eqb, int base, int je, int nb1, int cols,
-                                               const uint32_t (&wc)[2], uint32_t &cw, uint32_t &ncw, const FmaK &k) {
-  uint32_t row[TW];
-#pragma unroll
-  for (int m = 0; m < TW; m++) {
-    const int j = base + m;
-    row[m] = j <= je ? ring[j] : 0u;
-  }
-  eq_columns_fg<TW, PF>(row, eqb + 16ull * (uint64_t)min(base, nb1), wc, cols, cw, ncw, k);
-  int z = 0;
-#pragma unroll
-  for (int m = 0; m < TW; m++) {
-    const int j = base + m;
-    if (j <= je) {
-      ring[j] = row[m];
-      z += __popc(~row[m]);
-    }
-  }
-  return z;
-}
-
-template <class Ring>
-__device__ __forceinline__ int tiled_rem_eqfg(int rem, const Ring &ring, uint64_t eqb, int base, int je, int nb1,
-                                              int cols, const uint32_t (&wc)[2], uint32_t &cw, uint32_t &ncw,
-                                              const FmaK &k) {
-  constexpr int R = NGIA_REM_ROUND;
-  switch ((rem + R - 1) / R * R) {
-#define NGIA_REM(W) \
-  case W:           \
-    if (W % R == 0) return tiled_tile_eqfg<W % R == 0 ? W : 1, false, Ring>(ring, eqb, base, je, nb1, cols, wc, cw, ncw, k); \
     return 0;
     NGIA_REM_CASES(NGIA_REM)
 #undef NGIA_REM
