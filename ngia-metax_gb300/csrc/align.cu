@@ -214,9 +214,9 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     __syncthreads();
   }
   const uint32_t s_eq_s = smem_u32(s_eq);
-  // 1 and 4 as values ptxas cannot fold (nb1 is read from shared memory)
+  // powers of two as values ptxas cannot fold (nb1 is read from shared memory)
   const uint32_t one_rt = 1u + (uint32_t)(h.nb1 < 0);
-  const FmaK fk{one_rt, one_rt << 2};
+  const FmaK fk(one_rt);
   (void)s_eq_s;
   (void)fk;
   typename RingOf<RING>::T ring;
@@ -224,12 +224,11 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     ring.base = smem + (((db.max_nb * P + 3) & ~3) + kListWords) + threadIdx.x;
   } else {
     const int64_t TL = (int64_t)gridDim.x * blockDim.x;
-    if ((int64_t)(rb.ring_mask + 1) * TL > rb.scratch_words) {
+    if ((int64_t)rb.ring_rows * TL > rb.scratch_words) {
       if (threadIdx.x == 0) set_error(st, NGIA_ERR_SCRATCH, 20);
       return;
     }
     ring.base = rb.scratch + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    ring.mask = rb.ring_mask;
     ring.stride = TL;
   }
   const int lane = threadIdx.x & 31;
@@ -283,20 +282,17 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
         state = -1;
         busy = false;
       } else {
+        ring.reset();
         for (int j = 0; j <= je; j++) ring[j] = 0xFFFFFFFFu;
 #pragma unroll
         for (int p = 0; p < P; p++) cur[p] = __ldg(qpl + p);
         active = true;
       }
     }
-    // Warp-uniform tile sequence: the full MT-slot tiles every busy lane
-    // needs, then tiles sized for the largest remainder in the warp.
-    // Lanes with narrower windows compute padding slots instead of taking a
-    // different branch.
+    // The lanes run the tiles of the warp's widest window in step (padding
+    // slots instead of different branches).
     const int n = busy ? je - js + 1 : 0;
-    constexpr int MT = tiled_main(P);
-    const int full = (int)__reduce_min_sync(kFullMask, busy ? (unsigned)(n / MT) : 0xFFFFFFFFu);
-    int rem = (int)__reduce_max_sync(kFullMask, busy ? (unsigned)(n - MT * full) : 0u);
+    const int slots = (int)__reduce_max_sync(kFullMask, (unsigned)n);
     if (!busy) continue;
     const int cols = (i == nq - 1) ? lastcols : 32;
     n_done += (unsigned long long)n * cols;
@@ -304,39 +300,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
 #pragma unroll
       for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + (i + 1) * P + p);
     }
-    if constexpr (kEq) {
-      using Ring = typename RingOf<RING>::T;
-      uint32_t wc[2];
-      eq_codes_top(cur, wc);
-      uint32_t cw = 0, ncw = 0;
-      int base = js;
-      zw = 0;  // the tiles return their rows' zero counts
-      for (int t = 0; t < full; t++, base += MT) {
-        zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-        cw = ncw << (32 - cols);  // column 0's carry at bit 31
-        ncw = 0;
-      }
-      for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      if (rem > 0) zw += tiled_rem_eqf<Ring>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-    } else {
-      uint32_t cw = 0, ncw = 0;
-      int base = js;
-      for (int t = 0; t < full; t++, base += MT) {
-        zw += tiled_tile<P, MT, typename RingOf<RING>::T>(ring, s_pl, base, je, cols, cur, cw, ncw);
-        cw = ncw << (32 - cols);  // column 0's carry at bit 31
-        ncw = 0;
-      }
-      for (; rem >= MT; rem -= MT, base += MT) {
-        zw += tiled_tile<P, MT, typename RingOf<RING>::T>(ring, s_pl, base, je, cols, cur, cw, ncw);
-        cw = ncw << (32 - cols);
-        ncw = 0;
-      }
-      if (rem > 0) zw += tiled_rem<P, typename RingOf<RING>::T, MT>(rem, ring, s_pl, base, je, cols, cur, cw, ncw);
-    }
+    zw = tile_block<P, kEq>(ring, s_eq_s, s_pl, js, je, nb1, slots, cols, cur, fk);
     i++;
     bool finished = i >= nq;
     if (!finished) {

@@ -337,10 +337,8 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
   c->db.n = saved_n;
   const int g = ngia::generic_class(type);  // (class 1 is on the global ring too)
   rb.generic_lanes = std::max(c->grid_align[1], c->grid_align[g]) * ngia::align_threads();
-  uint32_t ring = 1;
-  while ((int)ring < c->cap_nb) ring <<= 1;
-  rb.ring_mask = ring - 1;
-  rb.scratch_words = (int64_t)rb.generic_lanes * ring;
+  rb.ring_rows = ngia::global_rows(c->cap_nb);
+  rb.scratch_words = ngia::class_used(type, g, c->cap_nb) ? (int64_t)rb.generic_lanes * rb.ring_rows : 1;
   if (dalloc(&rb.scratch, (size_t)rb.scratch_words) != cudaSuccess)
     return fail(NGIA_E_NOMEM, "ngia_open: device allocation of alignment scratch failed");
   return NGIA_OK;

@@ -26,8 +26,8 @@
 namespace ngia {
 namespace {
 
-// Pair classes: band windows <= 64 blocks, <= 128, wider, and queries of at
-// most kQueryRows blocks with a window above 64 (the query's blocks are the
+// Pair classes: band windows <= 48 blocks, <= 112, wider, and queries of at
+// most kQueryRows blocks with a window above 48 (the query's blocks are the
 // rows then).
 constexpr int kServeClasses = 4;
 constexpr unsigned long long kNoRep = ~0ull;
@@ -61,13 +61,13 @@ struct RoundBufs {
 };
 constexpr int kCtlClaimed = 4, kCtlPairs = 8, kCtlLeft = 12, kCtlErr = 13;
 
-__host__ __device__ inline int serve_class(int A) { return A <= 64 ? 0 : A <= 128 ? 1 : 2; }
+__host__ __device__ inline int serve_class(int A) { return A <= kSmallWindow ? 0 : A <= kWideWindow ? 1 : 2; }
 __host__ __device__ inline int round_class(int A, int L2) {
-  return A > 64 && L2 <= 32 * kQueryRows ? 3 : serve_class(A);
+  return A > kSmallWindow && L2 <= 32 * kQueryRows ? 3 : serve_class(A);
 }
 // Whether windows of up to max_nb blocks can put a pair in class c.
 __host__ __device__ inline bool serve_class_used(int c, int max_nb, bool rounds) {
-  return c == 0 || (max_nb > (c == 2 ? 128 : 64) && (c < 3 || rounds));
+  return c == 0 || (max_nb > (c == 2 ? kWideWindow : kSmallWindow) && (c < 3 || rounds));
 }
 
 // k-mer presence bitset of every representative (the list of k_prep).
@@ -214,7 +214,7 @@ __host__ __device__ constexpr int round_table_blocks(int max_nb) {
 template <int P, int RING, bool MASK, bool QROWS>
 __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     k_round_align(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int word_after, int wave_pairs,
-                  uint32_t *scratch, int64_t scratch_words, uint32_t ring_mask, int table_blocks) {
+                  uint32_t *scratch, int64_t scratch_words, int ring_rows, int table_blocks) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint32_t s_qn;
   if (threadIdx.x == 0) s_qn = round_wave(rb, cls, wave_pairs) ? 0u : (uint32_t)min((int64_t)rb.ctl[cls], rb.cap);
@@ -227,23 +227,21 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     ring.base = smem + threadIdx.x;
   } else {
     const int64_t TL = (int64_t)gridDim.x * blockDim.x;
-    if ((int64_t)(ring_mask + 1) * TL > scratch_words) return;  // the host sizes the grid to the scratch
+    if ((int64_t)ring_rows * TL > scratch_words) return;  // the host sizes the grid to the scratch
     ring.base = scratch + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    ring.mask = ring_mask;
     ring.stride = TL;
   }
   constexpr bool kTable = P == 2 && !QROWS;
   uint32_t *w_eq = smem + RING * kAlignThreads + (threadIdx.x >> 5) * 4 * table_blocks;  // this warp's match table
   const uint32_t w_eq_s = smem_u32(w_eq);
   (void)w_eq_s;
-  // 1 and 4 as values ptxas cannot fold (the FMA-pipe bookkeeping of tile.cuh)
+  // powers of two as values ptxas cannot fold (the FMA-pipe bookkeeping of tile.cuh)
   const uint32_t one_rt = 1u + (uint32_t)(qn == 0u);
-  const FmaK fk{one_rt, one_rt << 2};
+  const FmaK fk(one_rt);
   (void)fk;
   const int lane = threadIdx.x & 31;
   const float s = prm.s;
   const int hw = qdb.hw;
-  constexpr int MT = tiled_main(P);
   unsigned long long n_pairs = 0, n_cells = 0;
   int staged = -1, L1 = 0, net1 = 0, nb1 = 0;  // the warp's representative
   const uint32_t *rpl = nullptr;
@@ -299,6 +297,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     if (active) {
       n_pairs++;
       je = band_first_top(B, nbr, nr, cutoff);
+      ring.reset();
       for (int j = 0; j <= je; j++) ring[j] = 0xFFFFFFFFu;
 #pragma unroll
       for (int p = 0; p < P; p++) cur[p] = __ldg(cp + p);
@@ -306,8 +305,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
     // the group's lanes in step, one column block at a time (at most kMaxBlocks)
     while (__any_sync(kFullMask, active)) {
       const int n = active ? je - js + 1 : 0;
-      const int full = (int)__reduce_min_sync(kFullMask, active ? (unsigned)(n / MT) : 0xFFFFFFFFu);
-      int rem = (int)__reduce_max_sync(kFullMask, active ? (unsigned)(n - MT * full) : 0u);
+      const int slots = (int)__reduce_max_sync(kFullMask, (unsigned)n);
       if (!active) continue;
       const int cols = min(32, nc - 32 * i);
       n_cells += (unsigned long long)n * cols * 32;
@@ -315,38 +313,11 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
 #pragma unroll
         for (int p = 0; p < P; p++) nxt[p] = __ldg(cp + (i + 1) * P + p);
       }
-      uint32_t cw = 0, ncw = 0;
-      int base = js;
-      if (kTable && table) {
-        if constexpr (kTable) {
-          uint32_t wc[2];
-          eq_codes_top(cur, wc);
-          zw = 0;  // the tiles return their rows' zero counts
-          for (int t = 0; t < full; t++, base += MT) {
-            zw += tiled_tile_eqf<MT, NGIA_SERVE_PF, Ring>(ring, w_eq_s, base, je, nbr, cols, wc, cw, ncw, fk);
-            cw = ncw << (32 - cols);
-            ncw = 0;
-          }
-          for (; rem >= MT; rem -= MT, base += MT) {
-            zw += tiled_tile_eqf<MT, NGIA_SERVE_PF, Ring>(ring, w_eq_s, base, je, nbr, cols, wc, cw, ncw, fk);
-            cw = ncw << (32 - cols);
-            ncw = 0;
-          }
-          if (rem > 0) zw += tiled_rem_eqf<Ring>(rem, ring, w_eq_s, base, je, nbr, cols, wc, cw, ncw, fk);
-        }
-      } else {
-        for (int t = 0; t < full; t++, base += MT) {
-          zw += tiled_tile<P, MT, Ring>(ring, rp, base, je, cols, cur, cw, ncw);
-          cw = ncw << (32 - cols);
-          ncw = 0;
-        }
-        for (; rem >= MT; rem -= MT, base += MT) {
-          zw += tiled_tile<P, MT, Ring>(ring, rp, base, je, cols, cur, cw, ncw);
-          cw = ncw << (32 - cols);
-          ncw = 0;
-        }
-        if (rem > 0) zw += tiled_rem<P, Ring, MT>(rem, ring, rp, base, je, cols, cur, cw, ncw);
-      }
+      if constexpr (kTable)
+        zw = table ? tile_block<P, true>(ring, w_eq_s, rp, js, je, nbr, slots, cols, cur, fk)
+                   : tile_block<P, false>(ring, w_eq_s, rp, js, je, nbr, slots, cols, cur, fk);
+      else
+        zw = tile_block<P, false>(ring, w_eq_s, rp, js, je, nbr, slots, cols, cur, fk);
       i++;
       bool finished = i >= ncb;
       if (!finished) {
@@ -490,7 +461,7 @@ __global__ void __launch_bounds__(kAlignThreads)
 }
 
 // ---- launch ---------------------------------------------------------------------
-using RoundAlignFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, uint32_t *, int64_t, uint32_t, int);
+using RoundAlignFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, uint32_t *, int64_t, int, int);
 using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, int);
 
 template <int P, bool MASK>
@@ -533,7 +504,7 @@ struct RoundPlan {
   int wave_pairs[kServeClasses] = {0, 0, 0, 0};
   uint32_t *scratch = nullptr;  // global ring of class 2
   int64_t scratch_words = 0;
-  uint32_t ring_mask = 0;
+  int ring_rows = 0;
 };
 
 template <bool MASK>
@@ -573,10 +544,8 @@ cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
       // the clustering kernels' cut-off (api.cu)
       if (wave) pl.wave_pairs[c] = 56 * num_sms;
     }
-  uint32_t ring = 1;
-  while ((int)ring < rep_nb) ring <<= 1;
-  pl.ring_mask = ring - 1;
-  pl.scratch_words = serve_class_used(2, rep_nb, MASK) ? (int64_t)pl.grid[2] * kAlignThreads * ring : 1;
+  pl.ring_rows = global_rows(rep_nb);
+  pl.scratch_words = serve_class_used(2, rep_nb, MASK) ? (int64_t)pl.grid[2] * kAlignThreads * pl.ring_rows : 1;
   return cudaSuccess;
 }
 
@@ -594,7 +563,7 @@ cudaError_t round_launch(const RoundPlan &pl, const DevDB &qdb, const RepStore &
     int cls = c, wa = word_after, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb;
     uint32_t *scr = pl.scratch;
     int64_t sw = pl.scratch_words;
-    uint32_t rm = pl.ring_mask;
+    int rm = pl.ring_rows;
     void *args[] = {&db, &r, &p, &b, &cls, &wa, &wp, &scr, &sw, &rm, &tb};
     cudaError_t e = cudaLaunchKernel(round_fn<MASK>(pl.type, c, false), dim3(pl.grid[c]), dim3(kAlignThreads), args,
                                      round_align_smem(pl.type, c, pl.rep_nb), st);

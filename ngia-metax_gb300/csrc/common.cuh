@@ -16,21 +16,25 @@ constexpr int kRefGridThreads = 128 * 128;     // BLOCK*WARP of the reference la
 
 // Alignment work classes.  Pairs are queued by the width of the band window
 // their alignment can need (window_need, in rep blocks): the last three
-// classes of a type hold windows of up to 64 or 128 rows in a shared-memory
-// ring, or of any width on a global-memory ring.  Classes 0 and 1 are the
-// pairs of windows up to 128 and of any width whose query has at most
+// classes of a type hold windows of up to 48 or 112 blocks (kSmallWindow,
+// kWideWindow) in shared-memory rows, or of any width in global-memory rows.
+// Classes 0 and 1 are the pairs of windows up to 112 and of any width whose query has at most
 // kQueryRows blocks: short queries against a long representative, aligned by
 // 16 threads with the query's blocks as rows (wave.cuh) while they are few.
 // DNA numbers 2 and 3 are unused: class numbers in saved tunings, checkpoints
 // and statistics keep their meaning.
 constexpr int kNumClasses = 7;
 constexpr int kQueryRows = 16;
+constexpr int kSmallWindow = 48, kWideWindow = 112;
+// Global-memory rows per lane: every rep block, and the padding of a lane at
+// the last block whose warp's widest window is the whole representative.
+__host__ __device__ constexpr int global_rows(int max_nb) { return 2 * max_nb + 16; }
 __host__ __device__ inline int num_classes(int type) { return type == 0 ? 7 : 5; }
 __host__ __device__ inline int generic_class(int type) { return num_classes(type) - 1; }
 __host__ __device__ inline int base_class(int type) { return num_classes(type) - 3; }
 // Classes 0 and 1: rows are the query's.
 __host__ __device__ inline bool is_query_class(int c) { return c < 2; }
-// Ring rows of class c: 64, 128, or 0 (global-memory ring).
+// Shared-memory rows of class c: 64, 128, or 0 (global-memory rows).
 __host__ __device__ inline int class_ring(int type, int c) {
   if (is_query_class(c)) return c == 0 ? 128 : 0;
   return c >= generic_class(type) ? 0 : c == generic_class(type) - 1 ? 128 : 64;
@@ -40,7 +44,7 @@ __host__ __device__ inline int class_ring(int type, int c) {
 __host__ __device__ inline bool class_used(int type, int c, int max_nb) {
   if (c >= num_classes(type) || (c >= 2 && c < base_class(type))) return false;
   const int ring = class_ring(type, c);
-  return ring == 64 || max_nb > (ring == 128 ? 64 : 128);
+  return ring == 64 || max_nb > (ring == 128 ? kSmallWindow : kWideWindow);
 }
 // Parallel branch class c runs in: the two classes on the global ring share
 // its scratch and run one after the other.
@@ -50,9 +54,9 @@ __host__ __device__ inline int class_stream(int type, int c) {
 // The class of a pair whose window is A blocks and whose query has L2 (raw)
 // residues.
 __host__ __device__ inline int class_of(int type, int A, int L2) {
-  if (A <= 64) return base_class(type);
-  if (L2 <= 32 * kQueryRows) return A <= 128 ? 0 : 1;
-  return base_class(type) + (A <= 128 ? 1 : 2);
+  if (A <= kSmallWindow) return base_class(type);
+  if (L2 <= 32 * kQueryRows) return A <= kWideWindow ? 0 : 1;
+  return base_class(type) + (A <= kWideWindow ? 1 : 2);
 }
 
 // Device copy of the makeDB database plus per-sequence header arrays.
@@ -136,7 +140,7 @@ struct RunBufs {
   uint32_t *scratch;      // per-lane band rows of the widest class (global ring)
   int64_t scratch_words;
   int32_t generic_lanes;
-  uint32_t ring_mask;     // global ring size - 1 (power of two >= the widest record)
+  int32_t ring_rows;      // global-memory rows per lane: every rep block and a tile's padding
   // filter counters, 32 stripes x kFilterStats (one 64-byte line each),
   // added per CTA and folded into the run state by k_next
   unsigned long long *fstats;

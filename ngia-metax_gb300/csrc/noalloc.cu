@@ -11,7 +11,7 @@
 // Three kernels:
 //  * up to noalloc_groups pairs per SM, a group of threads per pair (wave.cuh:
 //    rows in registers, match table and query codes in shared memory);
-//  * above that, representatives of up to 128 blocks: a thread per pair, the
+//  * above that, representatives of up to 112 blocks: a thread per pair, the
 //    band rows in a shared-memory ring, register tiles (tile.cuh);
 //  * proteins whose match table does not fit shared memory: a thread per
 //    pair with its working row (one 32-bit word per 32 representative
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, ngia::tiled_min_blocks(P))
                     float s, int *__restrict__ scores, int cap_blocks) {
   using Ring = typename ngia::RingOf<RING>::T;
   extern __shared__ __align__(16) uint32_t s_mem[];
-  constexpr int hw = P == 2 ? 6 : 30, MT = ngia::tiled_main(P);
+  constexpr int hw = P == 2 ? 6 : 30;
   constexpr unsigned kAll = ngia::kFullMask;
   const uint32_t *rep = words + rep_off;
   const int L1 = (int)rep[0], net1 = (int)rep[1], nb1 = (net1 + 31) / 32;
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, ngia::tiled_min_blocks(P))
   const uint32_t s_eq_s = ngia::smem_u32(s_eq);
   (void)s_eq_s;
   const uint32_t one_rt = 1u + (uint32_t)(nb1 < 0);
-  const ngia::FmaK fk{one_rt, one_rt << 2};
+  const ngia::FmaK fk(one_rt);
   (void)fk;
   Ring ring;
   ring.base = s_mem + planes + threadIdx.x;
@@ -217,48 +217,20 @@ __global__ void __launch_bounds__(kThreads, ngia::tiled_min_blocks(P))
         qpl = q + hw;
         nq = (net2 + 31) / 32;
         je = min(B, nb1 - 1);
+        ring.reset();
         for (int j = 0; j <= je; j++) ring[j] = 0xFFFFFFFFu;
       }
     }
     for (int i = 0; __any_sync(kAll, i < nq); i++) {  // warp-uniform
       const bool busy = i < nq;
       const int rows = busy ? je - js + 1 : 0;
-      const int full = (int)__reduce_min_sync(kAll, busy ? (unsigned)(rows / MT) : 0xFFFFFFFFu);
-      int rem = (int)__reduce_max_sync(kAll, busy ? (unsigned)(rows - MT * full) : 0u);
+      const int slots = (int)__reduce_max_sync(kAll, (unsigned)rows);
       if (busy) {
         const int cols = min(32, net2 - 32 * i);
-        uint32_t cur[P], cw = 0, ncw = 0;
+        uint32_t cur[P];
 #pragma unroll
         for (int p = 0; p < P; p++) cur[p] = __ldg(qpl + i * P + p);
-        int base = js;
-        if constexpr (P == 2) {
-          uint32_t wc[2];
-          ngia::eq_codes_top(cur, wc);
-          zw = 0;
-          for (int t = 0; t < full; t++, base += MT) {
-            zw += ngia::tiled_tile_eqf<MT, true, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-            cw = ncw << (32 - cols);
-            ncw = 0;
-          }
-          for (; rem >= MT; rem -= MT, base += MT) {
-            zw += ngia::tiled_tile_eqf<MT, true, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-            cw = ncw << (32 - cols);
-            ncw = 0;
-          }
-          if (rem > 0) zw += ngia::tiled_rem_eqf<Ring>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-        } else {
-          for (int t = 0; t < full; t++, base += MT) {
-            zw += ngia::tiled_tile<P, MT, Ring>(ring, s_mem, base, je, cols, cur, cw, ncw);
-            cw = ncw << (32 - cols);
-            ncw = 0;
-          }
-          for (; rem >= MT; rem -= MT, base += MT) {
-            zw += ngia::tiled_tile<P, MT, Ring>(ring, s_mem, base, je, cols, cur, cw, ncw);
-            cw = ncw << (32 - cols);
-            ncw = 0;
-          }
-          if (rem > 0) zw += ngia::tiled_rem<P, Ring, MT>(rem, ring, s_mem, base, je, cols, cur, cw, ncw);
-        }
+        zw = ngia::tile_block<P, P == 2>(ring, s_eq_s, s_mem, js, je, nb1, slots, cols, cur, fk);
         const bool last = i + 1 >= nq || ngia::band_advance(ring, i + 1, B, nb1, net1, vlast, net2 - 32 * (i + 1),
                                                             ngia::kNoCut, js, je, frozen, zw) != ngia::kBandGo;
         if (last) {
@@ -336,15 +308,15 @@ extern "C" int ngia_rep_scores_noalloc(const uint32_t *d_words, int64_t rep_off,
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool many = n > noalloc_groups(P, nb1) * std::max(sms, 1) && nb1 <= 128;
+  const bool many = n > noalloc_groups(P, nb1) * std::max(sms, 1) && nb1 <= ngia::kWideWindow;
   const int form = nb1 <= 64 ? 0 : nb1 <= 128 ? 1 : 2;  // a warp, a CTA of one row word per thread, of up to 16
   NoAllocFn fn;
   size_t smem;
   int per;  // pairs per CTA
   if (many) {
-    const int ring = form == 0 ? 64 : 128;
-    fn = P == 2 ? (form == 0 ? k_noalloc_tiled<2, 64> : k_noalloc_tiled<2, 128>)
-                : (form == 0 ? k_noalloc_tiled<5, 64> : k_noalloc_tiled<5, 128>);
+    const int ring = nb1 <= ngia::kSmallWindow ? 64 : 128;
+    fn = P == 2 ? (ring == 64 ? k_noalloc_tiled<2, 64> : k_noalloc_tiled<2, 128>)
+                : (ring == 64 ? k_noalloc_tiled<5, 64> : k_noalloc_tiled<5, 128>);
     smem = 4 * (size_t)(((nb1 * P + 3) & ~3) + ring * kThreads + (P == 2 ? ngia::eq_words(nb1) : 0));
     per = kThreads;
   } else {
@@ -354,7 +326,7 @@ extern "C" int ngia_rep_scores_noalloc(const uint32_t *d_words, int64_t rep_off,
     smem = 4 * ((size_t)ngia::wave_table_words(P, nb1) + (size_t)per * ngia::kWaveRingWords);
   }
   if (smem <= kNoAllocSmemMost) {
-    e = noalloc_configure(fn, (P == 2 ? 0 : 8) + (many ? 4 : 0) + form, smem);
+    e = noalloc_configure(fn, (P == 2 ? 0 : 8) + (many ? 4 + (nb1 <= ngia::kSmallWindow ? 0 : 1) : form), smem);
     if (e != cudaSuccess) return ngia::fail(NGIA_E_CUDA, "ngia_rep_scores_noalloc: %s", cudaGetErrorString(e));
     const int grid = std::max(1, std::min(std::max(sms, 1) * 8, (n + per - 1) / per));
     fn<<<grid, kThreads, smem, st>>>(d_words, rep_off, d_query_off, n, similarity, d_scores, nb1);

@@ -71,7 +71,7 @@ struct PoolDev {
   uint32_t *done;        // [0] filter CTAs finished, [1] next CTAs finished (last one resets)
   uint32_t *scratch;     // global ring of the widest bucket
   int64_t scratch_words;
-  uint32_t ring_mask;
+  int32_t ring_rows;
   int32_t n_jobs, type, total_words;
   int32_t grid_align[kNumClasses];
 };
@@ -299,7 +299,6 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
   __shared__ uint32_t s_next;
   __shared__ unsigned long long s_qw;
   constexpr bool kEq = P == 2;
-  constexpr int MT = tiled_main(P);
   const int nj = pd.n_jobs;
   const int32_t *cb = pd.chunk_base + cls * (nj + 1);
   const int lane = threadIdx.x & 31;
@@ -313,9 +312,8 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
     ring.base = smem + (((max_nb * P + 3) & ~3) + kListWords) + threadIdx.x;
   } else {
     const int64_t TL = (int64_t)gridDim.x * blockDim.x;
-    if ((int64_t)(pd.ring_mask + 1) * TL > pd.scratch_words) return;  // the host sizes the grid to the scratch
+    if ((int64_t)pd.ring_rows * TL > pd.scratch_words) return;  // the host sizes the grid to the scratch
     ring.base = pd.scratch + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    ring.mask = pd.ring_mask;
     ring.stride = TL;
   }
   if (threadIdx.x == 0) mbar_init(&bar, 1);
@@ -326,9 +324,9 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
   // the staged job's representative
   int L1 = 0, net1 = 0, nb1 = 0, rep = 0, word_after = 0;
   uint32_t vlast = 0;
-  // 1 and 4 as values ptxas cannot fold (the FMA-pipe bookkeeping of tile.cuh)
+  // powers of two as values ptxas cannot fold (the FMA-pipe bookkeeping of tile.cuh)
   const uint32_t one_rt = 1u + (uint32_t)(max_nb < 0);
-  const FmaK fk{one_rt, one_rt << 2};
+  const FmaK fk(one_rt);
   (void)fk;
   for (;;) {
     if (threadIdx.x == 0) {
@@ -463,6 +461,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
           state = -1;
           busy = false;
         } else {
+          ring.reset();
           for (int jj = 0; jj <= je; jj++) ring[jj] = 0xFFFFFFFFu;
 #pragma unroll
           for (int p = 0; p < P; p++) cur[p] = __ldg(qpl + p);
@@ -470,8 +469,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
         }
       }
       const int n = busy ? je - js + 1 : 0;
-      const int full = (int)__reduce_min_sync(kFullMask, busy ? (unsigned)(n / MT) : 0xFFFFFFFFu);
-      int rem = (int)__reduce_max_sync(kFullMask, busy ? (unsigned)(n - MT * full) : 0u);
+      const int slots = (int)__reduce_max_sync(kFullMask, (unsigned)n);
       if (!busy) continue;
       const int cols = (i == nq - 1) ? lastcols : 32;
       n_done += (unsigned long long)n * cols;
@@ -479,39 +477,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
 #pragma unroll
         for (int p = 0; p < P; p++) nxt[p] = __ldg(qpl + (i + 1) * P + p);
       }
-      using Ring = typename RingOf<RING>::T;
-      if constexpr (kEq) {
-        uint32_t wc[2];
-        eq_codes_top(cur, wc);
-        uint32_t cw = 0, ncw = 0;
-        int base = js;
-        zw = 0;  // the tiles return their rows' zero counts
-        for (int t = 0; t < full; t++, base += MT) {
-          zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-          cw = ncw << (32 - cols);  // column 0's carry at bit 31
-          ncw = 0;
-        }
-        for (; rem >= MT; rem -= MT, base += MT) {
-          zw += tiled_tile_eqf<MT, NGIA_EQ_PF_MAIN, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-          cw = ncw << (32 - cols);
-          ncw = 0;
-        }
-        if (rem > 0) zw += tiled_rem_eqf<Ring>(rem, ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, fk);
-      } else {
-        uint32_t cw = 0, ncw = 0;
-        int base = js;
-        for (int t = 0; t < full; t++, base += MT) {
-          zw += tiled_tile<P, MT, Ring>(ring, s_pl, base, je, cols, cur, cw, ncw);
-          cw = ncw << (32 - cols);
-          ncw = 0;
-        }
-        for (; rem >= MT; rem -= MT, base += MT) {
-          zw += tiled_tile<P, MT, Ring>(ring, s_pl, base, je, cols, cur, cw, ncw);
-          cw = ncw << (32 - cols);
-          ncw = 0;
-        }
-        if (rem > 0) zw += tiled_rem<P, Ring, MT>(rem, ring, s_pl, base, je, cols, cur, cw, ncw);
-      }
+      zw = tile_block<P, kEq>(ring, s_eq_s, s_pl, js, je, nb1, slots, cols, cur, fk);
       i++;
       bool finished = i >= nq;
       if (!finished) {
@@ -690,12 +656,11 @@ int group_open(const std::vector<ngia_ctx *> &jobs, Group **out) {
     if (ring == 0) occ = std::min(occ, 2);
     pd.grid_align[k] = g->num_sms * occ;
   }
-  uint32_t rs = 1;
-  while ((int)rs < g->max_nb) rs <<= 1;
+  const int rs = global_rows(g->max_nb);
   // (class 1 is on the global ring too: it runs on the same stream)
   const int gcls = generic_class(type);
   pd.scratch_words = (int64_t)std::max(pd.grid_align[1], pd.grid_align[gcls]) * kAlignThreads * rs;
-  pd.ring_mask = rs - 1;
+  pd.ring_rows = rs;
   if (dalloc(&g->d_scratch, (size_t)pd.scratch_words) != cudaSuccess) {
     group_close(g);
     return fail(NGIA_E_NOMEM, "pool: device allocation of the alignment ring failed");

@@ -14,14 +14,12 @@
 //    CTAs per SM of the tiled kernel.
 //  NGIA_EQ_PF_MAIN  load the next column's match words during the current
 //    column in the main tiles of the clustering kernel.
-//  NGIA_SERVE_PF  the same in the kernel that takes the representative per
-//    pair: off (60.2k against 64.3k queries/s).
-//  Settled before the window followed the pair (band_advance), on windows of
-//  49 blocks: match words from the representative's table instead of plane
-//  registers +16%; columns unrolled 2/4/8 times 0.92x/0.64x/0.41x
-//  (instruction cache); code, address and carry bookkeeping as multiply-adds
-//  by run-time constants (FMA pipe) +2.9%; adds as IMAD.X 0.97x; straight
-//  tiles +3%.
+//  Swept with windows that follow their pair (20,000 DNA to the end | 400k
+//  DNA, 12 iterations, ms): 16 slots, 4 CTAs, prefetch 233 | 22.7; without
+//  prefetch 234 | 24.6; 5 CTAs 236 | 23.1; 12 slots 252 | 25.6 (5 CTAs); 8
+//  slots 260 | 27 (6, 7 CTAs); remainder tiles of even width 238 | 23.3.
+//  Columns unrolled, adds as IMAD.X and the like lost 3-60% earlier (the
+//  kernels are sensitive to their instruction footprint).
 #ifndef NGIA_TILED_MAIN_DNA
 #define NGIA_TILED_MAIN_DNA 16
 #endif
@@ -31,69 +29,97 @@
 #ifndef NGIA_EQ_PF_MAIN
 #define NGIA_EQ_PF_MAIN 1
 #endif
-#ifndef NGIA_SERVE_PF
-#define NGIA_SERVE_PF 0
-#endif
-// Remainder tiles: rounded up to a multiple of this many slots.  Two: windows
-// that follow their pair end at any width, and half as many tile bodies miss
-// less in the instruction cache (20,000 DNA to the end 286 -> 250 ms, four
-// 258 ms; 400k DNA, 12 iterations 27.3 -> 24.4, four 25.4).
-#ifndef NGIA_REM_ROUND
-#define NGIA_REM_ROUND 2
-#endif
-
 namespace ngia {
 
 constexpr int kAlignThreads = 128;  // threads per CTA of every alignment kernel
 
-// Band rows of one lane's pair, indexed by absolute rep block j.  Windows of
-// up to RING blocks keep them in shared memory (row j of thread t at
-// (j mod RING) * threads + t: the 32 lanes of a warp hit 32 banks); wider
-// windows keep them in global scratch with the same layout over all lanes
-// of the grid (a warp's accesses to one row are one 128-byte line).
-template <int RING>
+// Band rows of one lane's pair, indexed by absolute rep block j and one after
+// the other in memory, so that a tile's rows have immediate offsets from its
+// first.  A tile loads and stores all its rows: those above the window's top
+// (padding of a lane whose window is narrower than its warp's widest) hold
+// anything, and a row is set when it enters the window (band_advance).
+//
+// SmemRing: CAP rows per lane in shared memory, row j of thread t at
+// (j - off) * threads + t (the 32 lanes of a warp hit 32 banks); when a
+// window reaches the end its rows move to the start (fit), once in CAP minus
+// the warp's widest window query blocks (kSmallWindow, kWideWindow: 16 at
+// least).
+// GlobalRing: every rep block and the padding (global_rows) in global
+// scratch, with the same layout over all lanes of the grid (a warp's access
+// to one row is one 128-byte line).
+template <int CAP>
 struct SmemRing {
-  static constexpr int kSize = RING;
-  uint32_t *base;  // ring + threadIdx.x
-  __device__ __forceinline__ uint32_t &operator[](int j) const { return base[(j & (RING - 1)) * kAlignThreads]; }
-  __device__ __forceinline__ uint32_t *at(int j) const { return base + (j & (RING - 1)) * kAlignThreads; }
+  static constexpr int kPitch = kAlignThreads;
+  uint32_t *base;  // rows + threadIdx.x
+  int off = 0;     // rep block of the first row
+  __device__ __forceinline__ void reset() { off = 0; }
+  __device__ __forceinline__ uint32_t &operator[](int j) const { return base[(j - off) * kAlignThreads]; }
+  __device__ __forceinline__ void fit(int js, int je, int slots) {
+    if (js - off + slots < CAP) return;  // and a row for the block that enters next
+    for (int j = js; j <= je; j++) base[(j - js) * kAlignThreads] = base[(j - off) * kAlignThreads];
+    off = js;
+  }
 };
 struct GlobalRing {
-  static constexpr int kSize = 0;  // no straight-tile path
-  __device__ __forceinline__ uint32_t *at(int) const { return nullptr; }
+  static constexpr int kPitch = 0;
   uint32_t *base;  // scratch + global lane index
-  uint32_t mask;   // ring size - 1 (a power of two >= the widest window)
   int64_t stride;  // lanes of the grid
-  __device__ __forceinline__ uint32_t &operator[](int j) const { return base[(int64_t)(j & mask) * stride]; }
+  __device__ __forceinline__ void reset() {}
+  __device__ __forceinline__ uint32_t &operator[](int j) const { return base[(int64_t)j * stride]; }
+  __device__ __forceinline__ void fit(int, int, int) {}
 };
-template <int RING>
+template <int CAP>
 struct RingOf {
-  using T = SmemRing<RING>;
+  using T = SmemRing<CAP>;
 };
 template <>
 struct RingOf<0> {
   using T = GlobalRing;
 };
 
-// One tile: band rows base .. base+TW-1 (rows above je are padding) through
-// the `cols` columns of the current query block, whose P plane words are
-// cur[]; s_pl points at the representative's planes (shared or global
-// memory).  cw holds the column carries into the tile (column k at bit
-// 31-k after the shift below), ncw collects the carries out.  Returns the
-// change of the zero count over the tile's rows.
+template <int TW, class Ring>
+__device__ __forceinline__ void rows_load(const Ring &ring, int base, uint32_t (&row)[TW]) {
+  const uint32_t *rp = &ring[base];
+  if constexpr (Ring::kPitch > 0) {
+#pragma unroll
+    for (int m = 0; m < TW; m++) row[m] = rp[m * Ring::kPitch];
+  } else {
+#pragma unroll
+    for (int m = 0; m < TW; m++) row[m] = rp[m * ring.stride];
+  }
+}
+// Stores a tile's rows; returns their zero count.
+template <int TW, class Ring>
+__device__ __forceinline__ int rows_store(const Ring &ring, int base, const uint32_t (&row)[TW]) {
+  uint32_t *rp = &ring[base];
+  int ones = 0;
+  if constexpr (Ring::kPitch > 0) {
+#pragma unroll
+    for (int m = 0; m < TW; m++) rp[m * Ring::kPitch] = row[m];
+  } else {
+#pragma unroll
+    for (int m = 0; m < TW; m++) rp[m * ring.stride] = row[m];
+  }
+#pragma unroll
+  for (int m = 0; m < TW; m++) ones += __popc(row[m]);
+  return 32 * TW - ones;
+}
+
+// One tile from plane registers: rows base .. base+TW-1 through the `cols`
+// columns of the current block, whose P plane words are cur[]; planes points
+// at the rows' sequence (nbr blocks, shared or global memory).  cw holds the
+// column carries into the tile (column 0 at bit 31), ncw collects the
+// carries out.  Returns the rows' zero count.
 template <int P, int TW, class Ring>
-__device__ __forceinline__ int tiled_tile(const Ring &ring, const uint32_t *s_pl, int base, int je, int cols,
-                                          const uint32_t (&cur)[P], uint32_t &cw, uint32_t &ncw) {
+__device__ __forceinline__ int tile_planes(const Ring &ring, const uint32_t *planes, int base, int nbr, int cols,
+                                           const uint32_t (&cur)[P], uint32_t &cw, uint32_t &ncw) {
   uint32_t row[TW], pl[P][TW];
-  int zold = 0;
+  rows_load<TW>(ring, base, row);
 #pragma unroll
   for (int m = 0; m < TW; m++) {
-    const int j = base + m;
-    const bool in = j <= je;
-    row[m] = in ? ring[j] : 0u;
-    zold += in ? __popc(~row[m]) : 0;
+    const uint32_t *b = planes + min(base + m, nbr - 1) * P;
 #pragma unroll
-    for (int p = 0; p < P; p++) pl[p][m] = in ? s_pl[j * P + p] : 0u;
+    for (int p = 0; p < P; p++) pl[p][m] = b[p];
   }
   uint32_t rv[P];
 #pragma unroll
@@ -108,16 +134,7 @@ __device__ __forceinline__ int tiled_tile(const Ring &ring, const uint32_t *s_pl
     }
     dp_tile<P, TW>(row, pl, mk, cw, ncw);
   }
-  int znew = 0;
-#pragma unroll
-  for (int m = 0; m < TW; m++) {
-    const int j = base + m;
-    if (j <= je) {
-      ring[j] = row[m];
-      znew += __popc(~row[m]);
-    }
-  }
-  return znew - zold;
+  return rows_store<TW>(ring, base, row);
 }
 
 // DNA match table: for every rep block j its four match words, word 4j + c =
@@ -153,25 +170,23 @@ __device__ __forceinline__ void build_eq(const uint32_t *s_pl, int nb1, uint32_t
 // Run-time constants 1 and 4: ptxas cannot fold a multiply by them into a
 // shift or an add, so the multiply-adds below stay IMADs (FMA pipe).
 struct FmaK {
-  uint32_t one, four;
+  uint32_t one, two, four, eight;
+  __device__ __forceinline__ explicit FmaK(uint32_t one_rt) : one(one_rt), two(one_rt << 1), four(one_rt << 2), eight(one_rt << 3) {}
 };
 
-// Column codes of one 32-residue query block, first column on top: w[h]
-// holds columns 16h..16h+15, two bits each (plane-1 bit above plane-0 bit),
-// column 16h in bits 31..30.
-__device__ __forceinline__ void eq_codes_top(const uint32_t (&cur)[2], uint32_t (&w)[2]) {
-  const uint32_t r0 = __brev(cur[0]), r1 = __brev(cur[1]);
-  w[0] = spread16(r0 >> 16) | (spread16(r1 >> 16) << 1);
-  w[1] = spread16(r0) | (spread16(r1) << 1);
-}
-
-// Shared-memory address of the next column's match words: code = w >> 30,
-// w <<= 2, address = eb + 4 code — three multiply-adds.
-__device__ __forceinline__ uint32_t eq_next_addr(uint32_t &w, uint32_t eb, const FmaK &k) {
-  uint32_t c, a;
-  asm("mul.hi.u32 %0, %1, %2;" : "=r"(c) : "r"(w), "r"(k.four));
-  asm("mul.lo.u32 %0, %0, %1;" : "+r"(w) : "r"(k.four));
-  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(a) : "r"(c), "r"(k.four), "r"(eb));
+// Shared-memory address of the next column's match words: the code's two bits
+// are on top of the bit-reversed planes w[]; four high and low products by a
+// run-time 2 and two multiply-adds, all on the FMA pipe.  (Packing the codes
+// first takes half of these and 42 logic instructions per block of columns:
+// the same time.)
+__device__ __forceinline__ uint32_t eq_next_addr(uint32_t (&w)[2], uint32_t eb, const FmaK &k) {
+  uint32_t c0, c1, a;
+  asm("mul.hi.u32 %0, %1, %2;" : "=r"(c0) : "r"(w[0]), "r"(k.two));
+  asm("mul.hi.u32 %0, %1, %2;" : "=r"(c1) : "r"(w[1]), "r"(k.two));
+  asm("mul.lo.u32 %0, %0, %1;" : "+r"(w[0]) : "r"(k.two));
+  asm("mul.lo.u32 %0, %0, %1;" : "+r"(w[1]) : "r"(k.two));
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(a) : "r"(c0), "r"(k.four), "r"(eb));
+  asm("mad.lo.u32 %0, %1, %2, %0;" : "+r"(a) : "r"(c1), "r"(k.eight));
   return a;
 }
 
@@ -193,137 +208,89 @@ __device__ __forceinline__ void eq_load_s(uint32_t (&e)[TW], uint32_t a) {
   EqLoad<TW, TW>::run(e, a);
 }
 
-// eq_columns with the codes on top of w[] and the FMA-pipe bookkeeping.
+// All `cols` columns of one block through a tile whose match words start at
+// shared address eb; the tile takes column carries in cw and hands them out
+// in ncw.  PF: the next column's match words are loaded while the current
+// column updates (two columns per loop trip).
 template <int TW, bool PF>
-__device__ __forceinline__ void eq_columns_f(uint32_t (&row)[TW], uint32_t eb, const uint32_t (&wc)[2], int cols,
-                                             uint32_t &cw, uint32_t &ncw, const FmaK &k) {
+__device__ __forceinline__ void eq_columns(uint32_t (&row)[TW], uint32_t eb, const uint32_t (&cur)[2], int cols,
+                                           uint32_t &cw, uint32_t &ncw, const FmaK &k) {
+  uint32_t w[2] = {__brev(cur[0]), __brev(cur[1])};
+  if constexpr (PF) {
+    uint32_t ea[TW], eo[TW];
+    eq_load_s<TW>(ea, eq_next_addr(w, eb, k));
+    int c = 0;
 #pragma unroll 1
-  for (int h = 0; h < 2; h++) {
-    const int n = min(16, cols - 16 * h);
-    if (n <= 0) break;
-    uint32_t w = wc[h];
-    if constexpr (PF) {
-      uint32_t ea[TW], eo[TW];
-      eq_load_s<TW>(ea, eq_next_addr(w, eb, k));
-      int c = 0;
+    for (; c + 2 <= cols; c += 2) {
+      eq_load_s<TW>(eo, eq_next_addr(w, eb, k));
+      dp_tile_eqf<TW>(row, ea, cw, ncw, k.one);
+      eq_load_s<TW>(ea, eq_next_addr(w, eb, k));  // past the last column: some code, in bounds
+      dp_tile_eqf<TW>(row, eo, cw, ncw, k.one);
+    }
+    if (c < cols) dp_tile_eqf<TW>(row, ea, cw, ncw, k.one);
+  } else {
 #pragma unroll 1
-      for (; c + 2 <= n; c += 2) {
-        eq_load_s<TW>(eo, eq_next_addr(w, eb, k));
-        dp_tile_eqf<TW>(row, ea, cw, ncw, k.one);
-        eq_load_s<TW>(ea, eq_next_addr(w, eb, k));  // past the last column: code 0, in bounds
-        dp_tile_eqf<TW>(row, eo, cw, ncw, k.one);
-      }
-      if (c < n) dp_tile_eqf<TW>(row, ea, cw, ncw, k.one);
-    } else {
-#pragma unroll 1
-      for (int c = 0; c < n; c++) {
-        uint32_t ev[TW];
-        eq_load_s<TW>(ev, eq_next_addr(w, eb, k));
-        dp_tile_eqf<TW>(row, ev, cw, ncw, k.one);
-      }
+    for (int c = 0; c < cols; c++) {
+      uint32_t ev[TW];
+      eq_load_s<TW>(ev, eq_next_addr(w, eb, k));
+      dp_tile_eqf<TW>(row, ev, cw, ncw, k.one);
     }
   }
 }
 
-// Straight tile: rows base .. base+TW-1 all inside the lane's window
-// (<= je) and contiguous in the shared-memory ring (no wrap).  Its rows are
-// then at rp + m * threads, immediate offsets from one address.
-template <int TW, class Ring>
-__device__ __forceinline__ bool tile_straight(const Ring &ring, int base, int je, uint32_t *&rp) {
-  if constexpr (Ring::kSize >= TW) {
-    rp = ring.at(base);
-    return base + TW - 1 <= je && (base & (Ring::kSize - 1)) + TW <= Ring::kSize;
-  } else {
-    rp = nullptr;
-    return false;
-  }
-}
-template <int TW>
-__device__ __forceinline__ void tile_load_straight(uint32_t (&row)[TW], const uint32_t *rp) {
-#pragma unroll
-  for (int m = 0; m < TW; m++) row[m] = rp[m * kAlignThreads];
-}
-// Stores a straight tile's rows; returns their zero count.
-template <int TW>
-__device__ __forceinline__ int tile_store_straight(const uint32_t (&row)[TW], uint32_t *rp) {
-#pragma unroll
-  for (int m = 0; m < TW; m++) rp[m * kAlignThreads] = row[m];
-  int ones = 0;
-#pragma unroll
-  for (int m = 0; m < TW; m++) ones += __popc(row[m]);
-  return 32 * TW - ones;
-}
-
-// One tile of band rows base .. base+TW-1 (rows above je are padding) through
-// the block's columns, with the match table at shared address s_eq_s; returns
-// the zero count of the tile's rows after the block.
+// One DNA tile with the match table at shared address s_eq_s (per column one
+// load per slot and three integer instructions per 32 cells: AND, add with
+// carry, LOP3).  A tile past the last rep block (a lane with a narrower
+// window than its warp's widest) reads the table's zero blocks.
 template <int TW, bool PF, class Ring>
-__device__ __forceinline__ int tiled_tile_eqf(const Ring &ring, uint32_t s_eq_s, int base, int je, int nb1, int cols,
-                                              const uint32_t (&wc)[2], uint32_t &cw, uint32_t &ncw, const FmaK &k) {
+__device__ __forceinline__ int tile_eq(const Ring &ring, uint32_t s_eq_s, int base, int nbr, int cols,
+                                       const uint32_t (&cur)[2], uint32_t &cw, uint32_t &ncw, const FmaK &k) {
   uint32_t row[TW];
-  uint32_t *rp = nullptr;
-  const bool straight = tile_straight<TW>(ring, base, je, rp);
-  if (straight) {
-    tile_load_straight<TW>(row, rp);
-  } else {
-#pragma unroll
-    for (int m = 0; m < TW; m++) {
-      const int j = base + m;
-      row[m] = j <= je ? ring[j] : 0u;
-    }
+  rows_load<TW>(ring, base, row);
+  eq_columns<TW, PF>(row, s_eq_s + 16u * (uint32_t)min(base, nbr), cur, cols, cw, ncw, k);
+  return rows_store<TW>(ring, base, row);
+}
+
+// Main tile width of the tiled kernels.
+__host__ __device__ constexpr int tiled_main(int P) { return P == 2 ? NGIA_TILED_MAIN_DNA : 16; }
+__host__ __device__ constexpr int tiled_min_blocks(int P) { return P == 2 ? NGIA_TILED_BLOCKS_DNA : 2; }
+
+// One block of columns (planes cur[], cols of them) over a lane's window
+// [js, je] in tiles of `slots` rows altogether (the warp's widest window: the
+// lanes stay in step, narrower windows run padding slots).  TABLE: match words from
+// s_eq_s, else from the rows' planes.  Returns the window's zero count.
+template <int P, bool TABLE, class Ring>
+__device__ __forceinline__ int tile_block(Ring &ring, uint32_t s_eq_s, const uint32_t *planes, int js, int je, int nbr,
+                                          int slots, int cols, const uint32_t (&cur)[P], const FmaK &fk) {
+  constexpr int MT = tiled_main(P);
+  ring.fit(js, je, slots);
+  uint32_t cw = 0, ncw = 0;
+  int z = 0, base = js, left = slots;
+  for (; left >= MT; left -= MT, base += MT) {
+    if constexpr (TABLE)
+      z += tile_eq<MT, NGIA_EQ_PF_MAIN>(ring, s_eq_s, base, nbr, cols, cur, cw, ncw, fk);
+    else
+      z += tile_planes<P, MT>(ring, planes, base, nbr, cols, cur, cw, ncw);
+    cw = ncw << (32 - cols);  // column 0's carry at bit 31
+    ncw = 0;
   }
-  // A tile past the rep's last block (a lane with a narrower window than its
-  // warp's widest) is all padding: it reads the zero blocks after nb1.
-  eq_columns_f<TW, PF>(row, s_eq_s + 16u * (uint32_t)min(base, nb1), wc, cols, cw, ncw, k);
-  if (straight) return tile_store_straight<TW>(row, rp);
-  int z = 0;
-#pragma unroll
-  for (int m = 0; m < TW; m++) {
-    const int j = base + m;
-    if (j <= je) {
-      ring[j] = row[m];
-      z += __popc(~row[m]);
-    }
+  switch (left) {
+#define NGIA_REM(W)                                                                                            \
+  case W:                                                                                                      \
+    if constexpr (W < MT) {                                                              \
+      if constexpr (TABLE)                                                                                     \
+        z += tile_eq<W, false>(ring, s_eq_s, base, nbr, cols, cur, cw, ncw, fk);                                \
+      else                                                                                                     \
+        z += tile_planes<P, W>(ring, planes, base, nbr, cols, cur, cw, ncw);                                   \
+    }                                                                                                          \
+    break;
+    NGIA_REM(1) NGIA_REM(2) NGIA_REM(3) NGIA_REM(4) NGIA_REM(5) NGIA_REM(6) NGIA_REM(7) NGIA_REM(8)
+    NGIA_REM(9) NGIA_REM(10) NGIA_REM(11) NGIA_REM(12) NGIA_REM(13) NGIA_REM(14) NGIA_REM(15)
+#undef NGIA_REM
+    default: break;
   }
+  for (int j = je + 1; j < js + slots; j++) z -= __popc(~ring[j]);  // the padding's zeros
   return z;
-}
-
-// Remainder tile widths 1 .. 16, rounded up to a multiple of NGIA_REM_ROUND
-// (extra slots are padding).
-#define NGIA_REM_CASES(X) \
-  X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
-
-template <class Ring>
-__device__ __forceinline__ int tiled_rem_eqf(int rem, const Ring &ring, uint32_t s_eq_s, int base, int je, int nb1,
-                                             int cols, const uint32_t (&wc)[2], uint32_t &cw, uint32_t &ncw,
-                                             const FmaK &k) {
-  constexpr int R = NGIA_REM_ROUND;
-  switch ((rem + R - 1) / R * R) {
-#define NGIA_REM(W) \
-  case W:           \
-    if (W % R == 0) return tiled_tile_eqf<W % R == 0 ? W : 1, false, Ring>(ring, s_eq_s, base, je, nb1, cols, wc, cw, ncw, k); \
-    return 0;
-    NGIA_REM_CASES(NGIA_REM)
-#undef NGIA_REM
-    default:
-      return 0;
-  }
-}
-
-// The last tile of a block row, exactly `rem` (1..MT-1, warp-uniform) slots wide.
-template <int P, class Ring, int MT>
-__device__ __forceinline__ int tiled_rem(int rem, const Ring &ring, const uint32_t *s_pl, int base, int je, int cols,
-                                         const uint32_t (&cur)[P], uint32_t &cw, uint32_t &ncw) {
-  switch (rem) {
-#define NGIA_REM(W) \
-  case W:           \
-    if (W < MT) return tiled_tile<P, (W < MT ? W : 1), Ring>(ring, s_pl, base, je, cols, cur, cw, ncw); \
-    return 0;
-    NGIA_REM_CASES(NGIA_REM)
-#undef NGIA_REM
-    default:
-      return 0;
-  }
 }
 
 // Rep block a pair's window reaches in its first query block: blocks whose
@@ -383,9 +350,5 @@ __device__ __forceinline__ int band_advance(const Ring &ring, int i, int B, int 
   }
   return js > je ? kBandDone : kBandGo;
 }
-
-// Main tile width of the tiled kernel (16 slots; NGIA_TILED_MAIN_DNA for DNA).
-__host__ __device__ constexpr int tiled_main(int P) { return P == 2 ? NGIA_TILED_MAIN_DNA : 16; }
-__host__ __device__ constexpr int tiled_min_blocks(int P) { return P == 2 ? NGIA_TILED_BLOCKS_DNA : 2; }
 
 }  // namespace ngia

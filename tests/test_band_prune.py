@@ -127,3 +127,23 @@ def test_pruned_band_gives_the_oracles_accepted_scores(db_type, s):
             need = min(min(2 * B + 1, nb1) if B >= 0 else 0, max(0, L2 - cut) // 32 + max(0, L1 - cut) // 32 + 3)
             assert widest <= need, (a, b, widest, need)
     assert accepted > 20
+
+
+@pytest.mark.parametrize("cap,widest", [(64, 48), (128, 112)])
+def test_row_indices_stay_inside_the_shared_rows(cap, widest):
+    """SmemRing::fit (tile.cuh) restated: every row a tile touches, and the row
+    of the block that enters next, lie within the CAP rows of a lane."""
+    rng = np.random.default_rng(cap)
+    for _ in range(300):
+        off, js, je = 0, 0, int(rng.integers(0, widest))
+        for _ in range(150):
+            slots = int(rng.integers(je - js + 1, widest + 1))  # the warp's widest window
+            if not js - off + slots < cap:
+                assert je - off < cap
+                off = js
+            assert js >= off and js + slots - 1 - off < cap
+            js = min(js + int(rng.integers(0, 4)), je)
+            je -= int(rng.integers(0, je - js + 1)) if rng.random() < 0.2 else 0
+            if rng.random() < 0.8 and je - js + 1 < widest:
+                je += 1
+                assert je - off < cap
