@@ -132,7 +132,9 @@ __device__ __forceinline__ void finish_pair(const DevDB &db, const RunBufs &rb, 
     return;
   }
   bool pass = !(sum < cutoff);
-  if (pass && h.word_after) {
+  if (pass && h.word_after && cand == h.rep) {  // every word of its own
+    pass = !(max(0, h.net1 - prm.w + 1) < word_min(L2, prm.w, prm.s));
+  } else if (pass && h.word_after) {
     // short-word test of func.cu:376-396, evaluated only for aligned members
     int ws = 0;
     {
@@ -277,8 +279,11 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
         n_cells += (unsigned long long)band_cells(B, nb1, net2);
         atomicAdd(&s_qw, (unsigned long long)(nq * P));
       }
-      if (B < 0 || je < 0 || nq == 0) {
-        finish_pair<P>(db, rb, prm, h, score_mode, entry, cand, 0, cutoff, L2, net2, qpl, s_list, n_members);
+      // a sequence against itself: the band holds the diagonal, so the count
+      // is its net length (the reference's job list holds the representative)
+      const bool self = cand == h.rep && !score_mode;
+      if (B < 0 || je < 0 || nq == 0 || self) {
+        finish_pair<P>(db, rb, prm, h, score_mode, entry, cand, self ? h.net1 : 0, cutoff, L2, net2, qpl, s_list, n_members);
         state = -1;
         busy = false;
       } else {
@@ -375,7 +380,10 @@ __global__ void __launch_bounds__(kAlignThreads)
       atomicAdd(&s_qw, (unsigned long long)(nq * P));
     }
     int sum = 0;  // no band: score 0
-    if (B >= 0 && nb1 > 0 && nq > 0) {
+    const bool self = cand == h.rep && !score_mode;
+    if (self) {
+      sum = h.net1;  // the band holds the diagonal
+    } else if (B >= 0 && nb1 > 0 && nq > 0) {
       const int cut = score_mode ? kNoCut : cutoff;
       int lo, hi;
       if (!wave_band(B, h.net1, net2, cut, lo, hi)) continue;
@@ -387,7 +395,9 @@ __global__ void __launch_bounds__(kAlignThreads)
       continue;
     }
     bool pass = !(sum < cutoff);
-    if (pass && h.word_after && threadIdx.x / 32 == group * NW) {  // short-word test (func.cu:376-396): the group's first warp
+    if (pass && h.word_after && self) {
+      pass = !(max(0, net2 - prm.w + 1) < word_min(L2, prm.w, s));
+    } else if (pass && h.word_after && threadIdx.x / 32 == group * NW) {  // short-word test (func.cu:376-396): the group's first warp
       pass = !(word_count_warp_bits<P>(qpl, net2, prm.w, s_list) < word_min(L2, prm.w, s));
     }
     if (lead && pass) {

@@ -9,6 +9,7 @@
 //   ngia_close           finish (767-781)
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -164,7 +165,7 @@ int build_graph(ngia_ctx *c) {
 
 bool same_params(const ngia::RunParams &a, const ngia::RunParams &b) {
   return a.s == b.s && a.w == b.w && a.precise == b.precise && a.word_order == b.word_order && a.refill == b.refill &&
-         a.wait_polls == b.wait_polls;
+         a.wait_polls == b.wait_polls && a.word_can == b.word_can;
 }
 
 // The captured loop for the context's current parameters and tuning,
@@ -174,6 +175,14 @@ int ensure_graph(ngia_ctx *c) {
       c->graph_tune_gen == c->tune_gen)
     return NGIA_OK;
   return build_graph(c);
+}
+
+// Whether the short-word test can be worth doing first for some
+// representative of the database: the expected share of all words in the set
+// of its shortest record is below what a candidate needs.
+int word_can_pay(int type, int shortest, const ngia::RunParams &prm) {
+  const double words = std::max(0, shortest - prm.w + 1);
+  return !prm.precise && 1.0 - std::exp(-words / ngia::word_space(type, prm.w)) < ngia::word_need(prm);
 }
 
 int validate_params(int type, const ngia_params *p) {
@@ -264,6 +273,7 @@ int load_db(ngia_ctx *c, const ngia_db_view *v) {
   if (e != cudaSuccess) return fail(NGIA_E_CUDA, "ngia_open: copy: %s", cudaGetErrorString(e));
   c->n_words = v->n_words;
   c->longest = v->longest;
+  c->shortest = v->shortest;
   c->db.n = v->n;
   e = ngia::launch_loader(c, c->d_flags, c->d_flags + 1, c->d_flags + 2);
   if (e == cudaSuccess) e = cudaMemcpyAsync(c->h_flags, c->d_flags, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream);
@@ -508,6 +518,7 @@ int ngia::drv::begin_subset(ngia_ctx *c, const ngia_params *p, int32_t mode, con
   if (const char *rf = getenv("NGIA_REFILL")) c->prm.refill = std::max(1, std::min(32, atoi(rf)));
   if (!getenv("NGIA_WARP_PAIRS")) c->warp_pairs = c->tuned_warp_pairs >= 0 ? c->tuned_warp_pairs : c->warp_pairs_default;
   if (c->db.has_short && !c->prm.precise) c->prm.word_order = 1;  // exact path is word first
+  c->prm.word_can = word_can_pay(c->db.type, c->shortest, c->prm);
   // NGIA_WAIT_POLLS lowers the poll limit of the alignment kernels' staging
   // wait; at 0 every such wait gives up at once, which is how the tests make
   // the device-side error path (NGIA_E_DEVICE, context still usable) run

@@ -41,7 +41,7 @@ struct RepStore {
   const uint32_t *cnt;
   const uint32_t *lists;  // n x list_words k-mer bitsets (empty when net < 16)
   int32_t n, list_words;
-  const int32_t *count;   // when set: the representatives in use (on the device, <= n)
+  uint8_t *first;         // 1: the representative's short-word test goes before the alignment
 };
 
 // Buffers of the assignment rounds of one slot.
@@ -70,13 +70,15 @@ __host__ __device__ inline bool serve_class_used(int c, int max_nb, bool rounds)
   return c == 0 || (max_nb > (c == 2 ? kWideWindow : kSmallWindow) && (c < 3 || rounds));
 }
 
-// k-mer presence bitset of every representative (the list of k_prep).
+// k-mer presence bitset of every representative (the list of k_prep) and the
+// order of its tests.
 template <int P>
-__global__ void k_rep_lists(RepStore rs, int w, uint32_t *lists) {
+__global__ void k_rep_lists(RepStore rs, RunParams prm, uint32_t *lists) {
   __shared__ uint32_t s_list[kListWords];
-  const int r = blockIdx.x;
-  if (rs.count && r >= *rs.count) return;
+  __shared__ int s_bits;
+  const int r = blockIdx.x, w = prm.w;
   const int lw = rs.list_words;
+  if (threadIdx.x == 0) s_bits = 0;
   for (int i = threadIdx.x; i < lw; i += blockDim.x) s_list[i] = 0;
   __syncthreads();
   const uint32_t *rec = rs.words + rs.off[r];
@@ -93,7 +95,14 @@ __global__ void k_rep_lists(RepStore rs, int w, uint32_t *lists) {
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < lw; i += blockDim.x) lists[(int64_t)r * lw + i] = s_list[i];
+  int bits_set = 0;
+  for (int i = threadIdx.x; i < lw; i += blockDim.x) {
+    lists[(int64_t)r * lw + i] = s_list[i];
+    bits_set += __popc(s_list[i]);
+  }
+  if (bits_set) atomicAdd(&s_bits, bits_set);
+  __syncthreads();
+  if (threadIdx.x == 0) rs.first[r] = (uint8_t)word_first_of(P == 2 ? 0 : 1, prm, s_bits);
 }
 
 // Queues the survivors of one representative r among n_res tested queries of
@@ -134,9 +143,9 @@ __device__ __forceinline__ void queue_groups(const RoundBufs &rb, int r, int q0,
 // One CTA per representative of the chunk: composition test (and the
 // short-word test in word-first order) for every unassigned query.
 template <int P>
-__global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int r0,
-                                                      int word_first) {
-  extern __shared__ uint8_t s_res[];  // per query: 0 = out, 1 + class
+__global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int r0) {
+  extern __shared__ __align__(16) uint32_t s_list[];  // the representative's k-mer bitset, then per query:
+  uint8_t *s_res = reinterpret_cast<uint8_t *>(s_list + rs.list_words);  // 0 = out, 1 + class
   __shared__ uint32_t s_rc[28], s_cnt[kServeClasses], s_base[kServeClasses], s_pos[kServeClasses];
   constexpr int A = P == 2 ? 4 : 28;
   const int r = r0 + blockIdx.x;
@@ -146,8 +155,11 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
   __syncthreads();
   const int L1 = (int)rec[0], net1 = (int)rec[1], nb1 = (net1 + 31) / 32;
   const float s = prm.s;
-  const bool word_here = word_first && !prm.precise && net1 >= 16;
-  const uint32_t *rlist = rs.lists + (int64_t)r * rs.list_words;
+  const bool word_here = !prm.precise && net1 >= 16 && rs.first[r];
+  if (word_here) {
+    for (int t = threadIdx.x; t < rs.list_words; t += blockDim.x) s_list[t] = rs.lists[(int64_t)r * rs.list_words + t];
+    __syncthreads();
+  }
   const int n = qdb.n, nbw = (n + 31) / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int wi = warp; wi < nbw; wi += blockDim.x >> 5) {
@@ -162,10 +174,7 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
       bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cut);
       if (pass && word_here) {
         const int net2 = __ldg(qdb.net + q);
-        if (net2 >= 16) {
-          const uint32_t *planes = qdb.words + __ldg(qdb.off + q) + qdb.hw;
-          pass = !(word_count<P>(planes, net2, prm.w, rlist) < word_min(L2, prm.w, s));
-        }
+        if (net2 >= 16) pass = !(word_count_cand<P>(qdb, q, net2, prm.w, KmerBits{s_list}) < word_min(L2, prm.w, s));
       }
       if (pass) res = 1 + serve_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1));
     }
@@ -213,7 +222,7 @@ __host__ __device__ constexpr int round_table_blocks(int max_nb) {
 // the planes.
 template <int P, int RING, bool MASK, bool QROWS>
 __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
-    k_round_align(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int word_after, int wave_pairs,
+    k_round_align(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int wave_pairs,
                   uint32_t *scratch, int64_t scratch_words, int ring_rows, int table_blocks) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint32_t s_qn;
@@ -244,6 +253,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   const int hw = qdb.hw;
   unsigned long long n_pairs = 0, n_cells = 0;
   int staged = -1, L1 = 0, net1 = 0, nb1 = 0;  // the warp's representative
+  bool word_after = false;  // the short-word test follows the alignment
   const uint32_t *rpl = nullptr;
   bool table = false;
   for (;;) {
@@ -259,6 +269,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       net1 = (int)rrec[1];
       nb1 = (net1 + 31) >> 5;
       rpl = rrec + hw;
+      word_after = !prm.precise && net1 >= 16 && !rs.first[r];
       staged = r;
       if constexpr (kTable) {
         table = nb1 + kEqPad <= table_blocks;
@@ -286,7 +297,12 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
       cutoff = cutoff_of(L2, s);
       qpl = qdb.words + __ldg(qdb.off + x) + hw;
       active = B >= 0 && nb1 > 0 && net2 > 0;
-      if (!active && !(0 < cutoff)) round_accept<MASK>(rb, r, q, 0);  // no band: score 0
+      if (MASK && q == r) {  // a candidate against itself: the band holds the diagonal (align.cu)
+        active = false;
+        if (!(net1 < cutoff) && !(word_after && net1 - prm.w + 1 < word_min(L2, prm.w, s))) round_accept<MASK>(rb, r, q, net1);
+      } else if (!active && !(0 < cutoff)) {
+        round_accept<MASK>(rb, r, q, 0);  // no band: score 0
+      }
     }
     const uint32_t *rp = QROWS ? qpl : rpl, *cp = QROWS ? rpl : qpl;
     const int nr = QROWS ? net2 : net1, nbr = (nr + 31) >> 5;
@@ -332,7 +348,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
         int sum = frozen;
         for (int j = js; j <= je; j++) sum += __popc(~ring[j] & (j == nbr - 1 ? vlast : 0xFFFFFFFFu));
         bool pass = !(sum < cutoff);
-        if (pass && word_after && net1 >= 16 && net2 >= 16)
+        if (pass && word_after && net2 >= 16)
           pass = !(word_count<P>(qpl, net2, prm.w, rs.lists + (int64_t)r * rs.list_words) < word_min(L2, prm.w, s));
         if (pass) round_accept<MASK>(rb, r, q, sum);
         active = false;
@@ -359,8 +375,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
 // Shared memory: match table | code rings, or rep codes | match tables.
 template <int P, int NW, int WMAX, bool MASK>
 __global__ void __launch_bounds__(kAlignThreads)
-    k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int word_after, int wave_pairs,
-                 int cap_blocks) {
+    k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int wave_pairs, int cap_blocks) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr bool kQ = NW == 0;
   constexpr int GS = kQ ? kQueryGroup : 32 * NW, kGroups = kAlignThreads / GS;
@@ -375,6 +390,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   const int hw = qdb.hw, lane = threadIdx.x & 31;
   unsigned long long n_pairs = 0, n_cells = 0;
   int staged = -1, L1 = 0, net1 = 0, nb1 = 0;
+  bool word_after = false;  // the short-word test follows the alignment
   for (uint32_t e0 = blockIdx.x * kGroups; e0 < qn; e0 += gridDim.x * kGroups) {
     const int2 first = rb.queue[cls][e0];  // entries of one group: the padding comes last
     if (first.y < 0) continue;             // CTA-uniform
@@ -385,6 +401,7 @@ __global__ void __launch_bounds__(kAlignThreads)
       L1 = (int)rrec[0];
       net1 = (int)rrec[1];
       nb1 = (net1 + 31) >> 5;
+      word_after = !prm.precise && net1 >= 16 && !rs.first[r];
       const uint32_t vlast = (net1 & 31) ? ((1u << (net1 & 31)) - 1u) : 0xFFFFFFFFu;
       if constexpr (kQ) {
         for (int b = threadIdx.x; b < nb1; b += kAlignThreads) {
@@ -404,6 +421,7 @@ __global__ void __launch_bounds__(kAlignThreads)
     int L2 = 0, net2 = 0, nq = 0, B = 0, cutoff = 1, lo = 0, hi = 0, sum = 0;
     const uint32_t *qpl = qdb.words;
     // (a key can change while the group's threads look at it: one answer)
+    const bool self = MASK && q == r;  // a candidate against itself: the band holds the diagonal (align.cu)
     bool have = q >= 0 && (MASK || (rb.key[q] >> 32) > (unsigned long long)r), run = false;
     if constexpr (!MASK) {
       if constexpr (NW == 4)
@@ -419,7 +437,9 @@ __global__ void __launch_bounds__(kAlignThreads)
       B = band_blocks(L1, L2, s);
       cutoff = cutoff_of(L2, s);
       qpl = qdb.words + __ldg(qdb.off + x) + hw;
-      if (B >= 0 && nb1 > 0 && nq > 0) {
+      if (self) {
+        sum = net1;
+      } else if (B >= 0 && nb1 > 0 && nq > 0) {
         run = wave_band(B, net1, net2, cutoff, lo, hi);
         have = run;
         if (lead) n_pairs++;
@@ -436,7 +456,7 @@ __global__ void __launch_bounds__(kAlignThreads)
     }
     n_cells += 32 * cells;
     bool pass = have && !(sum < cutoff);
-    if (word_after && net1 >= 16) {  // short-word test (func.cu:376-396), a warp per member
+    if (word_after) {  // short-word test (func.cu:376-396), a warp per member
       const uint32_t *list = rs.lists + (int64_t)r * rs.list_words;
 #pragma unroll
       for (int k = 0; k < (kQ ? 2 : 1); k++) {
@@ -461,8 +481,8 @@ __global__ void __launch_bounds__(kAlignThreads)
 }
 
 // ---- launch ---------------------------------------------------------------------
-using RoundAlignFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, uint32_t *, int64_t, int, int);
-using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, int);
+using RoundAlignFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, uint32_t *, int64_t, int, int);
+using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int);
 
 template <int P, bool MASK>
 RoundAlignFn round_align_fn(int cls) {
@@ -553,23 +573,23 @@ cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
 // the round's pair counts decide on the device which of the two works.
 template <bool MASK>
 cudaError_t round_launch(const RoundPlan &pl, const DevDB &qdb, const RepStore &rs, const RunParams &prm,
-                         const RoundBufs &rb, int word_after, cudaStream_t st) {
+                         const RoundBufs &rb, cudaStream_t st) {
   for (int c = 0; c < kServeClasses; c++) {
     if (!serve_class_used(c, pl.rep_nb, MASK)) continue;
     DevDB db = qdb;
     RepStore r = rs;
     RunParams p = prm;
     RoundBufs b = rb;
-    int cls = c, wa = word_after, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb;
+    int cls = c, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb;
     uint32_t *scr = pl.scratch;
     int64_t sw = pl.scratch_words;
     int rm = pl.ring_rows;
-    void *args[] = {&db, &r, &p, &b, &cls, &wa, &wp, &scr, &sw, &rm, &tb};
+    void *args[] = {&db, &r, &p, &b, &cls, &wp, &scr, &sw, &rm, &tb};
     cudaError_t e = cudaLaunchKernel(round_fn<MASK>(pl.type, c, false), dim3(pl.grid[c]), dim3(kAlignThreads), args,
                                      round_align_smem(pl.type, c, pl.rep_nb), st);
     if (e != cudaSuccess) return e;
     if (wp <= 0) continue;
-    void *wargs[] = {&db, &r, &p, &b, &cls, &wa, &wp, &cap};
+    void *wargs[] = {&db, &r, &p, &b, &cls, &wp, &cap};
     e = cudaLaunchKernel(round_fn<MASK>(pl.type, c, true), dim3(pl.wave_grid[c]), dim3(kAlignThreads), wargs,
                          round_wave_smem(pl.type, c, pl.rep_nb), st);
     if (e != cudaSuccess) return e;

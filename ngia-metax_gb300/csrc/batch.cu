@@ -78,7 +78,7 @@ void destroy_batch_graph(ngia_batch *b) {
 
 bool same_prm(const ngia::RunParams &a, const ngia::RunParams &b) {
   return a.s == b.s && a.w == b.w && a.precise == b.precise && a.word_order == b.word_order && a.refill == b.refill &&
-         a.wait_polls == b.wait_polls;
+         a.wait_polls == b.wait_polls && a.word_can == b.word_can;
 }
 
 // Captures every job's iteration into the body of its own conditional WHILE

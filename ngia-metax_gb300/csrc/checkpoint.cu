@@ -174,6 +174,7 @@ extern "C" int ngia_cluster_resume(ngia_ctx *c, const char *path, int32_t mode) 
   c->prm.precise = h.precise;
   c->prm.word_order = h.word_order;
   c->prm.refill = h.refill;
+  c->prm.word_can = ngia::drv::word_can_pay(c->db.type, c->shortest, c->prm);
   st.iter_limit = INT64_MAX;
   *c->h_state = st;
   cudaError_t e = cudaMemcpyAsync(c->rb.st, c->h_state, sizeof(st), cudaMemcpyHostToDevice, c->stream);

@@ -23,7 +23,7 @@ struct ngia_ctx {
   uint32_t *d_cnt = nullptr;
   uint32_t *d_codes = nullptr;  // protein residue-code streams (DevDB::codes)
   int64_t n_words = 0;
-  int32_t longest = 0;
+  int32_t longest = 0, shortest = 0;
   // capacity of the allocations (a context can be reloaded with any database
   // within it: serving slots)
   int64_t cap_n = 0, cap_words = 0;
@@ -92,6 +92,7 @@ int pull_state(ngia_ctx *c);
 int enqueue_iteration(ngia_ctx *c, bool graph, cudaGraphConditionalHandle cond);
 void fill_stats(const ngia_ctx *c, ngia_stats *stats);
 int validate_params(int type, const ngia_params *p);
+int word_can_pay(int type, int shortest, const ngia::RunParams &prm);
 // spec.cu: speculative rounds (NGIA_MODE_SPEC)
 int spec_prepare(ngia_ctx *c);                 // buffers for the context's capacity; zeroed masks
 int spec_step(ngia_ctx *c, int64_t max_iters);  // up to max_iters representatives (<= 0: all)

@@ -121,7 +121,7 @@ __global__ void k_init_run(DevDB db, RunBufs rb, RunParams prm) {
     st->iter_limit = LLONG_MAX;
     for (int k = 0; k < kNumClasses; k++) st->qcount[k] = st->qhead[k] = 0;
     st->long_count = 0;
-    st->word_first = word_first_of(db.type, prm);
+    st->word_first = 0;
     st->word_active = 0;
     st->rep_nb = st->rep_len = st->rep_net = 0;
     st->st_candidates = st->st_base_pass = st->st_align_pairs = st->st_members = 0;
@@ -282,7 +282,7 @@ __device__ __forceinline__ void flush_stats(const RunBufs &rb, unsigned long lon
 #define NGIA_FILTER_HOIST 0
 #endif
 template <int P, int kFilterWordsPerWarp, bool kWord = true>
-__global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams prm, int exact) {
+__global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams prm, int exact, int turn) {
   constexpr int kFilterTileWords = 8 * kFilterWordsPerWarp;  // 256 threads
   RunState *st = rb.st;
   extern __shared__ __align__(16) uint32_t s_list[];
@@ -293,10 +293,11 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
   constexpr int A = P == 2 ? 4 : 28;
   if (threadIdx.x == 0) {
     const bool skip = st->done || st->iter >= st->iter_limit || st->err;
-    s_hdr[0] = skip;
+    const int word = (!exact && st->word_first && st->word_active) ? 1 : 0;
+    s_hdr[0] = skip || (turn >= 0 && turn != word);
     s_hdr[1] = st->rep_len;
     s_hdr[2] = st->rep_nb;
-    s_hdr[3] = (!exact && st->word_first && st->word_active) ? 1 : 0;
+    s_hdr[3] = word;
   }
   if (threadIdx.x < A) s_rc[threadIdx.x] = rb.rep_rec[2 + threadIdx.x];
   __syncthreads();
@@ -328,11 +329,12 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
   if (word_here && NGIA_FILTER_WARP_WORD) {
     // Short-word test here: the work per candidate grows with its length, so
     // warps run independently — each takes every W-th bitmap word of the
-    // length-sorted database (a share of every length) and queues its
-    // survivors with one atomic per class and word; no CTA barrier makes a
-    // warp wait for the CTA's longest candidates.
+    // length-sorted database, a CTA's warps words gridDim.x apart (a share of
+    // every length for each SM) — and queues its survivors with one atomic
+    // per class and word; no CTA barrier makes a warp wait for the CTA's
+    // longest candidates.
     const int W = gridDim.x * (blockDim.x >> 5);
-    for (int wi = blockIdx.x * (blockDim.x >> 5) + warp; wi < nbw; wi += W) {
+    for (int wi = warp * gridDim.x + blockIdx.x; wi < nbw; wi += W) {
       const uint32_t bits = rb.alive[wi];
       if (!bits) continue;  // warp-uniform
       const int c = wi * 32 + lane;
@@ -658,12 +660,16 @@ cudaError_t launch_filter(ngia_ctx *c) {
   const int grid_b = std::max(1, std::min(c->grid_filter, (nbw + 8 * kB - 1) / (8 * kB)));
   const int grid_w = std::max(1, std::min(c->grid_filter, (nbw + 8 * kW - 1) / (8 * kW)));
   if (!exact) {
-    // word-first order also holds the byte table (8 bytes per bitset byte)
-    if (word_first_of(c->db.type, c->prm)) {
+    // The instance with the short-word test, the one without, or (automatic
+    // order, when either may be wanted) both: the representative's order
+    // decides on the device which works.
+    const bool word = c->prm.word_order == 1 || (c->prm.word_order == 0 && c->prm.word_can);
+    const int turn = c->prm.word_order == 0 && c->prm.word_can ? 1 : -1;
+    if (word) {  // also holds the byte table (8 bytes per bitset byte)
       if (P == 2)
-        k_filter<2, kW><<<grid_w, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm, 0);
+        k_filter<2, kW><<<grid_w, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm, 0, turn);
       else
-        k_filter<5, kW><<<grid_w, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm, 0);
+        k_filter<5, kW><<<grid_w, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm, 0, turn);
       if (NGIA_FILTER_WARP_WORD && c->db.max_nb * 32 > kWarpWordLen) {  // some record is long
         const int grid_l = std::max(1, std::min(c->grid_filter, c->num_sms));
         if (P == 2)
@@ -671,23 +677,27 @@ cudaError_t launch_filter(ngia_ctx *c) {
         else
           k_filter_long<5><<<grid_l, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm);
       }
-    } else if (c->filter_tile == kW) {  // the tuner's choice: one bitmap word per warp and tile
-      if (P == 2)
-        k_filter<2, kW, !NGIA_FILTER_SPLIT><<<grid_w, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0);
-      else
-        k_filter<5, kW, !NGIA_FILTER_SPLIT><<<grid_w, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0);
-    } else {
-      if (P == 2)
-        k_filter<2, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0);
-      else
-        k_filter<5, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0);
+    }
+    if (!word || turn >= 0) {
+      const int other = turn >= 0 ? 0 : -1;
+      if (c->filter_tile == kW) {  // the tuner's choice: one bitmap word per warp and tile
+        if (P == 2)
+          k_filter<2, kW, !NGIA_FILTER_SPLIT><<<grid_w, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
+        else
+          k_filter<5, kW, !NGIA_FILTER_SPLIT><<<grid_w, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
+      } else {
+        if (P == 2)
+          k_filter<2, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
+        else
+          k_filter<5, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
+      }
     }
     return cudaGetLastError();
   }
   if (P == 2)
-    k_filter<2, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 1);
+    k_filter<2, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 1, -1);
   else
-    k_filter<5, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 1);
+    k_filter<5, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 1, -1);
   k_scan_words<<<1, 1024, 0, c->stream>>>(reinterpret_cast<const uint32_t *>(c->rb.flags), nbw, c->rb.scan_part);
   k_first_short<<<64, 256, 0, c->stream>>>(c->db, c->rb, 1);
   k_first_short<<<c->num_sms * 2, 256, 0, c->stream>>>(c->db, c->rb, 0);

@@ -450,11 +450,16 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P)) k_pool_ali
         n_pairs++;
         n_cells += (unsigned long long)band_cells(B, nb1, net2);
         atomicAdd(&s_qw, (unsigned long long)(nq * P));
-        if (B < 0 || je < 0 || nq == 0) {
+        const bool self = cand == rep;  // the band holds the diagonal: its net length (align.cu)
+        if (B < 0 || je < 0 || nq == 0 || self) {
           // no band: score 0 (func.cu never updates the rows)
-          if (!(0 < cutoff) && !(word_after && word_count<P>(qpl, net2, w, s_list) < word_min(L2, w, s))) {
+          const int sum = self ? net1 : 0;
+          bool pass = !(sum < cutoff);
+          if (pass && word_after)
+            pass = !((self ? max(0, net1 - w + 1) : word_count<P>(qpl, net2, w, s_list)) < word_min(L2, w, s));
+          if (pass) {
             cluster[cand] = rep;
-            ident[cand] = 0;
+            ident[cand] = sum;
             atomicAnd(&alive[cand >> 5], ~(1u << (cand & 31)));
             n_members++;
           }

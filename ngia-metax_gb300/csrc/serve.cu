@@ -159,9 +159,9 @@ struct ngia_server {
   int device = 0, type = 0, num_sms = 0;
   ngia_params params{};
   ngia::RunParams prm{};
-  int word_first = 0;
   ngia_ctx *reps = nullptr;  // the resident representatives' database
   uint32_t *d_lists = nullptr;
+  uint8_t *d_first = nullptr;  // the order of each representative's tests
   ngia::RepStore store{};
   int64_t cap_n = 0, cap_words = 0;
   int32_t cap_nb = 0;
@@ -201,7 +201,6 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
   RoundBufs rb = sl.rb;
   k_serve_init<<<std::max(1, std::min(c->num_sms, (n + 255) / 256)), 256, 0, st>>>(n, rb);
   CKS(cudaGetLastError());
-  const int word_after = !sv->word_first && !sv->prm.precise;
   // Representatives per round: kFirstChunk doubling up to kMaxChunk, and more
   // while the unassigned queries are few, so that a round holds at least
   // kFirstPairs (later kMaxPairs) pairs: a round takes a pair's latency
@@ -216,6 +215,7 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
     const char *m = getenv("NGIA_SERVE_MAX_CHUNK");
     return m ? std::max(kFirstChunk, std::min(kMaxChunk, atoi(m))) : INT_MAX;
   }();
+  const size_t fsm = 4 * (size_t)sv->store.list_words + (size_t)nbw * 32;
   int r0 = 0, chunk = kFirstChunk;
   int64_t pairs = kFirstPairs;
   uint32_t left = (uint32_t)n;
@@ -230,12 +230,12 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
     CKS(cudaMemsetAsync(rb.ctl, 0, kCtlWords * sizeof(uint32_t), st));
     if (ev[0]) cudaEventRecord(ev[0], st);
     if (sv->type == 0)
-      k_serve_filter<2><<<nr, 256, (size_t)nbw * 32, st>>>(c->db, sv->store, sv->prm, rb, r0, sv->word_first);
+      k_serve_filter<2><<<nr, 256, fsm, st>>>(c->db, sv->store, sv->prm, rb, r0);
     else
-      k_serve_filter<5><<<nr, 256, (size_t)nbw * 32, st>>>(c->db, sv->store, sv->prm, rb, r0, sv->word_first);
+      k_serve_filter<5><<<nr, 256, fsm, st>>>(c->db, sv->store, sv->prm, rb, r0);
     CKS(cudaGetLastError());
     if (ev[1]) cudaEventRecord(ev[1], st);
-    CKS(round_launch<false>(sl.plan, c->db, sv->store, sv->prm, rb, word_after, st));
+    CKS(round_launch<false>(sl.plan, c->db, sv->store, sv->prm, rb, st));
     if (ev[2]) cudaEventRecord(ev[2], st);
     k_serve_round_end<<<std::max(1, std::min(c->num_sms, (nbw + 255) / 256)), 256, 0, st>>>(n, rb);
     CKS(cudaGetLastError());
@@ -407,6 +407,7 @@ void destroy(ngia_server *sv) {
   for (auto &sl : sv->slots) free_slot(*sl);
   if (sv->reps) ngia_close(sv->reps);
   cudaFree(sv->d_lists);
+  cudaFree(sv->d_first);
   delete sv;
 }
 
@@ -456,7 +457,8 @@ extern "C" int ngia_serve_open(const ngia_db_view *reps, const ngia_params *para
   // queries/s
   sv->prm.refill = 32;
   if (const char *rf = getenv("NGIA_SERVE_REFILL")) sv->prm.refill = std::max(1, std::min(32, atoi(rf)));
-  sv->word_first = ngia::word_first_of(sv->type, sv->prm);
+  // representatives of a resident set come in any length: each its own order
+  sv->prm.word_can = !sv->prm.precise && ngia::word_need(sv->prm) > 0.0;
   sv->cap_n = cf.max_batch;
   sv->cap_words = cf.max_batch_words;
   sv->cap_nb = cf.max_record_blocks;
@@ -469,16 +471,17 @@ extern "C" int ngia_serve_open(const ngia_db_view *reps, const ngia_params *para
   const int bits = sv->type ? 5 : 2;
   const int lw = std::max(1, (int)((1u << (params->word_length * bits)) / 32u));
   ngia_ctx *rc_ctx = sv->reps;
-  if (cudaMalloc((void **)&sv->d_lists, 4 * (size_t)lw * (size_t)reps->n) != cudaSuccess) {
+  if (cudaMalloc((void **)&sv->d_lists, 4 * (size_t)lw * (size_t)reps->n) != cudaSuccess ||
+      cudaMalloc((void **)&sv->d_first, (size_t)reps->n) != cudaSuccess) {
     ngia::destroy(sv);
     return fail(NGIA_E_NOMEM, "ngia_serve_open: k-mer table allocation failed");
   }
   sv->store = ngia::RepStore{rc_ctx->db.words, rc_ctx->db.off, rc_ctx->db.len, rc_ctx->db.net, rc_ctx->db.cnt,
-                             sv->d_lists, rc_ctx->db.n, lw};
+                             sv->d_lists, rc_ctx->db.n, lw, sv->d_first};
   if (sv->type == 0)
-    ngia::k_rep_lists<2><<<reps->n, 256, 0, rc_ctx->stream>>>(sv->store, params->word_length, sv->d_lists);
+    ngia::k_rep_lists<2><<<reps->n, 256, 0, rc_ctx->stream>>>(sv->store, sv->prm, sv->d_lists);
   else
-    ngia::k_rep_lists<5><<<reps->n, 256, 0, rc_ctx->stream>>>(sv->store, params->word_length, sv->d_lists);
+    ngia::k_rep_lists<5><<<reps->n, 256, 0, rc_ctx->stream>>>(sv->store, sv->prm, sv->d_lists);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(rc_ctx->stream);
   if (e != cudaSuccess) {
@@ -489,6 +492,10 @@ extern "C" int ngia_serve_open(const ngia_db_view *reps, const ngia_params *para
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   const int64_t budget = cf.memory_budget > 0 ? cf.memory_budget : (int64_t)(free_b / 2);
+  const size_t fsm = 4 * (size_t)lw + (size_t)((sv->cap_n + 31) / 32 * 32);
+  if (fsm > 48 * 1024)
+    cudaFuncSetAttribute(sv->type == 0 ? (const void *)ngia::k_serve_filter<2> : (const void *)ngia::k_serve_filter<5>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(fsm, 226 * 1024));
   ngia::RoundPlan plan;
   e = ngia::round_plan<false>(plan, sv->type, rc_ctx->db.max_nb, sv->num_sms);
   if (e != cudaSuccess) {

@@ -79,6 +79,7 @@ struct SpecDev {
   SpecCtl *ctl;
   int64_t *rs_off;          // record offsets of the candidates (the RepStore's off)
   uint32_t *lists;          // k-mer bitsets of the candidates
+  uint8_t *first;           // and the order of their tests
 };
 
 // Round start (one CTA of 1,024 threads): lists the unclustered set (its
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(1024) k_spec_pick(DevDB db, RunBufs run, SpecD
 constexpr int kSpecTile = 1024;
 template <int P>
 __global__ void __launch_bounds__(256) k_spec_filter(DevDB db, SpecDev sd, RoundBufs rb, RunParams prm,
-                                                      int word_first, int list_words) {
+                                                      int list_words) {
   constexpr int A = P == 2 ? 4 : 28;
   extern __shared__ uint32_t s_list[];  // the candidate's k-mer bitset (word-first order)
   __shared__ uint32_t s_rc[A], s_cnt[kServeClasses], s_base[kServeClasses], s_pos[kServeClasses];
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(256) k_spec_filter(DevDB db, SpecDev sd, Round
   const int n = min(kSpecTile, alive - p0);
   const uint32_t *rec = db.words + sd.rs_off[i];
   const int L1 = (int)rec[0], net1 = (int)rec[1], nb1 = (net1 + 31) / 32;
-  const bool word_here = word_first && !prm.precise && net1 >= 16;
+  const bool word_here = !prm.precise && net1 >= 16 && sd.first[i];
   if (threadIdx.x < A) s_rc[threadIdx.x] = rec[2 + threadIdx.x];
   if (threadIdx.x < kServeClasses) s_cnt[threadIdx.x] = 0;
   if (word_here)
@@ -313,7 +314,7 @@ int spec_alloc(ngia_ctx *c) {
   sp->k_max = (int)std::max<int64_t>(1, std::min<int64_t>(kSpecMax, kSpecScoreWords / std::max<int64_t>(1, n)));
   const int lw = kListWords;
   if (dmalloc(&sp->d.list, (size_t)n) != cudaSuccess || dmalloc(&sp->d.rs_off, kSpecMax) != cudaSuccess ||
-      dmalloc(&sp->d.lists, (size_t)kSpecMax * lw) != cudaSuccess || dmalloc(&sp->d_ctl, kCtlBytes) != cudaSuccess ||
+      dmalloc(&sp->d.lists, (size_t)kSpecMax * lw) != cudaSuccess || dmalloc(&sp->d.first, kSpecMax) != cudaSuccess || dmalloc(&sp->d_ctl, kCtlBytes) != cudaSuccess ||
       cudaMallocHost((void **)&sp->h_ctl, kCtlBytes) != cudaSuccess ||
       dmalloc(&sp->rb.mask, (size_t)n) != cudaSuccess ||
       dmalloc(&sp->rb.score, (size_t)sp->k_max * (size_t)n) != cudaSuccess ||
@@ -352,23 +353,22 @@ int spec_launch_round(ngia_ctx *c, bool lists, int k, int alive) {
   cudaStream_t st = c->stream;
   const int P = c->db.type ? 5 : 2;
   const int lw = (int)std::max<uint32_t>(1u, (1u << (c->prm.w * (P == 2 ? 2 : 5))) / 32u);
-  const RepStore rs{c->db.words, sp->d.rs_off, nullptr, nullptr, nullptr, sp->d.lists, kSpecMax, lw, nullptr};
+  const RepStore rs{c->db.words, sp->d.rs_off, nullptr, nullptr, nullptr, sp->d.lists, kSpecMax, lw, sp->d.first};
   if (lists) {
     if (P == 2)
-      k_rep_lists<2><<<k, 256, 0, st>>>(rs, c->prm.w, sp->d.lists);
+      k_rep_lists<2><<<k, 256, 0, st>>>(rs, c->prm, sp->d.lists);
     else
-      k_rep_lists<5><<<k, 256, 0, st>>>(rs, c->prm.w, sp->d.lists);
+      k_rep_lists<5><<<k, 256, 0, st>>>(rs, c->prm, sp->d.lists);
     CKP(cudaGetLastError());
   }
-  const int word_first = word_first_of(c->db.type, c->prm);
   const dim3 fgrid((alive + kSpecTile - 1) / kSpecTile, k);
-  const size_t fsm = word_first && lists ? 4 * (size_t)lw : 0;
+  const size_t fsm = lists ? 4 * (size_t)lw : 0;
   if (P == 2)
-    k_spec_filter<2><<<fgrid, 256, fsm, st>>>(c->db, sp->d, sp->rb, c->prm, word_first, lw);
+    k_spec_filter<2><<<fgrid, 256, fsm, st>>>(c->db, sp->d, sp->rb, c->prm, lw);
   else
-    k_spec_filter<5><<<fgrid, 256, fsm, st>>>(c->db, sp->d, sp->rb, c->prm, word_first, lw);
+    k_spec_filter<5><<<fgrid, 256, fsm, st>>>(c->db, sp->d, sp->rb, c->prm, lw);
   CKP(cudaGetLastError());
-  CKP(round_launch<true>(sp->plan, c->db, rs, c->prm, sp->rb, !word_first && !c->prm.precise, st));
+  CKP(round_launch<true>(sp->plan, c->db, rs, c->prm, sp->rb, st));
   k_spec_assign<<<(alive + 255) / 256, 256, 0, st>>>(c->rb, sp->d, sp->rb);
   CKP(cudaGetLastError());
   return spec_pick(c);
@@ -409,6 +409,7 @@ void spec_free(ngia_ctx *c) {
   cudaFree(sp->d.list);
   cudaFree(sp->d.rs_off);
   cudaFree(sp->d.lists);
+  cudaFree(sp->d.first);
   cudaFree(sp->d_ctl);
   if (sp->h_ctl) cudaFreeHost(sp->h_ctl);
   cudaFree(sp->rb.mask);

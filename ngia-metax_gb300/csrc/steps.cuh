@@ -27,9 +27,10 @@ constexpr int kRepPlanes = 32;
 // change); otherwise the representative is st->rep.
 __device__ __forceinline__ void prep_body(const DevDB &db, const RunBufs &rb, const RunParams &prm, int score_rep) {
   RunState *st = rb.st;
-  __shared__ int s_skip;
+  __shared__ int s_skip, s_bits;
   __shared__ uint32_t s_list[kListWords];
   if (threadIdx.x == 0) {
+    s_bits = 0;
     int skip = 0;
     if (score_rep < 0) skip = st->done || st->iter >= st->iter_limit || st->err;
     s_skip = skip;
@@ -67,9 +68,16 @@ __device__ __forceinline__ void prep_body(const DevDB &db, const RunBufs &rb, co
       atomicOr(&s_list[word >> 5], 1u << (word & 31));
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < list_words; i += blockDim.x) rb.rep_list[i] = s_list[i];
+    int bits_set = 0;
+    for (int i = threadIdx.x; i < list_words; i += blockDim.x) {
+      rb.rep_list[i] = s_list[i];
+      bits_set += __popc(s_list[i]);
+    }
+    if (bits_set) atomicAdd(&s_bits, bits_set);
+    __syncthreads();
   }
   if (threadIdx.x == 0) {
+    st->word_first = word_first_of(db.type, prm, s_bits);
     st->rep_len = L1;
     st->rep_net = net1;
     st->rep_nb = nb1;
