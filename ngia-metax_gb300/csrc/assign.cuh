@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
       bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cut);
       if (pass && word_here) {
         const int net2 = __ldg(qdb.net + q);
-        if (net2 >= 16) pass = !(word_count_cand<P>(qdb, q, net2, prm.w, KmerBits{s_list}) < word_min(L2, prm.w, s));
+        if (net2 >= 16) pass = words_reach<P, 1>(qdb, q, net2, prm.w, word_min(L2, prm.w, s), KmerBits{s_list}, s_list);
       }
       if (pass) res = 1 + serve_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1));
     }

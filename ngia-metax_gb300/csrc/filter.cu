@@ -5,9 +5,9 @@
 // Reference counterparts (CUDA/signalNode/src/func.cu):
 //   k_loader        readData device half (104-154): header arrays per sequence
 //   k_prep          updateRepresent rep copy (213-235) + generateListGen/Pro (241-302)
-//   k_filter        kernel_baseFilterGen/Pro (323-354) and kernel_wordFilterGen/Pro
-//                   (357-447) fused, survivors compacted on the device instead of
-//                   updateJobs (305-320)
+//   k_filter, k_filter_word  kernel_baseFilterGen/Pro (323-354) and
+//                   kernel_wordFilterGen/Pro (357-447) fused, survivors compacted on
+//                   the device instead of updateJobs (305-320)
 //   k_next          updateRepresent assignment/selection (190-215): the next
 //                   representative is the first unclustered sequence
 #include <algorithm>
@@ -71,19 +71,10 @@ __global__ void k_codes(const uint32_t *__restrict__ words, const int64_t *__res
     const int nb = (len[c] + 31) >> 5;
     const int64_t base = off[c] + hw;
     for (int b = lane; b < nb; b += 32) {
-      uint32_t pl[5], st[5] = {0u, 0u, 0u, 0u, 0u};
+      uint32_t pl[5], st[5];
 #pragma unroll
       for (int p = 0; p < 5; p++) pl[p] = words[base + 5 * b + p];
-#pragma unroll
-      for (int j = 0; j < 32; j++) {
-        uint32_t cj = 0;
-#pragma unroll
-        for (int p = 0; p < 5; p++) cj |= ((pl[p] >> j) & 1u) << p;
-        const int t = 155 - 5 * j;  // the code's lowest bit in the 160-bit value
-        const int k = 4 - (t >> 5), sh = t & 31;
-        st[k] |= cj << sh;
-        if (sh > 27) st[k - 1] |= cj >> (32 - sh);  // the group crosses into the word above
-      }
+      protein_stream(pl, st);
 #pragma unroll
       for (int k = 0; k < 5; k++) codes[base + 5 * b + k] = st[k];
     }
@@ -147,66 +138,6 @@ cudaError_t launch_prep(ngia_ctx *c, int score_rep) {
   return cudaGetLastError();
 }
 
-// Short-word count of one candidate by the whole warp: lane l takes blocks
-// l, l+32, ...; each lane's history (the previous block) comes from the lane
-// below by a shuffle.  All 32 lanes call it with the same arguments.
-template <int P>
-__device__ int word_count_warp(const uint32_t *__restrict__ planes, int net2, int w, const uint8_t *tab) {
-  constexpr int bits = P == 2 ? 2 : 5;
-  const uint32_t mask = (1u << (w * bits)) - 1u;
-  const int lane = threadIdx.x & 31;
-  const int nb = (net2 + 31) >> 5;
-  int sum = 0;
-  uint32_t carry[P];  // planes (DNA: the stream's low word) of the block below lane 0's
-#pragma unroll
-  for (int p = 0; p < P; p++) carry[p] = 0u;
-  for (int b0 = 0; b0 < nb; b0 += 32) {
-    const int b = b0 + lane;
-    const bool have = b < nb;
-    const int lim = have ? min(32, net2 - 32 * b) : 0;
-    uint32_t pl[P];
-#pragma unroll
-    for (int p = 0; p < P; p++) pl[p] = have ? __ldg(planes + b * P + p) : 0u;
-    if (P == 2) {
-      uint32_t hi, lo;
-      dna_stream(pl[0], pl[1], hi, lo);
-      uint32_t prev = __shfl_up_sync(kFullMask, lo, 1);
-      if (lane == 0) prev = carry[0];
-      if (lim == 32) sum += dna_block_full(prev, hi, lo, mask, tab);
-      else if (lim > 0) sum += dna_block_part(prev, hi, lo, lim, mask, tab);
-      carry[0] = __shfl_sync(kFullMask, lo, 31);
-    } else {
-      uint32_t pv[P];
-#pragma unroll
-      for (int p = 0; p < P; p++) {
-        pv[p] = __shfl_up_sync(kFullMask, pl[p], 1);
-        if (lane == 0) pv[p] = carry[p];
-      }
-      // history: the last w-1 residues of the block below
-      uint32_t word = 0;
-      for (int j = 32 - (w - 1); j < 32; j++) word = ((word << bits) | code_of<P>(pv, j)) & mask;
-      if (lim > 0) sum += roll_block<P>(pl, lim, word, mask, tab);
-#pragma unroll
-      for (int p = 0; p < P; p++) carry[p] = __shfl_sync(kFullMask, pl[p], 31);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
-  if (P == 2) return sum - dna_head(planes, net2, w, mask, tab);
-  return sum - roll_head<P>(planes, net2, w, mask, tab);
-}
-
-template <int P>
-__device__ __forceinline__ int word_count_cand_warp(const DevDB &db, int c, int net2, int w, const uint8_t *tab) {
-  const int64_t o = __ldg(db.off + c) + db.hw;
-  if (P == 5 && db.codes) return word_count_codes_warp(db.codes + o, net2, w, tab);
-  return word_count_warp<P>(db.words + o, net2, w, tab);
-}
-
-// Candidates longer than this are counted by the whole warp.
-constexpr int kWarpWordLen = 2048;
-
-
 // Adds the filter counters of the calling CTA (every thread calls it) to one
 // of kFilterStripes counter stripes; k_next folds the stripes into the run
 // state.  One warp-level and one CTA-level reduction keep the global atomics
@@ -236,237 +167,90 @@ __device__ __forceinline__ void flush_stats(const RunBufs &rb, unsigned long lon
     atomicAdd(&rb.fstats[(blockIdx.x % kFilterStripes) * kFilterStats + threadIdx.x], s_acc[threadIdx.x]);
 }
 
-// Fused filter over the unclustered set, one tile of kFilterTileWords
-// bitmap words (8 warps x kFilterWordsPerWarp words) per CTA pass: each warp takes
-// kFilterWordsPerWarp consecutive words; lanes read the header arrays of 32
-// consecutive sequences (coalesced), apply the composition test and, in
-// word-first order, the short-word test (shared-memory k-mer bitset).
-// Survivors are compacted into the alignment class queues in two levels:
-// warp-aggregated shared-memory counters give each survivor its slot inside
-// the tile, then one global atomic per class and tile reserves the tile's
-// range, so the global queue counters see ~1/1,000 of the candidates.
-// `exact` = 1 runs the composition stage only and records the survivors
+// Composition test over the unclustered set, one tile of 8 x WPW bitmap words
+// per CTA pass: each warp takes WPW consecutive words; lanes read the header
+// arrays of 32 consecutive sequences (coalesced).  Survivors are compacted
+// into the alignment class queues in two levels: warp-aggregated shared-memory
+// counters give each survivor its slot inside the tile, then one global atomic
+// per class and tile reserves the tile's range, so the global queue counters
+// see ~1/1,000 of the candidates.  `exact` = 1 records the survivors instead
 // (bitmap in rb.flags) for the exact short-word path.
-// Bitmap words per warp and tile pass.  Swept on GB300 (1M DNA s=0.85 and
-// 200k protein s=0.9): the composition test alone is fastest with 8 (fewer,
-// fuller CTAs: 20.7 us vs 23.1 us with 4), the short-word test in the filter
-// with 1 (protein 0.21 ms vs 0.24 / 0.37 / 0.61 ms with 2 / 4 / 8: more
-// tiles share the long candidates; DNA s=0.95 is the same for 1 to 4).
-#ifndef NGIA_FILTER_WPW_BASE
-#define NGIA_FILTER_WPW_BASE 8
-#endif
-#ifndef NGIA_FILTER_WPW_WORD
-#define NGIA_FILTER_WPW_WORD 1
-#endif
+// Bitmap words per warp and tile pass, swept on GB300 (1M DNA s=0.85): fastest
+// with 8 (fewer, fuller CTAs: 20.7 us vs 23.1 us with 4).
 // (Issuing every header load of a warp's 8 bitmap words before the first
-// use, unpredicated per lane, made the composition-only launch slower on
-// GB300: 24.6 vs 18.1 us per iteration, 1M DNA s=0.85.)
-// NGIA_FILTER_WARP_WORD: with the short-word test in the filter, warps take
-// bitmap words independently (no tile barriers); 0 keeps the tiled loop.
-#ifndef NGIA_FILTER_WARP_WORD
-#define NGIA_FILTER_WARP_WORD 1
-#endif
+// use, unpredicated per lane, made the launch slower on GB300: 24.6 vs 18.1 us
+// per iteration, 1M DNA s=0.85; predicated on the unclustered bit 24.2 against
+// 17.8, 80 registers with spills against 57.)
+constexpr int kFilterWords = 8;
 
-// NGIA_FILTER_SPLIT: launches that cannot run the short-word test in the
-// filter (alignment-first order, the exact short-word path) use an instance
-// compiled without it (kWord = false): each CTA runs its code once, so the
-// kernel's size is paid in instruction fetches.
-#ifndef NGIA_FILTER_SPLIT
-#define NGIA_FILTER_SPLIT 1
-#endif
-// NGIA_FILTER_HOIST: in the composition-only DNA instance, load every header
-// of the warp's words before the first test (predicated on the unclustered
-// bit).  Off: on GB300 it ran at 24.2 against 17.8 us per iteration (80
-// registers with spills against 57).
-#ifndef NGIA_FILTER_HOIST
-#define NGIA_FILTER_HOIST 0
-#endif
-template <int P, int kFilterWordsPerWarp, bool kWord = true>
+// Both filters: whether this launch works, for a representative whose order is
+// decided on the device (st->word_first).  turn 0: alignment-first ones only,
+// 1: word-first ones only, -1: all.
+struct FilterHead {
+  int skip, L1, nb1, word;
+};
+__device__ __forceinline__ FilterHead filter_head(const RunState *st, int exact, int turn) {
+  FilterHead h;
+  h.word = (!exact && st->word_first && st->word_active) ? 1 : 0;
+  h.skip = st->done || st->iter >= st->iter_limit || st->err || (turn >= 0 && turn != h.word);
+  h.L1 = st->rep_len;
+  h.nb1 = st->rep_nb;
+  return h;
+}
+
+template <int P, int WPW>
 __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams prm, int exact, int turn) {
-  constexpr int kFilterTileWords = 8 * kFilterWordsPerWarp;  // 256 threads
   RunState *st = rb.st;
-  extern __shared__ __align__(16) uint32_t s_list[];
-  __shared__ uint64_t bar;
   __shared__ uint32_t s_rc[28];
-  __shared__ int s_hdr[4];
+  __shared__ FilterHead h;
   __shared__ uint32_t s_cnt[kNumClasses], s_base[kNumClasses];
   constexpr int A = P == 2 ? 4 : 28;
-  if (threadIdx.x == 0) {
-    const bool skip = st->done || st->iter >= st->iter_limit || st->err;
-    const int word = (!exact && st->word_first && st->word_active) ? 1 : 0;
-    s_hdr[0] = skip || (turn >= 0 && turn != word);
-    s_hdr[1] = st->rep_len;
-    s_hdr[2] = st->rep_nb;
-    s_hdr[3] = word;
-  }
+  if (threadIdx.x == 0) h = filter_head(st, exact, turn);
   if (threadIdx.x < A) s_rc[threadIdx.x] = rb.rep_rec[2 + threadIdx.x];
   __syncthreads();
-  if (s_hdr[0]) return;
-  const int L1 = s_hdr[1], nb1 = s_hdr[2], word_here = kWord ? s_hdr[3] : 0;
-  const int list_words = max(1, (int)((1u << (prm.w * (P == 2 ? 2 : 5))) / 32u));
-  // byte table of the k-mer bitset, right after the bitset
-  uint8_t *s_tab = reinterpret_cast<uint8_t *>(s_list + list_words);
-  if (word_here) {
-    if (!stage_to_smem(s_list, rb.rep_list, (uint32_t)list_words, &bar, st, 1)) return;
-    for (int i = threadIdx.x; i < list_words * 8; i += blockDim.x) {
-      const uint32_t nib = (s_list[i >> 3] >> (4 * (i & 7))) & 0xFu;  // 4 words -> 4 bytes
-      reinterpret_cast<uint32_t *>(s_tab)[i] = (nib & 1u) | ((nib & 2u) << 7) | ((nib & 4u) << 14) | ((nib & 8u) << 21);
-    }
-    __syncthreads();
-  }
+  if (h.skip) return;
+  const int L1 = h.L1, nb1 = h.nb1;
   const float s = prm.s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nbw = (db.n + 31) / 32;
-  const int tiles = (nbw + kFilterTileWords - 1) / kFilterTileWords;
-  // Bitmap word of slot k of a tile.  With the short-word test here, a
-  // tile's words are spread over the (length-sorted) database so that every
-  // tile holds a share of the long candidates; otherwise they are
-  // consecutive, which keeps neighbouring queue entries of similar length.
-  auto word_of = [&](int tile, int k) {
-    return word_here ? k * tiles + tile : tile * kFilterTileWords + k;
-  };
-  unsigned long long cand = 0, base = 0, bytes = 0, wchk = 0, wpass = 0;
-  if (word_here && NGIA_FILTER_WARP_WORD) {
-    // Short-word test here: the work per candidate grows with its length, so
-    // warps run independently — each takes every W-th bitmap word of the
-    // length-sorted database, a CTA's warps words gridDim.x apart (a share of
-    // every length for each SM) — and queues its survivors with one atomic
-    // per class and word; no CTA barrier makes a warp wait for the CTA's
-    // longest candidates.
-    const int W = gridDim.x * (blockDim.x >> 5);
-    for (int wi = warp * gridDim.x + blockIdx.x; wi < nbw; wi += W) {
-      const uint32_t bits = rb.alive[wi];
-      if (!bits) continue;  // warp-uniform
-      const int c = wi * 32 + lane;
-      const bool alive = (bits >> lane) & 1u;
-      bool pass = false, deferred = false;
-      int cls = 0;
-      if (alive) {
-        cand++;
-        bytes += 4 * (2 + A);
-        const int L2 = __ldg(db.len + c);
-        pass = !(base_sum<A>(db.cnt, c, s_rc) < cutoff_of(L2, s));
-        if (pass) {
-          base++;
-          const int net2 = __ldg(db.net + c);
-          wchk++;
-          bytes += 4ull * P * ((net2 + 31) / 32);
-          if (net2 <= kWarpWordLen) {
-            pass = !(word_count_cand<P>(db, c, net2, prm.w, s_tab) < word_min(L2, prm.w, s));
-            if (pass) wpass++;
-          } else {
-            deferred = true;
-          }
-        }
-        if (pass) cls = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
-      }
-      // long candidates go to k_filter_long, which gives each one a warp
-      const unsigned dm = __ballot_sync(kFullMask, deferred);
-      if (dm) {
-        const int leader = __ffs(dm) - 1;
-        uint32_t b = 0;
-        if (lane == leader) b = atomicAdd(&st->long_count, (uint32_t)__popc(dm));
-        b = __shfl_sync(kFullMask, b, leader);
-        if (deferred) rb.long_list[b + __popc(dm & ((1u << lane) - 1u))] = c;
-      }
-      push_queue(rb, st, pass && !deferred, cls, c);
-    }
-    flush_stats(rb, cand, base, bytes, wchk, wpass);
-    return;
-  }
+  const int tiles = (nbw + 8 * WPW - 1) / (8 * WPW);
+  unsigned long long cand = 0, base = 0, bytes = 0;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     if (threadIdx.x < kNumClasses) s_cnt[threadIdx.x] = 0;
     __syncthreads();
     // The warp's bitmap words first, then every header load of all its
     // words (independent of one another), then the compaction.
-    int slot[kFilterWordsPerWarp], cls_of[kFilterWordsPerWarp];
-    uint32_t bits_of[kFilterWordsPerWarp];
+    const int w0 = (tile * 8 + warp) * WPW;
+    int slot[WPW], cls_of[WPW];
+    uint32_t bits_of[WPW];
 #pragma unroll
-    for (int k = 0; k < kFilterWordsPerWarp; k++) {
-      const int wi = word_of(tile, warp * kFilterWordsPerWarp + k);
-      bits_of[k] = wi < nbw ? rb.alive[wi] : 0u;
-    }
-    // Composition-only DNA instance: the headers of all the warp's words are
-    // loaded before any test (predicated on the unclustered bit), so a warp
-    // waits for one round of loads rather than one per word.
-    constexpr bool kHoist = NGIA_FILTER_HOIST && !kWord && P == 2;
-    constexpr int kH = kHoist ? kFilterWordsPerWarp : 1;
-    int len_h[kH];
-    uint4 cnt_h[kH];
-    if constexpr (kHoist) {
-#pragma unroll
-      for (int k = 0; k < kFilterWordsPerWarp; k++) {
-        const int c = word_of(tile, warp * kFilterWordsPerWarp + k) * 32 + lane;
-        len_h[k] = 0;
-        cnt_h[k] = make_uint4(0u, 0u, 0u, 0u);
-        if ((bits_of[k] >> lane) & 1u) {
-          len_h[k] = __ldg(db.len + c);
-          cnt_h[k] = __ldg(reinterpret_cast<const uint4 *>(db.cnt) + c);
-        }
-      }
-    }
+    for (int k = 0; k < WPW; k++) bits_of[k] = w0 + k < nbw ? rb.alive[w0 + k] : 0u;
     unsigned pass_of = 0;  // bit k: this lane's candidate of word k survives
 #pragma unroll
-    for (int k = 0; k < kFilterWordsPerWarp; k++) {
+    for (int k = 0; k < WPW; k++) {
       cls_of[k] = 0;
       const uint32_t bits = bits_of[k];
       if (!bits) continue;  // warp-uniform
-      const int wi = word_of(tile, warp * kFilterWordsPerWarp + k);
-      const int c = wi * 32 + lane;
-      const bool alive = (bits >> lane) & 1u;
-      bool pass = false, deferred = false;
-      if (alive) {
+      const int c = (w0 + k) * 32 + lane;
+      if ((bits >> lane) & 1u) {
         cand++;
         bytes += 4 * (2 + A);
-        int L2, sum;
-        if constexpr (kHoist) {
-          L2 = len_h[k];
-          const uint4 q = cnt_h[k];
-          sum = (int)(min(q.x, s_rc[0]) + min(q.y, s_rc[1]) + min(q.z, s_rc[2]) + min(q.w, s_rc[3]));
-        } else {
-          L2 = __ldg(db.len + c);
-          sum = base_sum<A>(db.cnt, c, s_rc);
-        }
-        pass = !(sum < cutoff_of(L2, s));
-        if (pass) base++;
-        if (pass && word_here) {
-          const int net2 = __ldg(db.net + c);
-          wchk++;
-          bytes += 4ull * P * ((net2 + 31) / 32);
-          if (net2 <= kWarpWordLen) {
-            pass = !(word_count_cand<P>(db, c, net2, prm.w, s_tab) < word_min(L2, prm.w, s));
-            if (pass) wpass++;
-          } else {
-            deferred = true;
-          }
-        }
-        if (pass && !exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
-      }
-      // long candidates: the whole warp counts each one
-      for (unsigned dm = __ballot_sync(kFullMask, deferred); dm; dm &= dm - 1) {
-        const int src = __ffs(dm) - 1;
-        const int cc = wi * 32 + src;
-        const int ws = word_count_cand_warp<P>(db, cc, __ldg(db.net + cc), prm.w, s_tab);
-        if (lane == src) {
-          const int L2 = __ldg(db.len + cc);
-          pass = !(ws < word_min(L2, prm.w, s));
-          if (pass) {
-            wpass++;
-            if (!exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
-          }
+        const int L2 = __ldg(db.len + c), cut = cutoff_of(L2, s);
+        if (!(base_sum<A>(db.cnt, c, s_rc) < cut)) {
+          base++;
+          pass_of |= 1u << k;
+          if (!exact) cls_of[k] = class_of(db.type, window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1), L2);
         }
       }
-      if (pass) pass_of |= 1u << k;
     }
 #pragma unroll
-    for (int k = 0; k < kFilterWordsPerWarp; k++) {
+    for (int k = 0; k < WPW; k++) {
       slot[k] = -1;
-      const int wi = word_of(tile, warp * kFilterWordsPerWarp + k);
-      if (wi >= nbw) continue;  // warp-uniform
+      if (w0 + k >= nbw) continue;  // warp-uniform
       const bool pass = (pass_of >> k) & 1u;
       const unsigned pm = __ballot_sync(kFullMask, pass);
       if (exact) {
-        if (lane == 0) reinterpret_cast<uint32_t *>(rb.flags)[wi] = pm;
+        if (lane == 0) reinterpret_cast<uint32_t *>(rb.flags)[w0 + k] = pm;
         continue;
       }
       if (pass) {
@@ -484,14 +268,95 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
       s_base[threadIdx.x] = s_cnt[threadIdx.x] ? atomicAdd(&st->qcount[threadIdx.x], s_cnt[threadIdx.x]) : 0u;
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kFilterWordsPerWarp; k++) {
-      if (slot[k] >= 0) {
-        const int c = word_of(tile, warp * kFilterWordsPerWarp + k) * 32 + lane;
-        rb.queue[cls_of[k]][s_base[cls_of[k]] + (uint32_t)slot[k]] = c;
-      }
-    }
+    for (int k = 0; k < WPW; k++)
+      if (slot[k] >= 0) rb.queue[cls_of[k]][s_base[cls_of[k]] + (uint32_t)slot[k]] = (w0 + k) * 32 + lane;
   }
-  flush_stats(rb, cand, base, bytes, wchk, wpass);
+  flush_stats(rb, cand, base, bytes, 0, 0);
+}
+
+// ---- composition and short-word test -------------------------------------------
+// Launches that may put the short-word test first.  The work per candidate
+// grows with its length, so warps run independently — each takes every W-th
+// bitmap word of the length-sorted database, a CTA's warps words gridDim.x
+// apart (a share of every length for each SM) — and queues its survivors with
+// one atomic per class and word; no CTA barrier makes a warp wait for the CTA's
+// longest candidates.  Candidates longer than kWarpWordLen go to k_filter_long,
+// a warp each, spread over the grid: the longest sequences of the length-sorted
+// database share the first bitmap words.
+//
+// GB300, 200,000 DNA of 1,450 residues, w = 5, the whole filter per iteration:
+// s = 0.99 42 us (a byte per word and every word counted: 151), s = 0.97 77
+// (153); the first iterations of 100,000 proteins of 20 to 6,600 residues,
+// w = 3, s = 0.9: 44 us with cold caches (72), the longest candidate of a warp
+// and the composition counts; the table of w = 3 allows one word per lookup.
+// Two CTAs of 512 threads per SM: one of 1,024 waits for a whole SM when other
+// jobs share the GPU (12 mixed jobs 2% slower), 256 threads build the table
+// too often (s = 0.97 102 us), 40 registers for three CTAs of 512 spill (90 us).
+// kWarpWordLen: 1,024 is no faster, 512 makes the proteins 25% slower.
+constexpr int kWordThreads = 512, kWordCtas = 2, kWarpWordLen = 2048;
+
+// Shared memory: k-mer bitset | lookup table (word_table_bytes).
+template <int P, int M>
+__global__ void __launch_bounds__(kWordThreads, kWordCtas)
+    k_filter_word(DevDB db, RunBufs rb, RunParams prm, int turn) {
+  RunState *st = rb.st;
+  extern __shared__ __align__(16) uint32_t s_list[];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t s_rc[28];
+  __shared__ FilterHead h;
+  constexpr int A = P == 2 ? 4 : 28;
+  if (threadIdx.x == 0) h = filter_head(st, 0, turn);
+  if (threadIdx.x < A) s_rc[threadIdx.x] = rb.rep_rec[2 + threadIdx.x];
+  __syncthreads();
+  if (h.skip) return;
+  const int L1 = h.L1, nb1 = h.nb1, word_here = h.word;
+  const uint32_t list_words = list_words_of(db.type, prm.w);
+  uint8_t *s_tab = reinterpret_cast<uint8_t *>(s_list + list_words);
+  if (word_here) {
+    if (!stage_to_smem(s_list, rb.rep_list, list_words, &bar, st, 1)) return;
+    build_word_table<P, M>(s_tab, s_list, prm.w);
+  }
+  const float s = prm.s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nbw = (db.n + 31) / 32;
+  uint32_t cand = 0, base = 0, bytes = 0, wpass = 0;  // a thread sees fewer than 2^17 candidates of 22 KB
+  const int W = gridDim.x * (blockDim.x >> 5);
+  for (int wi = warp * gridDim.x + blockIdx.x; wi < nbw; wi += W) {
+    const uint32_t bits = rb.alive[wi];
+    if (!bits) continue;  // warp-uniform
+    const int c = wi * 32 + lane;
+    bool pass = false, deferred = false;
+    int cls = 0;
+    if ((bits >> lane) & 1u) {
+      cand++;
+      bytes += 4 * (2 + A);
+      const int L2 = __ldg(db.len + c), cut = cutoff_of(L2, s);
+      pass = !(base_sum<A>(db.cnt, c, s_rc) < cut);
+      if (pass) {
+        base++;
+        if (word_here) {
+          const int net2 = __ldg(db.net + c);
+          bytes += 4 * P * ((net2 + 31) / 32);
+          deferred = net2 > kWarpWordLen;
+          if (!deferred) {
+            pass = words_reach<P, M>(db, c, net2, prm.w, word_min(L2, prm.w, s), s_tab, s_list);
+            if (pass) wpass++;
+          }
+        }
+      }
+      if (pass) cls = class_of(db.type, window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1), L2);
+    }
+    const unsigned dm = __ballot_sync(kFullMask, deferred);
+    if (dm) {
+      const int leader = __ffs(dm) - 1;
+      uint32_t b = 0;
+      if (lane == leader) b = atomicAdd(&st->long_count, (uint32_t)__popc(dm));
+      b = __shfl_sync(kFullMask, b, leader);
+      if (deferred) rb.long_list[b + __popc(dm & ((1u << lane) - 1u))] = c;
+    }
+    push_queue(rb, st, pass && !deferred, cls, c);
+  }
+  flush_stats(rb, cand, base, bytes, word_here ? base : 0, wpass);
 }
 
 // ---- exact short-word path ---------------------------------------------------
@@ -591,18 +456,15 @@ __global__ void __launch_bounds__(256) k_word_exact(DevDB db, RunBufs rb, RunPar
   flush_stats(rb, 0, 0, bytes, wchk, wpass);
 }
 
-// Largest filter shared memory: DNA w=8 bitset (8 KB) + byte table (64 KB).
-// Short-word test of the candidates longer than kWarpWordLen residues that
-// k_filter queued in rb.long_list (word-first order): one warp per
-// candidate, spread over the grid, so that the longest sequences of the
-// length-sorted database (which share the first bitmap words) are counted
-// side by side; survivors join the alignment class queues.
-template <int P>
+// Short-word test of the candidates that k_filter_word queued in rb.long_list:
+// one warp per candidate, spread over the grid; survivors join the alignment
+// class queues.
+template <int P, int M>
 __global__ void __launch_bounds__(256) k_filter_long(DevDB db, RunBufs rb, RunParams prm) {
   RunState *st = rb.st;
   extern __shared__ __align__(16) uint32_t s_list[];
   __shared__ uint64_t bar;
-  __shared__ int s_hdr[4];
+  __shared__ int s_hdr[3];
   if (threadIdx.x == 0) {
     const bool skip = st->done || st->iter >= st->iter_limit || st->err;
     s_hdr[0] = skip ? 0 : (int)st->long_count;
@@ -611,93 +473,87 @@ __global__ void __launch_bounds__(256) k_filter_long(DevDB db, RunBufs rb, RunPa
   }
   __syncthreads();
   const int nlong = s_hdr[0];
-  if (nlong == 0) return;
+  if ((int)blockIdx.x * (int)(blockDim.x >> 5) >= nlong) return;
   const int L1 = s_hdr[1], nb1 = s_hdr[2];
-  const int list_words = max(1, (int)((1u << (prm.w * (P == 2 ? 2 : 5))) / 32u));
+  const uint32_t list_words = list_words_of(db.type, prm.w);
   uint8_t *s_tab = reinterpret_cast<uint8_t *>(s_list + list_words);
-  if (!stage_to_smem(s_list, rb.rep_list, (uint32_t)list_words, &bar, st, 2)) return;
-  for (int i = threadIdx.x; i < list_words * 8; i += blockDim.x) {
-    const uint32_t nib = (s_list[i >> 3] >> (4 * (i & 7))) & 0xFu;
-    reinterpret_cast<uint32_t *>(s_tab)[i] = (nib & 1u) | ((nib & 2u) << 7) | ((nib & 4u) << 14) | ((nib & 8u) << 21);
-  }
-  __syncthreads();
+  if (!stage_to_smem(s_list, rb.rep_list, list_words, &bar, st, 2)) return;
+  build_word_table<P, M>(s_tab, s_list, prm.w);
   const float s = prm.s;
   const int lane = threadIdx.x & 31;
   const int W = gridDim.x * (blockDim.x >> 5);
   unsigned long long wpass = 0;
   for (int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < nlong; k += W) {
     const int c = rb.long_list[k];
-    const int ws = word_count_cand_warp<P>(db, c, __ldg(db.net + c), prm.w, s_tab);
     const int L2 = __ldg(db.len + c);
-    const bool pass = lane == 0 && !(ws < word_min(L2, prm.w, s));
+    const bool pass = words_reach_warp<P, M>(db, c, __ldg(db.net + c), prm.w, word_min(L2, prm.w, s), s_tab, s_list) &&
+                      lane == 0;
     if (pass) wpass++;
-    push_queue(rb, st, pass, pass ? class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2) : 0, c);
+    push_queue(rb, st, pass,
+               pass ? class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2) : 0, c);
   }
   flush_stats(rb, 0, 0, 0, 0, wpass);
 }
 
+using FilterFn = void (*)(DevDB, RunBufs, RunParams, int, int);
+using WordFn = void (*)(DevDB, RunBufs, RunParams, int);
+using LongFn = void (*)(DevDB, RunBufs, RunParams);
+static WordFn word_fn(int type, int M) {
+  if (type) return M == 2 ? k_filter_word<5, 2> : k_filter_word<5, 1>;
+  return M == 4 ? k_filter_word<2, 4> : M == 2 ? k_filter_word<2, 2> : k_filter_word<2, 1>;
+}
+static LongFn long_fn(int type, int M) {
+  if (type) return M == 2 ? k_filter_long<5, 2> : k_filter_long<5, 1>;
+  return M == 4 ? k_filter_long<2, 4> : M == 2 ? k_filter_long<2, 2> : k_filter_long<2, 1>;
+}
+static size_t word_smem(int type, int w) {
+  return 4 * (size_t)list_words_of(type, w) + word_table_bytes(type, w, words_per_lookup(type, w));
+}
+
 cudaError_t filter_configure() {
-  const int most = 9 * (1 << 16) / 8;
-  const void *fns[] = {(const void *)k_filter<2, NGIA_FILTER_WPW_WORD>, (const void *)k_filter<5, NGIA_FILTER_WPW_WORD>,
-                       (const void *)k_filter_long<2>, (const void *)k_filter_long<5>};
-  for (const void *f : fns) {
-    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (e != cudaSuccess) return e;
-  }
+  constexpr size_t most = 72 * 1024;  // DNA w = 8: 8 KB bitset, 64 KB table
+  for (int type = 0; type < 2; type++)
+    for (int M = 1; M <= (type ? 2 : 4); M *= 2) {
+      cudaError_t e = cudaFuncSetAttribute((const void *)word_fn(type, M), cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void *)long_fn(type, M), cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      if (e != cudaSuccess) return e;
+    }
   return cudaSuccess;
 }
 
 cudaError_t launch_filter(ngia_ctx *c) {
-  const int P = c->db.P;
-  const int bits = c->db.type ? 5 : 2;
-  const int list_words = std::max(1, (int)((1u << (c->prm.w * bits)) / 32u));
-  const size_t smem = (size_t)list_words * 4;
+  const int type = c->db.type, P = c->db.P;
   // Exact path only matters when the short-word filter can run and some
   // record is shorter than 16 residues.
   const bool exact = c->db.has_short && !c->prm.precise;
   const int nbw = (c->db.n + 31) / 32;
-  constexpr int kB = NGIA_FILTER_WPW_BASE, kW = NGIA_FILTER_WPW_WORD;
-  const int grid_b = std::max(1, std::min(c->grid_filter, (nbw + 8 * kB - 1) / (8 * kB)));
-  const int grid_w = std::max(1, std::min(c->grid_filter, (nbw + 8 * kW - 1) / (8 * kW)));
+  const bool small = !exact && c->filter_tile == 1;  // the tuner's choice: one bitmap word per warp and tile
+  const int per = 8 * (small ? 1 : kFilterWords);
+  const int grid = std::max(1, std::min(c->grid_filter, (nbw + per - 1) / per));
+  const FilterFn fn = P == 2 ? (small ? k_filter<2, 1> : k_filter<2, kFilterWords>)
+                             : (small ? k_filter<5, 1> : k_filter<5, kFilterWords>);
   if (!exact) {
-    // The instance with the short-word test, the one without, or (automatic
+    // The filter with the short-word test, the one without, or (automatic
     // order, when either may be wanted) both: the representative's order
     // decides on the device which works.
     const bool word = c->prm.word_order == 1 || (c->prm.word_order == 0 && c->prm.word_can);
     const int turn = c->prm.word_order == 0 && c->prm.word_can ? 1 : -1;
-    if (word) {  // also holds the byte table (8 bytes per bitset byte)
-      if (P == 2)
-        k_filter<2, kW><<<grid_w, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm, 0, turn);
-      else
-        k_filter<5, kW><<<grid_w, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm, 0, turn);
-      if (NGIA_FILTER_WARP_WORD && c->db.max_nb * 32 > kWarpWordLen) {  // some record is long
+    if (word) {
+      const int M = words_per_lookup(type, c->prm.w);
+      const size_t smem = word_smem(type, c->prm.w);
+      const int grid_w = std::max(1, std::min(std::min(c->grid_filter, kWordCtas * c->num_sms), (nbw + 7) / 8));
+      word_fn(type, M)<<<grid_w, kWordThreads, smem, c->stream>>>(c->db, c->rb, c->prm, turn);
+      if (c->db.max_nb * 32 > kWarpWordLen) {  // some record is long
         const int grid_l = std::max(1, std::min(c->grid_filter, c->num_sms));
-        if (P == 2)
-          k_filter_long<2><<<grid_l, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm);
-        else
-          k_filter_long<5><<<grid_l, 256, smem * 9, c->stream>>>(c->db, c->rb, c->prm);
+        long_fn(type, M)<<<grid_l, 256, smem, c->stream>>>(c->db, c->rb, c->prm);
       }
     }
-    if (!word || turn >= 0) {
-      const int other = turn >= 0 ? 0 : -1;
-      if (c->filter_tile == kW) {  // the tuner's choice: one bitmap word per warp and tile
-        if (P == 2)
-          k_filter<2, kW, !NGIA_FILTER_SPLIT><<<grid_w, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
-        else
-          k_filter<5, kW, !NGIA_FILTER_SPLIT><<<grid_w, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
-      } else {
-        if (P == 2)
-          k_filter<2, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
-        else
-          k_filter<5, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 0, other);
-      }
-    }
+    if (!word || turn >= 0) fn<<<grid, 256, 0, c->stream>>>(c->db, c->rb, c->prm, 0, turn >= 0 ? 0 : -1);
     return cudaGetLastError();
   }
-  if (P == 2)
-    k_filter<2, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 1, -1);
-  else
-    k_filter<5, kB, !NGIA_FILTER_SPLIT><<<grid_b, 256, smem, c->stream>>>(c->db, c->rb, c->prm, 1, -1);
+  const size_t smem = 4 * (size_t)list_words_of(type, c->prm.w);
+  fn<<<grid, 256, 0, c->stream>>>(c->db, c->rb, c->prm, 1, -1);
   k_scan_words<<<1, 1024, 0, c->stream>>>(reinterpret_cast<const uint32_t *>(c->rb.flags), nbw, c->rb.scan_part);
   k_first_short<<<64, 256, 0, c->stream>>>(c->db, c->rb, 1);
   k_first_short<<<c->num_sms * 2, 256, 0, c->stream>>>(c->db, c->rb, 0);
@@ -812,7 +668,7 @@ __global__ void k_floor_empty(const RunBufs rb) {
 }
 
 __global__ void __launch_bounds__(256) k_floor_read(DevDB db, RunBufs rb, unsigned long long *sink) {
-  constexpr int kW = NGIA_FILTER_WPW_BASE, kTileWords = 8 * kW;
+  constexpr int kW = kFilterWords, kTileWords = 8 * kW;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nbw = (db.n + 31) / 32;
   const int tiles = (nbw + kTileWords - 1) / kTileWords;
@@ -847,7 +703,7 @@ extern "C" int ngia_measure_filter_floor(ngia_ctx *c, double *launch_us, double 
   if (!c->begun) return ngia::fail(NGIA_E_STATE, "ngia_measure_filter_floor before ngia_cluster_begin");
   if (c->db.type != 0) return ngia::fail(NGIA_E_ARG, "ngia_measure_filter_floor: DNA databases only");
   const int nbw = (c->db.n + 31) / 32;
-  constexpr int kB = NGIA_FILTER_WPW_BASE;
+  constexpr int kB = ngia::kFilterWords;
   const int grid = std::max(1, std::min(c->grid_filter, (nbw + 8 * kB - 1) / (8 * kB)));
   constexpr int kReps = 20;
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;

@@ -243,8 +243,7 @@ __global__ void __launch_bounds__(256) k_pool_filter(PoolDev pd, int ncls) {
           wchk = 1;
           bytes += 4ull * P * ((net2 + 31) / 32);
           if (net2 <= kPoolWarpWordLen) {
-            const uint32_t *planes = J->db.words + __ldg(J->db.off + c) + J->db.hw;
-            pass = !(word_count<P>(planes, net2, w, J->rb.rep_list) < word_min(L2, w, s));
+            pass = words_reach<P, 1>(J->db, c, net2, w, word_min(L2, w, s), KmerBits{J->rb.rep_list}, J->rb.rep_list);
             wpass = pass;
           } else {
             deferred = true;
@@ -256,11 +255,11 @@ __global__ void __launch_bounds__(256) k_pool_filter(PoolDev pd, int ncls) {
     for (unsigned dm = __ballot_sync(kFullMask, deferred); dm; dm &= dm - 1) {
       const int src = __ffs(dm) - 1;
       const int cc = wi * 32 + src;
-      const uint32_t *planes = J->db.words + __ldg(J->db.off + cc) + J->db.hw;
-      const int ws = word_count_warp_bits<P>(planes, __ldg(J->db.net + cc), w, J->rb.rep_list);
+      const int L2 = __ldg(J->db.len + cc);
+      const bool reach = words_reach_warp<P, 1>(J->db, cc, __ldg(J->db.net + cc), w, word_min(L2, w, s),
+                                                KmerBits{J->rb.rep_list}, J->rb.rep_list);
       if (lane == src) {
-        const int L2 = __ldg(J->db.len + cc);
-        pass = !(ws < word_min(L2, w, s));
+        pass = reach;
         wpass = pass;
         if (pass) cls = class_of(type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2);
       }

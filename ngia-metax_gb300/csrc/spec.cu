@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) k_spec_filter(DevDB db, SpecDev sd, Round
         bool pass = !(base_sum<A>(db.cnt, x, s_rc) < cut);
         if (pass && word_here) {
           const int net2 = __ldg(db.net + x);
-          if (net2 >= 16) pass = !(word_count_cand<P>(db, x, net2, prm.w, KmerBits{s_list}) < word_min(L2, prm.w, s));
+          if (net2 >= 16) pass = words_reach<P, 1>(db, x, net2, prm.w, word_min(L2, prm.w, s), KmerBits{s_list}, s_list);
         }
         if (pass) res = 1 + round_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1), L2);
       }
