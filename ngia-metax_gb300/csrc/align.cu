@@ -55,11 +55,11 @@ struct AlignHdr {
 // shared memory with bulk copies.  Returns false when there is no work.
 template <int P>
 // groups: pairs a CTA of the group-per-pair kernel works on at a time (it
-// takes classes with at most warp_pairs pairs), 0 for the thread-per-pair
-// kernels (classes with more); the other kernel of a class returns here,
-// before any staging.
+// takes classes with at most warp_pairs pairs; kAlignThreads / 32 once there
+// are more than `few`), 0 for the thread-per-pair kernels (classes with more);
+// the other kernel of a class returns here, before any staging.
 __device__ __forceinline__ bool align_setup(const DevDB &db, const RunBufs &rb, const RunParams &prm, int cls,
-                                            int score_mode, int warp_pairs, int groups, uint32_t *smem,
+                                            int score_mode, int warp_pairs, int groups, int few, uint32_t *smem,
                                             uint64_t *bar, AlignHdr &h) {
   __shared__ int s_hdr[6];
   RunState *st = rb.st;
@@ -67,7 +67,7 @@ __device__ __forceinline__ bool align_setup(const DevDB &db, const RunBufs &rb, 
     const bool skip = !score_mode && (st->done || st->iter >= st->iter_limit || st->err);
     const int qn = skip ? 0 : (int)st->qcount[cls];
     const bool mine = groups ? qn <= warp_pairs : qn > warp_pairs;
-    const bool idle = (int)blockIdx.x * groups >= qn;
+    const bool idle = (int)blockIdx.x * (qn > few ? max(groups, kAlignThreads / 32) : groups) >= qn;
     s_hdr[0] = mine && !(groups && idle) ? qn : 0;
     s_hdr[1] = st->rep_len;
     s_hdr[2] = st->rep_net;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   AlignHdr h;
   __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
   if (threadIdx.x == 0) s_qw = 0;
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, 0, smem, &bar, h)) return;
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, 0, 0, smem, &bar, h)) return;
   const uint32_t *s_pl = smem;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
   RunState *st = rb.st;
@@ -339,76 +339,105 @@ __host__ __device__ constexpr int wave_table_off(int P, int max_nb) { return ((m
 
 // ---- a group of threads per pair (wave.cuh) ------------------------------------------
 // For classes with few queued pairs the latency of one pair on one thread
-// bounds the iteration.  NW = 1: a warp per pair (windows up to 64 blocks);
-// NW = 4: the CTA per pair, W = 1 row word per thread for windows up to 128
-// blocks, up to 16 for any.
+// bounds the iteration.  Windows up to 64 blocks: a warp per pair.  Wider ones:
+// the CTA per pair for up to `few` pairs, one row word per thread for windows
+// up to 128 blocks, up to 16 for any; beyond, when every scheduler has a warp,
+// a warp per pair with up to 8 or 16 words, which takes half the instructions:
+// a step has 80 beside the columns' (5 + 4 W) each, and 2 nq + nb1 / W steps
+// are taken by one warp instead of four.
+struct WaveCounts {
+  unsigned long long pairs = 0, members = 0, cells = 0, done = 0;
+};
+
+// This CTA's share of the class's pairs, `per` neighbouring entries at a time.
+// MINE: -1 all, 1 the bands that a warp can hold, 0 the others.
+template <int P, int NW, int WMAX, int MINE>
+__device__ __forceinline__ void wave_entries(const DevDB &db, const RunBufs &rb, const RunParams &prm, int cls,
+                                             int score_mode, const AlignHdr &h, int per, const uint32_t *s_tab,
+                                             uint32_t *s_rings, const uint32_t *s_list, uint32_t *s_xch,
+                                             unsigned long long *s_qw, WaveCounts &n) {
+  constexpr int kGroups = kAlignThreads / 32 / NW;
+  const int group = (int)(threadIdx.x >> 5) / NW;
+  const bool lead = threadIdx.x % (32 * NW) == 0;
+  const float s = prm.s;
+  const int nb1 = h.nb1;
+  uint32_t *ring = s_rings + group * kWaveRingWords;
+  for (int e0 = blockIdx.x * per; e0 < h.qn; e0 += gridDim.x * per) {
+    for (int e = e0 + group; e < min(h.qn, e0 + per); e += kGroups) {
+      const int entry = rb.queue[cls][e];
+      const int cand = score_mode ? rb.score_cands[entry] : entry;
+      const int L2 = __ldg(db.len + cand), net2 = __ldg(db.net + cand);
+      const int nq = (net2 + 31) >> 5;
+      const int B = band_blocks(h.L1, L2, s);
+      const int cutoff = cutoff_of(L2, s), cut = score_mode ? kNoCut : cutoff;
+      const uint32_t *qpl = db.words + __ldg(db.off + cand) + db.hw;
+      const bool self = cand == h.rep && !score_mode, band = B >= 0 && nb1 > 0 && nq > 0;
+      int lo = 0, hi = 0;
+      const bool run = !self && band && wave_band(B, h.net1, net2, cut, lo, hi);
+      if constexpr (MINE >= 0)
+        if ((MINE != 0) == (run && !wave_holds(32, 16, lo, hi, nb1))) continue;
+      if (!score_mode && lead) {
+        n.pairs++;
+        n.cells += (unsigned long long)band_cells(B, nb1, net2);
+        atomicAdd(s_qw, (unsigned long long)(nq * P));
+      }
+      int sum = self ? h.net1 : 0;  // itself: the band holds the diagonal; no band: score 0
+      if (!self && band) {
+        if (!run) continue;  // no chain can reach the cutoff
+        sum = wave_any<P, NW, WMAX>(s_tab, nb1, qpl, nq, net2, lo, hi, cut, ring, s_xch, n.done);
+        if (sum < 0) continue;  // cannot reach the cutoff
+      }
+      if (score_mode) {
+        if (lead) rb.score_out[4 * entry + 2] = sum;
+        continue;
+      }
+      bool pass = !(sum < cutoff);
+      if (pass && h.word_after && self) {
+        pass = !(max(0, net2 - prm.w + 1) < word_min(L2, prm.w, s));
+      } else if (pass && h.word_after && threadIdx.x / 32 == group * NW) {  // short-word test (func.cu:376-396): the group's first warp
+        pass = !(word_count_warp_bits<P>(qpl, net2, prm.w, s_list) < word_min(L2, prm.w, s));
+      }
+      if (lead && pass) {
+        rb.cluster[cand] = h.rep;
+        rb.ident[cand] = sum;
+        atomicAnd(&rb.alive[cand >> 5], ~(1u << (cand & 31)));
+        n.members++;
+      }
+      __syncwarp();
+    }
+  }
+}
+
 template <int P, int NW, int WMAX>
 __global__ void __launch_bounds__(kAlignThreads)
-    k_align_wave(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs) {
+    k_align_wave(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs, int few) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint64_t bar;
   __shared__ uint32_t s_xch[4 * NW];
   AlignHdr h;
   __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
   if (threadIdx.x == 0) s_qw = 0;
-  constexpr int kGroups = kAlignThreads / 32 / NW;  // pairs per CTA
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kGroups, smem, &bar, h)) return;
-  const uint32_t *s_pl = smem;
+  constexpr int kWarps = kAlignThreads / 32;
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kWarps / NW, few, smem, &bar, h)) return;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
-  const int group = (int)(threadIdx.x >> 5) / NW;
-  const bool lead = threadIdx.x % (32 * NW) == 0;
-  RunState *st = rb.st;
-  const float s = prm.s;
-  const int nb1 = h.nb1;
   const uint32_t vlast = (h.net1 & 31) ? ((1u << (h.net1 & 31)) - 1u) : 0xFFFFFFFFu;
   uint32_t *s_tab = smem + wave_table_off(P, db.max_nb);
-  uint32_t *s_ring = s_tab + wave_table_words(P, db.max_nb) + group * kWaveRingWords;
-  wave_table<P>(s_pl, nb1, vlast, s_tab, threadIdx.x, kAlignThreads);
+  uint32_t *s_rings = s_tab + wave_table_words(P, db.max_nb);
+  wave_table<P>(smem, h.nb1, vlast, s_tab, threadIdx.x, kAlignThreads);
   __syncthreads();
-  unsigned long long n_pairs = 0, n_members = 0, n_cells = 0, n_done = 0;
-  for (int e = blockIdx.x * kGroups + group; e < h.qn; e += gridDim.x * kGroups) {
-    const int entry = rb.queue[cls][e];
-    const int cand = score_mode ? rb.score_cands[entry] : entry;
-    const int L2 = __ldg(db.len + cand), net2 = __ldg(db.net + cand);
-    const int nq = (net2 + 31) >> 5;
-    const int B = band_blocks(h.L1, L2, s);
-    const int cutoff = cutoff_of(L2, s);
-    const uint32_t *qpl = db.words + __ldg(db.off + cand) + db.hw;
-    if (!score_mode && lead) {
-      n_pairs++;
-      n_cells += (unsigned long long)band_cells(B, nb1, net2);
-      atomicAdd(&s_qw, (unsigned long long)(nq * P));
+  WaveCounts n;
+  if (NW == 1 || h.qn <= few) {
+    wave_entries<P, NW, WMAX, -1>(db, rb, prm, cls, score_mode, h, kWarps / NW, s_tab, s_rings, s_list, s_xch, &s_qw, n);
+  } else if constexpr (NW > 1) {
+    constexpr int WW = WMAX == 1 ? 8 : 16;  // one word for each of 128 threads: 8 for 32 hold as much
+    wave_entries<P, 1, WW, WMAX == 1 ? -1 : 1>(db, rb, prm, cls, score_mode, h, kWarps, s_tab, s_rings, s_list, s_xch,
+                                               &s_qw, n);
+    if (WMAX > 1 && h.nb1 > 32 * WW) {  // bands too wide for a warp
+      __syncthreads();
+      wave_entries<P, NW, WMAX, 0>(db, rb, prm, cls, score_mode, h, kWarps, s_tab, s_rings, s_list, s_xch, &s_qw, n);
     }
-    int sum = 0;  // no band: score 0
-    const bool self = cand == h.rep && !score_mode;
-    if (self) {
-      sum = h.net1;  // the band holds the diagonal
-    } else if (B >= 0 && nb1 > 0 && nq > 0) {
-      const int cut = score_mode ? kNoCut : cutoff;
-      int lo, hi;
-      if (!wave_band(B, h.net1, net2, cut, lo, hi)) continue;
-      sum = wave_any<P, NW, WMAX>(s_tab, nb1, qpl, nq, net2, lo, hi, cut, s_ring, s_xch, n_done);
-      if (sum < 0) continue;  // cannot reach the cutoff
-    }
-    if (score_mode) {
-      if (lead) rb.score_out[4 * entry + 2] = sum;
-      continue;
-    }
-    bool pass = !(sum < cutoff);
-    if (pass && h.word_after && self) {
-      pass = !(max(0, net2 - prm.w + 1) < word_min(L2, prm.w, s));
-    } else if (pass && h.word_after && threadIdx.x / 32 == group * NW) {  // short-word test (func.cu:376-396): the group's first warp
-      pass = !(word_count_warp_bits<P>(qpl, net2, prm.w, s_list) < word_min(L2, prm.w, s));
-    }
-    if (lead && pass) {
-      rb.cluster[cand] = h.rep;
-      rb.ident[cand] = sum;
-      atomicAnd(&rb.alive[cand >> 5], ~(1u << (cand & 31)));
-      n_members++;
-    }
-    __syncwarp();
   }
-  flush_align_stats(st, cls, n_pairs, n_members, n_cells, n_done, &s_qw);
+  flush_align_stats(rb.st, cls, n.pairs, n.members, n.cells, n.done, &s_qw);
 }
 
 // Classes 0 and 1 with few pairs: 16 threads per pair, the query's blocks as
@@ -423,7 +452,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
   if (threadIdx.x == 0) s_qw = 0;
   constexpr int kGroups = kAlignThreads / kQueryGroup;
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kGroups, smem, &bar, h)) return;
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kGroups, INT_MAX, smem, &bar, h)) return;
   const uint32_t *s_pl = smem;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
   const int lane = threadIdx.x & 31, g = lane & (kQueryGroup - 1);
@@ -496,12 +525,16 @@ __global__ void __launch_bounds__(kAlignThreads)
 // ---- dispatch ---------------------------------------------------------------------
 typedef void (*AlignFn)(DevDB, RunBufs, RunParams, int, int, int);
 
-static AlignFn wave_fn(int type, int cls) {
-  if (is_query_class(cls)) return type == 0 ? k_align_query<2> : k_align_query<5>;
+static const void *wave_fn(int type, int cls) {
+  if (is_query_class(cls)) return type == 0 ? (const void *)k_align_query<2> : (const void *)k_align_query<5>;
   const int ring = class_ring(type, cls);
   if (type == 0)
-    return ring == 64 ? k_align_wave<2, 1, 2> : ring == 128 ? k_align_wave<2, 4, 1> : k_align_wave<2, 4, 16>;
-  return ring == 64 ? k_align_wave<5, 1, 2> : ring == 128 ? k_align_wave<5, 4, 1> : k_align_wave<5, 4, 16>;
+    return ring == 64    ? (const void *)k_align_wave<2, 1, 2>
+           : ring == 128 ? (const void *)k_align_wave<2, 4, 1>
+                         : (const void *)k_align_wave<2, 4, 16>;
+  return ring == 64    ? (const void *)k_align_wave<5, 1, 2>
+         : ring == 128 ? (const void *)k_align_wave<5, 4, 1>
+                       : (const void *)k_align_wave<5, 4, 16>;
 }
 
 // Pairs a CTA of the class's group-per-pair kernel takes at a time.
@@ -524,7 +557,7 @@ static size_t wave_smem(int type, int cls, int max_nb) {
   if (is_query_class(cls))
     words += 8 * (size_t)max_nb + kAlignThreads * wave_codes(P);
   else
-    words += (size_t)wave_table_words(P, max_nb) + (size_t)wave_pairs_per_cta(type, cls) * kWaveRingWords;
+    words += (size_t)wave_table_words(P, max_nb) + (size_t)(kAlignThreads / 32) * kWaveRingWords;
   return 4u * words;
 }
 // Records of up to this many bytes of shared memory per CTA take the
@@ -556,7 +589,7 @@ cudaError_t align_configure(int type, int max_nb) {
       const int want = (int)(wave ? wave_smem(type, c, max_nb) : align_smem(type, max_nb, c));
       int &have = configured[dev][type ? 1 : 0][wave][c];
       if (want <= have) continue;
-      e = cudaFuncSetAttribute((const void *)(wave ? wave_fn(type, c) : align_fn(type, c)),
+      e = cudaFuncSetAttribute(wave ? wave_fn(type, c) : (const void *)align_fn(type, c),
                                cudaFuncAttributeMaxDynamicSharedMemorySize, want);
       if (e != cudaSuccess) return e;
       have = want;
@@ -569,7 +602,7 @@ cudaError_t align_configure(int type, int max_nb) {
 // wave: of its group-per-pair kernel.
 int align_occupancy(int type, int cls, int max_nb, bool wave) {
   int nb = 0;
-  const void *fn = (const void *)(wave ? wave_fn(type, cls) : align_fn(type, cls));
+  const void *fn = wave ? wave_fn(type, cls) : (const void *)align_fn(type, cls);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kAlignThreads,
                                                     wave ? wave_smem(type, cls, max_nb) : align_smem(type, max_nb, cls)) !=
       cudaSuccess)
@@ -597,11 +630,12 @@ cudaError_t launch_align(ngia_ctx *c, int cls, cudaStream_t s, int score_mode) {
     grid = std::min(grid, (score_mode + kAlignThreads - 1) / kAlignThreads);
     grid_wave = std::min(grid_wave, score_mode);
   }
-  void *args[] = {&db, &rb, &prm, &cls, &score_mode, &wp};
+  int few = wave_few(std::min(wp, c->warp_pairs_default));
+  void *args[] = {&db, &rb, &prm, &cls, &score_mode, &wp, &few};
   cudaError_t e = cudaLaunchKernel((const void *)align_fn(c->db.type, cls), dim3(grid), dim3(kAlignThreads), args,
                                    align_smem(c->db.type, c->db.max_nb, cls), s);
   if (e != cudaSuccess || wp <= 0) return e;  // no class goes to the group kernel
-  return cudaLaunchKernel((const void *)wave_fn(c->db.type, cls), dim3(grid_wave), dim3(kAlignThreads), args,
+  return cudaLaunchKernel(wave_fn(c->db.type, cls), dim3(grid_wave), dim3(kAlignThreads), args,
                           wave_smem(c->db.type, cls, c->db.max_nb), s);
 }
 

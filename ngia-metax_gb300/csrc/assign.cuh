@@ -368,107 +368,145 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   }
 }
 
-// The same for classes with few pairs, a group of threads per pair (wave.cuh).
-// NW 1 or 4: rows are the representative's; NW 0: 16 threads per pair, the
-// query's blocks as rows.  A CTA takes as many neighbouring entries as it has
-// groups: they share their representative.
+// One entry of the round by this thread's group (NW 1 or 4: 32 NW threads,
+// rows are the representative's; NW 0: 16 threads, the query's blocks as rows).
+// MINE: -1 all, 1 the bands that a warp can hold, 0 the others.
+struct RoundRep {
+  int r = -1, L1 = 0, net1 = 0, nb1 = 0;
+  bool word_after = false;  // the short-word test follows the alignment
+};
+template <int P, int NW, int WMAX, bool MASK, int MINE>
+__device__ __forceinline__ void round_wave_entry(const DevDB &qdb, const RepStore &rs, const RunParams &prm,
+                                                 const RoundBufs &rb, const RoundRep &h, int q, int cap_blocks,
+                                                 uint32_t *smem, uint32_t *s_xch, unsigned long long &n_pairs,
+                                                 unsigned long long &n_cells) {
+  constexpr bool kQ = NW == 0;
+  constexpr int GS = kQ ? kQueryGroup : 32 * NW;
+  const int r = h.r, nb1 = h.nb1, net1 = h.net1, lane = threadIdx.x & 31;
+  const bool lead = threadIdx.x % GS == 0;
+  const float s = prm.s;
+  int L2 = 0, net2 = 0, nq = 0, B = 0, cutoff = 1, lo = 0, hi = 0, sum = 0;
+  const uint32_t *qpl = qdb.words;
+  // (a key can change while the group's threads look at it: one answer)
+  const bool self = MASK && q == r;  // a candidate against itself: the band holds the diagonal (align.cu)
+  bool have = q >= 0 && (MASK || (rb.key[q] >> 32) > (unsigned long long)r), run = false;
+  if constexpr (!MASK) {
+    if constexpr (NW == 4)
+      have = __syncthreads_or(have) != 0;
+    else
+      have = __shfl_sync(kFullMask, (int)have, 0, GS) != 0;
+  }
+  if (have) {
+    const int x = MASK ? rb.list[q] : q;
+    L2 = __ldg(qdb.len + x);
+    net2 = __ldg(qdb.net + x);
+    nq = (net2 + 31) >> 5;
+    B = band_blocks(h.L1, L2, s);
+    cutoff = cutoff_of(L2, s);
+    qpl = qdb.words + __ldg(qdb.off + x) + qdb.hw;
+    if (self) {
+      sum = net1;
+    } else if (B >= 0 && nb1 > 0 && nq > 0) {
+      run = wave_band(B, net1, net2, cutoff, lo, hi);
+      have = run;
+    }
+    if constexpr (MINE >= 0)
+      if ((MINE != 0) == (run && !wave_holds(32, 16, lo, hi, nb1))) have = run = false;
+    if (run && lead) n_pairs++;
+  }
+  unsigned long long cells = 0;
+  if constexpr (kQ) {
+    uint32_t *tab = smem + 8 * cap_blocks + (threadIdx.x >> 5) * 32 * wave_codes(P);
+    const int got = wave_query<P>(smem, nb1, net1, qpl, run ? nq : 0, net2, lo, hi, tab, cells);
+    if (run) sum = got;
+  } else if (run) {  // uniform in the group
+    uint32_t *ring = smem + wave_table_words(P, cap_blocks) + (threadIdx.x / GS) * kWaveRingWords;
+    sum = wave_any<P, NW, WMAX>(smem, nb1, qpl, nq, net2, lo, hi, cutoff, ring, s_xch, cells);
+  }
+  n_cells += 32 * cells;
+  bool pass = have && !(sum < cutoff);
+  if (h.word_after) {  // short-word test (func.cu:376-396), a warp per member
+    const uint32_t *list = rs.lists + (int64_t)r * rs.list_words;
+#pragma unroll
+    for (int k = 0; k < (kQ ? 2 : 1); k++) {
+      const int src = k * kQueryGroup;
+      if (!__shfl_sync(kFullMask, (int)(pass && net2 >= 16), src)) continue;
+      const uint32_t *qp = reinterpret_cast<const uint32_t *>(__shfl_sync(kFullMask, (unsigned long long)qpl, src));
+      const int n2 = __shfl_sync(kFullMask, net2, src);
+      const int ws = word_count_warp_bits<P>(qp, n2, prm.w, list);
+      if (!kQ || lane / kQueryGroup == k) pass = !(ws < word_min(L2, prm.w, s));
+    }
+  }
+  if (pass && lead) round_accept<MASK>(rb, r, q, sum);
+}
+
+// The same for classes with few pairs, a group of threads per pair (wave.cuh):
+// NW as above; NW 4 is a warp per pair once there are more than `few` (align.cu).
+// A CTA takes as many neighbouring entries as it has groups: they share their
+// representative.
 // Shared memory: match table | code rings, or rep codes | match tables.
 template <int P, int NW, int WMAX, bool MASK>
 __global__ void __launch_bounds__(kAlignThreads)
     k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int wave_pairs, int cap_blocks) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr bool kQ = NW == 0;
-  constexpr int GS = kQ ? kQueryGroup : 32 * NW, kGroups = kAlignThreads / GS;
+  constexpr int GS = kQ ? kQueryGroup : 32 * NW, kGroups = kAlignThreads / GS, kWarps = kAlignThreads / 32;
+  constexpr int WW = WMAX == 1 ? 8 : 16;
   __shared__ uint32_t s_xch[kQ ? 1 : 4 * NW];
-  __shared__ uint32_t s_qn;
-  if (threadIdx.x == 0) s_qn = round_wave(rb, cls, wave_pairs) ? (uint32_t)min((int64_t)rb.ctl[cls], rb.cap) : 0u;
+  __shared__ uint32_t s_qn, s_many;
+  if (threadIdx.x == 0) {
+    s_qn = round_wave(rb, cls, wave_pairs) ? (uint32_t)min((int64_t)rb.ctl[cls], rb.cap) : 0u;
+    s_many = NW == 4 && rb.ctl[kCtlPairs + cls] > (uint32_t)wave_few(wave_pairs);
+  }
   __syncthreads();
   const uint32_t qn = s_qn;
-  const int group = threadIdx.x / GS;
-  const bool lead = threadIdx.x % GS == 0;
-  const float s = prm.s;
+  const bool many = NW == 4 && s_many;
+  const uint32_t per = many ? kWarps : kGroups;
   const int hw = qdb.hw, lane = threadIdx.x & 31;
   unsigned long long n_pairs = 0, n_cells = 0;
-  int staged = -1, L1 = 0, net1 = 0, nb1 = 0;
-  bool word_after = false;  // the short-word test follows the alignment
-  for (uint32_t e0 = blockIdx.x * kGroups; e0 < qn; e0 += gridDim.x * kGroups) {
+  RoundRep h;
+  for (uint32_t e0 = blockIdx.x * per; e0 < qn; e0 += gridDim.x * per) {
     const int2 first = rb.queue[cls][e0];  // entries of one group: the padding comes last
     if (first.y < 0) continue;             // CTA-uniform
     const int r = first.x;
-    if (r != staged) {
+    if (r != h.r) {
       __syncthreads();  // every group is through with the last representative
       const uint32_t *rrec = rs.words + rs.off[r];
-      L1 = (int)rrec[0];
-      net1 = (int)rrec[1];
-      nb1 = (net1 + 31) >> 5;
-      word_after = !prm.precise && net1 >= 16 && !rs.first[r];
-      const uint32_t vlast = (net1 & 31) ? ((1u << (net1 & 31)) - 1u) : 0xFFFFFFFFu;
+      h.L1 = (int)rrec[0];
+      h.net1 = (int)rrec[1];
+      h.nb1 = (h.net1 + 31) >> 5;
+      h.word_after = !prm.precise && h.net1 >= 16 && !rs.first[r];
+      const uint32_t vlast = (h.net1 & 31) ? ((1u << (h.net1 & 31)) - 1u) : 0xFFFFFFFFu;
       if constexpr (kQ) {
-        for (int b = threadIdx.x; b < nb1; b += kAlignThreads) {
+        for (int b = threadIdx.x; b < h.nb1; b += kAlignThreads) {
           uint32_t pl[P];
 #pragma unroll
           for (int p = 0; p < P; p++) pl[p] = rrec[hw + b * P + p];
           wave_unpack<P>(pl, reinterpret_cast<uint4 *>(smem) + 2 * b);
         }
       } else {
-        wave_table<P>(rrec + hw, nb1, vlast, smem, threadIdx.x, kAlignThreads);
+        wave_table<P>(rrec + hw, h.nb1, vlast, smem, threadIdx.x, kAlignThreads);
       }
       __syncthreads();
-      staged = r;
+      h.r = r;
     }
-    const int2 e = rb.queue[cls][e0 + group];
-    const int q = e.y;
-    int L2 = 0, net2 = 0, nq = 0, B = 0, cutoff = 1, lo = 0, hi = 0, sum = 0;
-    const uint32_t *qpl = qdb.words;
-    // (a key can change while the group's threads look at it: one answer)
-    const bool self = MASK && q == r;  // a candidate against itself: the band holds the diagonal (align.cu)
-    bool have = q >= 0 && (MASK || (rb.key[q] >> 32) > (unsigned long long)r), run = false;
-    if constexpr (!MASK) {
-      if constexpr (NW == 4)
-        have = __syncthreads_or(have) != 0;
-      else
-        have = __shfl_sync(kFullMask, (int)have, 0, GS) != 0;
-    }
-    if (have) {
-      const int x = MASK ? rb.list[q] : q;
-      L2 = __ldg(qdb.len + x);
-      net2 = __ldg(qdb.net + x);
-      nq = (net2 + 31) >> 5;
-      B = band_blocks(L1, L2, s);
-      cutoff = cutoff_of(L2, s);
-      qpl = qdb.words + __ldg(qdb.off + x) + hw;
-      if (self) {
-        sum = net1;
-      } else if (B >= 0 && nb1 > 0 && nq > 0) {
-        run = wave_band(B, net1, net2, cutoff, lo, hi);
-        have = run;
-        if (lead) n_pairs++;
+    if constexpr (NW == 4) {
+      if (many) {
+        const int q = rb.queue[cls][e0 + (threadIdx.x >> 5)].y;
+        round_wave_entry<P, 1, WW, MASK, WMAX == 1 ? -1 : 1>(qdb, rs, prm, rb, h, q, cap_blocks, smem, s_xch, n_pairs,
+                                                             n_cells);
+        if (WMAX > 1 && h.nb1 > 32 * WW) {  // bands too wide for a warp
+          __syncthreads();
+          for (int k = 0; k < kWarps; k++)
+            round_wave_entry<P, 4, WMAX, MASK, 0>(qdb, rs, prm, rb, h, rb.queue[cls][e0 + k].y, cap_blocks, smem, s_xch,
+                                                  n_pairs, n_cells);
+          __syncthreads();
+        }
+        continue;
       }
     }
-    unsigned long long cells = 0;
-    if constexpr (kQ) {
-      uint32_t *tab = smem + 8 * cap_blocks + (threadIdx.x >> 5) * 32 * wave_codes(P);
-      const int got = wave_query<P>(smem, nb1, net1, qpl, run ? nq : 0, net2, lo, hi, tab, cells);
-      if (run) sum = got;
-    } else if (run) {  // uniform in the group
-      uint32_t *ring = smem + wave_table_words(P, cap_blocks) + group * kWaveRingWords;
-      sum = wave_any<P, NW, WMAX>(smem, nb1, qpl, nq, net2, lo, hi, cutoff, ring, s_xch, cells);
-    }
-    n_cells += 32 * cells;
-    bool pass = have && !(sum < cutoff);
-    if (word_after) {  // short-word test (func.cu:376-396), a warp per member
-      const uint32_t *list = rs.lists + (int64_t)r * rs.list_words;
-#pragma unroll
-      for (int k = 0; k < (kQ ? 2 : 1); k++) {
-        const int src = k * kQueryGroup;
-        if (!__shfl_sync(kFullMask, (int)(pass && net2 >= 16), src)) continue;
-        const uint32_t *qp = reinterpret_cast<const uint32_t *>(__shfl_sync(kFullMask, (unsigned long long)qpl, src));
-        const int n2 = __shfl_sync(kFullMask, net2, src);
-        const int ws = word_count_warp_bits<P>(qp, n2, prm.w, list);
-        if (!kQ || lane / kQueryGroup == k) pass = !(ws < word_min(L2, prm.w, s));
-      }
-    }
-    if (pass && lead) round_accept<MASK>(rb, r, q, sum);
+    round_wave_entry<P, NW, WMAX, MASK, -1>(qdb, rs, prm, rb, h, rb.queue[cls][e0 + threadIdx.x / GS].y, cap_blocks,
+                                            smem, s_xch, n_pairs, n_cells);
   }
   for (int o = 16; o; o >>= 1) {
     n_pairs += __shfl_down_sync(kFullMask, n_pairs, o);
@@ -502,7 +540,6 @@ RoundWaveFn round_wave_fn(int cls) {
     default: return k_round_wave<P, 0, 1, MASK>;
   }
 }
-inline int round_wave_groups(int cls) { return cls == 0 ? 4 : cls == 3 ? kAlignThreads / kQueryGroup : 1; }
 
 inline size_t round_align_smem(int type, int cls, int rep_nb) {
   const size_t ring = cls == 2 ? 0 : (size_t)(cls == 1 ? 128 : 64) * kAlignThreads;
@@ -512,7 +549,7 @@ inline size_t round_align_smem(int type, int cls, int rep_nb) {
 inline size_t round_wave_smem(int type, int cls, int rep_nb) {
   const int P = type ? 5 : 2;
   return 4 * (cls == 3 ? 8 * (size_t)rep_nb + kAlignThreads * wave_codes(P)
-                       : (size_t)wave_table_words(P, rep_nb) + (size_t)round_wave_groups(cls) * kWaveRingWords);
+                       : (size_t)wave_table_words(P, rep_nb) + (size_t)(kAlignThreads / 32) * kWaveRingWords);
 }
 
 // The alignment launches of a round: shapes for representatives of up to

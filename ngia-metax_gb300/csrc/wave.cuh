@@ -25,7 +25,10 @@
 // carries over the lanes with two votes, 500 DNA pairs of 1,450 residues
 // 100-275 -> 65 us.  Tried: planes in registers instead of the table (370
 // us), the columns rolled by four (250), the carry as a value instead of the
-// carry flag (231), two row words per thread where one is enough (292).
+// carry flag (231), two row words per thread where one is enough (292), the
+// next step's codes loaded ahead (12 mixed jobs 5% slower).  Once every
+// scheduler has a warp the instructions count, (80 + 16 (5 + 4 W)) a step for
+// 32 W rows of a warp: then a warp per pair with more words (wave_few).
 #pragma once
 #include <stdint.h>
 
@@ -43,11 +46,23 @@ __host__ __device__ constexpr int wave_codes(int P) { return 1 << P; }          
 // that the last chunk's missing blocks read zeros).
 __host__ __device__ constexpr int wave_stride(int nb) { return (nb + 31) & ~31; }
 __host__ __device__ constexpr int wave_table_words(int P, int nb) { return wave_codes(P) * wave_stride(nb); }
+// Place of block j's word in its row: 16-byte units of a 128-byte line swapped
+// by the line, so that eight lanes reading one unit each of chunks of 8 or 16
+// words (32 or 64 bytes apart) find it in eight different bank groups.
+__host__ __device__ constexpr int wave_place(int j) { return j ^ (((j >> 5) & 3) << 2); }
 
 // Widest band (blocks a query block covers) a group of GS threads can take
 // with W row words per thread when chunks are reused: a thread must have left
 // chunk q - 1 + GS alone until its neighbour is through with chunk q.
 __host__ __device__ constexpr int wave_cap(int GS, int W) { return W * (GS - 2) + GS / kWaveUnits + 1; }
+
+// Pairs up to which a CTA per pair is faster than a warp per pair, when a group
+// per pair is up to `pairs` (56 per SM for a job that has the GPU to itself:
+// here one pair per SM, a warp for each scheduler).  GB300, 12 mixed jobs of
+// records up to 10,000 residues 47.5 ms with a CTA always; 30.6, 30.4, 30.3,
+// 29.7 ms from 4, 2, 1 and 1/2 pairs per SM on; 30,000 proteins at s = 0.5 10.5
+// ms, and 9.4, 9.4, 9.2, 9.8.
+__host__ __device__ constexpr int wave_few(int pairs) { return pairs / 56; }
 
 // Band of one pair in blocks below and above the diagonal.  With a cutoff,
 // only the diagonals a chain of that many matches can touch; false when no
@@ -78,7 +93,7 @@ __device__ __forceinline__ void wave_table(const uint32_t *rp, int nb1, uint32_t
       uint32_t m = valid;
 #pragma unroll
       for (int p = 0; p < P; p++) m &= (a >> p) & 1 ? pl[p] : ~pl[p];
-      tab[a * stride + j] = m;
+      tab[a * stride + wave_place(j)] = m;
     }
   }
 }
@@ -99,23 +114,24 @@ __device__ __forceinline__ void wave_unpack(const uint32_t (&pl)[P], uint4 *out)
   out[1] = make_uint4(v[4], v[5], v[6], v[7]);
 }
 
-// W consecutive match words (W-word aligned, at most four at a time).
-template <int W>
-__device__ __forceinline__ void wave_load(uint32_t (&e)[W], const char *a) {
+// The W match words of a chunk at row a of the table: off[k] is the byte offset
+// of its k-th unit of four words (of its first word, W < 4).
+template <int W, int U>
+__device__ __forceinline__ void wave_load(uint32_t (&e)[W], const char *tab, uint32_t a, const uint32_t (&off)[U]) {
   if constexpr (W == 1) {
-    e[0] = *reinterpret_cast<const uint32_t *>(a);
+    e[0] = *reinterpret_cast<const uint32_t *>(tab + (a + off[0]));
   } else if constexpr (W == 2) {
-    const uint2 v = *reinterpret_cast<const uint2 *>(a);
+    const uint2 v = *reinterpret_cast<const uint2 *>(tab + (a + off[0]));
     e[0] = v.x;
     e[1] = v.y;
   } else {
 #pragma unroll
-    for (int w = 0; w < W; w += 4) {
-      const uint4 v = *reinterpret_cast<const uint4 *>(a + 4 * w);
-      e[w] = v.x;
-      e[w + 1] = v.y;
-      e[w + 2] = v.z;
-      e[w + 3] = v.w;
+    for (int k = 0; k < U; k++) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(tab + (a + off[k]));
+      e[4 * k] = v.x;
+      e[4 * k + 1] = v.y;
+      e[4 * k + 2] = v.z;
+      e[4 * k + 3] = v.w;
     }
   }
 }
@@ -133,14 +149,16 @@ __device__ __forceinline__ int wave_pair(const uint32_t *tab, int nb1, const uin
   const int g = warp * 32 + lane;
   const int q_last = min(nb1 - 1, nq - 1 + hi) / W;
   const uint32_t row_bytes = 4u * (uint32_t)wave_stride(nb1);
-  uint32_t row[W];
-  const char *base = nullptr;
+  constexpr int U = W > 4 ? W / 4 : 1;
+  uint32_t row[W], off[U];
+  const char *tabc = reinterpret_cast<const char *>(tab);
   int q = g, u0 = 0, u1 = 0, acc = 0;
   auto open = [&]() {  // chunk q: rows all-ones
     const bool used = q <= q_last;
     u0 = used ? S * max(0, q * W - hi) : 0;
     u1 = used ? min(S * nq, S * (q * W + W + lo)) : 0;
-    base = reinterpret_cast<const char *>(tab + (used ? q * W : 0));
+#pragma unroll
+    for (int k = 0; k < U; k++) off[k] = used ? 4u * (uint32_t)wave_place(q * W + 4 * k) : 0u;
 #pragma unroll
     for (int w = 0; w < W; w++) row[w] = 0xFFFFFFFFu;
   };
@@ -224,7 +242,7 @@ __device__ __forceinline__ int wave_pair(const uint32_t *tab, int nb1, const uin
     uint32_t cw = ncol > 0 && q > 0 ? cin << (32 - ncol) : 0u, ncw = 0;
     auto column = [&](uint32_t c) {  // one column of residue code c
       uint32_t e[W];
-      wave_load<W>(e, base + c * row_bytes);
+      wave_load<W, U>(e, tabc, c * row_bytes, off);
       dp_wave<W>(row, e, act, cw, ncw);
     };
     if (t < S * nq - 2 || __all_sync(kFullMask, !active || ncol == C)) {
@@ -259,17 +277,20 @@ __device__ __forceinline__ int wave_pair(const uint32_t *tab, int nb1, const uin
   return sum;
 }
 
+// Whether a group of GS threads with up to W row words each can hold the band.
+__host__ __device__ constexpr bool wave_holds(int GS, int W, int lo, int hi, int nb1) {
+  return lo + hi + 1 <= wave_cap(GS, W) || nb1 <= GS * W;
+}
+
 // The same with the fewest row words per thread (up to WMAX) the band allows;
 // a group that holds every rep block at once takes any band.  The caller
 // makes sure that WMAX words do.
 template <int P, int NW, int WMAX>
 __device__ __forceinline__ int wave_any(const uint32_t *tab, int nb1, const uint32_t *qp, int nq, int net2, int lo,
                                         int hi, int cut, uint32_t *ring, uint32_t *xch, unsigned long long &n_done) {
-  constexpr int GS = 32 * NW;
-  const int n = lo + hi + 1;
-#define NGIA_WAVE(W)                                        \
-  if constexpr (W <= WMAX)                                  \
-    if (W == WMAX || n <= wave_cap(GS, W) || nb1 <= GS * W) \
+#define NGIA_WAVE(W)                                          \
+  if constexpr (W <= WMAX)                                    \
+    if (W == WMAX || wave_holds(32 * NW, W, lo, hi, nb1))     \
       return wave_pair<P, W, NW>(tab, nb1, qp, nq, net2, lo, hi, cut, ring, xch, n_done);
   NGIA_WAVE(1) NGIA_WAVE(2) NGIA_WAVE(4) NGIA_WAVE(8) NGIA_WAVE(16)
 #undef NGIA_WAVE
@@ -330,7 +351,7 @@ __device__ __forceinline__ int wave_query(const uint32_t *rep_codes, int nb1, in
     uint32_t cw = ncol > 0 && g > 0 ? cin << (32 - ncol) : 0u, ncw = 0;
     auto column = [&](uint32_t c) {
       uint32_t e[1];
-      wave_load<1>(e, base + c * 128u);
+      e[0] = *reinterpret_cast<const uint32_t *>(base + c * 128u);
       dp_wave<1>(row, e, act, cw, ncw);
     };
     if (__all_sync(kFullMask, !active || ncol == C)) {
