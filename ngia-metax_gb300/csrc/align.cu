@@ -622,7 +622,9 @@ cudaError_t launch_align(ngia_ctx *c, int cls, cudaStream_t s, int score_mode) {
   RunParams prm = c->prm;
   // per length bucket (class): its own cut-off and CTA count when the tuner
   // chose them; pair scores go by the context's grids
-  int wp = score_mode ? c->warp_pairs_default : c->cls_warp_pairs[cls] >= 0 ? c->cls_warp_pairs[cls] : c->warp_pairs;
+  const int pairs = score_mode ? c->warp_pairs_default : c->warp_pairs;
+  int wp = !score_mode && c->cls_warp_pairs[cls] >= 0 ? c->cls_warp_pairs[cls]
+                                                      : group_cut(class_ring(c->db.type, cls), pairs);
   if (!wave_fits(c->db.type, c->cap_nb)) wp = -1;
   int grid = std::max(1, c->grid_align[cls] / std::max(1, c->cls_grid_div[cls]));
   int grid_wave = c->grid_wave[cls];
@@ -630,7 +632,7 @@ cudaError_t launch_align(ngia_ctx *c, int cls, cudaStream_t s, int score_mode) {
     grid = std::min(grid, (score_mode + kAlignThreads - 1) / kAlignThreads);
     grid_wave = std::min(grid_wave, score_mode);
   }
-  int few = wave_few(std::min(wp, c->warp_pairs_default));
+  int few = wave_few(std::min(pairs, c->warp_pairs_default));
   void *args[] = {&db, &rb, &prm, &cls, &score_mode, &wp, &few};
   cudaError_t e = cudaLaunchKernel((const void *)align_fn(c->db.type, cls), dim3(grid), dim3(kAlignThreads), args,
                                    align_smem(c->db.type, c->db.max_nb, cls), s);

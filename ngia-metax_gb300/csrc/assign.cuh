@@ -447,7 +447,7 @@ __device__ __forceinline__ void round_wave_entry(const DevDB &qdb, const RepStor
 // Shared memory: match table | code rings, or rep codes | match tables.
 template <int P, int NW, int WMAX, bool MASK>
 __global__ void __launch_bounds__(kAlignThreads)
-    k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int wave_pairs, int cap_blocks) {
+    k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int wave_pairs, int cap_blocks, int few) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr bool kQ = NW == 0;
   constexpr int GS = kQ ? kQueryGroup : 32 * NW, kGroups = kAlignThreads / GS, kWarps = kAlignThreads / 32;
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   __shared__ uint32_t s_qn, s_many;
   if (threadIdx.x == 0) {
     s_qn = round_wave(rb, cls, wave_pairs) ? (uint32_t)min((int64_t)rb.ctl[cls], rb.cap) : 0u;
-    s_many = NW == 4 && rb.ctl[kCtlPairs + cls] > (uint32_t)wave_few(wave_pairs);
+    s_many = NW == 4 && rb.ctl[kCtlPairs + cls] > (uint32_t)few;
   }
   __syncthreads();
   const uint32_t qn = s_qn;
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(kAlignThreads)
 
 // ---- launch ---------------------------------------------------------------------
 using RoundAlignFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, uint32_t *, int64_t, int, int);
-using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int);
+using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, int);
 
 template <int P, bool MASK>
 RoundAlignFn round_align_fn(int cls) {
@@ -559,6 +559,7 @@ struct RoundPlan {
   int type = 0, rep_nb = 1;
   int grid[kServeClasses] = {0, 0, 0, 0}, wave_grid[kServeClasses] = {0, 0, 0, 0};
   int wave_pairs[kServeClasses] = {0, 0, 0, 0};
+  int few = 0;  // k_round_wave's
   uint32_t *scratch = nullptr;  // global ring of class 2
   int64_t scratch_words = 0;
   int ring_rows = 0;
@@ -583,6 +584,7 @@ cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   pl.type = type;
   pl.rep_nb = rep_nb;
+  pl.few = wave_few(56 * num_sms);
   std::lock_guard<std::mutex> lock(mu);
   for (int c = 0; c < kServeClasses; c++)
     for (int wave = 0; wave < 2; wave++) {
@@ -599,7 +601,7 @@ cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kAlignThreads, bytes) != cudaSuccess || occ < 1) occ = 1;
       (wave ? pl.wave_grid : pl.grid)[c] = num_sms * occ;
       // the clustering kernels' cut-off (api.cu)
-      if (wave) pl.wave_pairs[c] = 56 * num_sms;
+      if (wave) pl.wave_pairs[c] = group_cut(c == 2 ? 0 : 64, 56 * num_sms);
     }
   pl.ring_rows = global_rows(rep_nb);
   pl.scratch_words = serve_class_used(2, rep_nb, MASK) ? (int64_t)pl.grid[2] * kAlignThreads * pl.ring_rows : 1;
@@ -617,7 +619,7 @@ cudaError_t round_launch(const RoundPlan &pl, const DevDB &qdb, const RepStore &
     RepStore r = rs;
     RunParams p = prm;
     RoundBufs b = rb;
-    int cls = c, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb;
+    int cls = c, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb, few = pl.few;
     uint32_t *scr = pl.scratch;
     int64_t sw = pl.scratch_words;
     int rm = pl.ring_rows;
@@ -626,7 +628,7 @@ cudaError_t round_launch(const RoundPlan &pl, const DevDB &qdb, const RepStore &
                                      round_align_smem(pl.type, c, pl.rep_nb), st);
     if (e != cudaSuccess) return e;
     if (wp <= 0) continue;
-    void *wargs[] = {&db, &r, &p, &b, &cls, &wp, &cap};
+    void *wargs[] = {&db, &r, &p, &b, &cls, &wp, &cap, &few};
     e = cudaLaunchKernel(round_fn<MASK>(pl.type, c, true), dim3(pl.wave_grid[c]), dim3(kAlignThreads), wargs,
                          round_wave_smem(pl.type, c, pl.rep_nb), st);
     if (e != cudaSuccess) return e;

@@ -46,6 +46,16 @@ __host__ __device__ inline bool class_used(int type, int c, int max_nb) {
   const int ring = class_ring(type, c);
   return ring == 64 || max_nb > (ring == 128 ? kSmallWindow : kWideWindow);
 }
+// Pairs up to which a class takes its group-per-pair kernel, when those with
+// rows in shared memory do up to `pairs` (api.cu): four times as many where
+// the other kernel has its rows in global memory.  GB300, ms for 30,000
+// proteins at s = 0.5 (two seeds) and 12 mixed jobs: 9.3, 7.4, 30.0 at the
+// same, 9.6, 7.4, 30.6 at twice, 5.5, 4.8, 27.7 at four times, 5.4, 4.8, 28.9
+// at eight times as many; four times for rows in shared memory too: 28.5, and
+// 16 serving batches 28.1 -> 28.7.
+__host__ __device__ constexpr int group_cut(int ring, int pairs) {
+  return ring == 0 && pairs < (1 << 28) ? 4 * pairs : pairs;
+}
 // Parallel branch class c runs in: the two classes on the global ring share
 // its scratch and run one after the other.
 __host__ __device__ inline int class_stream(int type, int c) {
