@@ -634,9 +634,14 @@ cudaError_t launch_align(ngia_ctx *c, int cls, cudaStream_t s, int score_mode) {
   }
   int few = wave_few(std::min(pairs, c->warp_pairs_default));
   void *args[] = {&db, &rb, &prm, &cls, &score_mode, &wp, &few};
-  cudaError_t e = cudaLaunchKernel((const void *)align_fn(c->db.type, cls), dim3(grid), dim3(kAlignThreads), args,
-                                   align_smem(c->db.type, c->db.max_nb, cls), s);
-  if (e != cudaSuccess || wp <= 0) return e;  // no class goes to the group kernel
+  // a call's pairs are known here: with no more than the cut-off no class can
+  // go to the thread-per-pair kernel
+  if (!score_mode || score_mode > wp) {
+    cudaError_t e = cudaLaunchKernel((const void *)align_fn(c->db.type, cls), dim3(grid), dim3(kAlignThreads), args,
+                                     align_smem(c->db.type, c->db.max_nb, cls), s);
+    if (e != cudaSuccess) return e;
+  }
+  if (wp <= 0) return cudaSuccess;  // no class goes to the group kernel
   return cudaLaunchKernel(wave_fn(c->db.type, cls), dim3(grid_wave), dim3(kAlignThreads), args,
                           wave_smem(c->db.type, cls, c->db.max_nb), s);
 }

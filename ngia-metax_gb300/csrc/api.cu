@@ -11,6 +11,7 @@
 #include <climits>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <new>
 
@@ -28,11 +29,6 @@ using namespace ngia::drv;
 
 namespace ngia {
 namespace drv {
-
-template <class T>
-cudaError_t dalloc(T **p, size_t count) {
-  return cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(count, 1));
-}
 
 int check_device_error(ngia_ctx *c) {
   if (c->h_state->err)
@@ -131,6 +127,10 @@ void destroy_graph(ngia_ctx *c) {
 // node re-runs it until k_next clears the condition.
 int build_graph(ngia_ctx *c) {
   destroy_graph(c);
+  for (int k = 0; k < ngia::kNumClasses && !c->batch_member; k++) {
+    if (!c->side[k]) CK(cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking));
+    if (!c->join_ev[k]) CK(cudaEventCreateWithFlags(&c->join_ev[k], cudaEventDisableTiming));
+  }
   CK(cudaGraphCreate(&c->graph, 0));
   cudaGraphConditionalHandle cond;
   CK(cudaGraphConditionalHandleCreate(&cond, c->graph, 1, cudaGraphCondAssignDefault));
@@ -203,7 +203,6 @@ extern "C" int ngia_open(const ngia_db_view *v, ngia_ctx **out) { return ngia::d
 
 namespace {
 
-using ngia::drv::dalloc;
 
 // Streams and events of a context.
 int create_streams(ngia_ctx *c) {
@@ -213,11 +212,6 @@ int create_streams(ngia_ctx *c) {
     return fail(NGIA_E_CUDA, "cannot query SM count");
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(NGIA_E_CUDA, "cannot create stream");
-  for (int k = 0; k < ngia::kNumClasses; k++) {
-    if (cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->join_ev[k], cudaEventDisableTiming) != cudaSuccess)
-      return fail(NGIA_E_CUDA, "cannot create side streams");
-  }
   if (cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&c->ev_step0) != cudaSuccess || cudaEventCreate(&c->ev_step1) != cudaSuccess ||
       cudaEventCreate(&c->ev_p0) != cudaSuccess || cudaEventCreate(&c->ev_p1) != cudaSuccess ||
@@ -225,10 +219,18 @@ int create_streams(ngia_ctx *c) {
     return fail(NGIA_E_CUDA, "cannot create event");
   for (auto &ev : c->ev_cls)
     if (cudaEventCreate(&ev) != cudaSuccess) return fail(NGIA_E_CUDA, "cannot create event");
-  if (dalloc(&c->d_flags, 3) != cudaSuccess || cudaMallocHost((void **)&c->h_flags, 3 * sizeof(int32_t)) != cudaSuccess)
-    return fail(NGIA_E_NOMEM, "ngia_open: allocation failed");
-  if (cudaMallocHost((void **)&c->h_state, sizeof(ngia::RunState)) != cudaSuccess)
-    return fail(NGIA_E_NOMEM, "ngia_open: pinned allocation failed");
+  constexpr size_t kState = (sizeof(ngia::RunState) + 63) & ~(size_t)63;
+  constexpr size_t kMirror = kState + 64 + kMirrorCtl;
+  static_assert(kMirror % 64 == 0, "aligned_alloc");
+  void *mirror = nullptr;
+  if (!c->batch_member)
+    mirror = std::aligned_alloc(64, kMirror);
+  else if (cudaMallocHost(&mirror, kMirror) != cudaSuccess)
+    mirror = nullptr;
+  if (!mirror) return fail(NGIA_E_NOMEM, "ngia_open: host allocation failed");
+  c->h_state = reinterpret_cast<ngia::RunState *>(mirror);
+  c->h_flags = reinterpret_cast<int32_t *>((char *)mirror + kState);
+  c->h_ctl = (unsigned char *)mirror + kState + 64;
   std::memset(c->h_state, 0, sizeof(ngia::RunState));
   return NGIA_OK;
 }
@@ -240,10 +242,15 @@ int alloc_db(ngia_ctx *c, int type, int64_t cap_n, int64_t cap_words) {
   // the test reads the planes instead)
   const char *pc = getenv("NGIA_PROTEIN_CODES");
   const bool codes = type != 0 && !(pc && atoi(pc) == 0);
-  if (dalloc(&c->d_words, (size_t)cap_words + 4) != cudaSuccess || dalloc(&c->d_off, (size_t)cap_n) != cudaSuccess ||
-      dalloc(&c->d_len, (size_t)cap_n) != cudaSuccess || dalloc(&c->d_net, (size_t)cap_n) != cudaSuccess ||
-      dalloc(&c->d_cnt, (size_t)cap_n * A) != cudaSuccess ||
-      (codes && dalloc(&c->d_codes, (size_t)cap_words + 4) != cudaSuccess))
+  DevBlock &m = c->mem_db;
+  m.add(&c->d_flags, 3);
+  m.add(&c->d_words, (size_t)cap_words + 4);
+  m.add(&c->d_off, (size_t)cap_n);
+  m.add(&c->d_len, (size_t)cap_n);
+  m.add(&c->d_net, (size_t)cap_n);
+  m.add(&c->d_cnt, (size_t)cap_n * A);
+  if (codes) m.add(&c->d_codes, (size_t)cap_words + 4);
+  if (m.take() != cudaSuccess)
     return fail(NGIA_E_NOMEM, "ngia_open: device allocation of the database failed");
   c->cap_n = cap_n;
   c->cap_words = cap_words;
@@ -324,19 +331,20 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
   c->cap_nb = std::max(1, cap_nb);
   const size_t nbw = (size_t)(cap_n + 31) / 32;
   ngia::RunBufs &rb = c->rb;
-  bool ok = dalloc(&rb.st, 1) == cudaSuccess && dalloc(&rb.cluster, (size_t)cap_n) == cudaSuccess &&
-            dalloc(&rb.ident, (size_t)cap_n) == cudaSuccess && dalloc(&rb.alive, nbw) == cudaSuccess &&
-            dalloc(&rb.rep_rec, 32 + (size_t)ngia::kMaxBlocks * 5 + 64) == cudaSuccess &&
-            dalloc(&rb.rep_list, ngia::kListWords) == cudaSuccess &&
-            dalloc(&rb.first_short, ngia::kRefGridThreads) == cudaSuccess &&
-            dalloc(&rb.scan_part, nbw) == cudaSuccess && dalloc(&rb.long_list, (size_t)cap_n) == cudaSuccess;
-  ok = ok && cudaMalloc((void **)&rb.flags, 4 * std::max<size_t>(nbw, 1)) == cudaSuccess;
-  ok = ok && dalloc(&rb.fstats, (size_t)ngia::kFilterStripes * ngia::kFilterStats) == cudaSuccess;
-  for (int k = 0; ok && k < ngia::num_classes(type); k++)
-    if (ngia::class_used(type, k, c->cap_nb)) ok = dalloc(&rb.queue[k], (size_t)cap_n) == cudaSuccess;
-  if (!ok) return fail(NGIA_E_NOMEM, "ngia_open: device allocation of run buffers failed");
-  cudaMemsetAsync(rb.rep_list, 0, 4 * ngia::kListWords, c->stream);
-  cudaMemsetAsync(rb.fstats, 0, 8 * ngia::kFilterStripes * ngia::kFilterStats, c->stream);
+  DevBlock &m = c->mem_run;
+  m.add(&rb.st, 1);
+  m.add(&rb.cluster, (size_t)cap_n);
+  m.add(&rb.ident, (size_t)cap_n);
+  m.add(&rb.alive, nbw);
+  m.add(&rb.rep_rec, 32 + (size_t)ngia::kMaxBlocks * 5 + 64);
+  m.add(&rb.rep_list, ngia::kListWords);
+  m.add(&rb.first_short, ngia::kRefGridThreads);
+  m.add(&rb.scan_part, nbw);
+  m.add(&rb.long_list, (size_t)cap_n);
+  m.add((uint32_t **)&rb.flags, nbw);
+  m.add(&rb.fstats, (size_t)ngia::kFilterStripes * ngia::kFilterStats);
+  for (int k = 0; k < ngia::num_classes(type); k++)
+    if (ngia::class_used(type, k, c->cap_nb)) m.add(&rb.queue[k], (size_t)cap_n);
   if (ngia::align_configure(type, c->cap_nb) != cudaSuccess || ngia::filter_configure() != cudaSuccess)
     return fail(NGIA_E_CUDA, "ngia_open: kernel attributes");
   // the widest class keeps its rows in global scratch, sized for this
@@ -349,8 +357,10 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
   rb.generic_lanes = std::max(c->grid_align[1], c->grid_align[g]) * ngia::align_threads();
   rb.ring_rows = ngia::global_rows(c->cap_nb);
   rb.scratch_words = ngia::class_used(type, g, c->cap_nb) ? (int64_t)rb.generic_lanes * rb.ring_rows : 1;
-  if (dalloc(&rb.scratch, (size_t)rb.scratch_words) != cudaSuccess)
-    return fail(NGIA_E_NOMEM, "ngia_open: device allocation of alignment scratch failed");
+  m.add(&rb.scratch, (size_t)rb.scratch_words);
+  if (m.take() != cudaSuccess) return fail(NGIA_E_NOMEM, "ngia_open: device allocation of run buffers failed");
+  cudaMemsetAsync(rb.rep_list, 0, 4 * ngia::kListWords, c->stream);
+  cudaMemsetAsync(rb.fstats, 0, 8 * ngia::kFilterStripes * ngia::kFilterStats, c->stream);
   return NGIA_OK;
 }
 
@@ -450,29 +460,11 @@ extern "C" int ngia_close(ngia_ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   destroy_graph(c);
   ngia::drv::spec_free(c);
-  cudaFree(c->d_words);
-  cudaFree(c->d_off);
-  cudaFree(c->d_len);
-  cudaFree(c->d_net);
-  cudaFree(c->d_cnt);
-  cudaFree(c->d_codes);
-  ngia::RunBufs &rb = c->rb;
-  cudaFree(rb.st);
-  cudaFree(rb.cluster);
-  cudaFree(rb.ident);
-  cudaFree(rb.alive);
-  cudaFree(rb.rep_rec);
-  cudaFree(rb.rep_list);
-  cudaFree(rb.first_short);
-  cudaFree(rb.scan_part);
-  cudaFree(rb.long_list);
-  cudaFree(rb.flags);
-  cudaFree(rb.fstats);
-  cudaFree(rb.scratch);
-  for (int k = 0; k < ngia::kNumClasses; k++) cudaFree(rb.queue[k]);
-  if (c->h_state) cudaFreeHost(c->h_state);
-  cudaFree(c->d_flags);
-  if (c->h_flags) cudaFreeHost(c->h_flags);
+  c->mem_db.give();
+  c->mem_run.give();
+  c->mem_score.give();
+  if (c->batch_member && c->h_state) cudaFreeHost(c->h_state);
+  if (!c->batch_member) std::free(c->h_state);
   for (int k = 0; k < ngia::kNumClasses; k++) {
     if (c->side[k]) cudaStreamDestroy(c->side[k]);
     if (c->join_ev[k]) cudaEventDestroy(c->join_ev[k]);
@@ -667,21 +659,24 @@ extern "C" int ngia_pair_scores(ngia_ctx *c, const ngia_params *p, int32_t rep, 
   c->prm.precise = p->precise;
   c->prm.refill = 32;
   c->prm.wait_polls = ngia::kWaitPolls;
-  int32_t *d_c = nullptr, *d_o = nullptr;
-  CK(dalloc(&d_c, (size_t)n));
-  CK(dalloc(&d_o, 4 * (size_t)n));
-  c->rb.score_cands = d_c;
-  c->rb.score_out = d_o;
-  CK(cudaMemcpyAsync(d_c, cands, 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+  if (n > c->score_cap) {
+    c->mem_score.give();
+    c->score_cap = 0;
+    c->mem_score.add(&c->d_score_cands, (size_t)n);
+    c->mem_score.add(&c->d_score_out, 4 * (size_t)n);
+    CK(c->mem_score.take());
+    c->score_cap = n;
+  }
+  c->rb.score_cands = c->d_score_cands;
+  c->rb.score_out = c->d_score_out;
+  CK(cudaMemcpyAsync(c->d_score_cands, cands, 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemsetAsync(c->rb.st, 0, sizeof(ngia::RunState), c->stream));
   CK(ngia::launch_prep(c, rep));
   CK(ngia::launch_score_classify(c, n));
   for (int k = 0; k < ngia::num_classes(c->db.type); k++)
     if (ngia::class_used(c->db.type, k, c->db.max_nb)) CK(ngia::launch_align(c, k, c->stream, n));
-  CK(cudaMemcpyAsync(out, d_o, 16 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(out, c->d_score_out, 16 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
   rc = pull_state(c);
-  cudaFree(d_c);
-  cudaFree(d_o);
   c->rb.score_cands = nullptr;
   c->rb.score_out = nullptr;
   c->begun = false;

@@ -8,6 +8,41 @@
 #include "../../include/ngia.h"
 #include "common.cuh"
 
+// Several device arrays in one allocation, each on a 256-byte boundary: a
+// cudaMalloc and its cudaFree take 2 us of host time on GB300 where the driver
+// has room in a chunk of its own, else 60 to 110, and a context has some 30
+// arrays.  Opening, clustering and closing a database of 500 short records,
+// ms: 1.82; in three allocations 1.65; with the rounds' queues sized by the
+// database 1.52; without pinned memory 1.25.
+struct DevBlock {
+  template <class T>
+  void add(T **p, size_t count) {
+    items.push_back({(void **)p, (sizeof(T) * (count ? count : 1) + 255) & ~(size_t)255});
+  }
+  cudaError_t take() {
+    size_t total = 0;
+    for (const Item &i : items) total += i.bytes;
+    const cudaError_t e = cudaMalloc(&base, total);
+    char *at = (char *)base;
+    for (const Item &i : items) {
+      *i.p = e == cudaSuccess ? at : nullptr;
+      at += i.bytes;
+    }
+    items.clear();
+    return e;
+  }
+  void give() {
+    cudaFree(base);
+    base = nullptr;
+  }
+  struct Item {
+    void **p;
+    size_t bytes;
+  };
+  std::vector<Item> items;
+  void *base = nullptr;
+};
+
 struct ngia_spec;  // speculative-round driver state (spec.cu)
 static_assert(ngia::kNumClasses == 7, "per-class initialisers of ngia_ctx");
 
@@ -16,7 +51,8 @@ struct ngia_ctx {
   int num_sms = 0;
   cudaStream_t stream = nullptr;
   ngia::DevDB db{};
-  // owned device allocations of the database
+  // device arrays of the database (mem_db) and of a run (mem_run)
+  DevBlock mem_db, mem_run;
   uint32_t *d_words = nullptr;
   int64_t *d_off = nullptr;
   int32_t *d_len = nullptr, *d_net = nullptr;
@@ -29,10 +65,19 @@ struct ngia_ctx {
   int64_t cap_n = 0, cap_words = 0;
   int32_t cap_nb = 0;
   int32_t *d_flags = nullptr;  // loader results: max blocks, short record, bad record
-  int32_t *h_flags = nullptr;  // pinned mirror
+  int32_t *h_flags = nullptr;  // host mirror (behind h_state)
   // run buffers
   ngia::RunBufs rb{};
-  ngia::RunState *h_state = nullptr;  // pinned mirror
+  // Host mirror.  Pinned for contexts that share the GPU with others (a copy
+  // into it does not hold up the thread that drives them); pageable for a
+  // context of its own, which waits for each copy anyway: allocating and
+  // freeing a process's only pinned page takes 270 us on GB300, a copy into
+  // pageable memory a few more than into pinned.
+  ngia::RunState *h_state = nullptr;
+  unsigned char *h_ctl = nullptr;  // kMirrorCtl bytes of it: the speculative driver's (behind h_flags)
+  // pair scores: the calls' candidates and results, grown to the largest call
+  DevBlock mem_score;
+  int32_t score_cap = 0, *d_score_cands = nullptr, *d_score_out = nullptr;
   ngia::RunParams prm{};
   int mode = 0;
   bool begun = false;
@@ -59,7 +104,7 @@ struct ngia_ctx {
   cudaGraph_t graph = nullptr;
   bool graph_ready = false;
   ngia::RunParams graph_prm{};
-  cudaStream_t side[ngia::kNumClasses] = {nullptr};
+  cudaStream_t side[ngia::kNumClasses] = {nullptr};  // created with the first graph, as are join_ev
   cudaEvent_t fork_ev = nullptr, join_ev[ngia::kNumClasses] = {nullptr};
   // timing: whole steps, and (profiling, plain form) filter / align stages
   cudaEvent_t ev_step0 = nullptr, ev_step1 = nullptr, ev_p0 = nullptr, ev_p1 = nullptr, ev_p2 = nullptr;
@@ -70,6 +115,8 @@ struct ngia_ctx {
   float last_step_ms = 0.f;
   ngia_spec *spec = nullptr;  // NGIA_MODE_SPEC buffers, allocated on first use
 };
+
+constexpr size_t kMirrorCtl = 1024;
 
 namespace ngia {
 // api.cu: driver internals shared with batch.cu / serve.cu
@@ -89,6 +136,7 @@ int build_graph(ngia_ctx *c);
 int ensure_graph(ngia_ctx *c);  // build_graph unless the captured one is current
 void destroy_graph(ngia_ctx *c);
 int pull_state(ngia_ctx *c);
+int check_device_error(ngia_ctx *c);  // of the mirrored run state
 int enqueue_iteration(ngia_ctx *c, bool graph, cudaGraphConditionalHandle cond);
 void fill_stats(const ngia_ctx *c, ngia_stats *stats);
 int validate_params(int type, const ngia_params *p);

@@ -12,6 +12,7 @@
 //                   representative is the first unclustered sequence
 #include <algorithm>
 #include <climits>
+#include <mutex>
 
 #include "../host/host_common.h"
 #include "ctx.h"
@@ -512,6 +513,14 @@ static size_t word_smem(int type, int w) {
 
 cudaError_t filter_configure() {
   constexpr size_t most = 72 * 1024;  // DNA w = 8: 8 KB bitset, 64 KB table
+  static std::mutex mu;
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t d = cudaGetDevice(&dev);
+  if (d != cudaSuccess) return d;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done[dev]) return cudaSuccess;
   for (int type = 0; type < 2; type++)
     for (int M = 1; M <= (type ? 2 : 4); M *= 2) {
       cudaError_t e = cudaFuncSetAttribute((const void *)word_fn(type, M), cudaFuncAttributeMaxDynamicSharedMemorySize, most);
@@ -519,6 +528,7 @@ cudaError_t filter_configure() {
         e = cudaFuncSetAttribute((const void *)long_fn(type, M), cudaFuncAttributeMaxDynamicSharedMemorySize, most);
       if (e != cudaSuccess) return e;
     }
+  done[dev] = true;
   return cudaSuccess;
 }
 

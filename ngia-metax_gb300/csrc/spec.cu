@@ -72,6 +72,8 @@ struct SpecCtl {
   int32_t ramp;             // candidates allowed so far (0: first round)
   int32_t reserved;
   uint32_t prev[kCtlWords];  // the previous round's queue counters (RoundBufs ctl)
+  unsigned long long stats[2];  // RoundBufs::stats and the run state after the round: the host reads
+  RunState st;                  // a round's outcome in one copy
 };
 
 struct SpecDev {
@@ -147,6 +149,11 @@ __global__ void __launch_bounds__(1024) k_spec_pick(DevDB db, RunBufs run, SpecD
   for (int i = tid; i < s_k; i += blockDim.x) sd.rs_off[i] = db.off[sd.list[i]];
   // the plain iteration (and a checkpoint) take the representative from here
   if (tid == 0 && total > 0) st->rep = sd.list[0];
+  __syncthreads();
+  static_assert(sizeof(RunState) % 4 == 0, "copied by words");
+  if (tid < 2) sd.ctl->stats[tid] = rb.stats[tid];
+  for (int i = tid; i < (int)(sizeof(RunState) / 4); i += blockDim.x)
+    reinterpret_cast<uint32_t *>(&sd.ctl->st)[i] = reinterpret_cast<const uint32_t *>(st)[i];
 }
 
 // Filter of a round: candidate blockIdx.y against kSpecTile members of the
@@ -274,7 +281,9 @@ struct ngia_spec {
   ngia::SpecDev d{};
   ngia::RoundBufs rb{};
   ngia::RepStore rs{};
-  unsigned char *h_ctl = nullptr;  // pinned: RoundBufs ctl + SpecCtl
+  unsigned char *h_ctl = nullptr;  // the context's: RoundBufs ctl + SpecCtl
+  unsigned long long stats[2] = {0, 0};  // pairs and cells of the run's rounds
+  DevBlock mem;
   unsigned char *d_ctl = nullptr;
   ngia::RoundPlan plan;
   int budget = ngia::kSpecBudget;  // pairs per round (NGIA_SPEC_BUDGET lowers it)
@@ -293,12 +302,8 @@ namespace {
     if (e_ != cudaSuccess) return fail(NGIA_E_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
   } while (0)
 
-template <class T>
-cudaError_t dmalloc(T **p, size_t count) {
-  return cudaMalloc((void **)p, sizeof(T) * (count ? count : 1));
-}
-
 constexpr size_t kCtlBytes = kCtlWords * sizeof(uint32_t) + sizeof(SpecCtl);
+static_assert(kCtlBytes <= kMirrorCtl, "the mirror in the context");
 
 int spec_alloc(ngia_ctx *c) {
   ngia_spec *sp = c->spec;
@@ -313,17 +318,27 @@ int spec_alloc(ngia_ctx *c) {
   sp->type = c->db.type;
   sp->k_max = (int)std::max<int64_t>(1, std::min<int64_t>(kSpecMax, kSpecScoreWords / std::max<int64_t>(1, n)));
   const int lw = kListWords;
-  if (dmalloc(&sp->d.list, (size_t)n) != cudaSuccess || dmalloc(&sp->d.rs_off, kSpecMax) != cudaSuccess ||
-      dmalloc(&sp->d.lists, (size_t)kSpecMax * lw) != cudaSuccess || dmalloc(&sp->d.first, kSpecMax) != cudaSuccess || dmalloc(&sp->d_ctl, kCtlBytes) != cudaSuccess ||
-      cudaMallocHost((void **)&sp->h_ctl, kCtlBytes) != cudaSuccess ||
-      dmalloc(&sp->rb.mask, (size_t)n) != cudaSuccess ||
-      dmalloc(&sp->rb.score, (size_t)sp->k_max * (size_t)n) != cudaSuccess ||
-      dmalloc(&sp->rb.stats, 2) != cudaSuccess)
-    return fail(NGIA_E_NOMEM, "spec: device allocation failed");
-  // a tile of a candidate pads its last group of each class
-  const int64_t cap = kSpecBudget + 32ll * kSpecMax * ((n + kSpecTile - 1) / kSpecTile);
+  CKP(round_plan<true>(sp->plan, sp->type, nb, c->num_sms));
+  // a tile of a candidate pads its last group of each class (64 MB of queues
+  // for a small set cost its open and close 0.1 ms)
+  const int64_t cap = std::min<int64_t>(kSpecBudget, n * sp->k_max) + 32ll * kSpecMax * ((n + kSpecTile - 1) / kSpecTile);
+  DevBlock &m = sp->mem;
+  m.add(&sp->d.list, (size_t)n);
+  m.add(&sp->d.rs_off, kSpecMax);
+  m.add(&sp->d.lists, (size_t)kSpecMax * lw);
+  m.add(&sp->d.first, kSpecMax);
+  m.add(&sp->d_ctl, kCtlBytes);
+  m.add(&sp->rb.mask, (size_t)n);
+  m.add(&sp->rb.score, (size_t)sp->k_max * (size_t)n);
+  m.add(&sp->rb.stats, 2);
   for (int k = 0; k < kServeClasses; k++)
-    if (serve_class_used(k, nb, true) && dmalloc(&sp->rb.queue[k], (size_t)cap) != cudaSuccess) return fail(NGIA_E_NOMEM, "spec: queue allocation failed");
+    if (serve_class_used(k, nb, true)) m.add(&sp->rb.queue[k], (size_t)cap);
+  m.add(&sp->plan.scratch, (size_t)sp->plan.scratch_words);
+  if (m.take() != cudaSuccess) {
+    spec_free(c);
+    return fail(NGIA_E_NOMEM, "spec: device allocation failed");
+  }
+  sp->h_ctl = c->h_ctl;
   sp->rb.ctl = reinterpret_cast<uint32_t *>(sp->d_ctl);
   sp->d.ctl = reinterpret_cast<SpecCtl *>(sp->d_ctl + kCtlWords * sizeof(uint32_t));
   sp->rb.cap = cap;
@@ -331,9 +346,6 @@ int spec_alloc(ngia_ctx *c) {
   sp->rb.score_stride = n;
   sp->rb.key = nullptr;
   sp->rb.todo = nullptr;
-  CKP(round_plan<true>(sp->plan, sp->type, nb, c->num_sms));
-  if (dmalloc(&sp->plan.scratch, (size_t)sp->plan.scratch_words) != cudaSuccess)
-    return fail(NGIA_E_NOMEM, "spec: scratch allocation failed");
   return NGIA_OK;
 }
 
@@ -377,7 +389,12 @@ int spec_launch_round(ngia_ctx *c, bool lists, int k, int alive) {
 int spec_read(ngia_ctx *c) {
   ngia_spec *sp = c->spec;
   CKP(cudaMemcpyAsync(sp->h_ctl, sp->d_ctl, kCtlBytes, cudaMemcpyDeviceToHost, c->stream));
-  return pull_state(c);  // synchronises the stream
+  CKP(cudaStreamSynchronize(c->stream));
+  const SpecCtl *ctl = reinterpret_cast<const SpecCtl *>(sp->h_ctl + kCtlWords * sizeof(uint32_t));
+  *c->h_state = ctl->st;
+  sp->stats[0] = ctl->stats[0];
+  sp->stats[1] = ctl->stats[1];
+  return check_device_error(c);
 }
 
 }  // namespace
@@ -394,6 +411,7 @@ int spec_prepare(ngia_ctx *c) {
   if (rc) return rc;
   ngia_spec *sp = c->spec;
   CKP(cudaMemsetAsync(sp->rb.stats, 0, 2 * sizeof(unsigned long long), c->stream));
+  sp->stats[0] = sp->stats[1] = 0;
   CKP(cudaMemsetAsync(sp->d_ctl, 0, kCtlBytes, c->stream));
   sp->big = false;
   sp->budget = kSpecBudget;
@@ -406,17 +424,7 @@ int spec_prepare(ngia_ctx *c) {
 void spec_free(ngia_ctx *c) {
   ngia_spec *sp = c->spec;
   if (!sp) return;
-  cudaFree(sp->d.list);
-  cudaFree(sp->d.rs_off);
-  cudaFree(sp->d.lists);
-  cudaFree(sp->d.first);
-  cudaFree(sp->d_ctl);
-  if (sp->h_ctl) cudaFreeHost(sp->h_ctl);
-  cudaFree(sp->rb.mask);
-  cudaFree(sp->rb.score);
-  cudaFree(sp->rb.stats);
-  for (auto *q : sp->rb.queue) cudaFree(q);
-  cudaFree(sp->plan.scratch);
+  sp->mem.give();
   delete sp;
   c->spec = nullptr;
 }
@@ -488,13 +496,8 @@ int spec_step(ngia_ctx *c, int64_t max_iters) {
 }
 
 void spec_stats(const ngia_ctx *c, int64_t *pairs, int64_t *cells) {
-  *pairs = *cells = 0;
-  if (!c->spec) return;
-  unsigned long long h[2] = {0, 0};
-  if (cudaMemcpy(h, c->spec->rb.stats, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess) {
-    *pairs = (int64_t)h[0];
-    *cells = (int64_t)h[1];
-  }
+  *pairs = c->spec ? (int64_t)c->spec->stats[0] : 0;
+  *cells = c->spec ? (int64_t)c->spec->stats[1] : 0;
 }
 
 }  // namespace drv
