@@ -55,11 +55,11 @@ struct AlignHdr {
 // shared memory with bulk copies.  Returns false when there is no work.
 template <int P>
 // groups: pairs a CTA of the group-per-pair kernel works on at a time (it
-// takes classes with at most warp_pairs pairs; kAlignThreads / 32 once there
-// are more than `few`), 0 for the thread-per-pair kernels (classes with more);
+// takes classes with at most warp_pairs pairs; more once there are more than
+// `few`), 0 for the thread-per-pair kernels (classes with more);
 // the other kernel of a class returns here, before any staging.
 __device__ __forceinline__ bool align_setup(const DevDB &db, const RunBufs &rb, const RunParams &prm, int cls,
-                                            int score_mode, int warp_pairs, int groups, int few, uint32_t *smem,
+                                            int score_mode, int warp_pairs, int groups, int few, int subs, uint32_t *smem,
                                             uint64_t *bar, AlignHdr &h) {
   __shared__ int s_hdr[6];
   RunState *st = rb.st;
@@ -67,7 +67,8 @@ __device__ __forceinline__ bool align_setup(const DevDB &db, const RunBufs &rb, 
     const bool skip = !score_mode && (st->done || st->iter >= st->iter_limit || st->err);
     const int qn = skip ? 0 : (int)st->qcount[cls];
     const bool mine = groups ? qn <= warp_pairs : qn > warp_pairs;
-    const bool idle = (int)blockIdx.x * (qn > few ? max(groups, kAlignThreads / 32) : groups) >= qn;
+    const int per = qn > subs ? kAlignThreads / kSubGroup : qn > few ? max(groups, kAlignThreads / 32) : groups;
+    const bool idle = (int)blockIdx.x * per >= qn;
     s_hdr[0] = mine && !(groups && idle) ? qn : 0;
     s_hdr[1] = st->rep_len;
     s_hdr[2] = st->rep_net;
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
   AlignHdr h;
   __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
   if (threadIdx.x == 0) s_qw = 0;
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, 0, 0, smem, &bar, h)) return;
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, 0, 0, 0, smem, &bar, h)) return;
   const uint32_t *s_pl = smem;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
   RunState *st = rb.st;
@@ -344,13 +345,15 @@ __host__ __device__ constexpr int wave_table_off(int P, int max_nb) { return ((m
 // up to 128 blocks, up to 16 for any; beyond, when every scheduler has a warp,
 // a warp per pair with up to 8 or 16 words, which takes half the instructions:
 // a step has 80 beside the columns' (5 + 4 W) each, and 2 nq + nb1 / W steps
-// are taken by one warp instead of four.
+// are taken by one warp instead of four.  Classes of windows up to 112 blocks
+// go to four pairs per warp above `subs` pairs.
 struct WaveCounts {
   unsigned long long pairs = 0, members = 0, cells = 0, done = 0;
 };
 
 // This CTA's share of the class's pairs, `per` neighbouring entries at a time.
-// MINE: -1 all, 1 the bands that a warp can hold, 0 the others.
+// MINE: -1 all, 1 the bands that a warp can hold, 0 the others, 2 those that 8
+// threads cannot hold.
 template <int P, int NW, int WMAX, int MINE>
 __device__ __forceinline__ void wave_entries(const DevDB &db, const RunBufs &rb, const RunParams &prm, int cls,
                                              int score_mode, const AlignHdr &h, int per, const uint32_t *s_tab,
@@ -375,7 +378,7 @@ __device__ __forceinline__ void wave_entries(const DevDB &db, const RunBufs &rb,
       int lo = 0, hi = 0;
       const bool run = !self && band && wave_band(B, h.net1, net2, cut, lo, hi);
       if constexpr (MINE >= 0)
-        if ((MINE != 0) == (run && !wave_holds(32, 16, lo, hi, nb1))) continue;
+        if ((MINE == 1) == (run && !(MINE == 2 ? sub_holds(lo, hi, nb1) : wave_holds(32, 16, lo, hi, nb1)))) continue;
       if (!score_mode && lead) {
         n.pairs++;
         n.cells += (unsigned long long)band_cells(B, nb1, net2);
@@ -408,9 +411,75 @@ __device__ __forceinline__ void wave_entries(const DevDB &db, const RunBufs &rb,
   }
 }
 
+// The same, four pairs per warp.
+template <int P>
+__device__ __forceinline__ void sub_entries(const DevDB &db, const RunBufs &rb, const RunParams &prm, int cls,
+                                            int score_mode, const AlignHdr &h, const uint32_t *s_tab, uint32_t *s_rings,
+                                            const uint32_t *s_list, unsigned long long *s_qw, WaveCounts &n) {
+  constexpr int kGroups = kAlignThreads / kSubGroup;
+  const int lane = threadIdx.x & 31, group = threadIdx.x / kSubGroup, first = threadIdx.x / 32 * kSubs;
+  const bool lead = lane % kSubGroup == 0;
+  const float s = prm.s;
+  const int nb1 = h.nb1;
+  uint32_t *ring = s_rings + group * kSubRingWords;
+  for (int e0 = blockIdx.x * kGroups + first; e0 < h.qn; e0 += gridDim.x * kGroups) {  // warp-uniform
+    const int e = e0 + (group - first);
+    bool have = e < h.qn, run = false;
+    int entry = 0, cand = 0, L2 = 0, net2 = 0, nq = 0, cutoff = 0, lo = 0, hi = 0, sum = 0;
+    const uint32_t *qpl = db.words;
+    bool self = false;
+    if (have) {
+      entry = rb.queue[cls][e];
+      cand = score_mode ? rb.score_cands[entry] : entry;
+      L2 = __ldg(db.len + cand);
+      net2 = __ldg(db.net + cand);
+      nq = (net2 + 31) >> 5;
+      const int B = band_blocks(h.L1, L2, s);
+      cutoff = cutoff_of(L2, s);
+      qpl = db.words + __ldg(db.off + cand) + db.hw;
+      self = cand == h.rep && !score_mode;
+      const bool band = !self && B >= 0 && nb1 > 0 && nq > 0;
+      run = band && wave_band(B, h.net1, net2, score_mode ? kNoCut : cutoff, lo, hi);
+      if (run && !sub_holds(lo, hi, nb1)) have = run = false;  // the next pass takes it
+      if (have && !score_mode && lead) {
+        n.pairs++;
+        n.cells += (unsigned long long)band_cells(B, nb1, net2);
+        atomicAdd(s_qw, (unsigned long long)(nq * P));
+      }
+      if (self) sum = h.net1;
+      if (band && !run) have = false;  // no chain can reach the cutoff
+    }
+    const int got = sub_any<P>(s_tab, nb1, qpl, run ? nq : 0, net2, lo, hi, score_mode ? kNoCut : cutoff, ring, n.done);
+    if (run) sum = got;
+    if (score_mode) {
+      if (have && lead) rb.score_out[4 * entry + 2] = sum;
+      continue;
+    }
+    bool pass = have && !(sum < cutoff) && sum >= 0;
+    if (h.word_after) {  // short-word test (func.cu:376-396), a warp per member
+      for (int k = 0; k < kSubs; k++) {
+        const int src = k * kSubGroup;
+        if (!__shfl_sync(kFullMask, (int)pass, src)) continue;
+        const uint32_t *q = reinterpret_cast<const uint32_t *>(__shfl_sync(kFullMask, (unsigned long long)qpl, src));
+        const int n2 = __shfl_sync(kFullMask, net2, src);
+        const int ws = __shfl_sync(kFullMask, (int)self, src) ? max(0, n2 - prm.w + 1)
+                                                              : word_count_warp_bits<P>(q, n2, prm.w, s_list);
+        if (lane / kSubGroup == k) pass = !(ws < word_min(L2, prm.w, s));
+      }
+    }
+    if (pass && lead) {
+      rb.cluster[cand] = h.rep;
+      rb.ident[cand] = sum;
+      atomicAnd(&rb.alive[cand >> 5], ~(1u << (cand & 31)));
+      n.members++;
+    }
+    __syncwarp();
+  }
+}
+
 template <int P, int NW, int WMAX>
-__global__ void __launch_bounds__(kAlignThreads)
-    k_align_wave(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs, int few) {
+__global__ void __launch_bounds__(kAlignThreads, WMAX <= 2 ? 5 : 4)
+    k_align_wave(DevDB db, RunBufs rb, RunParams prm, int cls, int score_mode, int warp_pairs, int few, int subs) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ uint64_t bar;
   __shared__ uint32_t s_xch[4 * NW];
@@ -418,7 +487,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
   if (threadIdx.x == 0) s_qw = 0;
   constexpr int kWarps = kAlignThreads / 32;
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kWarps / NW, few, smem, &bar, h)) return;
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kWarps / NW, few, subs, smem, &bar, h)) return;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
   const uint32_t vlast = (h.net1 & 31) ? ((1u << (h.net1 & 31)) - 1u) : 0xFFFFFFFFu;
   uint32_t *s_tab = smem + wave_table_off(P, db.max_nb);
@@ -426,7 +495,14 @@ __global__ void __launch_bounds__(kAlignThreads)
   wave_table<P>(smem, h.nb1, vlast, s_tab, threadIdx.x, kAlignThreads);
   __syncthreads();
   WaveCounts n;
-  if (NW == 1 || h.qn <= few) {
+  if (WMAX <= 2 && h.qn > subs) {
+    sub_entries<P>(db, rb, prm, cls, score_mode, h, s_tab, s_rings, s_list, &s_qw, n);
+    if (h.nb1 > 16 * kSubGroup) {  // bands too wide for 8 threads
+      __syncthreads();
+      wave_entries<P, 1, NW == 1 ? WMAX : 8, 2>(db, rb, prm, cls, score_mode, h, kAlignThreads / kSubGroup, s_tab, s_rings,
+                                                s_list, s_xch, &s_qw, n);
+    }
+  } else if (NW == 1 || h.qn <= few) {
     wave_entries<P, NW, WMAX, -1>(db, rb, prm, cls, score_mode, h, kWarps / NW, s_tab, s_rings, s_list, s_xch, &s_qw, n);
   } else if constexpr (NW > 1) {
     constexpr int WW = WMAX == 1 ? 8 : 16;  // one word for each of 128 threads: 8 for 32 hold as much
@@ -452,7 +528,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   __shared__ unsigned long long s_qw;  // query plane words of the pairs taken (algorithmic bytes / 4)
   if (threadIdx.x == 0) s_qw = 0;
   constexpr int kGroups = kAlignThreads / kQueryGroup;
-  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kGroups, INT_MAX, smem, &bar, h)) return;
+  if (!align_setup<P>(db, rb, prm, cls, score_mode, warp_pairs, kGroups, INT_MAX, INT_MAX, smem, &bar, h)) return;
   const uint32_t *s_pl = smem;
   const uint32_t *s_list = smem + ((h.nb1 * P + 3) & ~3);
   const int lane = threadIdx.x & 31, g = lane & (kQueryGroup - 1);
@@ -633,7 +709,13 @@ cudaError_t launch_align(ngia_ctx *c, int cls, cudaStream_t s, int score_mode) {
     grid_wave = std::min(grid_wave, score_mode);
   }
   int few = wave_few(std::min(pairs, c->warp_pairs_default));
-  void *args[] = {&db, &rb, &prm, &cls, &score_mode, &wp, &few};
+  const int ring = class_ring(c->db.type, cls);
+  // (a batch member's smaller share does not move the four-pairs form: its
+  // chain of iterations wants the latency of one pair per warp; 12 mixed jobs
+  // 28.0 ms, 48.5 with it from the share on)
+  const int share = c->batch_member ? c->warp_pairs_default : std::min(pairs, c->warp_pairs_default);
+  int subs = ring && (c->db.P == 2 || score_mode) ? sub_from(c->db.P, ring == 128 ? 4 : 1, share) : INT_MAX;
+  void *args[] = {&db, &rb, &prm, &cls, &score_mode, &wp, &few, &subs};
   // a call's pairs are known here: with no more than the cut-off no class can
   // go to the thread-per-pair kernel
   if (!score_mode || score_mode > wp) {

@@ -369,8 +369,10 @@ __global__ void __launch_bounds__(kAlignThreads, tiled_min_blocks(P))
 }
 
 // One entry of the round by this thread's group (NW 1 or 4: 32 NW threads,
-// rows are the representative's; NW 0: 16 threads, the query's blocks as rows).
-// MINE: -1 all, 1 the bands that a warp can hold, 0 the others.
+// rows are the representative's; NW -1: the same with 8 threads; NW 0: 16
+// threads, the query's blocks as rows).  MINE: -1 all, 1 the bands that the
+// group (a warp, NW -1: 8 threads) can hold, 0 those a warp cannot hold, 2 those
+// 8 threads cannot hold.
 struct RoundRep {
   int r = -1, L1 = 0, net1 = 0, nb1 = 0;
   bool word_after = false;  // the short-word test follows the alignment
@@ -380,8 +382,8 @@ __device__ __forceinline__ void round_wave_entry(const DevDB &qdb, const RepStor
                                                  const RoundBufs &rb, const RoundRep &h, int q, int cap_blocks,
                                                  uint32_t *smem, uint32_t *s_xch, unsigned long long &n_pairs,
                                                  unsigned long long &n_cells) {
-  constexpr bool kQ = NW == 0;
-  constexpr int GS = kQ ? kQueryGroup : 32 * NW;
+  constexpr bool kQ = NW == 0, kSub = NW < 0;
+  constexpr int GS = kQ ? kQueryGroup : kSub ? kSubGroup : 32 * NW, kParts = GS < 32 ? 32 / GS : 1;
   const int r = h.r, nb1 = h.nb1, net1 = h.net1, lane = threadIdx.x & 31;
   const bool lead = threadIdx.x % GS == 0;
   const float s = prm.s;
@@ -411,7 +413,9 @@ __device__ __forceinline__ void round_wave_entry(const DevDB &qdb, const RepStor
       have = run;
     }
     if constexpr (MINE >= 0)
-      if ((MINE != 0) == (run && !wave_holds(32, 16, lo, hi, nb1))) have = run = false;
+      if ((MINE == 1) ==
+          (run && !(kSub || MINE == 2 ? sub_holds(lo, hi, nb1) : wave_holds(32, 16, lo, hi, nb1))))
+        have = run = false;
     if (run && lead) n_pairs++;
   }
   unsigned long long cells = 0;
@@ -419,22 +423,26 @@ __device__ __forceinline__ void round_wave_entry(const DevDB &qdb, const RepStor
     uint32_t *tab = smem + 8 * cap_blocks + (threadIdx.x >> 5) * 32 * wave_codes(P);
     const int got = wave_query<P>(smem, nb1, net1, qpl, run ? nq : 0, net2, lo, hi, tab, cells);
     if (run) sum = got;
+  } else if constexpr (kSub) {
+    uint32_t *ring = smem + wave_table_words(P, cap_blocks) + (threadIdx.x / GS) * kSubRingWords;
+    const int got = sub_any<P>(smem, nb1, qpl, run ? nq : 0, net2, lo, hi, cutoff, ring, cells);
+    if (run) sum = got;
   } else if (run) {  // uniform in the group
     uint32_t *ring = smem + wave_table_words(P, cap_blocks) + (threadIdx.x / GS) * kWaveRingWords;
     sum = wave_any<P, NW, WMAX>(smem, nb1, qpl, nq, net2, lo, hi, cutoff, ring, s_xch, cells);
   }
   n_cells += 32 * cells;
-  bool pass = have && !(sum < cutoff);
+  bool pass = have && sum >= 0 && !(sum < cutoff);
   if (h.word_after) {  // short-word test (func.cu:376-396), a warp per member
     const uint32_t *list = rs.lists + (int64_t)r * rs.list_words;
 #pragma unroll
-    for (int k = 0; k < (kQ ? 2 : 1); k++) {
-      const int src = k * kQueryGroup;
+    for (int k = 0; k < kParts; k++) {
+      const int src = k * GS % 32;
       if (!__shfl_sync(kFullMask, (int)(pass && net2 >= 16), src)) continue;
       const uint32_t *qp = reinterpret_cast<const uint32_t *>(__shfl_sync(kFullMask, (unsigned long long)qpl, src));
       const int n2 = __shfl_sync(kFullMask, net2, src);
       const int ws = word_count_warp_bits<P>(qp, n2, prm.w, list);
-      if (!kQ || lane / kQueryGroup == k) pass = !(ws < word_min(L2, prm.w, s));
+      if (kParts == 1 || lane / GS == k) pass = !(ws < word_min(L2, prm.w, s));
     }
   }
   if (pass && lead) round_accept<MASK>(rb, r, q, sum);
@@ -446,22 +454,25 @@ __device__ __forceinline__ void round_wave_entry(const DevDB &qdb, const RepStor
 // representative.
 // Shared memory: match table | code rings, or rep codes | match tables.
 template <int P, int NW, int WMAX, bool MASK>
-__global__ void __launch_bounds__(kAlignThreads)
-    k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int wave_pairs, int cap_blocks, int few) {
+__global__ void __launch_bounds__(kAlignThreads, NW == 0 ? 10 : WMAX <= 2 ? 5 : 4)
+    k_round_wave(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int cls, int wave_pairs, int cap_blocks, int few,
+                 int subs) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr bool kQ = NW == 0;
   constexpr int GS = kQ ? kQueryGroup : 32 * NW, kGroups = kAlignThreads / GS, kWarps = kAlignThreads / 32;
   constexpr int WW = WMAX == 1 ? 8 : 16;
   __shared__ uint32_t s_xch[kQ ? 1 : 4 * NW];
-  __shared__ uint32_t s_qn, s_many;
+  constexpr bool kSubOk = !kQ && WMAX <= 2;  // windows up to 112 blocks
+  __shared__ uint32_t s_qn, s_many, s_subs;
   if (threadIdx.x == 0) {
     s_qn = round_wave(rb, cls, wave_pairs) ? (uint32_t)min((int64_t)rb.ctl[cls], rb.cap) : 0u;
+    s_subs = kSubOk && rb.ctl[kCtlPairs + cls] > (uint32_t)subs;
     s_many = NW == 4 && rb.ctl[kCtlPairs + cls] > (uint32_t)few;
   }
   __syncthreads();
   const uint32_t qn = s_qn;
-  const bool many = NW == 4 && s_many;
-  const uint32_t per = many ? kWarps : kGroups;
+  const bool many = NW == 4 && s_many, sub = kSubOk && s_subs;
+  const uint32_t per = sub ? kAlignThreads / kSubGroup : many ? kWarps : kGroups;
   const int hw = qdb.hw, lane = threadIdx.x & 31;
   unsigned long long n_pairs = 0, n_cells = 0;
   RoundRep h;
@@ -489,6 +500,20 @@ __global__ void __launch_bounds__(kAlignThreads)
       }
       __syncthreads();
       h.r = r;
+    }
+    if constexpr (kSubOk) {
+      if (sub) {
+        const int q = rb.queue[cls][e0 + threadIdx.x / kSubGroup].y;
+        round_wave_entry<P, -1, 16, MASK, 1>(qdb, rs, prm, rb, h, q, cap_blocks, smem, s_xch, n_pairs, n_cells);
+        if (h.nb1 > 16 * kSubGroup) {  // bands too wide for 8 threads
+          __syncthreads();
+          for (int k = threadIdx.x >> 5; k < kAlignThreads / kSubGroup; k += kWarps)
+            round_wave_entry<P, 1, NW == 1 ? WMAX : 8, MASK, 2>(qdb, rs, prm, rb, h, rb.queue[cls][e0 + k].y, cap_blocks,
+                                                                smem, s_xch, n_pairs, n_cells);
+          __syncthreads();
+        }
+        continue;
+      }
     }
     if constexpr (NW == 4) {
       if (many) {
@@ -520,7 +545,7 @@ __global__ void __launch_bounds__(kAlignThreads)
 
 // ---- launch ---------------------------------------------------------------------
 using RoundAlignFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, uint32_t *, int64_t, int, int);
-using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, int);
+using RoundWaveFn = void (*)(DevDB, RepStore, RunParams, RoundBufs, int, int, int, int, int);
 
 template <int P, bool MASK>
 RoundAlignFn round_align_fn(int cls) {
@@ -559,7 +584,7 @@ struct RoundPlan {
   int type = 0, rep_nb = 1;
   int grid[kServeClasses] = {0, 0, 0, 0}, wave_grid[kServeClasses] = {0, 0, 0, 0};
   int wave_pairs[kServeClasses] = {0, 0, 0, 0};
-  int few = 0;  // k_round_wave's
+  int few = 0, subs[kServeClasses] = {0, 0, 0, 0};  // k_round_wave's
   uint32_t *scratch = nullptr;  // global ring of class 2
   int64_t scratch_words = 0;
   int ring_rows = 0;
@@ -601,6 +626,7 @@ cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kAlignThreads, bytes) != cudaSuccess || occ < 1) occ = 1;
       (wave ? pl.wave_grid : pl.grid)[c] = num_sms * occ;
       // the clustering kernels' cut-off (api.cu)
+      if (wave) pl.subs[c] = type == 0 ? sub_from(2, c == 1 ? 4 : 1, 56 * num_sms) : INT_MAX;
       if (wave) pl.wave_pairs[c] = group_cut(c == 2 ? 0 : 64, 56 * num_sms);
     }
   pl.ring_rows = global_rows(rep_nb);
@@ -619,7 +645,7 @@ cudaError_t round_launch(const RoundPlan &pl, const DevDB &qdb, const RepStore &
     RepStore r = rs;
     RunParams p = prm;
     RoundBufs b = rb;
-    int cls = c, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb, few = pl.few;
+    int cls = c, wp = pl.wave_pairs[c], tb = round_table_blocks(pl.rep_nb), cap = pl.rep_nb, few = pl.few, subs = pl.subs[c];
     uint32_t *scr = pl.scratch;
     int64_t sw = pl.scratch_words;
     int rm = pl.ring_rows;
@@ -628,7 +654,7 @@ cudaError_t round_launch(const RoundPlan &pl, const DevDB &qdb, const RepStore &
                                      round_align_smem(pl.type, c, pl.rep_nb), st);
     if (e != cudaSuccess) return e;
     if (wp <= 0) continue;
-    void *wargs[] = {&db, &r, &p, &b, &cls, &wp, &cap, &few};
+    void *wargs[] = {&db, &r, &p, &b, &cls, &wp, &cap, &few, &subs};
     e = cudaLaunchKernel(round_fn<MASK>(pl.type, c, true), dim3(pl.wave_grid[c]), dim3(kAlignThreads), wargs,
                          round_wave_smem(pl.type, c, pl.rep_nb), st);
     if (e != cudaSuccess) return e;

@@ -8,17 +8,18 @@
 // Such a caller already holds its inputs and outputs in device memory; this
 // entry point uses them as given and allocates nothing.
 //
-// Three kernels:
+// Three forms:
 //  * up to noalloc_groups pairs per SM, a group of threads per pair (wave.cuh:
-//    rows in registers, match table and query codes in shared memory);
+//    rows in registers, match table and query codes in shared memory), 8 of
+//    them for more than a few pairs;
 //  * above that, representatives of up to 112 blocks: a thread per pair, the
 //    band rows in a shared-memory ring, register tiles (tile.cuh);
 //  * proteins whose match table does not fit shared memory: a thread per
 //    pair with its working row (one 32-bit word per 32 representative
 //    residues) in a fixed file-scope device array, g_noalloc_rows, of
 //    kNoAllocWords words (4 MiB).
-// GB300, whole calls: 4,096 DNA queries of 1,450 residues 810 -> 168 us, 1,000
-// proteins of 380 residues 300 -> 49 us (against the third kernel for all).
+// GB300, whole calls: 4,096 DNA queries of 1,450 residues 747 -> 117 us, 1,000
+// proteins of 380 residues 278 -> 43 us (against the third kernel for all).
 //
 // Every GPU that loads this library keeps that array until the process
 // exits.  Its size caps the representative at 65,536 residues (2,048 words
@@ -53,10 +54,10 @@ constexpr int kThreads = 128;
 static_assert(kThreads == ngia::kAlignThreads, "the ring and the groups of four warps");
 // Pairs per SM up to which a group per pair is faster than a thread per pair,
 // which takes a pair's latency whatever their number.  GB300: DNA 1,450
-// residues 238 us for 6,000 pairs by groups, 292 from 9,000 to 16,000 by
-// threads; 300 residues 69 against 47; protein 380 residues 118 against 132,
-// 900 residues 232 against 525.
-constexpr int noalloc_groups(int P, int nb1) { return P == 2 && nb1 <= 16 ? 26 : 50; }
+// residues 242 us for 10,000 pairs by groups and 257 by threads, 274 and 268
+// for 14,000; 300 residues 69 against 47 for 6,000; protein 380 residues 119
+// and 119 for 10,000.
+constexpr int noalloc_groups(int P, int nb1) { return P == 5 ? 64 : nb1 <= 16 ? 26 : 80; }
 constexpr size_t kNoAllocSmemMost = 226 * 1024;
 
 __device__ __align__(256) uint32_t g_noalloc_rows[kNoAllocWords];
@@ -173,6 +174,38 @@ __global__ void __launch_bounds__(kThreads) k_noalloc_wave(const uint32_t *__res
       score = ngia::wave_any<P, NW, WMAX>(s_mem, nb1, q + hw, (net2 + 31) / 32, net2, B, B, ngia::kNoCut, ring, s_xch,
                                           cells);
     if (lead) scores[k] = score;
+  }
+}
+
+// Four pairs per warp (wave.cuh).  Shared memory: match table | code rings.
+template <int P>
+__global__ void __launch_bounds__(kThreads) k_noalloc_sub(const uint32_t *__restrict__ words, int64_t rep_off,
+                                                          const int64_t *__restrict__ query_off, int n, float s,
+                                                          int *__restrict__ scores, int cap_blocks) {
+  extern __shared__ __align__(16) uint32_t s_mem[];
+  constexpr int hw = P == 2 ? 6 : 30, kGroups = kThreads / ngia::kSubGroup;
+  const uint32_t *rep = words + rep_off;
+  const int L1 = (int)rep[0], net1 = (int)rep[1], nb1 = (net1 + 31) / 32;
+  if (nb1 > cap_blocks) return;  // the host sized shared memory for this many
+  const int group = threadIdx.x / ngia::kSubGroup;
+  const uint32_t vlast = (net1 & 31) ? ((1u << (net1 & 31)) - 1u) : 0xFFFFFFFFu;
+  uint32_t *ring = s_mem + ngia::wave_table_words(P, nb1) + group * ngia::kSubRingWords;
+  ngia::wave_table<P>(rep + hw, nb1, vlast, s_mem, threadIdx.x, kThreads);
+  __syncthreads();
+  unsigned long long cells = 0;
+  const int first = threadIdx.x / 32 * ngia::kSubs;  // the warp's first pair of the CTA's
+  for (int k0 = blockIdx.x * kGroups + first; k0 < n; k0 += gridDim.x * kGroups) {  // warp-uniform
+    const int k = k0 + (group - first);
+    const uint32_t *q = words;
+    int net2 = 0, B = 0, score = 0;
+    bool run = false;
+    if (k < n) {
+      q = words + query_off[k];
+      run = noalloc_pair(q, nb1, L1, s, net2, B, &score);
+    }
+    const int got = ngia::sub_any<P>(s_mem, nb1, q + hw, run ? (net2 + 31) / 32 : 0, net2, B, B, ngia::kNoCut, ring, cells);
+    if (run) score = got;
+    if (k < n && threadIdx.x % ngia::kSubGroup == 0) scores[k] = score;
   }
 }
 
@@ -313,12 +346,17 @@ extern "C" int ngia_rep_scores_noalloc(const uint32_t *d_words, int64_t rep_off,
   NoAllocFn fn;
   size_t smem;
   int per;  // pairs per CTA
+  const bool sub = !many && n > ngia::sub_from(P, nb1 > 64 ? 0 : 1, 56 * std::max(sms, 1)) && nb1 <= 16 * ngia::kSubGroup;
   if (many) {
     const int ring = nb1 <= ngia::kSmallWindow ? 64 : 128;
     fn = P == 2 ? (ring == 64 ? k_noalloc_tiled<2, 64> : k_noalloc_tiled<2, 128>)
                 : (ring == 64 ? k_noalloc_tiled<5, 64> : k_noalloc_tiled<5, 128>);
     smem = 4 * (size_t)(((nb1 * P + 3) & ~3) + ring * kThreads + (P == 2 ? ngia::eq_words(nb1) : 0));
     per = kThreads;
+  } else if (sub) {
+    fn = P == 2 ? k_noalloc_sub<2> : k_noalloc_sub<5>;
+    per = kThreads / ngia::kSubGroup;
+    smem = 4 * ((size_t)ngia::wave_table_words(P, nb1) + (size_t)per * ngia::kSubRingWords);
   } else {
     fn = P == 2 ? (form == 0 ? k_noalloc_wave<2, 1, 2> : form == 1 ? k_noalloc_wave<2, 4, 1> : k_noalloc_wave<2, 4, 16>)
                 : (form == 0 ? k_noalloc_wave<5, 1, 2> : form == 1 ? k_noalloc_wave<5, 4, 1> : k_noalloc_wave<5, 4, 16>);
@@ -326,7 +364,7 @@ extern "C" int ngia_rep_scores_noalloc(const uint32_t *d_words, int64_t rep_off,
     smem = 4 * ((size_t)ngia::wave_table_words(P, nb1) + (size_t)per * ngia::kWaveRingWords);
   }
   if (smem <= kNoAllocSmemMost) {
-    e = noalloc_configure(fn, (P == 2 ? 0 : 8) + (many ? 4 + (nb1 <= ngia::kSmallWindow ? 0 : 1) : form), smem);
+    e = noalloc_configure(fn, (P == 2 ? 0 : 8) + (many ? 4 + (nb1 <= ngia::kSmallWindow ? 0 : 1) : sub ? 6 : form), smem);
     if (e != cudaSuccess) return ngia::fail(NGIA_E_CUDA, "ngia_rep_scores_noalloc: %s", cudaGetErrorString(e));
     const int grid = std::max(1, std::min(std::max(sms, 1) * 8, (n + per - 1) / per));
     fn<<<grid, kThreads, smem, st>>>(d_words, rep_off, d_query_off, n, similarity, d_scores, nb1);

@@ -297,6 +297,156 @@ __device__ __forceinline__ int wave_any(const uint32_t *tab, int nb1, const uint
   return -1;
 }
 
+// ---- several pairs per warp -----------------------------------------------------
+// The same wavefront with GS = 8 threads per pair, four pairs per warp, once
+// there are more pairs than schedulers: for the windows of common records (up
+// to some 50 blocks) a warp per pair has one row word per thread, and 14
+// instructions per column and word instead of 5; here W = 8 words per thread
+// (4 and 16 for narrower and wider bands) and 2 nq + nb1 / 8 steps.
+constexpr int kSubGroup = 8, kSubs = 32 / kSubGroup;
+constexpr int kSubRing = 32, kSubFetch = 16;  // query blocks of codes a group keeps, and fetches at a time
+constexpr int kSubRingWords = kSubRing * 8;
+static_assert(kSubs * kSubRingWords == kWaveRingWords, "the kernels with both forms share the rings");
+
+// Each group's zero count (in all of its threads) or -1 once it cannot reach
+// `cut`.  All 32 lanes call it; arguments but tab, nb1 and cut differ by
+// group, nq = 0 for a group without a pair; ring: the group's.
+template <int P, int W>
+__device__ __forceinline__ int wave_sub(const uint32_t *tab, int nb1, const uint32_t *qp, int nq, int net2, int lo,
+                                        int hi, int cut, uint32_t *ring, unsigned long long &n_done) {
+  constexpr int GS = kSubGroup, C = kWaveCols, S = kWaveUnits, U = W > 4 ? W / 4 : 1;
+  const int lane = threadIdx.x & 31, g = lane & (GS - 1);
+  const int below = (lane & ~(GS - 1)) | ((g + GS - 1) & (GS - 1));
+  const uint32_t row_bytes = 4u * (uint32_t)wave_stride(nb1);
+  const char *tabc = reinterpret_cast<const char *>(tab);
+  int q_last = nq > 0 ? min(nb1 - 1, nq - 1 + hi) / W : -1;
+  uint32_t row[W], off[U];
+  int q = g, u0 = 0, u1 = 0, acc = 0;
+  auto open = [&]() {  // chunk q: rows all-ones
+    const bool used = q <= q_last;
+    u0 = used ? S * max(0, q * W - hi) : 0;
+    u1 = used ? min(S * nq, S * (q * W + W + lo)) : 0;
+#pragma unroll
+    for (int k = 0; k < U; k++) off[k] = used ? 4u * (uint32_t)wave_place(q * W + 4 * k) : 0u;
+#pragma unroll
+    for (int w = 0; w < W; w++) row[w] = 0xFFFFFFFFu;
+  };
+  open();
+  uint32_t cout = 0, cells = 0;
+  int low = 0, low_end = S * (W + lo), filled = 0;  // as in wave_pair; the other chunks are at most 4 blocks behind
+  bool dead = false;
+  const int steps = (int)__reduce_max_sync(kFullMask, (unsigned)(nq > 0 ? S * nq + q_last : 0));
+  __syncwarp();  // the warp is through with the last pairs' rings
+  for (int t = 0; t < steps; t++) {
+    if (t >= low_end) {
+      low++;
+      low_end += S * W + 1;
+    }
+    const bool fetch = ((t - low) >> 1) >= filled && filled < nq;
+    if (__any_sync(kFullMask, fetch)) {
+      if (fetch) {
+        for (int b = filled + g; b < min(nq, filled + kSubFetch); b += GS) {
+          uint32_t pl[P];
+#pragma unroll
+          for (int p = 0; p < P; p++) pl[p] = __ldg(qp + b * P + p);
+          wave_unpack<P>(pl, reinterpret_cast<uint4 *>(ring) + 2 * (b & (kSubRing - 1)));
+        }
+        filled += kSubFetch;
+      }
+      __syncwarp();
+    }
+    const uint32_t cin = __shfl_sync(kFullMask, cout, below);
+    if (cut != kNoCut && (t & 7) == 7) {  // wave_pair's bound, group by group
+      int z = acc;
+#pragma unroll
+      for (int w = 0; w < W; w++) z += __popc(~row[w]);
+#pragma unroll
+      for (int o = GS / 2; o; o >>= 1) z += __shfl_xor_sync(kFullMask, z, o);
+      int top = (t - 1 + S * hi) / (S * W + 1);
+      if (top * W <= hi) top = min(t - 1, hi / W);
+      top = min(top, q_last);
+      dead = dead || nq == 0 || z + max(0, net2 - C * (t - top)) < cut;
+      if (__all_sync(kFullMask, dead)) break;
+    }
+    const int u = t - q, i = u >> 1;
+    const bool active = !dead && u >= u0 && u < u1;
+    const int ncol = active ? max(0, min(C, net2 - C * u)) : 0;
+    uint32_t act[W];
+    int rows = 0;
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+      const int j = q * W + w;
+      const bool in = active && j >= i - lo && j <= i + hi;
+      act[w] = in ? 0xFFFFFFFFu : 0u;
+      rows += in ? 1 : 0;
+    }
+    cells += (uint32_t)(rows * ncol);
+    uint4 codes = make_uint4(0u, 0u, 0u, 0u);  // idle threads take code 0
+    if (active) codes = reinterpret_cast<const uint4 *>(ring)[2 * (i & (kSubRing - 1)) + (u & 1)];
+    const uint32_t code[4] = {codes.x, codes.y, codes.z, codes.w};
+    uint32_t cw = ncol > 0 && q > 0 ? cin << (32 - ncol) : 0u, ncw = 0;
+    auto column = [&](uint32_t c) {
+      uint32_t e[W];
+      wave_load<W, U>(e, tabc, c * row_bytes, off);
+      dp_wave<W>(row, e, act, cw, ncw);
+    };
+    if (__all_sync(kFullMask, !active || ncol == C)) {
+#pragma unroll 4
+      for (int k = 0; k < C; k++) column(__byte_perm(code[k >> 2], 0, 0x4440 | (k & 3)));
+    } else {  // some pair's last columns
+#pragma unroll 1
+      for (int k = 0; k < ncol; k++) {
+        const uint32_t w = k < 4 ? code[0] : k < 8 ? code[1] : k < 12 ? code[2] : code[3];
+        column((w >> (8 * (k & 3))) & 0xFFu);
+      }
+    }
+    cout = ncw;
+    if (u >= 0 && u + 1 >= u1 && q <= q_last) {  // the chunk has left the band
+#pragma unroll
+      for (int w = 0; w < W; w++) acc += __popc(~row[w]);
+      q += GS;
+      open();
+    }
+  }
+  n_done += cells;
+  int sum = acc;
+#pragma unroll
+  for (int o = GS / 2; o; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
+  return dead ? -1 : sum;
+}
+
+// Pairs above which a warp takes four, when a group per pair is up to `pairs`
+// (56 per SM).  other: words of row per thread in the form it replaces: 1 (a
+// warp per pair, bands of one word per thread), 4 (a warp, wider), 0 (a CTA).
+// GB300, score calls, us with the other form and with 8 threads per pair: DNA
+// 1,450 residues 73 and 84 for 1,000 pairs, 93 and 87 for 1,500, 168 and 112 for
+// 4,096; protein 380 residues 57 and 58 for 2,500, 71 and 57 for 4,096; DNA 2,600
+// residues, a CTA per pair, 142 and 131 for 400, 947 and 243 for 4,096.  Against
+// a warp with four words a pair takes three times as long, and 1.4 times fewer
+// instructions: a serving batch with 500 to 1,500 such pairs per round 1.42 ms,
+// 1.49 with 8 threads.  Proteins with a cut-off stay with a warp: most pairs
+// are out after a fifth of their length, and a warp of four runs as long as its
+// longest (100,000 proteins, s = 0.9, 8.4 ms, 9.3 with four).
+__host__ __device__ constexpr int sub_from(int P, int other, int pairs) {
+  return (int)((long long)pairs * (other == 0 ? 3 : other == 4 || P == 5 ? 20 : 9) / 56);
+}
+
+// Bands that 8 threads with 16 row words each can hold.
+__host__ __device__ constexpr bool sub_holds(int lo, int hi, int nb1) { return wave_holds(kSubGroup, 16, lo, hi, nb1); }
+
+// The same with the fewest row words per thread that hold every group's band;
+// the caller makes sure that 16 do.
+template <int P>
+__device__ __forceinline__ int sub_any(const uint32_t *tab, int nb1, const uint32_t *qp, int nq, int net2, int lo,
+                                       int hi, int cut, uint32_t *ring, unsigned long long &n_done) {
+  const int n = (int)__reduce_max_sync(kFullMask, (unsigned)(nq > 0 ? lo + hi + 1 : 0));
+  if (n <= wave_cap(kSubGroup, 4) || nb1 <= kSubGroup * 4)
+    return wave_sub<P, 4>(tab, nb1, qp, nq, net2, lo, hi, cut, ring, n_done);
+  if (n <= wave_cap(kSubGroup, 8) || nb1 <= kSubGroup * 8)
+    return wave_sub<P, 8>(tab, nb1, qp, nq, net2, lo, hi, cut, ring, n_done);
+  return wave_sub<P, 16>(tab, nb1, qp, nq, net2, lo, hi, cut, ring, n_done);
+}
+
 // ---- the query's blocks as rows -------------------------------------------------
 // Short queries against a long representative: GS = 16 threads per pair, two
 // pairs per warp, one query block per thread as its row word, the

@@ -73,3 +73,62 @@ def test_many_wide_pairs_in_rounds(cuda_device, L):
     with ngia.Context(db) as ctx:
         cl, ident = ctx.cluster(p, ngia.MODE_SPEC)[:2]
     assert (cl == ocl).all() and (ident == oid).all()
+
+
+# (type, similarity, length, dropped): blocks a query block's band covers
+@pytest.mark.parametrize("db_type,s,L,drop", [
+    (0, 0.9, 300, 20),     # one chunk row per thread and fewer
+    (0, 0.7, 1000, 200),   # 21, 32 blocks: 4 words
+    (0, 0.8, 2200, 300),   # 29
+    (0, 0.75, 2100, 300),  # 35: 8 words
+    (0, 0.6, 2047, 300),   # 53, 64 blocks
+    (0, 0.6, 2200, 60),    # 57: 16 words, the class of windows up to 112 and the narrower
+    (0, 0.6, 3900, 100),   # 99
+    (0, 0.7, 4090, 100),   # 79, 128 blocks
+    (0, 0.7, 5400, 100),   # 103: too wide for 8 threads
+    (0, 0.9, 12000, 100),  # 77, long records
+    (1, 0.5, 380, 100),
+    (1, 0.7, 900, 200),
+    (1, 0.7, 5400, 60),
+])
+def test_many_pairs_of_common_width(cuda_device, db_type, s, L, drop):
+    rng = np.random.default_rng(L + db_type)
+    alpha = np.frombuffer(b"ACGT" if db_type == 0 else b"ACDEFGHIKLMNPQRSTVWY", np.uint8)
+    base = alpha[rng.integers(0, len(alpha), L)]
+    seqs = [base.tobytes()] + _copies(rng, alpha, base, 30, 3 * (1 - s), 3) + _copies(rng, alpha, base, 17, 1 - s, drop)
+    db = seqs_to_db(db_type, seqs)
+    w = 5 if db_type == 0 else 2
+    for precise in (1, 0):  # 0: the short-word test follows the alignment
+        p = ngia.params_clamp(db_type, s, w, precise)
+        exp = np.stack([oracle.pair(db.words, db.rec_off, db_type, p.similarity, p.word_length, 0, i)
+                        for i in range(db.n)])
+        member = (exp[:, 4] != 0) & (exp[:, 6] != 0) & ((exp[:, 5] != 0) | (precise == 1))
+        member[0] = True
+        with ngia.Context(db) as ctx:
+            ctx.set_tuning(2, 32, 56)
+            for mode in (ngia.MODE_PLAIN, ngia.MODE_GRAPH):
+                ctx.begin(p, mode)
+                ctx.step(1)
+                cl, ident = ctx.end()[:2]
+                assert ((cl == 0) == member).all()
+                assert (ident[1:][member[1:]] == exp[1:, 2][member[1:]]).all()
+
+
+@pytest.mark.parametrize("db_type,s,L", [(0, 0.85, 700), (0, 0.8, 2400), (0, 0.7, 5200), (1, 0.6, 500)])
+def test_rounds_and_scores_of_common_width(cuda_device, db_type, s, L):
+    rng = np.random.default_rng(L)
+    alpha = np.frombuffer(b"ACGT" if db_type == 0 else b"ACDEFGHIKLMNPQRSTVWY", np.uint8)
+    seqs = []
+    for _ in range(8):
+        base = alpha[rng.integers(0, len(alpha), L)]
+        seqs += _copies(rng, alpha, base, 70, 1.5 * (1 - s), 40)
+    db = seqs_to_db(db_type, seqs)
+    p = ngia.params_clamp(db_type, s, 5 if db_type == 0 else 2, 0)
+    ocl, oid, _ = oracle.cluster(db.words, db.rec_off, db_type, p.similarity, p.word_length, p.precise)
+    with ngia.Context(db) as ctx:
+        cl, ident = ctx.cluster(p, ngia.MODE_SPEC)[:2]
+        got = ctx.pair_scores(p, 0, np.arange(db.n))
+    assert (cl == ocl).all() and (ident == oid).all()
+    exp = np.stack([oracle.pair(db.words, db.rec_off, db_type, p.similarity, p.word_length, 0, i)
+                    for i in range(db.n)])
+    assert (got[:, 2] == exp[:, 2]).all()
