@@ -25,6 +25,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -388,14 +389,8 @@ def run_ours(args, dist: Dist):
     total_cands = dist.reduce(float(r["cands"]), "sum")
     total_cells = dist.reduce(float(r["cells"]), "sum")
     tuning = r["tuning"]
-    # per iteration: prep, filter, next, and per class the thread-per-pair and
-    # the warp-per-pair kernel; k_filter_long when short words go first and
-    # records exceed 2,048 residues
-    launches_per_iter = 3 + 2 * ngia_classes(cfg["type"])
-    wo = tuning["word_order"] if tuning else 0
-    word_first = wo == 1 or (wo == 0 and (cfg["type"] == 1 or p.similarity >= 0.93))
-    if word_first and not p.precise and int(db.words[db.rec_off + 1].max()) > 2048:
-        launches_per_iter += 1
+    tuning_order = tuning["word_order"] if tuning else 0
+    launches_per_iter = launches_of(cfg["type"], db, p, tuning_order)
 
     out = None
     if dist.rank == 0:
@@ -580,8 +575,24 @@ def reference_gpu_compare(args) -> dict:
         return {"error": repr(e)}
 
 
-def ngia_classes(db_type: int) -> int:
-    return 3  # alignment classes in use (64 and 128 ring rows, any width)
+def launches_of(db_type: int, db, p, word_order: int) -> int:
+    """Kernels of one greedy iteration: prep, next, the filter with the
+    short-word test and the one without (either or, in the automatic order when
+    the test can pay for some representative, both), k_filter_long for records
+    above 2,048 residues, and two kernels (a thread or a group per pair) for
+    each class that the longest record allows (windows up to 48, 112 and more
+    blocks; the wider two also as classes of short queries)."""
+    longest = int(db.words[db.rec_off + 1].max())
+    blocks = (longest + 31) // 32
+    classes = 1 + (2 if blocks > 48 else 0) + (2 if blocks > 112 else 0)
+    space = (4.0 if db_type == 0 else 20.0) ** p.word_length
+    words = max(0, int(db.read_len.min()) - p.word_length + 1)
+    can = not p.precise and 1.0 - math.exp(-words / space) < 1.0 - p.word_length * (1.0 - p.similarity)
+    word = word_order == 1 or (word_order == 0 and can)
+    filters = (1 if word else 0) + (1 if not word or word_order == 0 else 0)
+    if word and longest > 2048:
+        filters += 1
+    return 2 + filters + 2 * classes
 
 
 def run_e2e(args, db, p, S):

@@ -389,9 +389,9 @@ int ngia_cluster_resume(ngia_ctx *ctx, const char *path, int32_t mode);
  * the speed of a run, never its result: the order of the two cheap tests
  * (short-word test before or after the alignment), the number of idle lanes
  * a warp of the tiled alignment waits for before it claims new pairs, the
- * pair count up to which a class is aligned warp-per-pair, and per length
+ * pair count up to which a class is aligned by a group of threads per pair, and per length
  * bucket (alignment class: pairs grouped by band window) its own
- * warp-per-pair cut-off and CTA count, and the composition filter's tile.
+ * such cut-off and CTA count, and the composition filter's tile.
  * ngia_autotune times candidate settings on the first `iters` greedy
  * iterations of a fresh run of this context's database (graph driver, device
  * time), keeps the fastest for later runs of the context and reports it;
@@ -402,11 +402,11 @@ int ngia_cluster_resume(ngia_ctx *ctx, const char *path, int32_t mode);
 typedef struct ngia_tuning {
     int32_t word_order;   /* 0 by similarity, 1 short words first, 2 alignment first */
     int32_t refill;       /* 1..32 idle lanes                                        */
-    int32_t warp_pairs;   /* warp-per-pair up to this many pairs; -1 = default      */
+    int32_t warp_pairs;   /* group-per-pair up to this many pairs; -1 = default     */
     int32_t candidates;   /* settings timed (ngia_autotune)                          */
     double  ms_per_iter;  /* device time per iteration of the chosen setting         */
     double  default_ms_per_iter;  /* the same for the default setting                */
-    int32_t class_warp_pairs[8];  /* per length bucket: its warp-per-pair cut-off,   */
+    int32_t class_warp_pairs[8];  /* per length bucket: its group-per-pair cut-off,  */
                                   /* -1 = warp_pairs                                 */
     int32_t class_grid_div[8];    /* per length bucket: its CTAs divided by 1 or 2   */
     int32_t filter_tile;          /* composition filter: bitmap words per warp and   */
@@ -421,7 +421,7 @@ int ngia_set_tuning(ngia_ctx *ctx, const ngia_tuning *t);
  * whole batch over the first `iters` greedy iterations of every job:
  *   NGIA_BATCH_POLICY_THREAD  every length bucket of every job aligned
  *                             thread per pair;
- *   NGIA_BATCH_POLICY_CUTOFF  each job's default warp-per-pair cut-off;
+ *   NGIA_BATCH_POLICY_CUTOFF  each job's whole default group-per-pair cut-off;
  *   NGIA_BATCH_POLICY_TUNED   each job's own ngia_autotune settings, found
  *                             with the job alone on the GPU (cached by
  *                             database shape and parameters).

@@ -57,7 +57,7 @@ struct ngia_batch {
   std::vector<int> ptune;                 // their tuning generation at capture
   cudaStream_t pstream = nullptr;         // capture and launch stream of the pooled graph
   // the per-job-loop form's policy chosen by ngia_batch_autotune
-  // (NGIA_BATCH_POLICY_*; -1 before) and each job's warp-per-pair cut-off
+  // (NGIA_BATCH_POLICY_*; -1 before) and each job's group-per-pair cut-off
   // under it, restored on every NGIA_MODE_GRAPH run
   int policy = -1;
   std::vector<int> policy_wp;
@@ -357,7 +357,7 @@ extern "C" int ngia_batch_run(ngia_batch *b, const ngia_params *params, int32_t 
       // the group-per-pair kernels up to the job's share of the pairs at
       // which they pay (many jobs: thread per pair, the form with the fewest
       // instructions per cell; 12 jobs of 1,000-4,000 sequences on GB300, 32
-      // iterations each: 281 ms with every class thread per pair, 52
+      // iterations each: 281 ms with every class thread per pair, 27
       // with the share); NGIA_BATCH_WARP=1 keeps each job's own cut-off
       // after ngia_batch_autotune, the chosen policy's settings
       if (b->policy >= 0 && b->policy_wp.size() == nj)
@@ -412,7 +412,7 @@ namespace {
 
 // The settings of one job under a batch policy: the untuned settings with
 // every bucket thread per pair, the untuned settings with the job's default
-// warp-per-pair cut-off, or the job's own tuning.
+// group-per-pair cut-off, or the job's own tuning.
 ngia_tuning policy_setting(int policy, const ngia_tuning &own) {
   if (policy == NGIA_BATCH_POLICY_TUNED) return own;
   ngia_tuning t;

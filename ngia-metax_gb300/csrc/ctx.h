@@ -89,9 +89,9 @@ struct ngia_ctx {
   int warp_pairs_default = -1;  // the above as sized for this context's grids
   // settings that change speed only (set by ngia_autotune / ngia_set_tuning):
   // test order (0 auto, 1 short words first, 2 alignment first), lockstep
-  // refill threshold, warp-per-pair cut-off (-1: keep warp_pairs_default)
+  // refill threshold, group-per-pair cut-off (-1: keep warp_pairs_default)
   int tuned_word_order = 0, tuned_refill = 32, tuned_warp_pairs = -1;
-  // per length bucket (alignment class): warp-per-pair cut-off (-1: the
+  // per length bucket (alignment class): group-per-pair cut-off (-1: the
   // context's) and CTA divisor; the composition filter's words per warp
   int cls_warp_pairs[ngia::kNumClasses] = {-1, -1, -1, -1, -1, -1, -1};
   int cls_grid_div[ngia::kNumClasses] = {1, 1, 1, 1, 1, 1, 1};

@@ -1,14 +1,14 @@
 // tune.cu — run-time tuning of the settings that change the speed of a run
 // but never its result: the order of the two cheap tests, the lockstep
-// refill threshold of the tiled alignment, the warp-per-pair cut-off, and per
+// refill threshold of the tiled alignment, the group-per-pair cut-off, and per
 // length bucket (alignment class: the pairs of one band-window range) the
-// class's own warp-per-pair cut-off and CTA count, plus the composition
+// class's own group-per-pair cut-off and CTA count, plus the composition
 // filter's tile.  Each candidate is timed (device time, graph driver) on the
 // first greedy iterations of a fresh run of the context's database; the
 // fastest is kept for the context's later runs.  Coordinate-wise: the
 // default; each test order; refill 24 and 28; the global cut-off at a
 // quarter, half and twice the default; then for every bucket that queued
-// pairs, thread-per-pair only, warp-per-pair up to four times the cut-off,
+// pairs, thread-per-pair only, group-per-pair up to four times the cut-off,
 // and half its CTAs; then the filter tile of one bitmap word per warp.  The
 // winner is cached in the process by database shape and parameters.
 #include <cstring>
@@ -178,7 +178,7 @@ extern "C" int ngia_autotune(ngia_ctx *c, const ngia_params *p, int32_t iters, n
     for (int v = 0; v < 3 && !rc; v++) {
       Setting s = best_s;
       if (v == 0) s.cls_wp[k] = 0;        // thread per pair only
-      if (v == 1) s.cls_wp[k] = 4 * cut;  // warp per pair up to 4x the cut-off
+      if (v == 1) s.cls_wp[k] = 4 * cut;  // group per pair up to 4x the cut-off
       if (v == 2) s.cls_div[k] = 2;       // half the CTAs
       if (v == 1 && cut <= 0) continue;
       rc = trial(s);

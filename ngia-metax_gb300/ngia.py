@@ -218,12 +218,14 @@ CONFIGS = {
 
 
 def class_kernels(db_type: int) -> list[str]:
-    """Thread-per-pair kernel of each alignment work class (by the width of
-    the band window a pair can need, in 32-residue blocks; the first classes
-    are unused); every class in use also launches the warp-per-pair kernel,
-    which does the class's work instead when it has few pairs."""
-    P, unused = (2, 4) if db_type == 0 else (5, 2)
-    return ["(unused)"] * unused + [f"k_align_tiled<{P},{r}>" for r in (64, 128, 0)]
+    """Thread-per-pair kernel of each alignment work class: the first two hold
+    short queries against wide windows, the last three go by the width of the
+    band window a pair can need, in 32-residue blocks (DNA leaves two between
+    unused).  Every class in use also launches its group-per-pair kernel, which
+    does the class's work instead when it has few pairs."""
+    P, unused = (2, 2) if db_type == 0 else (5, 0)
+    short = [f"k_align_tiled<{P},{r}>" for r in (128, 0)]
+    return short + ["(unused)"] * unused + [f"k_align_tiled<{P},{r}>" for r in (64, 128, 0)]
 
 
 class Seqs:
