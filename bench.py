@@ -578,20 +578,17 @@ def reference_gpu_compare(args) -> dict:
 def launches_of(db_type: int, db, p, word_order: int) -> int:
     """Kernels of one greedy iteration: prep, next, the filter with the
     short-word test and the one without (either or, in the automatic order when
-    the test can pay for some representative, both), k_filter_long for records
-    above 2,048 residues, and two kernels (a thread or a group per pair) for
-    each class that the longest record allows (windows up to 48, 112 and more
-    blocks; the wider two also as classes of short queries)."""
-    longest = int(db.words[db.rec_off + 1].max())
-    blocks = (longest + 31) // 32
+    the test can pay for some representative, both), and two kernels (a thread
+    or a group per pair) for each class that the longest record allows (windows
+    up to 48, 112 and more blocks; the wider two also as classes of short
+    queries)."""
+    blocks = (int(db.words[db.rec_off + 1].max()) + 31) // 32
     classes = 1 + (2 if blocks > 48 else 0) + (2 if blocks > 112 else 0)
     space = (4.0 if db_type == 0 else 20.0) ** p.word_length
     words = max(0, int(db.read_len.min()) - p.word_length + 1)
     can = not p.precise and 1.0 - math.exp(-words / space) < 1.0 - p.word_length * (1.0 - p.similarity)
     word = word_order == 1 or (word_order == 0 and can)
     filters = (1 if word else 0) + (1 if not word or word_order == 0 else 0)
-    if word and longest > 2048:
-        filters += 1
     return 2 + filters + 2 * classes
 
 

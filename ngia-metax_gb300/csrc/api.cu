@@ -243,7 +243,7 @@ int alloc_db(ngia_ctx *c, int type, int64_t cap_n, int64_t cap_words) {
   const char *pc = getenv("NGIA_PROTEIN_CODES");
   const bool codes = type != 0 && !(pc && atoi(pc) == 0);
   DevBlock &m = c->mem_db;
-  m.add(&c->d_flags, 3);
+  m.add(&c->d_flags, 4);
   m.add(&c->d_words, (size_t)cap_words + 4);
   m.add(&c->d_off, (size_t)cap_n);
   m.add(&c->d_len, (size_t)cap_n);
@@ -276,19 +276,20 @@ int load_db(ngia_ctx *c, const ngia_db_view *v) {
       cudaMemcpyAsync(c->d_words, v->words, sizeof(uint32_t) * (size_t)v->n_words, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(c->d_off, v->rec_off, sizeof(int64_t) * (size_t)v->n, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_flags, 0, 3 * sizeof(int32_t), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(c->d_flags, 0, 4 * sizeof(int32_t), c->stream);
   if (e != cudaSuccess) return fail(NGIA_E_CUDA, "ngia_open: copy: %s", cudaGetErrorString(e));
   c->n_words = v->n_words;
   c->longest = v->longest;
   c->shortest = v->shortest;
   c->db.n = v->n;
-  e = ngia::launch_loader(c, c->d_flags, c->d_flags + 1, c->d_flags + 2);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(c->h_flags, c->d_flags, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream);
+  e = ngia::launch_loader(c, c->d_flags, c->d_flags + 1, c->d_flags + 2, c->d_flags + 3);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(c->h_flags, c->d_flags, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return fail(NGIA_E_CUDA, "ngia_open: loader: %s", cudaGetErrorString(e));
   if (c->h_flags[2]) return fail(NGIA_E_FORMAT, "ngia_open: a record offset or header is out of range");
   c->db.max_nb = std::max(1, c->h_flags[0]);
   c->db.has_short = c->h_flags[1];
+  c->db.long_n = c->db.n - c->h_flags[3];
   return NGIA_OK;
 }
 
@@ -340,7 +341,6 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
   m.add(&rb.rep_list, ngia::kListWords);
   m.add(&rb.first_short, ngia::kRefGridThreads);
   m.add(&rb.scan_part, nbw);
-  m.add(&rb.long_list, (size_t)cap_n);
   m.add((uint32_t **)&rb.flags, nbw);
   m.add(&rb.fstats, (size_t)ngia::kFilterStripes * ngia::kFilterStats);
   for (int k = 0; k < ngia::num_classes(type); k++)
@@ -444,7 +444,7 @@ int ngia::drv::reload_ctx(ngia_ctx *c, const ngia_db_view *v) {
   size_grids(c, c->batch_member);
   // a captured graph holds the kernel arguments (sizes) and grids: it stays
   // valid when the database has the same shape
-  const bool same = before.n == c->db.n && before.max_nb == c->db.max_nb && before.has_short == c->db.has_short &&
+  const bool same = before.n == c->db.n && before.max_nb == c->db.max_nb && before.has_short == c->db.has_short && before.long_n == c->db.long_n &&
                     grids_before == c->grid_filter && warp_before == c->warp_pairs_default;
   if (!same) destroy_graph(c);
   return NGIA_OK;

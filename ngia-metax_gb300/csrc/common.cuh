@@ -77,6 +77,7 @@ struct DevDB {
   const int32_t *net;     // net length (record word 1)
   const uint32_t *cnt;    // residue counts, 4 (DNA) or 28 (protein) per sequence
   const uint32_t *codes;  // protein: each record's residue codes as a bit stream
+  int32_t long_n;         // records before the first of at most kWarpWordLen residues (filter.cu)
                           // (5 words per 32-residue block, at the planes'
                           // offsets); null for DNA
   int32_t n, type;
@@ -95,7 +96,7 @@ struct RunState {
   int64_t iter_limit;     // graph loop stops when iter reaches it
   uint32_t qcount[kNumClasses];  // pairs queued per class this iteration
   uint32_t qhead[kNumClasses];   // pairs claimed per class
-  uint32_t long_count;    // candidates left for k_filter_long this iteration
+  uint32_t long_count;    // unused (the run state's layout is that of saved checkpoints)
   int32_t word_first;     // 1: short-word filter before alignment
   int32_t word_active;    // 1: short-word filter applies this iteration
   int32_t rep_nb;         // plane blocks of the representative (net)
@@ -161,7 +162,6 @@ struct RunBufs {
   int32_t *pos;           // position of a base survivor in the job list
   int32_t *first_short;   // per reference thread: first job with net < 16
   uint32_t *scan_part;    // scan partials
-  int32_t *long_list;     // candidates whose short-word count k_filter_long takes (one warp each)
   uint32_t *scratch;      // per-lane band rows of the widest class (global ring)
   int64_t scratch_words;
   int32_t generic_lanes;

@@ -64,7 +64,7 @@ struct ngia_ctx {
   // within it: serving slots)
   int64_t cap_n = 0, cap_words = 0;
   int32_t cap_nb = 0;
-  int32_t *d_flags = nullptr;  // loader results: max blocks, short record, bad record
+  int32_t *d_flags = nullptr;  // loader results: max blocks, short record, bad record, n - db.long_n
   int32_t *h_flags = nullptr;  // host mirror (behind h_state)
   // run buffers
   ngia::RunBufs rb{};
@@ -149,7 +149,7 @@ bool spec_exact(const ngia_ctx *c);            // rounds reproduce the greedy lo
 void spec_stats(const ngia_ctx *c, int64_t *pairs, int64_t *cells);
 }  // namespace drv
 // loader.cu / filter.cu
-cudaError_t launch_loader(ngia_ctx *c, int32_t *d_maxnb, int32_t *d_short, int32_t *d_bad);
+cudaError_t launch_loader(ngia_ctx *c, int32_t *d_maxnb, int32_t *d_short, int32_t *d_bad, int32_t *d_end);
 cudaError_t launch_init_run(ngia_ctx *c);
 cudaError_t launch_prep(ngia_ctx *c, int score_rep);
 cudaError_t launch_filter(ngia_ctx *c);

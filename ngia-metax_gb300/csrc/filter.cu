@@ -21,12 +21,16 @@
 
 namespace ngia {
 
+// The short-word test of longer candidates takes a warp (k_filter_word).
+constexpr int kWarpWordLen = 2048;
+
 // ---- loader ---------------------------------------------------------------
+// from_end: n - the first record of at most kWarpWordLen residues.
 __global__ void k_loader(const uint32_t *__restrict__ words, const int64_t *__restrict__ off, int64_t n_words,
                          int n, int type, int32_t *len, int32_t *net, uint32_t *cnt, int32_t *max_nb,
-                         int32_t *has_short, int32_t *bad) {
+                         int32_t *has_short, int32_t *bad, int32_t *from_end) {
   const int A = type ? 28 : 4, hw = type ? 30 : 6, P = type ? 5 : 2;
-  int local_max = 0, local_short = 0, local_bad = 0;
+  int local_max = 0, local_short = 0, local_bad = 0, local_end = 0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     const int64_t o = off[c];
     if (o < 0 || o + hw > n_words) {
@@ -49,10 +53,12 @@ __global__ void k_loader(const uint32_t *__restrict__ words, const int64_t *__re
     for (int a = 0; a < A; a++) cnt[(int64_t)c * A + a] = r[2 + a];
     local_max = max(local_max, (int)((N + 31) / 32));
     local_short |= (N < 16);
+    if (L <= (uint32_t)kWarpWordLen) local_end = max(local_end, n - c);
   }
   atomicMax(max_nb, local_max);
   if (local_short) atomicOr(has_short, 1);
   if (local_bad) atomicOr(bad, 1);
+  atomicMax(from_end, local_end);
 }
 
 // Protein residue-code streams, one warp per record (lanes over its
@@ -82,10 +88,10 @@ __global__ void k_codes(const uint32_t *__restrict__ words, const int64_t *__res
   }
 }
 
-cudaError_t launch_loader(ngia_ctx *c, int32_t *d_maxnb, int32_t *d_short, int32_t *d_bad) {
+cudaError_t launch_loader(ngia_ctx *c, int32_t *d_maxnb, int32_t *d_short, int32_t *d_bad, int32_t *d_end) {
   int grid = c->num_sms * 4;
   k_loader<<<grid, 256, 0, c->stream>>>(c->d_words, c->d_off, c->n_words, c->db.n, c->db.type, c->d_len,
-                                        c->d_net, c->d_cnt, d_maxnb, d_short, d_bad);
+                                        c->d_net, c->d_cnt, d_maxnb, d_short, d_bad, d_end);
   if (c->db.type != 0 && c->d_codes)
     k_codes<<<grid, 256, 0, c->stream>>>(c->d_words, c->d_off, c->d_len, c->db.n, c->db.hw, c->d_codes);
   return cudaGetLastError();
@@ -281,9 +287,12 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
 // bitmap word of the length-sorted database, a CTA's warps words gridDim.x
 // apart (a share of every length for each SM) — and queues its survivors with
 // one atomic per class and word; no CTA barrier makes a warp wait for the CTA's
-// longest candidates.  Candidates longer than kWarpWordLen go to k_filter_long,
-// a warp each, spread over the grid: the longest sequences of the length-sorted
-// database share the first bitmap words.
+// longest candidates.  The records before the first of at most kWarpWordLen
+// residues (db.long_n; the longest share the first bitmap words) get a warp
+// each, from the grid's last warp on, which has the fewest words to do; a longer
+// record further on (a database that is not sorted) gets its lane's warp.  (A
+// launch of their own behind this one took 10 us of a 119 us iteration of
+// 100,000 proteins.)
 //
 // GB300, 200,000 DNA of 1,450 residues, w = 5, the whole filter per iteration:
 // s = 0.99 42 us (a byte per word and every word counted: 151), s = 0.97 77
@@ -294,7 +303,7 @@ __global__ void __launch_bounds__(256) k_filter(DevDB db, RunBufs rb, RunParams 
 // jobs share the GPU (12 mixed jobs 2% slower), 256 threads build the table
 // too often (s = 0.97 102 us), 40 registers for three CTAs of 512 spill (90 us).
 // kWarpWordLen: 1,024 is no faster, 512 makes the proteins 25% slower.
-constexpr int kWordThreads = 512, kWordCtas = 2, kWarpWordLen = 2048;
+constexpr int kWordThreads = 512, kWordCtas = 2;
 
 // Shared memory: k-mer bitset | lookup table (word_table_bytes).
 template <int P, int M>
@@ -321,14 +330,29 @@ __global__ void __launch_bounds__(kWordThreads, kWordCtas)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nbw = (db.n + 31) / 32;
   uint32_t cand = 0, base = 0, bytes = 0, wpass = 0;  // a thread sees fewer than 2^17 candidates of 22 KB
-  const int W = gridDim.x * (blockDim.x >> 5);
-  for (int wi = warp * gridDim.x + blockIdx.x; wi < nbw; wi += W) {
+  const int W = gridDim.x * (blockDim.x >> 5), gw = warp * gridDim.x + blockIdx.x;
+  const int n_long = word_here ? db.long_n : 0;
+  for (int c = W - 1 - gw; c < n_long; c += W) {  // a warp per record
+    if (!((rb.alive[c >> 5] >> (c & 31)) & 1u)) continue;
+    const int L2 = __ldg(db.len + c), net2 = __ldg(db.net + c), cut = cutoff_of(L2, s);
+    const bool comp = !(base_sum<A>(db.cnt, c, s_rc) < cut);
+    if (lane == 0) {
+      cand++;
+      base += comp;
+      bytes += 4 * (2 + A) + (comp ? 4 * P * ((net2 + 31) / 32) : 0);
+    }
+    if (!comp) continue;  // warp-uniform
+    const bool pass = words_reach_warp<P, M>(db, c, net2, prm.w, word_min(L2, prm.w, s), s_tab, s_list) && lane == 0;
+    if (pass) wpass++;
+    push_queue(rb, st, pass, pass ? class_of(db.type, window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1), L2) : 0, c);
+  }
+  for (int wi = gw; wi < nbw; wi += W) {
     const uint32_t bits = rb.alive[wi];
     if (!bits) continue;  // warp-uniform
     const int c = wi * 32 + lane;
     bool pass = false, deferred = false;
     int cls = 0;
-    if ((bits >> lane) & 1u) {
+    if (((bits >> lane) & 1u) && c >= n_long) {
       cand++;
       bytes += 4 * (2 + A);
       const int L2 = __ldg(db.len + c), cut = cutoff_of(L2, s);
@@ -347,15 +371,16 @@ __global__ void __launch_bounds__(kWordThreads, kWordCtas)
       }
       if (pass) cls = class_of(db.type, window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1), L2);
     }
-    const unsigned dm = __ballot_sync(kFullMask, deferred);
-    if (dm) {
-      const int leader = __ffs(dm) - 1;
-      uint32_t b = 0;
-      if (lane == leader) b = atomicAdd(&st->long_count, (uint32_t)__popc(dm));
-      b = __shfl_sync(kFullMask, b, leader);
-      if (deferred) rb.long_list[b + __popc(dm & ((1u << lane) - 1u))] = c;
+    for (unsigned dm = __ballot_sync(kFullMask, deferred); dm; dm &= dm - 1) {
+      const int src = __ffs(dm) - 1, cc = wi * 32 + src;
+      const bool reach = words_reach_warp<P, M>(db, cc, __ldg(db.net + cc), prm.w, word_min(__ldg(db.len + cc), prm.w, s),
+                                                s_tab, s_list);
+      if (lane == src) {
+        pass = reach;
+        if (pass) wpass++;
+      }
     }
-    push_queue(rb, st, pass && !deferred, cls, c);
+    push_queue(rb, st, pass, cls, c);
   }
   flush_stats(rb, cand, base, bytes, word_here ? base : 0, wpass);
 }
@@ -457,55 +482,11 @@ __global__ void __launch_bounds__(256) k_word_exact(DevDB db, RunBufs rb, RunPar
   flush_stats(rb, 0, 0, bytes, wchk, wpass);
 }
 
-// Short-word test of the candidates that k_filter_word queued in rb.long_list:
-// one warp per candidate, spread over the grid; survivors join the alignment
-// class queues.
-template <int P, int M>
-__global__ void __launch_bounds__(256) k_filter_long(DevDB db, RunBufs rb, RunParams prm) {
-  RunState *st = rb.st;
-  extern __shared__ __align__(16) uint32_t s_list[];
-  __shared__ uint64_t bar;
-  __shared__ int s_hdr[3];
-  if (threadIdx.x == 0) {
-    const bool skip = st->done || st->iter >= st->iter_limit || st->err;
-    s_hdr[0] = skip ? 0 : (int)st->long_count;
-    s_hdr[1] = st->rep_len;
-    s_hdr[2] = st->rep_nb;
-  }
-  __syncthreads();
-  const int nlong = s_hdr[0];
-  if ((int)blockIdx.x * (int)(blockDim.x >> 5) >= nlong) return;
-  const int L1 = s_hdr[1], nb1 = s_hdr[2];
-  const uint32_t list_words = list_words_of(db.type, prm.w);
-  uint8_t *s_tab = reinterpret_cast<uint8_t *>(s_list + list_words);
-  if (!stage_to_smem(s_list, rb.rep_list, list_words, &bar, st, 2)) return;
-  build_word_table<P, M>(s_tab, s_list, prm.w);
-  const float s = prm.s;
-  const int lane = threadIdx.x & 31;
-  const int W = gridDim.x * (blockDim.x >> 5);
-  unsigned long long wpass = 0;
-  for (int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < nlong; k += W) {
-    const int c = rb.long_list[k];
-    const int L2 = __ldg(db.len + c);
-    const bool pass = words_reach_warp<P, M>(db, c, __ldg(db.net + c), prm.w, word_min(L2, prm.w, s), s_tab, s_list) &&
-                      lane == 0;
-    if (pass) wpass++;
-    push_queue(rb, st, pass,
-               pass ? class_of(db.type, window_need(L1, L2, cutoff_of(L2, s), band_blocks(L1, L2, s), nb1), L2) : 0, c);
-  }
-  flush_stats(rb, 0, 0, 0, 0, wpass);
-}
-
 using FilterFn = void (*)(DevDB, RunBufs, RunParams, int, int);
 using WordFn = void (*)(DevDB, RunBufs, RunParams, int);
-using LongFn = void (*)(DevDB, RunBufs, RunParams);
 static WordFn word_fn(int type, int M) {
   if (type) return M == 2 ? k_filter_word<5, 2> : k_filter_word<5, 1>;
   return M == 4 ? k_filter_word<2, 4> : M == 2 ? k_filter_word<2, 2> : k_filter_word<2, 1>;
-}
-static LongFn long_fn(int type, int M) {
-  if (type) return M == 2 ? k_filter_long<5, 2> : k_filter_long<5, 1>;
-  return M == 4 ? k_filter_long<2, 4> : M == 2 ? k_filter_long<2, 2> : k_filter_long<2, 1>;
 }
 static size_t word_smem(int type, int w) {
   return 4 * (size_t)list_words_of(type, w) + word_table_bytes(type, w, words_per_lookup(type, w));
@@ -524,8 +505,6 @@ cudaError_t filter_configure() {
   for (int type = 0; type < 2; type++)
     for (int M = 1; M <= (type ? 2 : 4); M *= 2) {
       cudaError_t e = cudaFuncSetAttribute((const void *)word_fn(type, M), cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute((const void *)long_fn(type, M), cudaFuncAttributeMaxDynamicSharedMemorySize, most);
       if (e != cudaSuccess) return e;
     }
   done[dev] = true;
@@ -554,10 +533,6 @@ cudaError_t launch_filter(ngia_ctx *c) {
       const size_t smem = word_smem(type, c->prm.w);
       const int grid_w = std::max(1, std::min(std::min(c->grid_filter, kWordCtas * c->num_sms), (nbw + 7) / 8));
       word_fn(type, M)<<<grid_w, kWordThreads, smem, c->stream>>>(c->db, c->rb, c->prm, turn);
-      if (c->db.max_nb * 32 > kWarpWordLen) {  // some record is long
-        const int grid_l = std::max(1, std::min(c->grid_filter, c->num_sms));
-        long_fn(type, M)<<<grid_l, 256, smem, c->stream>>>(c->db, c->rb, c->prm);
-      }
     }
     if (!word || turn >= 0) fn<<<grid, 256, 0, c->stream>>>(c->db, c->rb, c->prm, 0, turn >= 0 ? 0 : -1);
     return cudaGetLastError();

@@ -53,3 +53,33 @@ def test_word_passes_of_one_iteration(cuda_device, db_type, w, s):
             assert sum(st["class_pairs"]) - 1 == word_ok.sum()
             member = word_ok & (exp[:, 6] != 0)
             assert ((cl[1:] == 0) == member).all()
+
+
+@pytest.mark.parametrize("db_type,w,s", [(0, 5, 0.97), (1, 3, 0.9)])
+def test_word_passes_of_records_in_any_order(cuda_device, db_type, w, s):
+    """Long records behind short ones (the filter gives a warp each to those in
+    front): candidates of one representative, the rest in random order."""
+    rng = np.random.default_rng(7 + db_type)
+    alpha = np.frombuffer(b"ACGT" if db_type == 0 else b"ACDEFGHIKLMNPQRSTVWY", np.uint8)
+    base = np.resize(alpha[rng.integers(0, len(alpha), 400 if db_type == 0 else 3200)], 4100)
+    seqs = [base.tobytes()]
+    for L in (40, 300, 2040, 2049, 2600, 4000) * 20:
+        x = base[:L].copy()
+        hit = rng.random(L) < rng.choice([0.0, 0.02, 0.1, 1.0])
+        x[hit] = alpha[rng.integers(0, len(alpha), int(hit.sum()))]
+        seqs.append(x.tobytes())
+    db = seqs_to_db(db_type, seqs)
+    order = np.concatenate([[0], 1 + rng.permutation(db.n - 1)])
+    recs = ngia.Records(db_type, np.ascontiguousarray(db.words), np.ascontiguousarray(db.rec_off[order]))
+    p = ngia.params_clamp(db_type, s, w, 0)
+    exp = np.stack([oracle.pair(db.words, db.rec_off, db_type, p.similarity, w, 0, i) for i in order])
+    ok = (exp[:, 4] != 0) & (exp[:, 5] != 0)
+    ok[0] = True
+    with ngia.Context(recs) as ctx:
+        ctx.set_tuning(1, 32, -1)
+        ctx.begin(p, ngia.MODE_GRAPH)
+        ctx.step(1)
+        st = ctx.stats()
+        cl = ctx.end()[0]
+    assert sum(st["class_pairs"]) == ok.sum()
+    assert ((cl == 0) == (ok & ((exp[:, 6] != 0) | (np.arange(len(ok)) == 0)))).all()
