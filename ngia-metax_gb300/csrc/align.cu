@@ -24,9 +24,9 @@
 //   IADD3.X, LOP3); protein builds it from the rep's planes held in registers
 //   (one LOP3 per plane).
 //
-// k_align_wave<P,NW>, k_align_query<P>  classes with few queued pairs: a warp
-//   (windows up to 64 blocks) or a CTA of four warps per pair; 16 threads for
-//   a short query against a long representative (wave.cuh).
+// k_align_wave<P,NW,WMAX>, k_align_query<P>  classes with few queued pairs: 8,
+//   32 or 128 threads per pair by their number and the width of their windows;
+//   16 threads for a short query against a long representative (wave.cuh).
 //
 // In clustering both keep only the rows that a score of at least the cutoff
 // can use (band_advance in tile.cuh) and stop a pair once it provably cannot

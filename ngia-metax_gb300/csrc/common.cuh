@@ -18,9 +18,10 @@ constexpr int kRefGridThreads = 128 * 128;     // BLOCK*WARP of the reference la
 // their alignment can need (window_need, in rep blocks): the last three
 // classes of a type hold windows of up to 48 or 112 blocks (kSmallWindow,
 // kWideWindow) in shared-memory rows, or of any width in global-memory rows.
-// Classes 0 and 1 are the pairs of windows up to 112 and of any width whose query has at most
-// kQueryRows blocks: short queries against a long representative, aligned by
-// 16 threads with the query's blocks as rows (wave.cuh) while they are few.
+// Classes 0 and 1 are the pairs of windows of 49 to 112 and of more blocks
+// whose query has at most kQueryRows blocks: short queries against a long
+// representative, aligned by 16 threads with the query's blocks as rows
+// (wave.cuh) while they are few.
 // DNA numbers 2 and 3 are unused: class numbers in saved tunings, checkpoints
 // and statistics keep their meaning.
 constexpr int kNumClasses = 7;

@@ -19,11 +19,11 @@
 //    residues) in a fixed file-scope device array, g_noalloc_rows, of
 //    kNoAllocWords words (4 MiB).
 // GB300, whole calls: 4,096 DNA queries of 1,450 residues 747 -> 117 us, 1,000
-// proteins of 380 residues 278 -> 43 us (against the third kernel for all).
+// proteins of 380 residues 278 -> 43 us (against the third form for all).
 //
 // Every GPU that loads this library keeps that array until the process
 // exits.  Its size caps the representative at 65,536 residues (2,048 words
-// per thread row); the grid of the third kernel is sized so that every
+// per thread row); the grid of the third form is sized so that every
 // thread's row fits.
 //
 // Host code must not use the array's name as a device address: the first call

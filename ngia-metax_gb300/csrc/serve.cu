@@ -7,8 +7,7 @@
 // Resident state (ngia_serve_open): the representatives as a device
 // database (records and header arrays, loaded by the same loader as
 // ngia_open) plus one k-mer bitset per representative, built on the device.
-// The per-pair kernels are shared with
-// the speculative rounds (assign.cuh).
+// The per-pair kernels are shared with the speculative rounds (assign.cuh).
 //
 // One batch runs on one slot — a context of fixed capacity with its own
 // stream, driven by its own host thread:
