@@ -141,52 +141,88 @@ __device__ __forceinline__ void queue_groups(const RoundBufs &rb, int r, int q0,
 }
 
 // One CTA per representative of the chunk: composition test (and the
-// short-word test in word-first order) for every unassigned query.
+// short-word test in word-first order) for every unassigned query, kServeTile
+// queries at a time, whose outcomes lie in shared memory until they are queued:
+// a batch of any size takes the same bounded amount.  (One byte per query of
+// the whole batch had to be allowed for by each service's own size, and a
+// batch of more than some 220,000 did not fit.)  A tile pads its last group of
+// each class; batches of up to 65,536 have one tile.
+constexpr int kServeTile = 1 << 16;
+// Entries of one representative and class for `left` queries in `tiles` tiles.
+__host__ __device__ constexpr int64_t serve_entries(int64_t left, int64_t tiles) { return (left + 31 * tiles) & ~31ll; }
+__host__ __device__ constexpr int64_t serve_tiles(int64_t n) { return (n + kServeTile - 1) / kServeTile; }
+// Dynamic shared memory: the k-mer bitset, then a byte per query of a tile.
+__host__ __device__ constexpr size_t serve_filter_smem(int list_words, int64_t n) {
+  return 4 * (size_t)list_words + (size_t)(n < kServeTile ? (n + 31) & ~31ll : kServeTile);
+}
 template <int P>
 __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, RunParams prm, RoundBufs rb, int r0) {
-  extern __shared__ __align__(16) uint32_t s_list[];  // the representative's k-mer bitset, then per query:
+  extern __shared__ __align__(16) uint32_t s_list[];  // the representative's k-mer bitset, then per query of the tile:
   uint8_t *s_res = reinterpret_cast<uint8_t *>(s_list + rs.list_words);  // 0 = out, 1 + class
   __shared__ uint32_t s_rc[28], s_cnt[kServeClasses], s_base[kServeClasses], s_pos[kServeClasses];
   constexpr int A = P == 2 ? 4 : 28;
   const int r = r0 + blockIdx.x;
   const uint32_t *rec = rs.words + rs.off[r];
   if (threadIdx.x < A) s_rc[threadIdx.x] = rec[2 + threadIdx.x];
-  if (threadIdx.x < kServeClasses) s_cnt[threadIdx.x] = 0;
-  __syncthreads();
   const int L1 = (int)rec[0], net1 = (int)rec[1], nb1 = (net1 + 31) / 32;
   const float s = prm.s;
   const bool word_here = !prm.precise && net1 >= 16 && rs.first[r];
-  if (word_here) {
+  if (word_here)
     for (int t = threadIdx.x; t < rs.list_words; t += blockDim.x) s_list[t] = rs.lists[(int64_t)r * rs.list_words + t];
-    __syncthreads();
-  }
-  const int n = qdb.n, nbw = (n + 31) / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int wi = warp; wi < nbw; wi += blockDim.x >> 5) {
-    const uint32_t bits = rb.todo[wi];
-    const int q = wi * 32 + lane;
-    int res = 0;
-    if ((bits >> lane) & 1u) {
-      // a smaller representative of this round may already hold q
-      const bool open = (rb.key[q] >> 32) > (unsigned long long)r;
-      const int L2 = __ldg(qdb.len + q);
-      const int cut = cutoff_of(L2, s);
-      bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cut);
-      if (pass && word_here) {
-        const int net2 = __ldg(qdb.net + q);
-        if (net2 >= 16) pass = words_reach<P, 1>(qdb, q, net2, prm.w, word_min(L2, prm.w, s), KmerBits{s_list}, s_list);
+  for (int q0 = 0; q0 < qdb.n; q0 += kServeTile) {
+    const int n = min(kServeTile, qdb.n - q0), nbw = (n + 31) / 32;
+    if (threadIdx.x < kServeClasses) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    for (int wi = warp; wi < nbw; wi += blockDim.x >> 5) {
+      const uint32_t bits = rb.todo[q0 / 32 + wi];
+      const int k = wi * 32 + lane, q = q0 + k;
+      int res = 0;
+      if ((bits >> lane) & 1u) {
+        // a smaller representative of this round may already hold q
+        const bool open = (rb.key[q] >> 32) > (unsigned long long)r;
+        const int L2 = __ldg(qdb.len + q);
+        const int cut = cutoff_of(L2, s);
+        bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cut);
+        if (pass && word_here) {
+          const int net2 = __ldg(qdb.net + q);
+          if (net2 >= 16)
+            pass = words_reach<P, 1>(qdb, q, net2, prm.w, word_min(L2, prm.w, s), KmerBits{s_list}, s_list);
+        }
+        if (pass) res = 1 + serve_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1));
       }
-      if (pass) res = 1 + serve_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1));
+      if (k < n) s_res[k] = (uint8_t)res;
+      const unsigned pm = __ballot_sync(kFullMask, res != 0);
+      if (res) {
+        const unsigned peers = __match_any_sync(pm, res);
+        if (lane == __ffs(peers) - 1) atomicAdd(&s_cnt[res - 1], (uint32_t)__popc(peers));
+      }
     }
-    if (q < n) s_res[q] = (uint8_t)res;
-    const unsigned pm = __ballot_sync(kFullMask, res != 0);
-    if (res) {
-      const unsigned peers = __match_any_sync(pm, res);
-      if (lane == __ffs(peers) - 1) atomicAdd(&s_cnt[res - 1], (uint32_t)__popc(peers));
-    }
+    __syncthreads();
+    queue_groups(rb, r, q0, n, s_res, s_cnt, s_base, s_pos);
+    __syncthreads();  // the tile's outcomes and places are read
   }
-  __syncthreads();
-  queue_groups(rb, r, 0, n, s_res, s_cnt, s_base, s_pos);
+}
+
+// The filter's dynamic shared memory limit, the largest any service can need:
+// it belongs to the kernel on the device, and is set once, so that no service
+// changes it under another.
+inline cudaError_t serve_filter_configure() {
+  static std::mutex mu;
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done[dev]) return cudaSuccess;
+  constexpr int most = (int)serve_filter_smem(kListWords, kServeTile);
+  for (const void *fn : {(const void *)k_serve_filter<2>, (const void *)k_serve_filter<5>}) {
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return e;
+  }
+  done[dev] = true;
+  return cudaSuccess;
 }
 
 // Whether the class's pairs of this round go to the group-per-pair kernel

@@ -58,6 +58,7 @@ namespace {
 constexpr int kFirstChunk = 64;     // representatives in the first round
 constexpr int kMaxChunk = 1024;     // ... doubling up to this many per round
 constexpr int64_t kFirstPairs = 1 << 16, kMaxPairs = 1 << 18;  // pairs a round takes more representatives for
+constexpr int64_t kMaxEntries = 0xFFF00000ll;  // of a class queue: claims run past its end by less than 2^20
 
 __global__ void k_serve_init(int n, RoundBufs rb) {
   const int nbw = (n + 31) / 32;
@@ -214,7 +215,7 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
     const char *m = getenv("NGIA_SERVE_MAX_CHUNK");
     return m ? std::max(kFirstChunk, std::min(kMaxChunk, atoi(m))) : INT_MAX;
   }();
-  const size_t fsm = 4 * (size_t)sv->store.list_words + (size_t)nbw * 32;
+  const size_t fsm = serve_filter_smem(sv->store.list_words, n);
   int r0 = 0, chunk = kFirstChunk;
   int64_t pairs = kFirstPairs;
   uint32_t left = (uint32_t)n;
@@ -222,8 +223,9 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
   if (trace())
     for (auto &e : ev) cudaEventCreate(&e);
   while (r0 < sv->store.n && left > 0) {
-    // at most the queue's capacity: a representative's entries pad to 32
-    const int64_t fit = rb.cap / (((int64_t)left + 31) & ~31ll);
+    // at most the queue's capacity and what its 32-bit counters hold: a
+    // representative's entries pad to 32 in each tile of the filter
+    const int64_t fit = std::min(rb.cap, kMaxEntries) / serve_entries(left, serve_tiles(n));
     const int64_t want = std::min<int64_t>({std::max<int64_t>(chunk, pairs / left), fit, (int64_t)max_chunk});
     const int nr = (int)std::min<int64_t>(want, sv->store.n - r0);
     CKS(cudaMemsetAsync(rb.ctl, 0, kCtlWords * sizeof(uint32_t), st));
@@ -491,12 +493,9 @@ extern "C" int ngia_serve_open(const ngia_db_view *reps, const ngia_params *para
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   const int64_t budget = cf.memory_budget > 0 ? cf.memory_budget : (int64_t)(free_b / 2);
-  const size_t fsm = 4 * (size_t)lw + (size_t)((sv->cap_n + 31) / 32 * 32);
-  if (fsm > 48 * 1024)
-    cudaFuncSetAttribute(sv->type == 0 ? (const void *)ngia::k_serve_filter<2> : (const void *)ngia::k_serve_filter<5>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(fsm, 226 * 1024));
   ngia::RoundPlan plan;
-  e = ngia::round_plan<false>(plan, sv->type, rc_ctx->db.max_nb, sv->num_sms);
+  e = ngia::serve_filter_configure();
+  if (e == cudaSuccess) e = ngia::round_plan<false>(plan, sv->type, rc_ctx->db.max_nb, sv->num_sms);
   if (e != cudaSuccess) {
     ngia::destroy(sv);
     return fail(NGIA_E_CUDA, "ngia_serve_open: kernel attributes: %s", cudaGetErrorString(e));

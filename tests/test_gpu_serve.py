@@ -88,3 +88,28 @@ def test_serve_poll_and_errors(cuda_device):
             srv.submit(prot)
         assert ex.value.code == -1
         assert srv.wait(srv.submit(batches[1]))[2]["done"] == 1
+
+
+def test_large_batches_of_services_side_by_side(cuda_device):
+    """A service for batches that take several tiles of the filter, and one of
+    other limits opened after it: full batches, whole tiles and one query more."""
+    rng = np.random.default_rng(96)
+    alpha = np.frombuffer(b"ACGT", np.uint8)
+    base = alpha[rng.integers(0, 4, (7, 64))]  # four representatives, three novel families
+    p = ngia.params_clamp(0, 0.8, 4, 0)
+    reps = seqs_to_db(0, [b.tobytes() for b in base[:4]])
+
+    def batch(n):
+        x = base[np.where(rng.random(n) < 0.002, rng.integers(4, 7, n), rng.integers(0, 4, n))]
+        hit = rng.random(x.shape) < 0.12 * rng.random((n, 1))
+        x[hit] = alpha[rng.integers(0, 4, int(hit.sum()))]
+        length = rng.integers(52, 65, n)
+        return seqs_to_db(0, [r[:k].tobytes() for r, k in zip(x, length)])
+
+    with ngia.Server(reps, p, slots=1, max_batch=240_000, max_record_blocks=4) as large, \
+            ngia.Server(reps, p, slots=1, max_batch=60_000, max_record_blocks=4) as small:
+        for srv, n in ((large, 240_000), (small, 60_000), (large, 65_536), (large, 65_537), (large, 3)):
+            b = batch(n)
+            got = srv.wait(srv.submit(b))
+            exp = _expected(p, reps, b)
+            assert np.array_equal(got[0], exp[0]) and np.array_equal(got[1], exp[1]), n
