@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kThreads) k_noalloc_wave(const uint32_t *__res
   ngia::wave_table<P>(rep + hw, nb1, vlast, s_mem, threadIdx.x, kThreads);
   __syncthreads();
   unsigned long long cells = 0;
-  for (int k = blockIdx.x * kGroups + group; k < n; k += gridDim.x * kGroups) {
+  for (int64_t k = blockIdx.x * kGroups + group; k < n; k += gridDim.x * kGroups) {
     const uint32_t *q = words + query_off[k];
     int net2 = 0, B = 0, score = 0;
     if (noalloc_pair(q, nb1, L1, s, net2, B, &score))
@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(kThreads) k_noalloc_sub(const uint32_t *__rest
   __syncthreads();
   unsigned long long cells = 0;
   const int first = threadIdx.x / 32 * ngia::kSubs;  // the warp's first pair of the CTA's
-  for (int k0 = blockIdx.x * kGroups + first; k0 < n; k0 += gridDim.x * kGroups) {  // warp-uniform
-    const int k = k0 + (group - first);
+  for (int64_t k0 = blockIdx.x * kGroups + first; k0 < n; k0 += gridDim.x * kGroups) {  // warp-uniform
+    const int64_t k = k0 + (group - first);
     const uint32_t *q = words;
     int net2 = 0, B = 0, score = 0;
     bool run = false;
@@ -239,9 +239,9 @@ __global__ void __launch_bounds__(kThreads, ngia::tiled_min_blocks(P))
   (void)fk;
   Ring ring;
   ring.base = s_mem + planes + threadIdx.x;
-  const int lane = threadIdx.x & 31, warps = gridDim.x * (kThreads / 32);
-  for (int k0 = (blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * 32; k0 < n; k0 += warps * 32) {
-    const int k = k0 + lane;
+  const int lane = threadIdx.x & 31;
+  for (int64_t k0 = blockIdx.x * kThreads + threadIdx.x - lane; k0 < n; k0 += gridDim.x * kThreads) {
+    const int64_t k = k0 + lane;
     int net2 = 0, B = 0, score = 0, nq = 0, js = 0, je = -1, frozen = 0, zw = 0;
     const uint32_t *qpl = words;
     if (k < n) {
@@ -366,14 +366,14 @@ extern "C" int ngia_rep_scores_noalloc(const uint32_t *d_words, int64_t rep_off,
   if (smem <= kNoAllocSmemMost) {
     e = noalloc_configure(fn, (P == 2 ? 0 : 8) + (many ? 4 + (nb1 <= ngia::kSmallWindow ? 0 : 1) : sub ? 6 : form), smem);
     if (e != cudaSuccess) return ngia::fail(NGIA_E_CUDA, "ngia_rep_scores_noalloc: %s", cudaGetErrorString(e));
-    const int grid = std::max(1, std::min(std::max(sms, 1) * 8, (n + per - 1) / per));
+    const int grid = (int)std::min<int64_t>(std::max(sms, 1) * 8, ((int64_t)n + per - 1) / per);
     fn<<<grid, kThreads, smem, st>>>(d_words, rep_off, d_query_off, n, similarity, d_scores, nb1);
   } else {  // a protein's table of more than 1,700 blocks
     // Every thread owns one row of nb1 words; the grid is as large as the
     // array allows (at least 4 CTAs: 2,048-word rows x 512 threads).
     const int64_t max_lanes = kNoAllocWords / (nb1 > 0 ? nb1 : 1);
     int grid = (int)std::min<int64_t>((int64_t)std::max(sms, 1) * 4, max_lanes / kThreads);
-    grid = std::max(1, std::min(grid, (n + kThreads - 1) / kThreads));
+    grid = (int)std::max<int64_t>(1, std::min<int64_t>(grid, ((int64_t)n + kThreads - 1) / kThreads));
     const int64_t lanes = (int64_t)grid * kThreads;
     const int cap_blocks = (int)(kNoAllocWords / lanes);
     k_noalloc_scores<5><<<grid, kThreads, sizeof(uint32_t) * (size_t)(nb1 * P), st>>>(
