@@ -53,11 +53,26 @@ constexpr int kNoAllocWords = 1 << 20;  // 4 MiB of per-thread rows
 constexpr int kThreads = 128;
 static_assert(kThreads == ngia::kAlignThreads, "the ring and the groups of four warps");
 // Pairs per SM up to which a group per pair is faster than a thread per pair,
-// which takes a pair's latency whatever their number.  GB300: DNA 1,450
-// residues 242 us for 10,000 pairs by groups and 257 by threads, 274 and 268
-// for 14,000; 300 residues 69 against 47 for 6,000; protein 380 residues 119
-// and 119 for 10,000.
-constexpr int noalloc_groups(int P, int nb1) { return P == 5 ? 64 : nb1 <= 16 ? 26 : 80; }
+// which takes a pair's latency whatever their number.  That latency grows
+// faster with the representative than a group's share of an SM, where a step's
+// fixed costs count (DNA of 4 to 46 blocks: 34 to 256 us for a thread, 41 to
+// 224 for groups of 8 with 80 pairs per SM), so the line rises with its blocks.
+// GB300, us for 8 threads per pair and for a thread, at the pairs per SM on
+// both sides of the line:
+//   DNA, 7 blocks        42, 42 (20)   42, 41 (26)
+//       13               55, 61 (32)   65, 61 (40)
+//       19               80, 88 (40)   93, 87 (50)
+//       25               99, 117 (40)  116, 116 (56)
+//       32               140, 153 (64) 167, 153 (72)
+//       46               224, 256 (80) 256, 255 (90)
+//      107               893, 1,070 (64) 1,084, 1,069 (80)
+//   protein, 7 blocks    45, 48 (14)   49, 47 (26)   (seven operations per match
+//       12               73, 77 (40)   83, 78 (50)    word of a thread instead of
+//       19               133, 142 (72) 158, 142 (90)  three: later)
+//       29               235, 262 (105)
+constexpr int noalloc_groups(int P, int nb1) {
+  return P == 2 ? std::min(std::min(12 + 2 * nb1, 26 + 5 * nb1 / 4), 80) : std::max(12, std::min(4 * nb1, 112));
+}
 constexpr size_t kNoAllocSmemMost = 226 * 1024;
 
 __device__ __align__(256) uint32_t g_noalloc_rows[kNoAllocWords];
