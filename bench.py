@@ -828,7 +828,7 @@ def run_batch(args, dist: Dist, emit: bool = True):
                       "jobs": len(tun), "cached": int(sum(t["cached"] for t in tun)),
                       "policy": ["thread", "cutoff", "tuned"][b.policy()],
                       "ms_per_iter": round(tun[0]["ms_per_iter"], 3),
-                      "thread_ms_per_iter": round(tun[0]["default_ms_per_iter"], 3)}
+                      "default_ms_per_iter": round(tun[0]["default_ms_per_iter"], 3)}
         for mode, name in ((ngia.MODE_POOL, "batch"), (ngia.MODE_GRAPH, "loops"), (ngia.MODE_SPEC, "rounds"),
                            (ngia.MODE_PLAIN, "plain")):
             for _ in range(args.warmup):

@@ -421,17 +421,18 @@ int ngia_set_tuning(ngia_ctx *ctx, const ngia_tuning *t);
  * whole batch over the first `iters` greedy iterations of every job:
  *   NGIA_BATCH_POLICY_THREAD  every length bucket of every job aligned
  *                             thread per pair;
- *   NGIA_BATCH_POLICY_CUTOFF  each job's whole default group-per-pair cut-off;
+ *   NGIA_BATCH_POLICY_CUTOFF  the untuned batch's settings: each job's
+ *                             buckets go to the group-per-pair kernels up to
+ *                             the default cut-off divided by the number of
+ *                             jobs;
  *   NGIA_BATCH_POLICY_TUNED   each job's own ngia_autotune settings, found
  *                             with the job alone on the GPU (cached by
  *                             database shape and parameters).
- * The thread-per-pair policy is chosen unless another is at least 2% faster.
- * (Before any choice, a job's buckets go to the group-per-pair kernels up to
- * the default cut-off divided by the number of jobs.)
+ * The untuned batch's settings are chosen unless others are at least 2% faster.
  * Later NGIA_MODE_GRAPH runs apply the chosen policy; out[j] (may be NULL)
  * receives job j's settings under it (candidates = 3, ms_per_iter and
  * default_ms_per_iter the batch's wall time per iteration under the chosen
- * and the thread-per-pair policy).  Results never change.  No reference
+ * policy and the untuned settings).  Results never change.  No reference
  * counterpart. */
 #define NGIA_BATCH_POLICY_THREAD 0
 #define NGIA_BATCH_POLICY_CUTOFF 1

@@ -186,6 +186,19 @@ bool batch_warp() {
   return on;
 }
 
+// A job's group-per-pair cut-off in the per-job-loop form when no policy sets
+// another.  Jobs running side by side share the GPU: each class of a job goes
+// to the group-per-pair kernels up to the job's share of the pairs at which
+// they pay (many jobs: thread per pair, the form with the fewest instructions
+// per cell).  GB300, ms per 16 iterations with the share, every class thread
+// per pair, and each job's whole cut-off (NGIA_BATCH_WARP=1): 12 mixed jobs of
+// 1,000-4,000 records of up to 10,000 residues 15.9, 78.0, 17.3; 32 of them
+// 20.3, 81.8, 27.7; 32 jobs of 2,000 DNA of 1,450 residues 5.5, 4.9, 10.7; 8
+// protein jobs 4.2, 16.1, 4.7.
+int job_cut(const ngia_batch *b, const ngia_ctx *c) {
+  return batch_warp() ? -1 : c->warp_pairs_default / (int)b->jobs.size();
+}
+
 // A job the pools can take: its greedy loop needs no per-job exact
 // short-word path (no record of net length < 16 while the test is on).
 bool poolable(const ngia_ctx *c) { return !(c->db.has_short && !c->prm.precise); }
@@ -353,17 +366,11 @@ extern "C" int ngia_batch_run(ngia_batch *b, const ngia_params *params, int32_t 
     bool rebuild = !b->exec || b->prm.size() != nj;
     for (size_t j = 0; j < nj; j++) {
       ngia_ctx *c = b->jobs[j];
-      // jobs running side by side share the GPU: each class of a job goes to
-      // the group-per-pair kernels up to the job's share of the pairs at
-      // which they pay (many jobs: thread per pair, the form with the fewest
-      // instructions per cell; 12 jobs of 1,000-4,000 sequences on GB300, 32
-      // iterations each: 281 ms with every class thread per pair, 27
-      // with the share); NGIA_BATCH_WARP=1 keeps each job's own cut-off
       // after ngia_batch_autotune, the chosen policy's settings
       if (b->policy >= 0 && b->policy_wp.size() == nj)
         c->tuned_warp_pairs = b->policy_wp[j];
       else
-        c->tuned_warp_pairs = batch_warp() ? -1 : c->warp_pairs_default / (int)nj;
+        c->tuned_warp_pairs = job_cut(b, c);
       int rc = ngia_cluster_begin(c, &params[j], NGIA_MODE_PLAIN);  // no per-job graph
       if (rc) return rc;
       c->mode = NGIA_MODE_GRAPH;
@@ -411,15 +418,15 @@ extern "C" int ngia_batch_run(ngia_batch *b, const ngia_params *params, int32_t 
 namespace {
 
 // The settings of one job under a batch policy: the untuned settings with
-// every bucket thread per pair, the untuned settings with the job's default
-// group-per-pair cut-off, or the job's own tuning.
-ngia_tuning policy_setting(int policy, const ngia_tuning &own) {
+// every bucket thread per pair, the untuned settings with the batch's default
+// cut-off (job_cut), or the job's own tuning.
+ngia_tuning policy_setting(int policy, int cut, const ngia_tuning &own) {
   if (policy == NGIA_BATCH_POLICY_TUNED) return own;
   ngia_tuning t;
   std::memset(&t, 0, sizeof(t));
   t.word_order = 0;
   t.refill = 32;
-  t.warp_pairs = policy == NGIA_BATCH_POLICY_THREAD ? 0 : -1;
+  t.warp_pairs = policy == NGIA_BATCH_POLICY_THREAD ? 0 : cut;
   for (int k = 0; k < 8; k++) {
     t.class_warp_pairs[k] = -1;
     t.class_grid_div[k] = 1;
@@ -432,7 +439,7 @@ int apply_policy(ngia_batch *b, int policy, const std::vector<ngia_tuning> &own)
   b->policy = policy;
   b->policy_wp.assign(b->jobs.size(), 0);
   for (size_t j = 0; j < b->jobs.size(); j++) {
-    const ngia_tuning t = policy_setting(policy, own[j]);
+    const ngia_tuning t = policy_setting(policy, job_cut(b, b->jobs[j]), own[j]);
     int rc = ngia_set_tuning(b->jobs[j], &t);
     if (rc) return rc;
     b->policy_wp[j] = t.warp_pairs;
@@ -456,7 +463,7 @@ extern "C" int ngia_batch_autotune(ngia_batch *b, const ngia_params *params, int
   // each policy timed on the whole batch, the first `iters` iterations of
   // every job in one graph launch: one untimed launch (graph capture), then
   // the faster of two
-  const int policies[3] = {NGIA_BATCH_POLICY_THREAD, NGIA_BATCH_POLICY_CUTOFF, NGIA_BATCH_POLICY_TUNED};
+  const int policies[3] = {NGIA_BATCH_POLICY_CUTOFF, NGIA_BATCH_POLICY_THREAD, NGIA_BATCH_POLICY_TUNED};
   double ms[3];
   for (int q = 0; q < 3; q++) {
     int rc = apply_policy(b, policies[q], own);
@@ -470,7 +477,7 @@ extern "C" int ngia_batch_autotune(ngia_batch *b, const ngia_params *params, int
       if (r > 0) ms[q] = std::min(ms[q], t);
     }
   }
-  // the thread-per-pair policy stays unless another is 2% faster (the
+  // the untuned batch's settings stay unless others are 2% faster (the
   // timings of one policy differ by about 1% between launches)
   int best = 0;
   for (int q = 1; q < 3; q++)
@@ -479,7 +486,7 @@ extern "C" int ngia_batch_autotune(ngia_batch *b, const ngia_params *params, int
   if (rc) return rc;
   if (out)
     for (size_t j = 0; j < nj; j++) {
-      out[j] = policy_setting(policies[best], own[j]);
+      out[j] = policy_setting(policies[best], job_cut(b, b->jobs[j]), own[j]);
       out[j].candidates = 3;
       out[j].ms_per_iter = ms[best] / iters;
       out[j].default_ms_per_iter = ms[0] / iters;

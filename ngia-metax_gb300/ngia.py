@@ -596,8 +596,8 @@ class Batch:
         return cls, ids, st.as_dict()
 
     def autotune(self, params: list, iters: int = 4) -> list:
-        """Times the three batch policies (thread per pair, default cut-off,
-        each job's own tuning) and keeps the fastest; returns each job's
+        """Times the three batch policies (the untuned settings, thread per
+        pair, each job's own tuning) and keeps the fastest; returns each job's
         settings under it."""
         n = len(self.dbs)
         ps = (Params * n)(*params)

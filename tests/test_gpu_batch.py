@@ -72,3 +72,37 @@ def test_batch_autotune_keeps_results(cuda_device):
             cls, ids, st = b.run(params, ngia.MODE_GRAPH)
             for (ocl, oid), cl, ident in zip(want, cls, ids):
                 assert np.array_equal(cl, ocl) and np.array_equal(ident, oid)
+
+
+def test_autotune_is_no_slower_than_not_calling_it(cuda_device):
+    """Jobs of long records, where a thread per pair is many times slower than
+    the untuned settings: autotune reports those as the default, and neither
+    its choice nor the policy that names them is much slower."""
+    import time
+
+    dbs = []
+    for k in range(4):
+        seqs = ngia.synth(type=0, n_seqs=300, n_ancestors=8, len_dist=2, len_a=200.0, len_b=9000.0, len_min=200,
+                          len_max=9000, subst_max=0.2, indel_max=3, seed=700 + k)
+        dbs.append(ngia.DB.pack(0, seqs, seqs.off))
+    params = [ngia.params_clamp(0, 0.9, 5, 0)] * 4
+    iters = 6
+
+    def per_iter(b):
+        best = float("inf")
+        for _ in range(4):
+            t = time.perf_counter()
+            b.run(params, ngia.MODE_GRAPH, max_iters=iters)
+            best = min(best, time.perf_counter() - t)
+        return 1e3 * best / iters
+
+    with ngia.Batch(dbs) as b:
+        untuned = per_iter(b)
+        b.set_policy(ngia.POLICY_THREAD)
+        thread = per_iter(b)
+        assert thread > 3 * untuned  # what the bounds below tell apart
+        tun = b.autotune(params, iters)
+        assert tun[0]["default_ms_per_iter"] < 2 * untuned
+        assert per_iter(b) < 1.5 * untuned
+        b.set_policy(ngia.POLICY_CUTOFF)
+        assert per_iter(b) < 1.5 * untuned
