@@ -235,8 +235,9 @@ int create_streams(ngia_ctx *c) {
   return NGIA_OK;
 }
 
-// Device arrays of a database of up to cap_n records and cap_words words.
-int alloc_db(ngia_ctx *c, int type, int64_t cap_n, int64_t cap_words) {
+// Device arrays of a database of up to cap_n records and cap_words words
+// (listed in mem_db, not allocated).
+void layout_db(ngia_ctx *c, int type, int64_t cap_n, int64_t cap_words) {
   const int A = ngia::count_words(type);
   // protein residue-code streams for the short-word test (NGIA_PROTEIN_CODES=0:
   // the test reads the planes instead)
@@ -250,7 +251,11 @@ int alloc_db(ngia_ctx *c, int type, int64_t cap_n, int64_t cap_words) {
   m.add(&c->d_net, (size_t)cap_n);
   m.add(&c->d_cnt, (size_t)cap_n * A);
   if (codes) m.add(&c->d_codes, (size_t)cap_words + 4);
-  if (m.take() != cudaSuccess)
+}
+
+int alloc_db(ngia_ctx *c, int type, int64_t cap_n, int64_t cap_words) {
+  layout_db(c, type, cap_n, cap_words);
+  if (c->mem_db.take() != cudaSuccess)
     return fail(NGIA_E_NOMEM, "ngia_open: device allocation of the database failed");
   c->cap_n = cap_n;
   c->cap_words = cap_words;
@@ -264,7 +269,7 @@ int alloc_db(ngia_ctx *c, int type, int64_t cap_n, int64_t cap_words) {
   c->db.type = type;
   c->db.hw = ngia::header_words(type);
   c->db.P = ngia::plane_count(type);
-  c->db.A = A;
+  c->db.A = ngia::count_words(type);
   c->db.max_nb = 1;
   return NGIA_OK;
 }
@@ -326,9 +331,8 @@ void size_grids(ngia_ctx *c, bool by_size) {
 }
 
 // Run buffers for up to cap_n sequences whose records have up to cap_nb
-// plane blocks (grids sized for that capacity).
-int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
-  const int type = c->db.type;
+// plane blocks (grids sized for that capacity; listed in mem_run, not allocated).
+int layout_run(ngia_ctx *c, int type, int64_t cap_n, int cap_nb) {
   c->cap_nb = std::max(1, cap_nb);
   const size_t nbw = (size_t)(cap_n + 31) / 32;
   ngia::RunBufs &rb = c->rb;
@@ -349,16 +353,24 @@ int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
     return fail(NGIA_E_CUDA, "ngia_open: kernel attributes");
   // the widest class keeps its rows in global scratch, sized for this
   // context's grid at capacity (every later grid of the context is within)
-  const int32_t saved_n = c->db.n;
+  const ngia::DevDB saved = c->db;
   c->db.n = (int32_t)cap_n;
+  c->db.type = type;
   size_grids(c, c->batch_member);
-  c->db.n = saved_n;
+  c->db = saved;
   const int g = ngia::generic_class(type);  // (class 1 is on the global ring too)
   rb.generic_lanes = std::max(c->grid_align[1], c->grid_align[g]) * ngia::align_threads();
   rb.ring_rows = ngia::global_rows(c->cap_nb);
   rb.scratch_words = ngia::class_used(type, g, c->cap_nb) ? (int64_t)rb.generic_lanes * rb.ring_rows : 1;
   m.add(&rb.scratch, (size_t)rb.scratch_words);
-  if (m.take() != cudaSuccess) return fail(NGIA_E_NOMEM, "ngia_open: device allocation of run buffers failed");
+  return NGIA_OK;
+}
+
+int alloc_run(ngia_ctx *c, int64_t cap_n, int cap_nb) {
+  int rc = layout_run(c, c->db.type, cap_n, cap_nb);
+  if (rc) return rc;
+  ngia::RunBufs &rb = c->rb;
+  if (c->mem_run.take() != cudaSuccess) return fail(NGIA_E_NOMEM, "ngia_open: device allocation of run buffers failed");
   cudaMemsetAsync(rb.rep_list, 0, 4 * ngia::kListWords, c->stream);
   cudaMemsetAsync(rb.fstats, 0, 8 * ngia::kFilterStripes * ngia::kFilterStats, c->stream);
   return NGIA_OK;
@@ -390,6 +402,16 @@ int ngia::drv::open_ctx(const ngia_db_view *v, bool batch_member, ngia_ctx **out
   }
   *out = c;
   return NGIA_OK;
+}
+
+int ngia::drv::ctx_bytes(int type, int64_t cap_n, int64_t cap_words, int cap_nb, int num_sms, int64_t *bytes) {
+  ngia_ctx c;
+  c.batch_member = true;
+  c.num_sms = num_sms;
+  layout_db(&c, type, cap_n, cap_words);
+  const int rc = layout_run(&c, type, cap_n, cap_nb);
+  *bytes = (int64_t)(c.mem_db.bytes() + c.mem_run.bytes());
+  return rc;
 }
 
 int ngia::drv::open_ctx_capacity(int type, int64_t cap_n, int64_t cap_words, int cap_nb, ngia_ctx **out) {

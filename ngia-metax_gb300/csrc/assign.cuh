@@ -16,6 +16,7 @@
 #pragma once
 #include <stdint.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -634,9 +635,11 @@ const void *round_fn(int type, int cls, bool wave) {
 
 // Kernel attributes (the dynamic shared memory limit only grows: launches of
 // other open servers or contexts may need more) and grids.  The scratch is the
-// caller's to allocate (scratch_words) and free.
+// caller's to allocate (scratch_words) and free; it has rows for the pairs that
+// a round can queue (`pairs` at most), none where their number always takes
+// the group-per-pair kernel.
 template <bool MASK>
-cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
+cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms, int64_t pairs) {
   static std::mutex mu;
   static size_t have[64][2][2][kServeClasses] = {};
   int dev = 0;
@@ -665,8 +668,10 @@ cudaError_t round_plan(RoundPlan &pl, int type, int rep_nb, int num_sms) {
       if (wave) pl.subs[c] = type == 0 ? sub_from(2, c == 1 ? 4 : 1, 56 * num_sms) : INT_MAX;
       if (wave) pl.wave_pairs[c] = group_cut(c == 2 ? 0 : 64, 56 * num_sms);
     }
+  pl.grid[2] = (int)std::min<int64_t>(pl.grid[2], std::max<int64_t>(1, (pairs + kAlignThreads - 1) / kAlignThreads));
   pl.ring_rows = global_rows(rep_nb);
-  pl.scratch_words = serve_class_used(2, rep_nb, MASK) ? (int64_t)pl.grid[2] * kAlignThreads * pl.ring_rows : 1;
+  const bool rows = serve_class_used(2, rep_nb, MASK) && pairs > pl.wave_pairs[2];
+  pl.scratch_words = rows ? (int64_t)pl.grid[2] * kAlignThreads * pl.ring_rows : 1;
   return cudaSuccess;
 }
 

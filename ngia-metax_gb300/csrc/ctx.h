@@ -137,6 +137,8 @@ int open_ctx(const ngia_db_view *v, bool batch_member, ngia_ctx **out);
 // A context with room for cap_n records, cap_words record words and records
 // of up to cap_nb plane blocks, holding no database until reload_ctx.
 int open_ctx_capacity(int type, int64_t cap_n, int64_t cap_words, int cap_nb, ngia_ctx **out);
+// Its device bytes.
+int ctx_bytes(int type, int64_t cap_n, int64_t cap_words, int cap_nb, int num_sms, int64_t *bytes);
 // Loads a database within the capacity (stream-ordered copies on the
 // context's stream; waits for that stream only).
 int reload_ctx(ngia_ctx *c, const ngia_db_view *v);
@@ -157,6 +159,9 @@ int word_can_pay(int type, int shortest, const ngia::RunParams &prm);
 int spec_prepare(ngia_ctx *c);                 // buffers for the context's capacity; zeroed masks
 int spec_step(ngia_ctx *c, int64_t max_iters);  // up to max_iters representatives (<= 0: all)
 void spec_free(ngia_ctx *c);
+// Device bytes of the driver of a context of this capacity, and those of its
+// widest class's rows among them.
+int spec_bytes(int type, int64_t n, int nb, int num_sms, int64_t *bytes, int64_t *rows);
 bool spec_exact(const ngia_ctx *c);            // rounds reproduce the greedy loop exactly
 void spec_stats(const ngia_ctx *c, int64_t *pairs, int64_t *cells);
 }  // namespace drv

@@ -356,23 +356,30 @@ void free_slot(Slot &sl) {
   sl = Slot{};
 }
 
-// Device bytes of one slot (context, round buffers, scratch).
-int64_t slot_bytes(const ngia_server *sv, int64_t scratch) {
-  const int A = sv->type ? 28 : 4;
-  const int64_t ctx = 4 * sv->cap_words + sv->cap_n * (8 + 4 + 4 + 4 * A) +
-                      sv->cap_n * (4 + 4 + 4 * ngia::kNumClasses) + (int64_t)sv->cap_n / 8 * 3;
-  const int64_t rounds = 3ll * kMaxChunk * sv->cap_n * 8 + sv->cap_n * 8 + sv->cap_n / 8;
-  // speculative leftover rounds: masks, up to 64 scores per record, pair
-  // queues of 2^20 pairs per class, their own global ring
-  const int64_t spec = sv->cap_n * (8 + 64 * 4) + (int64_t)kServeClasses * (1 << 20) * 8 + scratch;
-  return ctx + rounds + scratch + spec + (16 << 20);
+// Entries of a class queue: a round of kMaxChunk representatives against every
+// query, a representative's pairs padded to 32.
+int64_t queue_entries(const ngia_server *sv) { return (int64_t)kMaxChunk * ((sv->cap_n + 31) & ~31ll); }
+
+// Device bytes of one slot, and of them the rows of the leftover driver's
+// widest class.
+int slot_bytes(const ngia_server *sv, int64_t scratch_words, int64_t *bytes, int64_t *rows) {
+  int64_t ctx = 0, spec = 0;
+  *rows = 0;
+  int rc = drv::ctx_bytes(sv->type, sv->cap_n, sv->cap_words, sv->cap_nb, sv->num_sms, &ctx);
+  if (!rc && leftover_mode() == NGIA_MODE_SPEC)
+    rc = drv::spec_bytes(sv->type, sv->cap_n, sv->cap_nb, sv->num_sms, &spec, rows);
+  int64_t rounds = sv->cap_n * 8 + sv->cap_n / 8 + 4 * scratch_words;
+  for (int k = 0; k < kServeClasses; k++)
+    if (serve_class_used(k, sv->reps->db.max_nb, false)) rounds += (int64_t)sizeof(int2) * queue_entries(sv);
+  *bytes = ctx + rounds + spec + (16 << 20);  // and what allocations round up to
+  return rc;
 }
 
 int open_slot(ngia_server *sv, Slot &sl, int index) {
   sl.index = index;
   int rc = drv::open_ctx_capacity(sv->type, sv->cap_n, sv->cap_words, sv->cap_nb, &sl.ctx);
   if (rc) return rc;
-  const int64_t cap = (int64_t)kMaxChunk * ((sv->cap_n + 31) & ~31ll);  // a representative's pairs pad to 32
+  const int64_t cap = queue_entries(sv);
   for (int k = 0; k < kServeClasses; k++)
     if (serve_class_used(k, sv->reps->db.max_nb, false) &&
         cudaMalloc((void **)&sl.rb.queue[k], sizeof(int2) * (size_t)cap) != cudaSuccess)
@@ -386,7 +393,7 @@ int open_slot(ngia_server *sv, Slot &sl, int index) {
       cudaMallocHost((void **)&sl.h_stats, 2 * sizeof(unsigned long long)) != cudaSuccess)
     return fail(NGIA_E_NOMEM, "serve: slot allocation failed");
   sl.rb.cap = cap;
-  if (round_plan<false>(sl.plan, sv->type, sv->reps->db.max_nb, sv->num_sms) != cudaSuccess)
+  if (round_plan<false>(sl.plan, sv->type, sv->reps->db.max_nb, sv->num_sms, INT64_MAX / 2) != cudaSuccess)
     return fail(NGIA_E_CUDA, "serve: kernel attributes");
   if (cudaMalloc((void **)&sl.plan.scratch, 4 * (size_t)sl.plan.scratch_words) != cudaSuccess)
     return fail(NGIA_E_NOMEM, "serve: scratch allocation failed");
@@ -495,13 +502,19 @@ extern "C" int ngia_serve_open(const ngia_db_view *reps, const ngia_params *para
   const int64_t budget = cf.memory_budget > 0 ? cf.memory_budget : (int64_t)(free_b / 2);
   ngia::RoundPlan plan;
   e = ngia::serve_filter_configure();
-  if (e == cudaSuccess) e = ngia::round_plan<false>(plan, sv->type, rc_ctx->db.max_nb, sv->num_sms);
+  if (e == cudaSuccess) e = ngia::round_plan<false>(plan, sv->type, rc_ctx->db.max_nb, sv->num_sms, INT64_MAX / 2);
   if (e != cudaSuccess) {
     ngia::destroy(sv);
     return fail(NGIA_E_CUDA, "ngia_serve_open: kernel attributes: %s", cudaGetErrorString(e));
   }
-  const int64_t per = ngia::slot_bytes(sv, 4 * plan.scratch_words);
-  const int n_slots = (int)std::min<int64_t>(cf.slots, budget / per);
+  int64_t per = 0, rows = 0;
+  rc = ngia::slot_bytes(sv, plan.scratch_words, &per, &rows);
+  if (rc) {
+    ngia::destroy(sv);
+    return rc;
+  }
+  int n_slots = (int)std::min<int64_t>(cf.slots, budget / per);
+  if (n_slots < 1 && budget >= per - rows) n_slots = 1;  // one slot even if only those rows are beyond the budget
   if (n_slots < 1) {
     ngia::destroy(sv);
     return fail(NGIA_E_NOMEM, "ngia_serve_open: one slot needs %lld bytes, the budget is %lld", (long long)per,

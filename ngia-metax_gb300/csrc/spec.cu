@@ -305,23 +305,18 @@ namespace {
 constexpr size_t kCtlBytes = kCtlWords * sizeof(uint32_t) + sizeof(SpecCtl);
 static_assert(kCtlBytes <= kMirrorCtl, "the mirror in the context");
 
-int spec_alloc(ngia_ctx *c) {
-  ngia_spec *sp = c->spec;
-  const int64_t n = std::max<int64_t>(c->cap_n, c->db.n);
-  const int nb = std::max(c->cap_nb, c->db.max_nb);
-  if (sp && sp->cap_n >= n && sp->type == c->db.type && sp->plan.rep_nb >= nb) return NGIA_OK;
-  spec_free(c);
-  sp = new (std::nothrow) ngia_spec();
-  if (!sp) return fail(NGIA_E_NOMEM, "spec: out of host memory");
-  c->spec = sp;
+// The plan and the device arrays (listed in sp->mem, not allocated) for up to
+// n sequences of records of up to nb blocks.
+int spec_layout(ngia_spec *sp, int type, int64_t n, int nb, int num_sms) {
   sp->cap_n = n;
-  sp->type = c->db.type;
+  sp->type = type;
   sp->k_max = (int)std::max<int64_t>(1, std::min<int64_t>(kSpecMax, kSpecScoreWords / std::max<int64_t>(1, n)));
   const int lw = kListWords;
-  CKP(round_plan<true>(sp->plan, sp->type, nb, c->num_sms));
+  const int64_t pairs = std::min<int64_t>(kSpecBudget, n * sp->k_max);
+  CKP(round_plan<true>(sp->plan, type, nb, num_sms, pairs));
   // a tile of a candidate pads its last group of each class (64 MB of queues
   // for a small set cost its open and close 0.1 ms)
-  const int64_t cap = std::min<int64_t>(kSpecBudget, n * sp->k_max) + 32ll * kSpecMax * ((n + kSpecTile - 1) / kSpecTile);
+  const int64_t cap = pairs + 32ll * kSpecMax * ((n + kSpecTile - 1) / kSpecTile);
   DevBlock &m = sp->mem;
   m.add(&sp->d.list, (size_t)n);
   m.add(&sp->d.rs_off, kSpecMax);
@@ -334,14 +329,28 @@ int spec_alloc(ngia_ctx *c) {
   for (int k = 0; k < kServeClasses; k++)
     if (serve_class_used(k, nb, true)) m.add(&sp->rb.queue[k], (size_t)cap);
   m.add(&sp->plan.scratch, (size_t)sp->plan.scratch_words);
-  if (m.take() != cudaSuccess) {
+  sp->rb.cap = cap;
+  return NGIA_OK;
+}
+
+int spec_alloc(ngia_ctx *c) {
+  ngia_spec *sp = c->spec;
+  const int64_t n = std::max<int64_t>(c->cap_n, c->db.n);
+  const int nb = std::max(c->cap_nb, c->db.max_nb);
+  if (sp && sp->cap_n >= n && sp->type == c->db.type && sp->plan.rep_nb >= nb) return NGIA_OK;
+  spec_free(c);
+  sp = new (std::nothrow) ngia_spec();
+  if (!sp) return fail(NGIA_E_NOMEM, "spec: out of host memory");
+  c->spec = sp;
+  int rc = spec_layout(sp, c->db.type, n, nb, c->num_sms);
+  if (!rc && sp->mem.take() != cudaSuccess) rc = fail(NGIA_E_NOMEM, "spec: device allocation failed");
+  if (rc) {
     spec_free(c);
-    return fail(NGIA_E_NOMEM, "spec: device allocation failed");
+    return rc;
   }
   sp->h_ctl = c->h_ctl;
   sp->rb.ctl = reinterpret_cast<uint32_t *>(sp->d_ctl);
   sp->d.ctl = reinterpret_cast<SpecCtl *>(sp->d_ctl + kCtlWords * sizeof(uint32_t));
-  sp->rb.cap = cap;
   sp->rb.list = sp->d.list;
   sp->rb.score_stride = n;
   sp->rb.key = nullptr;
@@ -419,6 +428,14 @@ int spec_prepare(ngia_ctx *c) {
   sp->max_alive = kSpecMaxAlive;
   if (const char *m = getenv("NGIA_SPEC_MAX_ALIVE")) sp->max_alive = std::max(2, atoi(m));
   return NGIA_OK;
+}
+
+int spec_bytes(int type, int64_t n, int nb, int num_sms, int64_t *bytes, int64_t *rows) {
+  ngia_spec sp;
+  const int rc = spec_layout(&sp, type, n, nb, num_sms);
+  *bytes = (int64_t)sp.mem.bytes();
+  *rows = 4 * sp.plan.scratch_words;
+  return rc;
 }
 
 void spec_free(ngia_ctx *c) {

@@ -113,3 +113,20 @@ def test_large_batches_of_services_side_by_side(cuda_device):
             got = srv.wait(srv.submit(b))
             exp = _expected(p, reps, b)
             assert np.array_equal(got[0], exp[0]) and np.array_equal(got[1], exp[1]), n
+
+
+@pytest.mark.parametrize("max_batch,blocks", [(512, 128), (64, 1024), (4096, 96), (4096, 256)])
+def test_slots_stay_within_the_memory_budget(cuda_device, max_batch, blocks):
+    torch = pytest.importorskip("torch")
+    p, reps, batches = _workload(0, 0.9, 5, 300, 6, [40], seed=91)
+    with ngia.Server(reps, p, slots=1, max_batch=64, max_record_blocks=blocks) as srv:  # what loads once
+        srv.wait(srv.submit(batches[0]))
+    free = torch.cuda.mem_get_info()[0]
+    budget = 1 << 30
+    with ngia.Server(reps, p, slots=64, max_batch=max_batch, max_record_blocks=blocks, memory_budget=budget) as srv:
+        used = free - torch.cuda.mem_get_info()[0]
+        assert srv.slots >= 1
+        assert used <= budget + (64 << 20)  # the representatives are not counted
+        e = _expected(p, reps, batches[0])
+        got = srv.wait(srv.submit(batches[0]))
+        assert np.array_equal(got[0], e[0]) and np.array_equal(got[1], e[1])
