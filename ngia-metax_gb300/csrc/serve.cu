@@ -459,12 +459,6 @@ extern "C" int ngia_serve_open(const ngia_db_view *reps, const ngia_params *para
   sv->prm.precise = params->precise;
   sv->prm.word_order = 0;
   if (const char *wo = getenv("NGIA_SERVE_WORD_ORDER")) sv->prm.word_order = std::max(0, std::min(2, atoi(wo)));
-  // lockstep refill (NGIA_SERVE_REFILL: idle lanes a warp waits for before it
-  // claims); swept on GB300 (200 DNA query batches, 14,077
-  // representatives): 32, 24, 16, 8 lanes gave 53.4k, 52.2k, 48.8k, 49.9k
-  // queries/s
-  sv->prm.refill = 32;
-  if (const char *rf = getenv("NGIA_SERVE_REFILL")) sv->prm.refill = std::max(1, std::min(32, atoi(rf)));
   // representatives of a resident set come in any length: each its own order
   sv->prm.word_can = !sv->prm.precise && ngia::word_need(sv->prm) > 0.0;
   sv->cap_n = cf.max_batch;
