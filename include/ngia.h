@@ -400,14 +400,16 @@ int ngia_cluster_resume(ngia_ctx *ctx, const char *path, int32_t mode);
  * and a later ngia_autotune with the same key applies it without timing
  * (cached = 1).  ngia_set_tuning applies settings found before. */
 typedef struct ngia_tuning {
-    int32_t word_order;   /* 0 by similarity, 1 short words first, 2 alignment first */
+    int32_t word_order;   /* 0 per representative, 1 short words first, 2 last       */
     int32_t refill;       /* 1..32 idle lanes                                        */
     int32_t warp_pairs;   /* group-per-pair up to this many pairs; -1 = default     */
     int32_t candidates;   /* settings timed (ngia_autotune)                          */
     double  ms_per_iter;  /* device time per iteration of the chosen setting         */
     double  default_ms_per_iter;  /* the same for the default setting                */
     int32_t class_warp_pairs[8];  /* per length bucket: its group-per-pair cut-off,  */
-                                  /* -1 = warp_pairs                                 */
+                                  /* -1 = warp_pairs (0, 1: short queries against    */
+                                  /* wide windows; the last three of a type: by the  */
+                                  /* window)                                         */
     int32_t class_grid_div[8];    /* per length bucket: its CTAs divided by 1 or 2   */
     int32_t filter_tile;          /* composition filter: bitmap words per warp and   */
                                   /* tile, 8 (default) or 1                          */

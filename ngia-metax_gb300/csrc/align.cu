@@ -53,11 +53,11 @@ struct AlignHdr {
 // Reads the iteration header and stages the representative's planes (and,
 // when the short-word test follows the alignment, its k-mer bitset) into
 // shared memory with bulk copies.  Returns false when there is no work.
-template <int P>
 // groups: pairs a CTA of the group-per-pair kernel works on at a time (it
 // takes classes with at most warp_pairs pairs; more once there are more than
 // `few`), 0 for the thread-per-pair kernels (classes with more);
 // the other kernel of a class returns here, before any staging.
+template <int P>
 __device__ __forceinline__ bool align_setup(const DevDB &db, const RunBufs &rb, const RunParams &prm, int cls,
                                             int score_mode, int warp_pairs, int groups, int few, int subs, uint32_t *smem,
                                             uint64_t *bar, AlignHdr &h) {
@@ -340,9 +340,9 @@ __host__ __device__ constexpr int wave_table_off(int P, int max_nb) { return ((m
 
 // ---- a group of threads per pair (wave.cuh) ------------------------------------------
 // For classes with few queued pairs the latency of one pair on one thread
-// bounds the iteration.  Windows up to 64 blocks: a warp per pair.  Wider ones:
+// bounds the iteration.  Windows up to 48 blocks: a warp per pair.  Wider ones:
 // the CTA per pair for up to `few` pairs, one row word per thread for windows
-// up to 128 blocks, up to 16 for any; beyond, when every scheduler has a warp,
+// up to 112 blocks, up to 16 for any; beyond, when every scheduler has a warp,
 // a warp per pair with up to 8 or 16 words, which takes half the instructions:
 // a step has 80 beside the columns' (5 + 4 W) each, and 2 nq + nb1 / W steps
 // are taken by one warp instead of four.  Classes of windows up to 112 blocks

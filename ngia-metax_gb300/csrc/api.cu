@@ -323,8 +323,8 @@ void size_grids(ngia_ctx *c, bool by_size) {
   // A class with at most this many pairs goes to its group-per-pair kernel.
   // One thread per pair takes a pair's latency whatever their number (DNA
   // 1,450 residues: 275-345 us from 1,500 to 24,000 pairs on GB300), a group
-  // per pair 33 us per 1,000 pairs once it fills the GPU: equal at about
-  // 9,000 (150 SMs x 56).
+  // per pair 33 us per 1,000 pairs once it fills the GPU: equal between 8,300
+  // and 10,400 pairs; 56 per SM of 152 are 8,512.
   c->warp_pairs = 56 * c->num_sms;
   if (const char *w = getenv("NGIA_WARP_PAIRS")) c->warp_pairs = atoi(w);
   c->warp_pairs_default = c->warp_pairs;

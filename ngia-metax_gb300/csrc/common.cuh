@@ -22,8 +22,11 @@ constexpr int kRefGridThreads = 128 * 128;     // BLOCK*WARP of the reference la
 // whose query has at most kQueryRows blocks: short queries against a long
 // representative, aligned by 16 threads with the query's blocks as rows
 // (wave.cuh) while they are few.
-// DNA numbers 2 and 3 are unused: class numbers in saved tunings, checkpoints
-// and statistics keep their meaning.
+// DNA numbers 2 and 3 are unused, so that the last three classes keep their
+// numbers.  Tunings and checkpoints saved when classes 0 and 1 (DNA: 0 to 3)
+// were the narrowest windows are still taken: a cut-off of theirs then steers the
+// short-query classes, and a resumed run's statistics add those up with the
+// windows'.  Speed and statistics only.
 constexpr int kNumClasses = 7;
 constexpr int kQueryRows = 16;
 constexpr int kSmallWindow = 48, kWideWindow = 112;
@@ -78,9 +81,9 @@ struct DevDB {
   const int32_t *net;     // net length (record word 1)
   const uint32_t *cnt;    // residue counts, 4 (DNA) or 28 (protein) per sequence
   const uint32_t *codes;  // protein: each record's residue codes as a bit stream
-  int32_t long_n;         // records before the first of at most kWarpWordLen residues (filter.cu)
                           // (5 words per 32-residue block, at the planes'
                           // offsets); null for DNA
+  int32_t long_n;         // records before the first of at most kWarpWordLen residues (filter.cu)
   int32_t n, type;
   int32_t hw, P, A;       // header words, planes, count words
   int32_t max_nb;         // max plane blocks over all records

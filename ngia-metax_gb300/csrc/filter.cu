@@ -329,7 +329,10 @@ __global__ void __launch_bounds__(kWordThreads, kWordCtas)
   const float s = prm.s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nbw = (db.n + 31) / 32;
-  uint32_t cand = 0, base = 0, bytes = 0, wpass = 0;  // a thread sees fewer than 2^17 candidates of 22 KB
+  // 32 bits: a candidate is at most 41 KB (a protein of 65,536 residues), and a
+  // thread sees at most 13,800 of the bitmap's words' (2^31 records, 4,864
+  // warps) besides its warp's share of the long records, which fit the device
+  uint32_t cand = 0, base = 0, bytes = 0, wpass = 0;
   const int W = gridDim.x * (blockDim.x >> 5), gw = warp * gridDim.x + blockIdx.x;
   const int n_long = word_here ? db.long_n : 0;
   for (int c = W - 1 - gw; c < n_long; c += W) {  // a warp per record

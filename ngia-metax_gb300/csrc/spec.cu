@@ -46,12 +46,14 @@ namespace {
 
 constexpr int kSpecMax = 64;              // candidate representatives per round (one mask bit each)
 constexpr int kSpecBudget = 1 << 20;      // pairs per round at most (K x unclustered)
-// Rounds start once the unclustered set is this small: a one-representative
-// iteration over a larger set fills the GPU, and the round kernels (the
-// representative taken per pair) run at about half the clustering kernels'
-// cell rate (GB300, 1M DNA s=0.85: 7.3 ms for 1M pairs in the clustering
-// kernel; a greedy iteration over 32k sequences is bounded by the latency of
-// its slowest pair, 0.2-0.3 ms).
+// Rounds start once the unclustered set is this small.  The line is that of an
+// earlier round kernel, which took the representative per pair, at half the
+// clustering kernels' cell rate; with groups of one representative it lies too
+// low.  GB300, ms to the end with rounds from 2^13, 2^14, 2^15 and 2^16
+// unclustered sequences on: 60,000 DNA of 600 residues, s = 0.85, 2,350, 1,993,
+// 1,380 and 524; 60,000 of 300, s = 0.9, 1,541, 1,307, 896 and 258; 50,000 of
+// 1,450 4,984, 4,147, 2,694 and 1,302; 200,000 of 600 from 2^15 to 2^18 10,034,
+// 9,039, 7,559 and 6,234 (NGIA_SPEC_MAX_ALIVE).
 constexpr int kSpecMaxAlive = 1 << 15;
 constexpr int kSpecRecheck = 8;  // graph iterations between looks at the unclustered set
 constexpr int64_t kSpecScoreWords = 1ll << 26;  // K x n scores at most (256 MB)

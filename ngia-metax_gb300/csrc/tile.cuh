@@ -141,8 +141,9 @@ __device__ __forceinline__ int tile_planes(const Ring &ring, const uint32_t *pla
 // the rows of block j whose residue is c (c = plane-0 bit | plane-1 bit << 1),
 // i.e. ~(p0 ^ m0) & ~(p1 ^ m1) for the masks of residue c — the same words
 // the plane form builds per column.  kEqPad zero blocks follow the last rep
-// block, so a tile's padding slots (rows above je, whose row words are 0 and
-// mask whatever they read) stay inside the table.
+// block, so a tile's padding slots (rows above je) read inside the table.  Their
+// rows hold anything: carries only go up, away from the window's rows, and
+// tile_block takes their zeros off the count.
 constexpr int kEqPad = 32;
 __host__ __device__ constexpr int eq_words(int max_nb) { return 4 * (max_nb + kEqPad); }
 // Word offset of the match table in the tiled kernel's dynamic shared memory:
