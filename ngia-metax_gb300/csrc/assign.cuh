@@ -141,13 +141,15 @@ __device__ __forceinline__ void queue_groups(const RoundBufs &rb, int r, int q0,
   }
 }
 
-// One CTA per representative of the chunk: composition test (and the
-// short-word test in word-first order) for every unassigned query, kServeTile
-// queries at a time, whose outcomes lie in shared memory until they are queued:
-// a batch of any size takes the same bounded amount.  (One byte per query of
-// the whole batch had to be allowed for by each service's own size, and a
-// batch of more than some 220,000 did not fit.)  A tile pads its last group of
-// each class; batches of up to 65,536 have one tile.
+// One CTA per representative of the chunk and tile of kServeTile queries:
+// composition test (and the short-word test in word-first order) for every
+// unassigned query.  The outcomes lie in shared memory until they are queued,
+// a byte each, so a batch of any size takes the same bounded amount.  (A byte
+// per query of the whole batch had to be allowed for by each service's own
+// size, and a batch of more than some 220,000 did not fit.)  A tile pads its
+// last group of each class; batches of up to 65,536 queries have one tile.
+// (Tiles in turn by one CTA cost services of a few queries 3%: 465 -> 478 us for
+// five requests of up to three queries against 1,400 representatives.)
 constexpr int kServeTile = 1 << 16;
 // Entries of one representative and class for `left` queries in `tiles` tiles.
 __host__ __device__ constexpr int64_t serve_entries(int64_t left, int64_t tiles) { return (left + 31 * tiles) & ~31ll; }
@@ -162,47 +164,45 @@ __global__ void __launch_bounds__(256) k_serve_filter(DevDB qdb, RepStore rs, Ru
   uint8_t *s_res = reinterpret_cast<uint8_t *>(s_list + rs.list_words);  // 0 = out, 1 + class
   __shared__ uint32_t s_rc[28], s_cnt[kServeClasses], s_base[kServeClasses], s_pos[kServeClasses];
   constexpr int A = P == 2 ? 4 : 28;
-  const int r = r0 + blockIdx.x;
+  const int r = r0 + blockIdx.x, q0 = blockIdx.y * kServeTile;
   const uint32_t *rec = rs.words + rs.off[r];
   if (threadIdx.x < A) s_rc[threadIdx.x] = rec[2 + threadIdx.x];
+  if (threadIdx.x < kServeClasses) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
   const int L1 = (int)rec[0], net1 = (int)rec[1], nb1 = (net1 + 31) / 32;
   const float s = prm.s;
   const bool word_here = !prm.precise && net1 >= 16 && rs.first[r];
-  if (word_here)
+  if (word_here) {
     for (int t = threadIdx.x; t < rs.list_words; t += blockDim.x) s_list[t] = rs.lists[(int64_t)r * rs.list_words + t];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int q0 = 0; q0 < qdb.n; q0 += kServeTile) {
-    const int n = min(kServeTile, qdb.n - q0), nbw = (n + 31) / 32;
-    if (threadIdx.x < kServeClasses) s_cnt[threadIdx.x] = 0;
     __syncthreads();
-    for (int wi = warp; wi < nbw; wi += blockDim.x >> 5) {
-      const uint32_t bits = rb.todo[q0 / 32 + wi];
-      const int k = wi * 32 + lane, q = q0 + k;
-      int res = 0;
-      if ((bits >> lane) & 1u) {
-        // a smaller representative of this round may already hold q
-        const bool open = (rb.key[q] >> 32) > (unsigned long long)r;
-        const int L2 = __ldg(qdb.len + q);
-        const int cut = cutoff_of(L2, s);
-        bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cut);
-        if (pass && word_here) {
-          const int net2 = __ldg(qdb.net + q);
-          if (net2 >= 16)
-            pass = words_reach<P, 1>(qdb, q, net2, prm.w, word_min(L2, prm.w, s), KmerBits{s_list}, s_list);
-        }
-        if (pass) res = 1 + serve_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1));
-      }
-      if (k < n) s_res[k] = (uint8_t)res;
-      const unsigned pm = __ballot_sync(kFullMask, res != 0);
-      if (res) {
-        const unsigned peers = __match_any_sync(pm, res);
-        if (lane == __ffs(peers) - 1) atomicAdd(&s_cnt[res - 1], (uint32_t)__popc(peers));
-      }
-    }
-    __syncthreads();
-    queue_groups(rb, r, q0, n, s_res, s_cnt, s_base, s_pos);
-    __syncthreads();  // the tile's outcomes and places are read
   }
+  const int n = min(kServeTile, qdb.n - q0), nbw = (n + 31) / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int wi = warp; wi < nbw; wi += blockDim.x >> 5) {
+    const uint32_t bits = rb.todo[q0 / 32 + wi];
+    const int k = wi * 32 + lane, q = q0 + k;
+    int res = 0;
+    if ((bits >> lane) & 1u) {
+      // a smaller representative of this round may already hold q
+      const bool open = (rb.key[q] >> 32) > (unsigned long long)r;
+      const int L2 = __ldg(qdb.len + q);
+      const int cut = cutoff_of(L2, s);
+      bool pass = open && !(base_sum<A>(qdb.cnt, q, s_rc) < cut);
+      if (pass && word_here) {
+        const int net2 = __ldg(qdb.net + q);
+        if (net2 >= 16) pass = words_reach<P, 1>(qdb, q, net2, prm.w, word_min(L2, prm.w, s), KmerBits{s_list}, s_list);
+      }
+      if (pass) res = 1 + serve_class(window_need(L1, L2, cut, band_blocks(L1, L2, s), nb1));
+    }
+    if (k < n) s_res[k] = (uint8_t)res;
+    const unsigned pm = __ballot_sync(kFullMask, res != 0);
+    if (res) {
+      const unsigned peers = __match_any_sync(pm, res);
+      if (lane == __ffs(peers) - 1) atomicAdd(&s_cnt[res - 1], (uint32_t)__popc(peers));
+    }
+  }
+  __syncthreads();
+  queue_groups(rb, r, q0, n, s_res, s_cnt, s_base, s_pos);
 }
 
 // The filter's dynamic shared memory limit, the largest any service can need:

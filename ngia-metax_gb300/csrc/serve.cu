@@ -228,12 +228,13 @@ int run_batch(ngia_server *sv, Slot &sl, Request &rq) {
     const int64_t fit = std::min(rb.cap, kMaxEntries) / serve_entries(left, serve_tiles(n));
     const int64_t want = std::min<int64_t>({std::max<int64_t>(chunk, pairs / left), fit, (int64_t)max_chunk});
     const int nr = (int)std::min<int64_t>(want, sv->store.n - r0);
+    const dim3 grid(nr, (unsigned)serve_tiles(n));
     CKS(cudaMemsetAsync(rb.ctl, 0, kCtlWords * sizeof(uint32_t), st));
     if (ev[0]) cudaEventRecord(ev[0], st);
     if (sv->type == 0)
-      k_serve_filter<2><<<nr, 256, fsm, st>>>(c->db, sv->store, sv->prm, rb, r0);
+      k_serve_filter<2><<<grid, 256, fsm, st>>>(c->db, sv->store, sv->prm, rb, r0);
     else
-      k_serve_filter<5><<<nr, 256, fsm, st>>>(c->db, sv->store, sv->prm, rb, r0);
+      k_serve_filter<5><<<grid, 256, fsm, st>>>(c->db, sv->store, sv->prm, rb, r0);
     CKS(cudaGetLastError());
     if (ev[1]) cudaEventRecord(ev[1], st);
     CKS(round_launch<false>(sl.plan, c->db, sv->store, sv->prm, rb, st));
